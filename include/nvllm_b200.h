@@ -289,6 +289,20 @@ NVLLM_API int nvllm_decode_step_inputs(const void* staged, int64_t tokens_off, i
                              int64_t bt_row_stride, void* stream);
 
 /*
+ * The same with the staging block left in pinned host memory: `staged_host` is the host block
+ * itself (page-locked memory that the device can address), read by the kernel over PCIe, so a step
+ * costs one launch and no copy; the caller must not rewrite the block before the launch has
+ * completed.  When `temperatures_out` is not NULL the fp32[batch] section at temperatures_off is
+ * copied to it (device memory).  No counterpart in the reference beyond those named above
+ * (prepare_sample, nanovllm/engine/model_runner.py:251-258, for the temperatures).
+ */
+NVLLM_API int nvllm_decode_step_inputs_pinned(const void* staged_host, int64_t tokens_off, int64_t lens_off, int64_t offsets_off,
+                             int64_t blocks_off, int64_t temperatures_off, float* temperatures_out, int32_t batch,
+                             int32_t graph_batch, int32_t used_width, int32_t table_width, int64_t* input_ids,
+                             int64_t* positions, int32_t* slot_mapping, int32_t* context_lens, int32_t* block_tables,
+                             int64_t bt_row_stride, void* stream);
+
+/*
  * All-reduce (sum, bf16) over peer memory for tensor-parallel ranks on one node, one process per
  * GPU.  Replaces dist.all_reduce in RowParallelLinear.forward (nanovllm/layers/linear.py:195-199)
  * for tensors up to `max_bytes`.  Set-up, once per process and device, outside stream capture:

@@ -42,6 +42,9 @@ SIGNATURES = {
     "nvllm_sample_unpack": (c_int32, [c_void_p, c_void_p, c_int32, c_void_p]),
     "nvllm_decode_step_inputs": (c_int32, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32,
                                            c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
+    "nvllm_decode_step_inputs_pinned": (c_int32, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p, c_int32,
+                                                  c_int32, c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
+                                                  c_int64, c_void_p]),
     "nvllm_ar_handle_bytes": (c_int64, []),
     "nvllm_ar_init": (c_int32, [c_int32, c_int32, c_int64, c_void_p]),
     "nvllm_ar_connect": (c_int32, [c_void_p]),
@@ -68,6 +71,7 @@ SIGNATURES = {
 }
 
 _lib = None
+_host = None
 
 
 class NvllmError(RuntimeError):
@@ -93,6 +97,22 @@ def load() -> ctypes.CDLL:
             fn.argtypes = argtypes
         _lib = lib
     return _lib
+
+
+def host():
+    """The extension module that holds the entry points' host path (csrc/host.cpp), bound to the
+    library that ``load`` opened."""
+    global _host
+    if _host is None:
+        load()
+        try:
+            from . import _host as module
+        except ImportError as e:
+            raise ImportError("nano_vllm_b200._host is missing or does not load: build it with "
+                              "`python -m nano_vllm_b200.build`") from e
+        module.bind(str(LIB_PATH), check)
+        _host = module
+    return _host
 
 
 def last_error() -> str:
