@@ -101,3 +101,28 @@ def test_recorded_reference_modules(cuda, name):
     _bf16_ulp_close(q_d.reshape(n, hq, d), c["q"], "q")
     _bf16_ulp_close(k_d.reshape(n, hkv, d), c["k"], "k")
     assert torch.equal(v_d, c["qkv"][:, (hq + hkv) * d:])
+
+
+@pytest.mark.parametrize("hq,hkv,d,n,norm", [(16, 8, 128, 2401, True), (3, 1, 128, 16001, True), (5, 5, 64, 10243, True),
+                                             (14, 2, 64, 9003, False)])
+def test_launches_of_four_heads_per_lane_group_equal_those_of_one(cuda, hq, hkv, d, n, norm):
+    """A large launch gives each lane group four heads, a small one gives it one: the same bits, at head
+    counts that put q, k and v heads (or fewer than four) into one group."""
+    g = torch.Generator(device=cuda).manual_seed(n)
+    qkv = (torch.randn(n, (hq + 2 * hkv) * d, generator=g, device=cuda) * 3).bfloat16()
+    positions = torch.randint(0, 512, (n,), generator=g, device=cuda)
+    qw, kw = ((1 + 0.1 * torch.randn(d, generator=g, device=cuda)).bfloat16() if norm else None for _ in range(2))
+    cache = R.rotary_cache_ref(d, 512, 1e6).to(cuda)
+    blocks = (n + 255) // 256 + 1
+    slots = torch.randperm(blocks * 256, generator=g, device=cuda)[:n].to(torch.int32)
+    slots[1::7] = -1
+    results = []
+    for step in (n, 997):
+        x, kv = qkv.clone(), torch.zeros(2, blocks, 256, hkv, d, dtype=torch.bfloat16, device=cuda)
+        for a in range(0, n, step):
+            A.qk_norm_rope_store(x[a:a + step], positions[a:a + step], qw, kw, cache, 1e-6, slots[a:a + step], kv[0], kv[1],
+                                 hq, hkv, d)
+        results.append((x, kv))
+    assert torch.equal(results[0][0].view(torch.int16), results[1][0].view(torch.int16))
+    assert torch.equal(results[0][1].view(torch.int16), results[1][1].view(torch.int16))
+    assert _lib.read_status() == 0
