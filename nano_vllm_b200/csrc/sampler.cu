@@ -18,9 +18,23 @@
 //
 // A row is read by one thread-block cluster of 1, 2, 4 or 8 blocks of 256 threads (the fewer
 // the rows, the more blocks each gets, so that a decode batch of any size spreads over the 148
-// SMs); 16-byte loads, four in flight per thread.  Each block reduces to one candidate, block 0
-// of the cluster collects the others' candidates from their shared memory.  Ties go to the
-// lowest index.
+// SMs).  A thread takes groups of 16 bytes (8 bf16 or 4 fp32 logits), loaded one step ahead.  Each
+// block reduces to one candidate, block 0 of the cluster collects the others' candidates from
+// their shared memory.  Ties go to the lowest index.
+//
+// What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
+// per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
+// (now 53, of which the rounds are most; greedy rows 32 -> 20).  The logarithms are only needed for elements that can still win: since e >= v, where v is the uniform
+// draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
+// the group's largest x and the smallest of its draws decide that for the whole group, against the
+// best score that any warp of the block has seen; only groups that pass (a few per warp and row)
+// compute their scores.  A warp whose groups cannot pass even with the smallest possible draw
+// (x < b - 22) skips the generator as well, which is where most of the vocabulary of a peaked
+// distribution ends.  Greedy rows compare the group's maximum with the thread's best, two packed bf16 at a time.
+//
+// Groups start at multiples of four global positions (the generator's counter).  Where such a
+// group does not start on a 16-byte boundary (rows of an odd vocabulary, slices), it is shifted
+// out of two aligned loads; the up to fifteen elements around the whole groups go one at a time.
 //
 // Tensor parallelism: nano-vllm's LM head leaves every rank with the logits of its own slice of
 // the vocabulary and then gathers all slices on rank 0 and concatenates them
@@ -31,6 +45,8 @@
 // would have picked from the concatenated row, because the noise is generated from the global
 // index.  nvllm_sample_unpack turns the winning candidates into token ids.
 #include <cooperative_groups.h>
+
+#include <type_traits>
 
 #include "common.cuh"
 
@@ -49,26 +65,52 @@ struct SampleParams {
   int candidates;
 };
 
+// Float bits as a signed integer of the same order.
+__device__ __forceinline__ int ordered(float x) {
+  const int i = __float_as_int(x);
+  return i >= 0 ? i : i ^ 0x7fffffff;
+}
+__device__ __forceinline__ float from_ordered(int i) { return __int_as_float(i >= 0 ? i : i ^ 0x7fffffff); }
+
 // (score, index) as one int64 that orders like "higher score, then lower index".
 __device__ __forceinline__ long long pack_candidate(float score, int idx) {
-  int s = __float_as_int(score);
-  s = s >= 0 ? s : s ^ 0x7fffffff;  // order-preserving map of float bits to a signed integer
+  const int s = ordered(score);
   return (static_cast<long long>(s) << 32) | static_cast<long long>(0xffffffffu - static_cast<unsigned int>(idx));
 }
 
-// Philox4x32 with 10 rounds (Salmon et al., "Parallel random numbers: as easy as 1, 2, 3", SC'11).
-__device__ __forceinline__ uint4 philox4x32_10(uint4 ctr, uint2 key) {
-  constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
-#pragma unroll
-  for (int r = 0; r < 10; ++r) {
-    const uint32_t hi0 = __umulhi(M0, ctr.x), lo0 = M0 * ctr.x;
-    const uint32_t hi1 = __umulhi(M1, ctr.z), lo1 = M1 * ctr.z;
-    ctr = make_uint4(hi1 ^ ctr.y ^ key.x, lo1, hi0 ^ ctr.w ^ key.y, lo0);
-    key.x += W0;
-    key.y += W1;
+// Philox4x32 with 10 rounds (Salmon et al., "Parallel random numbers: as easy as 1, 2, 3", SC'11),
+// for counters (c0, row, step lo, step hi) of which only c0 differs between the calls of a thread:
+// one product of round 1 and one of round 2 do not depend on it and are made once.  High and low
+// words are separate multiplications on purpose: the 64-bit product is one instruction but slower
+// (64 us against 56 for the whole kernel at batch 256).
+struct Philox {
+  static constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
+  uint2 key;
+  uint32_t a, b, c, d;  // key and counter words that are the same for every c0
+  __device__ __forceinline__ Philox(uint64_t seed, uint32_t row, uint64_t step) {
+    key = make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+    const uint32_t lo = static_cast<uint32_t>(step), hi = static_cast<uint32_t>(step >> 32);
+    a = hi ^ key.y;                            // round 1: z = hi(M0 c0) ^ a, w = lo(M0 c0)
+    const uint32_t x1 = __umulhi(M1, lo) ^ row ^ key.x;
+    b = (M1 * lo) ^ (key.x + W0);              // round 2: x = hi(M1 z) ^ b, y = lo(M1 z)
+    c = __umulhi(M0, x1) ^ (key.y + W1);       //          z = w ^ c
+    d = M0 * x1;                               //          w = d
   }
-  return ctr;
-}
+  __device__ __forceinline__ uint4 operator()(uint32_t c0) const {
+    const uint32_t z1 = __umulhi(M0, c0) ^ a, w1 = M0 * c0;
+    uint4 s = make_uint4(__umulhi(M1, z1) ^ b, M1 * z1, w1 ^ c, d);
+    uint32_t k0 = key.x + W0, k1 = key.y + W1;
+#pragma unroll
+    for (int r = 2; r < 10; ++r) {
+      k0 += W0;
+      k1 += W1;
+      const uint32_t hi0 = __umulhi(M0, s.x), lo0 = M0 * s.x;
+      const uint32_t hi1 = __umulhi(M1, s.z), lo1 = M1 * s.z;
+      s = make_uint4(hi1 ^ s.y ^ k0, lo1, hi0 ^ s.w ^ k1, lo0);
+    }
+    return s;
+  }
+};
 
 // ln of an Exponential(1) draw made from 32 random bits.  v = (bits + 0.5) / 2^32 is uniform in
 // (0,1) and e = -ln(1 - v); for small v the series keeps the relative precision that 1 - v
@@ -97,7 +139,7 @@ __device__ __forceinline__ void take(Best& b, float s, int i) {
     b.idx = i;
   }
 }
-// Same for a thread's own elements, which it visits in rising index order.
+// Same for the groups of a thread, which it visits in rising index order.
 __device__ __forceinline__ void take_next(Best& b, float s, int i) {
   if (s > b.score) {
     b.score = s;
@@ -105,25 +147,97 @@ __device__ __forceinline__ void take_next(Best& b, float s, int i) {
   }
 }
 
+// A group is one 16-byte piece of a row: its elements as fp32, and their maximum (NaN ignored).
 template <typename T>
-__device__ __forceinline__ float to_f32(T x);
+struct Group;
 template <>
-__device__ __forceinline__ float to_f32<float>(float x) { return x; }
+struct Group<__nv_bfloat16> {
+  static constexpr int N = 8;
+  static __device__ __forceinline__ void unpack(const uint4& w, float (&x)[N]) {
+    const uint32_t u[4] = {w.x, w.y, w.z, w.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      x[2 * i] = __uint_as_float(u[i] << 16);
+      x[2 * i + 1] = __uint_as_float(u[i] & 0xffff0000u);
+    }
+  }
+  static __device__ __forceinline__ float max(const uint4& w) {
+    auto h = [](uint32_t u) { return *reinterpret_cast<__nv_bfloat162*>(&u); };
+    const __nv_bfloat162 m = __hmax2(__hmax2(h(w.x), h(w.y)), __hmax2(h(w.z), h(w.w)));
+    return fmaxf(__low2float(m), __high2float(m));
+  }
+};
 template <>
-__device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 x) { return __bfloat162float(x); }
+struct Group<float> {
+  static constexpr int N = 4;
+  static __device__ __forceinline__ void unpack(const uint4& w, float (&x)[N]) {
+    x[0] = __uint_as_float(w.x);
+    x[1] = __uint_as_float(w.y);
+    x[2] = __uint_as_float(w.z);
+    x[3] = __uint_as_float(w.w);
+  }
+  static __device__ __forceinline__ float max(const uint4& w) {
+    return fmaxf(fmaxf(__uint_as_float(w.x), __uint_as_float(w.y)), fmaxf(__uint_as_float(w.z), __uint_as_float(w.w)));
+  }
+};
 
-// Build-time shape (measurement aid): resident blocks per SM the register budget is held to, and
-// 16-byte loads in flight per thread.
+// 16 bytes that start `shift` bytes (a multiple of the element size, 0..15, uniform over the block)
+// into the pair (a, b).
+template <int ELEM>
+__device__ __forceinline__ uint4 shift_pair(const uint4& a, const uint4& b, int shift) {
+  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+  if (shift & 8) {
+#pragma unroll
+    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
+  }
+  if (shift & 4) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
+  }
+  if (ELEM == 2 && (shift & 2)) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], 16);
+  }
+  return make_uint4(w[0], w[1], w[2], w[3]);
+}
+
+// Build-time shape (measurement aid): resident blocks per SM the register budget is held to.
 #ifndef NVLLM_SAMPLER_MINBLOCKS
 #define NVLLM_SAMPLER_MINBLOCKS 4
 #endif
-#ifndef NVLLM_SAMPLER_UNROLL
-#define NVLLM_SAMPLER_UNROLL 4
-#endif
+
+// Calls f(pieces, first group, stride between the pieces' groups) for this thread's share of the
+// `n_groups` groups of a row that start at `first`, C pieces at a time; the next C are loaded before
+// the current ones are looked at.  All lanes of a warp make the same calls; pieces of groups past
+// the end are zero.
+template <bool ALIGNED, int C, typename T, class F>
+__device__ __forceinline__ void for_groups(const T* first, int n_groups, int tid, int nthreads, F&& f) {
+  const int lane = tid & 31;
+  const int shift = ALIGNED ? 0 : static_cast<int>(reinterpret_cast<uintptr_t>(first) & 15u);
+  const uint4* base = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(first) - shift);
+  auto load = [&](uint4 (&raw)[C], int g) {
+#pragma unroll
+    for (int c = 0; c < C; ++c, g += nthreads) {
+      const bool live = g < n_groups;
+      raw[c] = live ? __ldg(base + g) : make_uint4(0, 0, 0, 0);
+      if constexpr (!ALIGNED) raw[c] = shift_pair<sizeof(T)>(raw[c], live ? __ldg(base + g + 1) : make_uint4(0, 0, 0, 0), shift);
+    }
+  };
+  uint4 raw[C], next[C];
+  int g0 = tid - lane;
+  load(next, g0 + lane);
+  for (; g0 < n_groups; g0 += C * nthreads) {
+#pragma unroll
+    for (int c = 0; c < C; ++c) raw[c] = next[c];
+    load(next, g0 + C * nthreads + lane);
+    f(raw, g0 + lane, nthreads);
+  }
+}
 
 template <typename T>
 __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(const SampleParams p) {
-  constexpr int VEC = 16 / sizeof(T);  // elements per 16-byte load: 8 bf16 or 4 fp32
+  using G = Group<T>;
+  constexpr int N = G::N;
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   const int csize = static_cast<int>(cluster.num_blocks()), crank = static_cast<int>(cluster.block_rank());
@@ -135,61 +249,138 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
   const float t = p.temperatures[row];
   const bool greedy = !(t > 0.f) && !(t < 0.f);  // T == 0 (or NaN): plain argmax, as torch.where(T == 0, ...)
   const float inv_t = greedy ? 1.f : 1.f / t;
-  const uint2 key = make_uint2(static_cast<uint32_t>(p.seed), static_cast<uint32_t>(p.seed >> 32));
+  const Philox draw4(p.seed, static_cast<uint32_t>(row), p.step);  // unique per element and call
+  __shared__ int s_best;  // best score of the block so far, ordered()
+  if (threadIdx.x == 0) s_best = ordered(-INFINITY);
+  __syncthreads();
 
   Best best{-INFINITY, 0x7fffffff};
-  // score of element i given its logit; `bits` only used by the generator path
-  auto score_of = [&](float logit, int i, uint32_t bits) {
-    float s = logit * inv_t;
-    if (!greedy) s -= nz ? __logf(nz[i] + 1e-10f) : ln_exponential(bits);
-    return s;
-  };
-
-  // 16-byte loads need an aligned row, and a slice that starts on a group of four positions
-  // (one Philox call covers four consecutive global positions)
   const int off = static_cast<int>(p.offset);
-  const bool vec_ok = (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && (off & 3) == 0;
-  const int n_vec = vec_ok ? p.vocab / VEC : 0;
-  auto consume = [&](const uint4& raw, int v) {
-    const T* e = reinterpret_cast<const T*>(&raw);
-    uint32_t bits[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    if (!greedy && !nz) {
+  // whole groups of this row: they start at multiples of four global positions
+  const int lead = (4 - (off & 3)) & 3;
+  const int n_groups = p.vocab > lead ? (p.vocab - lead) / N : 0;
+  const T* first = x + lead;
+
+  auto scan = [&](auto aligned) {
+    constexpr bool A = decltype(aligned)::value;
+    if (greedy) {
+      for_groups<A, 4>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[4], int g, int stride) {
 #pragma unroll
-      for (int h = 0; h < VEC / 4; ++h) {
-        // counter: (group of 4 positions, row, step lo, step hi) -- unique per element and call
-        const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>((off >> 2) + v * (VEC / 4) + h), static_cast<uint32_t>(row),
-                                                 static_cast<uint32_t>(p.step), static_cast<uint32_t>(p.step >> 32)),
-                                      key);
-        bits[4 * h] = r.x; bits[4 * h + 1] = r.y; bits[4 * h + 2] = r.z; bits[4 * h + 3] = r.w;
+        for (int c = 0; c < 4; ++c, g += stride) {
+          if (g >= n_groups || !(G::max(raw[c]) > best.score)) continue;
+          float e[N];
+          G::unpack(raw[c], e);
+#pragma unroll
+          for (int k = 0; k < N; ++k) take_next(best, e[k], off + lead + g * N + k);
+        }
+      });
+    } else if (nz) {
+      for_groups<A, 1>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[1], int g, int) {
+        if (g >= n_groups) return;
+        float e[N];
+        G::unpack(raw[0], e);
+        const float* z = nz + lead + g * N;
+#pragma unroll
+        for (int k = 0; k < N; ++k) take_next(best, e[k] * inv_t - __logf(z[k] + 1e-10f), off + lead + g * N + k);
+      });
+    } else {
+      // log2 of 2^32 times the largest v with which x reaches a score b: x log2(e) / T - bar_of(b).  The slack
+      // covers the rounding of the scores, of the exponential and of v.
+      const float x_scale = inv_t * 1.4426950408889634f;
+      auto bar_of = [](float b) { return fmaf(b, 1.4426950408889634f, -32.01f - 1e-6f * fabsf(b)); };
+      // draws up to this can win; NaN (nothing seen yet, infinities) and T < 0 let everything pass
+      auto limit_of = [&](const uint4& raw, float bar) { return t < 0.f ? INFINITY : fast_exp2(fmaf(G::max(raw), x_scale, -bar)); };
+      // two pieces at a time, so that the chains of their generator calls overlap
+      constexpr int C = 2;
+      float bar = bar_of(-INFINITY);
+      int seen = ordered(-INFINITY);
+      for_groups<A, C>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[C], int g, int stride) {
+        const int now = *static_cast<volatile int*>(&s_best);
+        if (now != seen) {
+          seen = now;
+          bar = bar_of(from_ordered(now));
+        }
+        float limit[C];
+        bool any = false;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          limit[c] = limit_of(raw[c], bar);
+          any |= g + c * stride < n_groups && !(limit[c] < 0.25f);
+        }
+        if (!__any_sync(0xffffffffu, any)) return;
+        uint32_t bits[C][N];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+#pragma unroll
+          for (int h = 0; h < N / 4; ++h) {
+            const uint4 r = draw4(static_cast<uint32_t>((off + lead + (g + c * stride) * N) >> 2) + h);
+            bits[c][4 * h] = r.x; bits[c][4 * h + 1] = r.y; bits[c][4 * h + 2] = r.z; bits[c][4 * h + 3] = r.w;
+          }
+        }
+        if (seen == ordered(-INFINITY)) {
+          // Nothing is known of the row yet: take a bar from these elements.  -ln(e) >= -ln(v) - 0.33 for
+          // v < 1/2 (e <= 1.39 v), and the exponent and mantissa bits of v read as a number give log2(v)
+          // to within 0.09, so this is a score that some element reaches, found without logarithms.
+          float reach = -INFINITY;
+#pragma unroll
+          for (int c = 0; c < C; ++c) {
+            float e[N];
+            G::unpack(raw[c], e);
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+              const float log2v = fmaf(static_cast<float>(__float_as_int(static_cast<float>(bits[c][k]) + 0.5f)),
+                                       1.1920928955078125e-07f, -159.f);
+              const float s = fmaf(log2v + 0.1f, -0.69314718f, fmaf(e[k], inv_t, -0.33f));
+              if (bits[c][k] < 0x80000000u && g + c * stride < n_groups) reach = fmaxf(reach, s);
+            }
+          }
+          const int reached = __reduce_max_sync(0xffffffffu, ordered(reach));
+          if ((threadIdx.x & 31) == 0) atomicMax(&s_best, reached);
+#pragma unroll
+          for (int c = 0; c < C; ++c) limit[c] = limit_of(raw[c], bar_of(from_ordered(reached)));
+        }
+        bool pass = false;
+        uint32_t below[C];
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          below[c] = limit[c] < 4.2e9f ? __float2uint_ru(limit[c]) : 0xffffffffu;  // NaN: everything passes
+          uint32_t least = min(min(bits[c][0], bits[c][1]), min(bits[c][2], bits[c][3]));
+          if constexpr (N == 8) least = min(least, min(min(bits[c][4], bits[c][5]), min(bits[c][6], bits[c][7])));
+          pass |= g + c * stride < n_groups && least <= below[c];
+        }
+        if (!__any_sync(0xffffffffu, pass)) return;
+#pragma unroll
+        for (int c = 0; c < C; ++c) {
+          float e[N];
+          G::unpack(raw[c], e);
+#pragma unroll
+          for (int k = 0; k < N; ++k)
+            if (bits[c][k] <= below[c] && g + c * stride < n_groups)
+              take_next(best, e[k] * inv_t - ln_exponential(bits[c][k]), off + lead + (g + c * stride) * N + k);
+        }
+        const int warp_best = __reduce_max_sync(0xffffffffu, ordered(best.score));
+        if ((threadIdx.x & 31) == 0 && warp_best > now) atomicMax(&s_best, warp_best);
+      });
+    }
+  };
+  if ((reinterpret_cast<uintptr_t>(first) & 15u) == 0) scan(std::true_type{});
+  else scan(std::false_type{});
+  // the elements before and after the whole groups, one at a time, same counters
+  const int n_edge = p.vocab - n_groups * N, head = min(lead, p.vocab);
+  for (int k = tid; k < n_edge; k += nthreads) {
+    const int i = k < head ? k : k + n_groups * N;
+    float s = static_cast<float>(x[i]) * inv_t;
+    if (!greedy) {
+      if (nz) {
+        s -= __logf(nz[i] + 1e-10f);
+      } else {
+        const int gi = off + i;  // global position
+        const uint4 r = draw4(static_cast<uint32_t>(gi >> 2));
+        const uint32_t w[4] = {r.x, r.y, r.z, r.w};
+        s -= ln_exponential(w[gi & 3]);
       }
     }
-#pragma unroll
-    for (int k = 0; k < VEC; ++k) take_next(best, score_of(to_f32<T>(e[k]), v * VEC + k, bits[k]), off + v * VEC + k);
-  };
-  // four 16-byte loads in flight per thread before any of them is used
-  constexpr int UNROLL = NVLLM_SAMPLER_UNROLL;
-  const uint4* xv = reinterpret_cast<const uint4*>(x);
-  int v = tid;
-  for (; v + (UNROLL - 1) * nthreads < n_vec; v += UNROLL * nthreads) {
-    uint4 raw[UNROLL];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) raw[u] = xv[v + u * nthreads];
-#pragma unroll
-    for (int u = 0; u < UNROLL; ++u) consume(raw[u], v + u * nthreads);
-  }
-  for (; v < n_vec; v += nthreads) consume(xv[v], v);
-  // tail (and whole rows that are not 16-byte aligned): one element at a time, same counters
-  for (int i = n_vec * VEC + tid; i < p.vocab; i += nthreads) {
-    uint32_t b = 0;
-    if (!greedy && !nz) {
-      const int gi = off + i;  // global position
-      const uint4 r = philox4x32_10(make_uint4(static_cast<uint32_t>(gi >> 2), static_cast<uint32_t>(row),
-                                               static_cast<uint32_t>(p.step), static_cast<uint32_t>(p.step >> 32)),
-                                    key);
-      const uint32_t w[4] = {r.x, r.y, r.z, r.w};
-      b = w[gi & 3];
-    }
-    take_next(best, score_of(to_f32<T>(x[i]), i, b), off + i);
+    take(best, s, off + i);
   }
 
   // block argmax: shuffle inside a warp, shared memory across the warps; then across the cluster
@@ -311,13 +502,13 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   p.vocab = vocab;
   p.offset = vocab_offset;
   p.candidates = candidates;
-  // rows whose start is not 16-byte aligned take the element-wise path inside the kernel.
-  // Blocks per row: as many (1, 2, 4, 8) as keep the grid within one resident wave of
-  // 8 blocks on every SM of this device, and no more than the row has work for.
   const int sms = num_sms();
   if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: no CUDA device is usable");
-  int csize = 8;
-  while (csize > 1 && (static_cast<int64_t>(batch) * csize > static_cast<int64_t>(sms) * (NVLLM_SAMPLER_MINBLOCKS > 4 ? NVLLM_SAMPLER_MINBLOCKS : 8) || vocab < csize * 256 * 8)) csize >>= 1;
+  // Blocks per row: as few (1, 2, 4, 8) as give every SM three blocks, since every block pays its start
+  // and its merge; more would only help the balance, fewer leave the SMs short of warps (measured at
+  // batch 8 to 512).  No more than the row has work for.
+  int csize = 1;
+  while (csize < 8 && static_cast<int64_t>(batch) * csize < 3ll * sms && vocab >= csize * 2 * 256 * 8) csize *= 2;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(batch) * csize, 1, 1);
   cfg.blockDim = dim3(256, 1, 1);

@@ -14,7 +14,7 @@ import cases as C  # noqa: E402
 
 GOLDEN = C.GOLDEN_DIR
 
-from nano_vllm_b200 import attention as A
+from nano_vllm_b200 import _lib, attention as A
 from oracle import paged_attention_ref as R
 
 pytestmark = pytest.mark.gpu
@@ -187,3 +187,27 @@ def test_sharded_candidates_pick_the_token_of_the_one_rank_kernel(cuda, ranks, v
     real = logits[:, :per].contiguous()
     merged = _merge([A.sample_candidates(real, temps, 0, seed=5, step=1), A.sample_candidates(nan_slice, temps, per, seed=5, step=1)])
     assert torch.equal(A.sample_unpack(merged), A.sample_tokens(real, temps, seed=5, step=1))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab", [3, 8, 1000, 151643])
+@pytest.mark.parametrize("peak", [0.0, 60.0])
+def test_rows_at_any_alignment_pick_the_same_tokens(cuda, dtype, vocab, peak):
+    """The same logits, starting at each element offset within a 16-byte piece: groups shifted out of two
+    loads, elements at the edges, and (with a peak) whole warps that skip the generator.  The generated
+    noise depends on the position only, so the tokens must not change; nor may they differ from a
+    plain evaluation of the same row in slices, which sees another history of best scores."""
+    g = torch.Generator().manual_seed(vocab)
+    logits = (torch.randn(5, vocab, generator=g) * 3).to(dtype)
+    logits[:, vocab // 2] += peak
+    temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.6], device=cuda)
+    want = A.sample_tokens(logits.to(cuda), temps, seed=11, step=5)
+    for shift in range(1, 16 // logits.element_size()):
+        buf = torch.full((5, vocab + 8), 1e4, dtype=dtype, device=cuda)  # what lies around the row must not be seen
+        rows = buf[:, shift:shift + vocab]
+        rows.copy_(logits)
+        assert torch.equal(A.sample_tokens(rows, temps, seed=11, step=5), want), f"shift {shift}"
+    cuts = sorted({0, vocab // 3, vocab // 2 + 1, vocab})
+    cand = torch.stack([A.sample_candidates(logits[:, a:b].to(cuda), temps, a, seed=11, step=5) for a, b in zip(cuts, cuts[1:])])
+    assert torch.equal(A.sample_unpack(cand.max(0).values), want)
+    assert _lib.read_status() == 0
