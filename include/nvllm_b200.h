@@ -214,6 +214,38 @@ NVLLM_API int nvllm_prefill_varlen(const void* q, int64_t q_row_stride,
                          float scale, int64_t num_blocks, void* stream);
 
 /*
+ * nvllm_store_kvcache followed by nvllm_decode_paged / nvllm_prefill_varlen, as the attention layer
+ * does for every step (nanovllm/layers/attention.py:65-77), with the same arguments and results.
+ * Two launches; the attention kernel sums its lengths while the store is still running, which the
+ * two separate calls may not do because they do not know what ran before them.  n_new / total_k:
+ * rows of key / value and entries of slot_mapping (all of them are stored, as by
+ * nvllm_store_kvcache: num_slots = 256 * num_blocks).  Prefill reads key / value where
+ * block_tables is NULL, and the cache through the table otherwise.
+ */
+NVLLM_API int nvllm_attention_decode(const void* q, int64_t q_row_stride,
+                      const void* key, int64_t key_row_stride,
+                      const void* value, int64_t value_row_stride,
+                      const int32_t* slot_mapping, int64_t n_new,
+                      void* k_cache, void* v_cache,
+                      const int32_t* context_lens,
+                      const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks,
+                      void* out, int64_t out_row_stride,
+                      int32_t batch, int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim,
+                      float scale, int64_t num_blocks,
+                      void* workspace, int64_t workspace_bytes, void* stream);
+NVLLM_API int nvllm_attention_prefill(const void* q, int64_t q_row_stride,
+                         const void* key, int64_t key_row_stride,
+                         const void* value, int64_t value_row_stride,
+                         const int32_t* slot_mapping, void* k_cache, void* v_cache,
+                         const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks,
+                         void* out, int64_t out_row_stride,
+                         const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k,
+                         int64_t total_q, int64_t total_k,
+                         int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k,
+                         int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim,
+                         float scale, int64_t num_blocks, void* stream);
+
+/*
  * Fused pre-attention step over the fused qkv activation [n_tokens, (Hq + 2*Hkv) * D] (bf16,
  * row stride given): per-head RMSNorm of q and k (skipped when both weights are NULL), NeoX
  * rotary embedding of q and k from a [max_position, D] fp32 table (cos half, then sin half),

@@ -32,6 +32,12 @@ SIGNATURES = {
     "nvllm_prefill_varlen": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64,
                                        c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int32,
                                        c_int32, c_int32, c_int32, c_int32, c_int32, c_float, c_int64, c_void_p]),
+    "nvllm_attention_decode": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
+                                         c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_int64, c_int32, c_int32,
+                                         c_int32, c_int32, c_float, c_int64, c_void_p, c_int64, c_void_p]),
+    "nvllm_attention_prefill": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_void_p, c_void_p,
+                                          c_void_p, c_int64, c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64,
+                                          c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_float, c_int64, c_void_p]),
     "nvllm_qk_norm_rope_store": (c_int32, [c_void_p, c_int64, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_float,
                                            c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int32, c_int32, c_int32,
                                            c_void_p]),

@@ -64,14 +64,6 @@ int num_sms() {
 
 void count_launch(int n) { g_launches.fetch_add(n, std::memory_order_relaxed); }
 
-bool pdl_enabled() {
-  static const bool on = [] {
-    const char* s = std::getenv("NVLLM_PDL");
-    return s && s[0] == '1';
-  }();
-  return on;
-}
-
 int check_launch(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "%s: %s", what, cudaGetErrorString(e));

@@ -22,12 +22,6 @@ int check_launch(const char* what);
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
-// True when NVLLM_PDL=1 (read once per process): the decode and combine kernels are launched with
-// programmatic stream serialization, so that their blocks are already resident when the
-// predecessor in the stream drains.  Off by default: it measured +0.3 % on a 0.8 ms decode
-// step and +1 % on a 0.12 ms one.
-bool pdl_enabled();
-
 constexpr int kBlockSize = NVLLM_BLOCK_SIZE;
 
 // Multiprocessor count of the current device (queried once per device); 0 when no device is
@@ -38,15 +32,21 @@ int num_sms();
 // ---- device side -----------------------------------------------------------------------
 #ifdef __CUDACC__
 
-// Programmatic dependent launch.  Every kernel that may be launched with the attribute calls
-// pdl_prologue() as its first statement: it lets the next kernel in the stream start launching,
-// then blocks until the previous kernel has completed and its writes are visible.  Because every
-// block waits before it does anything else, completion stays transitive along the stream, and a
-// kernel launched without the attribute (or after a kernel that never signals) sees both
-// instructions as no-ops.
+// Programmatic dependent launch.  The attention kernels are launched with the attribute
+// (launch_kernel), so that their blocks may become resident while the predecessor in the stream
+// drains: about 1 us of every launch in a chain.  Each of them passes pdl_wait(), which returns when
+// the previous kernel has completed and its writes are visible, before it touches anything that
+// another kernel may have written, and so completion stays transitive along the stream.
+// pdl_trigger() lets the next kernel in the stream start launching once every block has reached
+// it (kernels that were not launched with the attribute are unaffected).
+// A kernel whose predecessor was issued by the same entry point, and calls pdl_wait() before
+// pdl_trigger(), may read what neither of the two writes before its own pdl_wait(): everything
+// older is then complete.
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_prologue() {
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  pdl_trigger();
+  pdl_wait();
 }
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -58,8 +58,10 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
   asm volatile("cp.async.cg.shared.global.L2::128B [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes));
 }
-__device__ __forceinline__ void st_shared16(uint32_t dst, const uint4& v) {
-  asm volatile("st.shared.v4.u32 [%0], {%1,%2,%3,%4};\n" ::"r"(dst), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+__device__ __forceinline__ uint4 ld_shared16(uint32_t src) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4];\n" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(src) : "memory");
+  return v;
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -132,10 +134,10 @@ __device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
   return r;
 }
 
-// Launch with (or, when `pdl` is false, without) programmatic stream serialization.
+// Launch with programmatic stream serialization; counts the launch and reports a refusal.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, bool pdl,
-                                 Args&&... args) {
+inline int launch_kernel(const char* what, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                         Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
@@ -145,8 +147,12 @@ inline cudaError_t launch_kernel(void (*kernel)(KArgs...), dim3 grid, dim3 block
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = pdl ? 1 : 0;
-  return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+  count_launch();
+  if (e == cudaSuccess) return NVLLM_OK;
+  (void)cudaGetLastError();
+  return fail(NVLLM_E_CUDA, "%s launch: %s", what, cudaGetErrorString(e));
 }
 
 #endif  // __CUDACC__

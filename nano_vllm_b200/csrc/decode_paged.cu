@@ -26,11 +26,21 @@
 //   * When a range leaves a sequence, the NW warps merge their (max, sum, O) through a
 //     dedicated patch of shared memory.  A sequence that lies inside one range is normalised
 //     and written as bf16 at once.  A sequence cut by a range boundary gives one fp32 partial
-//     per range; the block that delivers the last partial (an arrival counter per (sequence,
-//     KV head) in the workspace, no waiting) merges them in range order and writes the row, so
-//     there is no second launch.  The counters are returned to zero by that block.
+//     per range, written without waiting for anything; only its first and its last sequence can
+//     be cut, so a block reports its (at most two) partials when its range is done.  The block
+//     that reports the last partial (an arrival counter per (sequence, KV head) in the workspace,
+//     no waiting) merges them in range order and writes the row, so there is no second launch.
+//     The counters are returned to zero by that block.
 //   * Step variant: the block that streams token ctx-1 of a sequence takes that row from the
-//     new K/V activation instead of the cache and writes it to its cache slot on the way.
+//     new K/V activation instead of the cache (with the same asynchronous copies) and writes it to
+//     its cache slot when the tile is used.
+//
+// Small batches are bound by a chain of trips to memory: lengths, block table, K/V, then for cut
+// sequences partials out, arrival, partials in.  Table lines are fetched under the lengths, the
+// arrivals wait for nothing in the middle of a range, and a merge takes one trip for eight parts.
+// One launch in a chain, from a graph (head_dim 128, 16 / 8 heads): one sequence of 317 tokens 8.7 ->
+// 6.2 us, one of 4096 20.0 -> 10.7, 8 of 100-1024 16.3 -> 11.9, 16 of them 18.1 -> 14.9, 64 of them
+// 35.3 -> 32.7; 256 sequences of 2048-8192 tokens (32 / 8 heads, step variant) 795 -> 747.
 #include <cstdlib>
 
 #include "common.cuh"
@@ -77,6 +87,7 @@ struct DecodeParams {
   int64_t v_new_stride;
   const int32_t* slot_mapping;
   int n_ranges;
+  bool lengths_early;      // lengths and tables were complete before the previous kernel in the stream let this one start
   unsigned int* counters;  // [batch * hkv], zero between launches
   float* ws_o;             // [n_ranges + batch][hq][D]
   float* ws_ml;            // [n_ranges + batch][hq][2] = (running max in log2 units, sum)
@@ -105,17 +116,30 @@ struct DecodeCfg {
 // The sequence a block is working in: index, global index of its first unit, units, length.
 struct SeqCursor {
   int b, first, units, ctx;
+  int slot;  // step variant: slot of the new token (-1: nothing is stored)
 };
+
+// A sequence whose units lie in several ranges: n of them, from r_first on.
+struct Cut {
+  int b, r_first, n;
+};
+
+// Cost of a streamed unit over the cost of a merged partial: of 1, 2, 4, 8 and no limit, 8 was the best or
+// within 0.6 us of it at every size of one to eight sequences of 300 to 32000 tokens (one sequence of
+// 32000 in the head_dim 64 geometry: 16.1 us, 26.1 without a limit).
+constexpr float kSplitBalance = 8.f;
 
 template <class C>
 __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const DecodeParams p) {
   constexpr int D = C::D, TT = C::TT, NST = C::NST, NW = C::NW, UNIT = C::UNIT, NT = NW * 32;
+  constexpr int QUADS = D / 4, GROUPS = NT / QUADS;  // lanes that hold a head four columns each; such groups in a block
   extern __shared__ __align__(128) unsigned char smem[];
   __shared__ int s_scan[NW];
-  __shared__ int s_start[2];
-  __shared__ int s_last_arrival;
+  __shared__ int s_start[3];
+  __shared__ int s_last_arrival[2];
 
-  pdl_prologue();
+  pdl_trigger();
+  if (!p.lengths_early) pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gid = lane >> 2, tig = lane & 3;
   const int kvh = blockIdx.x % p.hkv;
@@ -130,9 +154,14 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   // ---- 1. units per sequence, block-wide scan, this block's range of the unit list ------
   const int per_thread = (p.batch + NT - 1) / NT;
   const int b_lo = min(tid * per_thread, p.batch), b_hi = min(b_lo + per_thread, p.batch);
-  int local = 0;
+  // The first table line of every sequence on its way to this SM while the lengths are summed: the
+  // block does not know yet whose it needs (beyond this batch the stream hides the trip).
+  if (p.batch <= NT && tid < p.batch)
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(p.block_tables + tid * p.bt_stride));
+  int local = 0, len_lo = 0;
   for (int b = b_lo; b < b_hi; ++b) {
     const int c = length_of(b);
+    if (b == b_lo) len_lo = c;
     local += units_of(c);
     if (c == 0 && b % p.n_ranges == range) {  // empty context: defined output (zeros), no cache access
       uint4* dst = reinterpret_cast<uint4*>(p.out + b * p.out_stride + static_cast<int64_t>(kvh * p.g) * D);
@@ -154,44 +183,56 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     total += s_scan[w];
   }
   const int excl = before + incl - local;
-  // No more ranges than units, so that every range in use holds at least one unit and the
-  // ranges that share a sequence are consecutive.
-  const int n_ranges = min(p.n_ranges, total);
-  if (range >= n_ranges) return;  // block-uniform (also when the whole batch is empty)
-  const int u0 = static_cast<int>(static_cast<int64_t>(total) * range / n_ranges);
-  const int u1 = static_cast<int>(static_cast<int64_t>(total) * (range + 1) / n_ranges);
+  // No more ranges than units, so that every range in use holds at least one unit and the ranges
+  // that share a sequence are consecutive.  And where sequences are few, no more than balance the
+  // two costs of a cut: a range streams total / n units and a sequence's merge reads n / batch
+  // partials, so that the sum is least at n = sqrt(c total batch).
+  const int n_ranges = max(1, min(min(p.n_ranges, total), static_cast<int>(sqrtf(kSplitBalance * total * p.batch))));
+  if (range >= n_ranges || total == 0) return;  // block-uniform (also when the whole batch is empty)
+  // the first `longer` ranges hold one unit more than the others
+  const int per_range = total / n_ranges, longer = total - per_range * n_ranges;
+  const int u0 = range * per_range + min(range, longer);
+  const int u1 = u0 + per_range + (range < longer ? 1 : 0);
   if (local > 0 && excl <= u0 && u0 < excl + local) {  // the one thread whose sequences hold unit u0
     int first = excl;
     for (int b = b_lo;; ++b) {
-      const int n = units_of(length_of(b));
+      const int len = b == b_lo ? len_lo : length_of(b), n = units_of(len);
       if (u0 < first + n) {
         s_start[0] = b;
         s_start[1] = first;
+        s_start[2] = len;
         break;
       }
       first += n;
     }
   }
   __syncthreads();
-  // the range that holds global unit u (ranges are [total*s/n, total*(s+1)/n))
+  // the range that holds global unit u
   auto range_of = [&](int u) {
-    return static_cast<int>((static_cast<int64_t>(u + 1) * n_ranges - 1) / total);
+    const int split = longer * (per_range + 1);
+    return u < split ? u / (per_range + 1) : longer + (u - split) / per_range;
   };
 
+  auto slot_of = [&](int b) { return p.k_new != nullptr ? p.slot_mapping[b] : -1; };
   SeqCursor cc;  // compute side
   cc.b = s_start[0];
   cc.first = s_start[1];
-  cc.ctx = length_of(cc.b);
+  cc.ctx = s_start[2];
   cc.units = units_of(cc.ctx);
+  cc.slot = slot_of(cc.b);
   SeqCursor pc = cc;  // load side, NST-1 units ahead
   auto seek = [&](SeqCursor& c, int u) {  // u < total, so c.b stays inside the batch
-    while (u >= c.first + c.units) {
+    if (u < c.first + c.units) return;
+    do {
       c.first += c.units;
       ++c.b;
       c.ctx = length_of(c.b);
       c.units = units_of(c.ctx);
-    }
+    } while (u >= c.first + c.units);
+    c.slot = slot_of(c.b);
   };
+
+  if (p.lengths_early) pdl_wait();  // from here on the cache is read
 
   // Q^T as the B operand: lane (gid, tig) holds q[head gid][16*ks + 2*tig .. +1] and [.. + 8].
   auto load_q = [&](uint32_t (&dst)[C::KS][2], int b) {
@@ -215,7 +256,9 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   const uint32_t warp_smem = smem_u32(smem) + warp * C::WARP_BYTES;
   const int64_t row_elems = static_cast<int64_t>(p.hkv) * D;
 
+  unsigned fresh = 0;  // step variant: stages whose tile holds the new token's row
   auto load_tile = [&](const SeqCursor& c, int u, int stage) {
+    fresh &= ~(1u << stage);
     const int t0 = (u - c.first) * UNIT + warp * TT;
     if (t0 >= c.ctx) return;  // this warp has no token in the sequence's last unit
     int64_t blk = p.block_tables[c.b * p.bt_stride + t0 / kBlockSize];
@@ -225,15 +268,16 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       blk = 0;
     }
     const int64_t slot0 = blk * kBlockSize + (t0 % kBlockSize);
-    // Step variant: token ctx-1 is the one being decoded.  Its row comes from the activation
-    // and goes to the cache from here, provided slot_mapping agrees with the block table.
+    // Step variant: token ctx-1 is the one being decoded.  Its row comes from the activation,
+    // provided slot_mapping agrees with the block table, and goes to the cache when the tile is used.
     const int last = c.ctx - 1;
-    bool take_new = false;
-    if (p.k_new != nullptr && last < t0 + TT) {  // last >= t0 holds because t0 < ctx
-      const int32_t slot = p.slot_mapping[c.b];
-      if (slot >= 0) {
-        if (blk_ok && slot == slot0 + (last - t0)) take_new = true;
-        else if (lane == 0) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
+    int new_row = -1;
+    if (p.k_new != nullptr && last < t0 + TT && c.slot >= 0) {  // last >= t0 holds because t0 < ctx
+      if (blk_ok && c.slot == slot0 + (last - t0)) {
+        new_row = last - t0;
+        fresh |= 1u << stage;
+      } else if (lane == 0) {
+        atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
       }
     }
     const uint32_t kdst = warp_smem + stage * C::STAGE_BYTES;
@@ -243,19 +287,15 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       const int r = idx / C::CPR, col = idx % C::CPR;
       const int bytes = (blk_ok && t0 + r < c.ctx) ? 16 : 0;
       const int64_t off = bytes ? (slot0 + r) * row_elems + kvh * D + col * 8 : 0;
-      const uint32_t dst = kdst + r * C::ROW_BYTES + ((col ^ (r & 7)) << 4);
-      if (take_new && t0 + r == last) {
+      const __nv_bfloat16 *ksrc = p.k_cache + off, *vsrc = p.v_cache + off;
+      if (r == new_row) {
         const int64_t in_row = static_cast<int64_t>(kvh) * D + col * 8;
-        const uint4 kk = *reinterpret_cast<const uint4*>(p.k_new + c.b * p.k_new_stride + in_row);
-        const uint4 vv = *reinterpret_cast<const uint4*>(p.v_new + c.b * p.v_new_stride + in_row);
-        *reinterpret_cast<uint4*>(p.k_cache + off) = kk;
-        *reinterpret_cast<uint4*>(p.v_cache + off) = vv;
-        st_shared16(dst, kk);
-        st_shared16(dst + C::TILE_BYTES, vv);
-      } else {
-        cp_async16(dst, p.k_cache + off, bytes);
-        cp_async16(dst + C::TILE_BYTES, p.v_cache + off, bytes);
+        ksrc = p.k_new + c.b * p.k_new_stride + in_row;
+        vsrc = p.v_new + c.b * p.v_new_stride + in_row;
       }
+      const uint32_t dst = kdst + r * C::ROW_BYTES + ((col ^ (r & 7)) << 4);
+      cp_async16(dst, ksrc, bytes);
+      cp_async16(dst + C::TILE_BYTES, vsrc, bytes);
     }
   };
 
@@ -271,6 +311,21 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
 
   float* sm_o = reinterpret_cast<float*>(smem + C::RING_BYTES);  // [NW][8][D]
   float* sm_ml = sm_o + NW * 8 * D;                              // [NW][8][2]
+
+  auto add_scaled = [](float4& acc, const float4& v, float f) {
+    acc.x += v.x * f;
+    acc.y += v.y * f;
+    acc.z += v.z * f;
+    acc.w += v.w * f;
+  };
+  auto write_quad = [&](int b, int h, int d4, const float4& acc, float L) {
+    const float inv = L > 0.f ? 1.f / L : 0.f;
+    *reinterpret_cast<uint2*>(p.out + b * p.out_stride + static_cast<int64_t>(kvh * p.g + h) * D + d4 * 4) =
+        make_uint2(pack_bf16x2(acc.x * inv, acc.y * inv), pack_bf16x2(acc.z * inv, acc.w * inv));
+  };
+
+  Cut cut0{}, cut1{};  // this range's sequences that other ranges share
+  int n_cut = 0;
 
   // Leaves sequence cc.b: merges the NW warps' states and writes the output row or a partial.
   auto flush = [&]() {
@@ -295,64 +350,121 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       sm_ml[(warp * 8 + 2 * tig + 1) * 2 + 0] = m1;
       sm_ml[(warp * 8 + 2 * tig + 1) * 2 + 1] = l1;
     }
-    __syncthreads();
     const int r_first = range_of(cc.first), r_last = range_of(cc.first + cc.units - 1);
     const int n_parts = r_last - r_first + 1;  // ranges that hold a piece of this sequence
-    for (int idx = tid; idx < p.g * D; idx += NT) {
-      const int h = idx / D, d = idx % D;
-      float mm = -INFINITY;
-#pragma unroll
-      for (int w = 0; w < NW; ++w) mm = fmaxf(mm, sm_ml[(w * 8 + h) * 2]);
-      float L = 0.f, acc = 0.f;
+    __syncthreads();
+    for (int quad = tid; quad < p.g * QUADS; quad += NT) {  // four columns of a head per thread
+      const int h = quad / QUADS, d4 = quad % QUADS;
+      float m[NW], mm = -INFINITY, L = 0.f;
 #pragma unroll
       for (int w = 0; w < NW; ++w) {
-        const float mw = sm_ml[(w * 8 + h) * 2];
-        const float f = (mw == -INFINITY) ? 0.f : fast_exp2(mw - mm);
-        L += sm_ml[(w * 8 + h) * 2 + 1] * f;
-        acc += sm_o[(w * 8 + h) * D + d] * f;
+        m[w] = sm_ml[(w * 8 + h) * 2];
+        mm = fmaxf(mm, m[w]);
       }
-      const int head = kvh * p.g + h;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int w = 0; w < NW; ++w) {
+        const float f = m[w] == -INFINITY ? 0.f : fast_exp2(m[w] - mm);
+        const float4 v = *reinterpret_cast<const float4*>(sm_o + (w * 8 + h) * D + d4 * 4);
+        L += sm_ml[(w * 8 + h) * 2 + 1] * f;
+        add_scaled(acc, v, f);
+      }
       if (n_parts == 1) {
-        p.out[cc.b * p.out_stride + static_cast<int64_t>(head) * D + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
+        write_quad(cc.b, h, d4, acc, L);
       } else {
         // partial slot range + b: strictly increasing along the (range, sequence) pieces of the list
-        const int64_t row = static_cast<int64_t>(range + cc.b) * p.hq + head;
-        p.ws_o[row * D + d] = acc;
-        if (d == 0) {
-          p.ws_ml[row * 2 + 0] = mm;
-          p.ws_ml[row * 2 + 1] = L;
-        }
+        const int64_t row = static_cast<int64_t>(range + cc.b) * p.hq + kvh * p.g + h;
+        *reinterpret_cast<float4*>(p.ws_o + row * D + d4 * 4) = acc;
+        if (d4 == 0) *reinterpret_cast<float2*>(p.ws_ml + row * 2) = make_float2(mm, L);
       }
     }
-    if (n_parts > 1) {  // block-uniform
-      __threadfence();
-      __syncthreads();
-      if (tid == 0) {
-        const unsigned int arrived = atomicAdd(&p.counters[cc.b * p.hkv + kvh], 1u);
-        s_last_arrival = arrived == static_cast<unsigned int>(n_parts - 1);
+    if (n_parts > 1) {  // block-uniform; reported at the end of the range
+      if (n_cut == 0) cut0 = {cc.b, r_first, n_parts};
+      else cut1 = {cc.b, r_first, n_parts};
+      ++n_cut;
+    }
+  };
+
+  // Merges the partials of a cut sequence, all of which are in the workspace, and writes its rows.
+  // QUADS lanes take a head (four columns each); lane l of them also holds the statistics of one
+  // part of every chunk of QUADS parts, so that a chunk's statistics and its first rows are in
+  // flight together and the weights go round by shuffle: one trip to L2 for up to eight parts.
+  // Lane groups left over split the parts of a head between them.
+  auto merge_cut = [&](const Cut& c) {
+    constexpr int AHEAD = 8;
+    const int group = tid / QUADS, gl = tid % QUADS;
+    const int n_split = max(1, GROUPS / p.g);
+    for (int h0 = 0; h0 < p.g; h0 += GROUPS) {
+      const bool narrow = p.g < GROUPS;
+      const int split = narrow ? group / p.g : 0, head = narrow ? group % p.g : min(h0 + group, p.g - 1);
+      const bool active = narrow ? split < n_split : h0 + group < p.g;
+      const int64_t row0 = static_cast<int64_t>(c.r_first + c.b) * p.hq + kvh * p.g + head;
+      auto row_of = [&](int j) { return __ldcg(reinterpret_cast<const float4*>(p.ws_o + (row0 + static_cast<int64_t>(j) * p.hq) * D) + gl); };
+      float mm = -INFINITY, L = 0.f;
+      float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+      auto rebase = [&](float m_new) {
+        const float keep = mm == -INFINITY ? 0.f : fast_exp2(mm - m_new);
+        L *= keep;
+        acc.x *= keep;
+        acc.y *= keep;
+        acc.z *= keep;
+        acc.w *= keep;
+        mm = m_new;
+      };
+      for (int j0 = 0; j0 < c.n; j0 += QUADS * n_split) {  // block-uniform; a group's parts are split + n_split * k
+        float4 rows[AHEAD];
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+          const int j = j0 + k * n_split + split;
+          if (active && j < c.n) rows[k] = row_of(j);
+        }
+        const int mine = j0 + gl * n_split + split;
+        float2 ml = make_float2(-INFINITY, 0.f);
+        if (active && mine < c.n)
+          ml = __ldcg(reinterpret_cast<const float2*>(p.ws_ml + (row0 + static_cast<int64_t>(mine) * p.hq) * 2));
+        float m_new = fmaxf(mm, ml.x);
+#pragma unroll
+        for (int sh = QUADS / 2; sh > 0; sh >>= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, sh));
+        rebase(m_new);
+        const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - m_new);
+        float sum = ml.y * f;
+#pragma unroll
+        for (int sh = QUADS / 2; sh > 0; sh >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, sh);
+        L += sum;
+#pragma unroll
+        for (int k = 0; k < AHEAD; ++k) {
+          const float fk = __shfl_sync(0xffffffffu, f, k, QUADS);
+          if (active && j0 + k * n_split + split < c.n) add_scaled(acc, rows[k], fk);
+        }
+        const int n_here = min(QUADS, (c.n - j0 + n_split - 1) / n_split);
+#pragma unroll 8
+        for (int k = AHEAD; k < n_here; ++k) {
+          const int j = j0 + k * n_split + split;
+          const float fk = __shfl_sync(0xffffffffu, f, k, QUADS);
+          if (active && j < c.n) add_scaled(acc, row_of(j), fk);
+        }
       }
-      __syncthreads();
-      if (s_last_arrival) {  // every piece is in the workspace: merge them in range order
-        __threadfence();
-        for (int idx = tid; idx < p.g * D; idx += NT) {
-          const int h = idx / D, d = idx % D;
-          const int head = kvh * p.g + h;
-          const int64_t row0 = static_cast<int64_t>(r_first + cc.b) * p.hq + head;
-          float mm = -INFINITY;
-          for (int j = 0; j < n_parts; ++j) mm = fmaxf(mm, __ldcg(p.ws_ml + (row0 + static_cast<int64_t>(j) * p.hq) * 2));
-          float L = 0.f, acc = 0.f;
-          for (int j = 0; j < n_parts; ++j) {
-            const int64_t row = row0 + static_cast<int64_t>(j) * p.hq;
-            const float mj = __ldcg(p.ws_ml + row * 2);
-            const float f = (mj == -INFINITY) ? 0.f : fast_exp2(mj - mm);
-            L += __ldcg(p.ws_ml + row * 2 + 1) * f;
-            acc += __ldcg(p.ws_o + row * D + d) * f;
+      if (n_split > 1) {  // block-uniform
+        float* patch = sm_o + group * (D + 4);
+        if (active && split > 0) {
+          *reinterpret_cast<float4*>(patch + gl * 4) = acc;
+          if (gl == 0) *reinterpret_cast<float2*>(patch + D) = make_float2(mm, L);
+        }
+        __syncthreads();
+        if (active && split == 0)
+          for (int k = 1; k < n_split; ++k) {
+            const float* other = sm_o + (group + k * p.g) * (D + 4);
+            const float2 ml = *reinterpret_cast<const float2*>(other + D);
+            rebase(fmaxf(mm, ml.x));
+            const float f = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
+            L += ml.y * f;
+            add_scaled(acc, *reinterpret_cast<const float4*>(other + gl * 4), f);
           }
-          p.out[cc.b * p.out_stride + static_cast<int64_t>(head) * D + d] = __float2bfloat16(L > 0.f ? acc / L : 0.f);
-        }
-        if (tid == 0) p.counters[cc.b * p.hkv + kvh] = 0u;  // ready for the next launch
+        __syncthreads();
       }
+      if (active && split == 0) write_quad(c.b, head, gl, acc, L);
     }
+    if (tid == 0) p.counters[c.b * p.hkv + kvh] = 0u;  // ready for the next launch
   };
 
   // ---- 2. stream the range ------------------------------------------------------------------
@@ -398,6 +510,15 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     const int t_end = cc.ctx;
     const uint32_t kbase = warp_smem + (i % NST) * C::STAGE_BYTES;
     const uint32_t vbase = kbase + C::TILE_BYTES;
+    if (fresh >> (i % NST) & 1u) {  // step variant: the new token's row, on its way to the cache
+      const int r = cc.ctx - 1 - t0;
+      if (lane < 2 * C::CPR) {  // K pieces, then V pieces (for head_dim 128 one per lane)
+        const int col = lane % C::CPR;
+        const uint4 v = ld_shared16((lane < C::CPR ? kbase : vbase) + r * C::ROW_BYTES + ((col ^ (r & 7)) << 4));
+        *reinterpret_cast<uint4*>((lane < C::CPR ? p.k_cache : p.v_cache) + static_cast<int64_t>(cc.slot) * row_elems + kvh * D +
+                                  col * 8) = v;
+      }
+    }
 
     // S^T = K Q^T
     float s[C::MT][4];
@@ -474,6 +595,18 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     }
   }
   cp_async_wait<0>();
+  if (n_cut == 0) return;  // block-uniform
+  __syncthreads();         // every thread's partials are written
+  if (tid < n_cut) {
+    const Cut& c = tid == 0 ? cut0 : cut1;
+    unsigned int arrived;  // releases the block's partials (the barrier ordered them before), acquires the others'
+    asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
+                 : "=r"(arrived) : "l"(p.counters + c.b * p.hkv + kvh) : "memory");
+    s_last_arrival[tid] = arrived == static_cast<unsigned int>(c.n - 1);
+  }
+  __syncthreads();
+  if (s_last_arrival[0]) merge_cut(cut0);
+  if (n_cut > 1 && s_last_arrival[1]) merge_cut(cut1);
 }
 
 // ---- host side -------------------------------------------------------------------------
@@ -533,14 +666,8 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
     attr_set[dev] = true;
   }
   const int grid = p.n_ranges * p.hkv;
-  cudaError_t e = launch_kernel(decode_paged_kernel<C>, dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream,
-                                pdl_enabled(), p);
-  count_launch();
-  if (e != cudaSuccess) {
-    (void)cudaGetLastError();
-    return fail(NVLLM_E_CUDA, "decode_paged launch: %s", cudaGetErrorString(e));
-  }
-  return NVLLM_OK;
+  return launch_kernel("decode_paged", decode_paged_kernel<C>, dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream,
+                       p);
 }
 
 // Shared body of nvllm_decode_paged and nvllm_decode_step.
@@ -549,7 +676,7 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
                          void* v_cache, const int32_t* context_lens, const int32_t* block_tables, int64_t bt_row_stride,
                          int32_t max_blocks, void* out, int64_t out_row_stride, int32_t batch, int32_t num_q_heads,
                          int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks, void* workspace,
-                         int64_t workspace_bytes, void* stream, bool with_store) {
+                         int64_t workspace_bytes, void* stream, bool with_store, bool lengths_early) {
   int rc = check_decode_geometry(who, batch, max_blocks, num_q_heads, num_kv_heads, head_dim);
   if (rc) return rc;
   if (batch == 0) return NVLLM_OK;
@@ -599,6 +726,7 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
   p.v_new = with_store ? static_cast<const __nv_bfloat16*>(v_new) : nullptr;
   p.v_new_stride = v_new_row_stride;
   p.slot_mapping = slot_mapping;
+  p.lengths_early = lengths_early;
   p.n_ranges = ranges_for(decode_ctas(), num_kv_heads);
   const int64_t rows = (static_cast<int64_t>(ranges_for(kMaxDecodeCtas, num_kv_heads)) + batch) * num_q_heads;
   p.counters = static_cast<unsigned int*>(workspace);
@@ -638,7 +766,7 @@ extern "C" int nvllm_decode_paged(const void* q, int64_t q_row_stride, const voi
   return nvllm::decode_common("decode_paged", q, q_row_stride, nullptr, 0, nullptr, 0, nullptr, const_cast<void*>(k_cache),
                               const_cast<void*>(v_cache), context_lens, block_tables, bt_row_stride, max_blocks, out,
                               out_row_stride, batch, num_q_heads, num_kv_heads, head_dim, scale, num_blocks, workspace,
-                              workspace_bytes, stream, false);
+                              workspace_bytes, stream, false, false);
 }
 
 extern "C" int nvllm_decode_step(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
@@ -650,7 +778,21 @@ extern "C" int nvllm_decode_step(const void* q, int64_t q_row_stride, const void
   return nvllm::decode_common("decode_step", q, q_row_stride, key, key_row_stride, value, value_row_stride, slot_mapping,
                               k_cache, v_cache, context_lens, block_tables, bt_row_stride, max_blocks, out, out_row_stride,
                               batch, num_q_heads, num_kv_heads, head_dim, scale, num_blocks, workspace, workspace_bytes,
-                              stream, true);
+                              stream, true, false);
+}
+
+extern "C" int nvllm_attention_decode(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
+                                      const void* value, int64_t value_row_stride, const int32_t* slot_mapping, int64_t n_new,
+                                      void* k_cache, void* v_cache, const int32_t* context_lens, const int32_t* block_tables,
+                                      int64_t bt_row_stride, int32_t max_blocks, void* out, int64_t out_row_stride,
+                                      int32_t batch, int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim, float scale,
+                                      int64_t num_blocks, void* workspace, int64_t workspace_bytes, void* stream) {
+  const int rc = nvllm_store_kvcache(key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_new,
+                                     num_kv_heads * head_dim, num_blocks * nvllm::kBlockSize, stream);
+  if (rc) return rc;
+  return nvllm::decode_common("attention_decode", q, q_row_stride, nullptr, 0, nullptr, 0, nullptr, k_cache, v_cache, context_lens,
+                              block_tables, bt_row_stride, max_blocks, out, out_row_stride, batch, num_q_heads, num_kv_heads,
+                              head_dim, scale, num_blocks, workspace, workspace_bytes, stream, false, n_new > 0);
 }
 
 // ---- decode without a caller-provided workspace ---------------------------------------------

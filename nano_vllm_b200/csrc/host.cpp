@@ -47,6 +47,8 @@ struct Api {
   decltype(&nvllm_decode_step) decode_step;
   decltype(&nvllm_decode_workspace_bytes) decode_workspace_bytes;
   decltype(&nvllm_prefill_varlen) prefill_varlen;
+  decltype(&nvllm_attention_decode) attention_decode;
+  decltype(&nvllm_attention_prefill) attention_prefill;
   decltype(&nvllm_qk_norm_rope_store) qk_norm_rope_store;
   decltype(&nvllm_sample_tokens) sample_tokens;
   decltype(&nvllm_sample_candidates) sample_candidates;
@@ -148,21 +150,26 @@ struct Rows {
   int64_t n, stride;
 };
 
-void store(const Rows& k, const Rows& v, int64_t row, const at::Tensor& k_cache, const at::Tensor& v_cache,
-           const at::Tensor& slot_mapping) {
+void check_store(const Rows& k, int64_t row, const at::Tensor& k_cache, const at::Tensor& v_cache, const at::Tensor& slot_mapping) {
   require(k_cache.dim() > 1 && k_cache.stride(1) == row && v_cache.dim() > 1 && v_cache.stride(1) == row,
           "k_cache.stride(1) == D and v_cache.stride(1) == D");
   require(slot_mapping.numel() == k.n, "slot_mapping.numel() == N");
   require_cuda_bf16("k_cache", k_cache);
   require_cuda_bf16("v_cache", v_cache);
   require_i32("slot_mapping", slot_mapping);
+}
+
+void store(const Rows& k, const Rows& v, int64_t row, const at::Tensor& k_cache, const at::Tensor& v_cache,
+           const at::Tensor& slot_mapping) {
+  check_store(k, row, k_cache, v_cache, slot_mapping);
   check(api.store_kvcache(k.p, k.stride, v.p, v.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(slot_mapping), k.n,
                           static_cast<int32_t>(row), k_cache.numel() / row, stream_of(k_cache)));
 }
 
-struct Step {  // the new token's rows, for the one-launch store + decode
+struct Step {  // the new tokens' rows, for a call that stores as well
   Rows k, v;
   const int32_t* slots;
+  bool one_launch;  // decode_step's rules; otherwise store_kvcache's, in a launch of its own
 };
 
 void decode(const Rows& q, int64_t hq, int64_t d, const at::Tensor& k_cache, const at::Tensor& v_cache,
@@ -187,7 +194,12 @@ void decode(const Rows& q, int64_t hq, int64_t d, const at::Tensor& k_cache, con
   const int32_t B = static_cast<int32_t>(q.n), HQ = static_cast<int32_t>(hq), HKV = static_cast<int32_t>(hkv),
                 D = static_cast<int32_t>(d);
   void* st = stream_of(k_cache);
-  if (step)
+  if (step && !step->one_launch)
+    check(api.attention_decode(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots, step->k.n,
+                               k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens), ptr<int32_t>(block_tables),
+                               block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D, static_cast<float>(scale),
+                               num_blocks, ws, ws_size, st));
+  else if (step)
     check(api.decode_step(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots, k_cache.data_ptr(),
                           v_cache.data_ptr(), ptr<int32_t>(context_lens), ptr<int32_t>(block_tables), block_tables.stride(0),
                           width, out.p, out.stride, B, HQ, HKV, D, static_cast<float>(scale), num_blocks, ws, ws_size, st));
@@ -213,7 +225,8 @@ KV paged_kv(const at::Tensor& k, const at::Tensor& v, const at::Tensor& block_ta
 }
 
 void prefill(const Rows& q, int64_t hq, int64_t d, const KV& kv, const at::Tensor& cu_q, const at::Tensor& cu_k, int64_t max_q,
-             int64_t max_k, double scale, const Rows& out, void* stream) {
+             int64_t max_k, double scale, const Rows& out, void* stream, const Step* step = nullptr,
+             const at::Tensor* k_cache = nullptr, const at::Tensor* v_cache = nullptr) {
   require_i32("cu_seqlens_q", cu_q);
   require_i32("cu_seqlens_k", cu_k);
   const int64_t batch = cu_q.numel() - 1;
@@ -221,6 +234,16 @@ void prefill(const Rows& q, int64_t hq, int64_t d, const KV& kv, const at::Tenso
   const at::Tensor* bt = kv.block_tables;
   if (bt)
     require(bt->dim() == 2 && bt->size(0) == batch, "block_tables.dim() == 2 and block_tables.shape[0] == batch");
+  if (step) {
+    check(api.attention_prefill(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots,
+                                k_cache->data_ptr(), v_cache->data_ptr(), bt ? ptr<int32_t>(*bt) : nullptr, bt ? bt->stride(0) : 0,
+                                bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride, ptr<int32_t>(cu_q),
+                                ptr<int32_t>(cu_k), q.n, step->k.n, static_cast<int32_t>(batch), static_cast<int32_t>(max_q),
+                                static_cast<int32_t>(max_k), static_cast<int32_t>(hq), static_cast<int32_t>(kv.hkv),
+                                static_cast<int32_t>(d), static_cast<float>(scale),
+                                k_cache->numel() / (NVLLM_BLOCK_SIZE * kv.hkv * d), stream));
+    return;
+  }
   if (q.n == 0 || batch == 0) return;
   check(api.prefill_varlen(q.p, q.stride, kv.k.p, kv.k.stride, kv.v.p, kv.v.stride, bt ? ptr<int32_t>(*bt) : nullptr,
                            bt ? bt->stride(0) : 0, bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride,
@@ -294,7 +317,7 @@ PyObject* decode_step(PyObject* const* a) {
     require(t->dim() == 3 && t->size(0) == B && t->size(1) == hkv && t->size(2) == D,
             "key.shape == (B, Hkv, D) and value.shape == (B, Hkv, D)");
   const Step step = {rows3(key, "key.stride(-1) == 1 and key.stride(1) == D"),
-                     rows3(value, "value.stride(-1) == 1 and value.stride(1) == D"), ptr<int32_t>(slots)};
+                     rows3(value, "value.stride(-1) == 1 and value.stride(1) == D"), ptr<int32_t>(slots), true};
   require(slots.numel() == B, "slot_mapping.numel() == B");
   const c10::cuda::CUDAGuard guard(q.device());
   Rows o;
@@ -374,9 +397,18 @@ PyObject* attention_forward(PyObject* const* a) {
   }
   require_cuda_bf16("q", q);
   const c10::cuda::CUDAGuard guard(q.device());
+  Ref slots(PyObject_GetAttr(ctx, names.slot_mapping));
+  Step step{};
+  const Step* with_store = nullptr;
   if (do_store) {
-    Ref slots(PyObject_GetAttr(ctx, names.slot_mapping));
-    store(kr, vr, hkv * d, k_cache, v_cache, tensor(slots.o, "slot_mapping"));
+    const at::Tensor& sm = tensor(slots.o, "slot_mapping");
+    if (qr.n > 0 && k_cache.numel() % (NVLLM_BLOCK_SIZE * hkv * d) == 0) {
+      check_store(kr, hkv * d, k_cache, v_cache, sm);
+      step = {kr, vr, ptr<int32_t>(sm), false};
+      with_store = &step;
+    } else {
+      store(kr, vr, hkv * d, k_cache, v_cache, sm);
+    }
   }
   at::Tensor out = at::empty({qr.n, hq * d}, q.options());
   const Rows o = {out.data_ptr(), qr.n, hq * d};
@@ -386,10 +418,11 @@ PyObject* attention_forward(PyObject* const* a) {
     const at::Tensor* table = maybe_tensor(bt.o, "block_tables");
     // prefix cache: every key is read through the table
     const KV kv = table ? paged_kv(k_cache, v_cache, *table) : KV{kr, vr, hkv, nullptr, 0};
-    prefill(qr, hq, d, kv, tensor(cq.o, "cu_seqlens_q"), tensor(ck.o, "cu_seqlens_k"), mq, mk, scale, o, stream_of(q));
+    prefill(qr, hq, d, kv, tensor(cq.o, "cu_seqlens_q"), tensor(ck.o, "cu_seqlens_k"), mq, mk, scale, o, stream_of(q), with_store,
+            &k_cache, &v_cache);
   } else {
     Ref lens(PyObject_GetAttr(ctx, names.context_lens));
-    decode(qr, hq, d, k_cache, v_cache, tensor(lens.o, "context_lens"), tensor(bt.o, "block_tables"), scale, o, nullptr);
+    decode(qr, hq, d, k_cache, v_cache, tensor(lens.o, "context_lens"), tensor(bt.o, "block_tables"), scale, o, with_store);
   }
   return wrap(std::move(out));
 }
@@ -622,6 +655,8 @@ PyObject* bind(PyObject* const* a) {  // library path, check
   RESOLVE(decode_step);
   RESOLVE(decode_workspace_bytes);
   RESOLVE(prefill_varlen);
+  RESOLVE(attention_decode);
+  RESOLVE(attention_prefill);
   RESOLVE(qk_norm_rope_store);
   RESOLVE(sample_tokens);
   RESOLVE(sample_candidates);

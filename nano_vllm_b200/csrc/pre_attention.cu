@@ -176,9 +176,8 @@ static int launch_pre_attention(const PreAttnParams& p, cudaStream_t stream) {
   const int64_t units = p.n_tokens * ((p.hq + 2 * p.hkv + HPT - 1) / HPT);
   constexpr int per_block = kPreThreads / (D / 8);
   if (units > 0x7fffffffLL) return fail(NVLLM_E_GEOMETRY, "qk_norm_rope_store: too many tokens for one launch");
-  pre_attention_kernel<D, HPT><<<static_cast<unsigned>((units + per_block - 1) / per_block), kPreThreads, 0, stream>>>(p);
-  count_launch();
-  return check_launch("qk_norm_rope_store launch");
+  return launch_kernel("qk_norm_rope_store", pre_attention_kernel<D, HPT>,
+                       dim3(static_cast<unsigned>((units + per_block - 1) / per_block)), dim3(kPreThreads), 0, stream, p);
 }
 
 }  // namespace nvllm

@@ -4,14 +4,14 @@
 #include "common.cuh"
 #include "prefill.cuh"
 
-extern "C" int nvllm_prefill_varlen(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride,
-                                    const void* v, int64_t v_row_stride, const int32_t* block_tables,
-                                    int64_t bt_row_stride, int32_t max_blocks, void* out, int64_t out_row_stride,
-                                    const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int64_t total_q,
-                                    int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads,
-                                    int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks,
-                                    void* stream) {
-  using namespace nvllm;
+namespace nvllm {
+
+static int prefill_common(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride, const void* v,
+                          int64_t v_row_stride, const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks, void* out,
+                          int64_t out_row_stride, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int64_t total_q,
+                          int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads,
+                          int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks, void* stream,
+                          bool lengths_early) {
   if (head_dim != 64 && head_dim != 128)
     return fail(NVLLM_E_GEOMETRY, "prefill_varlen: head_dim=%d unsupported (64 or 128)", head_dim);
   if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads)
@@ -74,6 +74,42 @@ extern "C" int nvllm_prefill_varlen(const void* q, int64_t q_row_stride, const v
   p.pack = 1;
   p.scale_log2e = scale * 1.4426950408889634f;
   p.num_blocks = num_blocks;
+  p.lengths_early = lengths_early;
   if (use_mma) return launch_prefill_mma(p, static_cast<cudaStream_t>(stream));
   return launch_prefill_tcp(p, total_q, total_k, static_cast<cudaStream_t>(stream));
+}
+
+}  // namespace nvllm
+
+extern "C" int nvllm_prefill_varlen(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride,
+                                    const void* v, int64_t v_row_stride, const int32_t* block_tables,
+                                    int64_t bt_row_stride, int32_t max_blocks, void* out, int64_t out_row_stride,
+                                    const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int64_t total_q,
+                                    int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads,
+                                    int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks,
+                                    void* stream) {
+  return nvllm::prefill_common(q, q_row_stride, k, k_row_stride, v, v_row_stride, block_tables, bt_row_stride, max_blocks, out,
+                               out_row_stride, cu_seqlens_q, cu_seqlens_k, total_q, total_k, batch, max_seqlen_q, max_seqlen_k,
+                               num_q_heads, num_kv_heads, head_dim, scale, num_blocks, stream, false);
+}
+
+extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
+                                       const void* value, int64_t value_row_stride, const int32_t* slot_mapping, void* k_cache,
+                                       void* v_cache, const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks,
+                                       void* out, int64_t out_row_stride, const int32_t* cu_seqlens_q,
+                                       const int32_t* cu_seqlens_k, int64_t total_q, int64_t total_k, int32_t batch,
+                                       int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads, int32_t num_kv_heads,
+                                       int32_t head_dim, float scale, int64_t num_blocks, void* stream) {
+  using namespace nvllm;
+  const int rc = nvllm_store_kvcache(key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, total_k,
+                                     num_kv_heads * head_dim, num_blocks * kBlockSize, stream);
+  if (rc) return rc;
+  const void *k = key, *v = value;
+  if (block_tables) {  // prefix cache: every key is read through the table
+    k = k_cache;
+    v = v_cache;
+  }
+  return prefill_common(q, q_row_stride, k, key_row_stride, v, value_row_stride, block_tables, bt_row_stride, max_blocks, out,
+                        out_row_stride, cu_seqlens_q, cu_seqlens_k, total_q, total_k, batch, max_seqlen_q, max_seqlen_k,
+                        num_q_heads, num_kv_heads, head_dim, scale, num_blocks, stream, total_k > 0);
 }

@@ -24,6 +24,7 @@ struct PrefillParams {
   float scale_log2e;
   int64_t num_blocks;
   int* status;
+  bool lengths_early;  // cu_q / cu_k were complete before the previous kernel in the stream let this one start
 };
 
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).

@@ -123,6 +123,8 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   // their end, and the packed heads share every K/V tile.
   const int pack = p.pack, BMT = BM / pack;
 
+  pdl_trigger();
+  if (!p.lengths_early) pdl_wait();
   // Rank the sequences by key length, longest first (ties by index): rank = how many come before.
   if (p.batch <= SORT_BATCH) {
     for (int b = tid; b < p.batch; b += NTHREADS_P) prefix[b] = p.cu_k[b + 1] - p.cu_k[b];  // lengths, for a moment
@@ -188,6 +190,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     }
   }
   if (warp == 9) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+  if (p.lengths_early) pdl_wait();  // from here on q, k and v are read
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -597,9 +600,8 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   if (max_items < grid) grid = static_cast<int>(max_items);
   // the two head_dim instantiations share the counter array: give each its own half
   const int slot = static_cast<int>(launch_seq.fetch_add(1) % (tcp::NUM_SLOTS / 2)) + (D == 64 ? tcp::NUM_SLOTS / 2 : 0);
-  prefill_tcp_kernel<D><<<grid, tcp::NTHREADS_P, G::SMEM, stream>>>(p, mq, mk, mv, slot);
-  count_launch();
-  return check_launch("prefill (tcgen05, persistent) launch");
+  return launch_kernel("prefill (tcgen05, persistent)", prefill_tcp_kernel<D>, dim3(grid), dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq,
+                       mk, mv, slot);
 }
 
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream) {

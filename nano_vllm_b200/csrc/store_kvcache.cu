@@ -15,7 +15,8 @@ store_kvcache_kernel(const uint4* __restrict__ key, int64_t key_stride16,      /
                      uint4* __restrict__ k_cache, uint4* __restrict__ v_cache,
                      const int32_t* __restrict__ slot_mapping,
                      int64_t n_tokens, int pieces_per_row, int64_t num_slots, int* __restrict__ status) {
-  pdl_prologue();  // lets the attention kernel that follows get its blocks resident early
+  pdl_wait();
+  pdl_trigger();  // after the wait: the attention kernel that follows may read its metadata early
   const int64_t total = n_tokens * pieces_per_row;
   const int64_t base = (static_cast<int64_t>(blockIdx.x) * kStoreThreads) * kStoreUnroll + threadIdx.x;
 
@@ -78,9 +79,8 @@ extern "C" int nvllm_store_kvcache(const void* key, int64_t key_row_stride,
   const int64_t per_block = static_cast<int64_t>(kStoreThreads) * kStoreUnroll;
   const int64_t blocks = (total + per_block - 1) / per_block;
   if (blocks > 0x7fffffffLL) return fail(NVLLM_E_GEOMETRY, "store_kvcache: too many tokens for one launch");
-  store_kvcache_kernel<<<static_cast<unsigned>(blocks), kStoreThreads, 0, static_cast<cudaStream_t>(stream)>>>(
-      static_cast<const uint4*>(key), key_row_stride / 8, static_cast<const uint4*>(value), value_row_stride / 8,
-      static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), slot_mapping, n_tokens, pieces, num_slots, status);
-  count_launch();
-  return check_launch("store_kvcache launch");
+  return launch_kernel("store_kvcache", store_kvcache_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kStoreThreads), 0,
+                       static_cast<cudaStream_t>(stream), static_cast<const uint4*>(key), key_row_stride / 8,
+                       static_cast<const uint4*>(value), value_row_stride / 8, static_cast<uint4*>(k_cache),
+                       static_cast<uint4*>(v_cache), slot_mapping, n_tokens, pieces, num_slots, status);
 }

@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from conftest import assert_close_to_oracle
-from nano_vllm_b200 import _lib, attention as A, workloads as W
+from nano_vllm_b200 import _lib, attention as A, context as C, workloads as W
 from oracle import paged_attention_ref as R
 
 pytestmark = pytest.mark.gpu
@@ -202,6 +202,22 @@ def test_strided_q_and_cuda_graph_replay(cuda):
     torch.cuda.synchronize()
     ref = R.decode_ref(case.q, case.k_cache, case.v_cache, shorter, case.block_tables, case.scale)
     assert_close_to_oracle(out, ref, "graph replay, shorter contexts")
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(1, 1, 128), (3, 1, 128), (16, 2, 128), (1, 1, 64), (5, 1, 64), (8, 1, 64), (28, 4, 64)])
+@pytest.mark.parametrize("lens", [[32000], [20000, 1, 0, 9001], [129, 65, 64, 63]])
+def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
+    """Merges of two to a hundred and more partials, with lane groups to spare (parts split between
+    them), as many as heads, and fewer; also through the layer, where the lengths are read early."""
+    case = W.make_decode_case(29, len(lens), 1, 1, hq, hkv, d, context_lens=lens)
+    _check(cuda, case, f"hq{hq} hkv{hkv} d{d} {lens}")
+    dev = case.to(cuda)
+    layer = A.Attention(hq, d, dev.scale, hkv)
+    layer.k_cache, layer.v_cache = dev.k_cache, dev.v_cache
+    C.set_context(False, slot_mapping=dev.slot_mapping, context_lens=dev.context_lens, block_tables=dev.block_tables)
+    got = layer(dev.q.view(len(lens), -1), dev.k_new.view(len(lens), -1), dev.v_new.view(len(lens), -1))
+    C.reset_context()
+    assert torch.equal(got.view_as(dev.q), A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, dev.scale))
 
 
 @pytest.mark.parametrize("tp", [2, 4, 8])
