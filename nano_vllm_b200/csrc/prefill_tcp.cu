@@ -212,7 +212,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
    if (warp == 8) {
     // ------------------------------------------------------------------ producer lane
-    if (lane == 0) {
+    if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
       int T = 0;   // key tiles loaded so far in this block's life
@@ -304,7 +304,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     }
    } else if (warp == 9) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc(BM, BN, 0, 0);
       constexpr uint32_t idesc_pv = umma_idesc(BM, D, 0, 1);
       const uint64_t q_desc = umma_desc(base + OFF_Q, 16, 1024);
@@ -595,6 +595,10 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   }
   // an upper bound of the work items known to the host: no more blocks than that
   const int64_t max_items = static_cast<int64_t>((p.max_seqlen_q + bmt - 1) / bmt) * (p.hq / pack) * p.batch;
+  if (const char* e = std::getenv("NVLLM_PREFILL_IMPL"); e && e[0] == 'p') {
+    p.tiles = max_items <= num_sms() ? 1 : 2;
+    return launch_prefill_pair(p, mq, mk, mv, max_items, stream);
+  }
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
   if (max_items < grid) grid = static_cast<int>(max_items);
