@@ -1,7 +1,5 @@
 // Parameters shared by the prefill kernels and their host-side dispatcher.
 #pragma once
-#include <cuda.h>  // CUtensorMap (types only)
-
 #include "common.cuh"
 
 namespace nvllm {
@@ -23,7 +21,6 @@ struct PrefillParams {
   int batch, max_seqlen_q, max_seqlen_k;
   int hq, hkv, g, d;
   int pack;  // persistent tcgen05 kernel only: query heads packed into one tile (1..8)
-  int tiles;  // prefill_pair.cu only: query tiles of an item (1 or 2)
   float scale_log2e;
   int64_t num_blocks;
   int* status;
@@ -37,11 +34,8 @@ constexpr int kPrefillMaxBatch = 1024;
 // Warp-level mma.sync kernel: every supported geometry; cross-check and A/B baseline only
 // (batch <= 65535).
 int launch_prefill_mma(const PrefillParams& p, cudaStream_t stream);
-// tcgen05 / TMEM / TMA kernels in persistent blocks that pull (sequence, query tile, head) items
+// tcgen05 / TMEM / TMA kernel in persistent blocks that pull (sequence, query tile, head) items
 // from a global counter; batch <= kPrefillMaxBatch.  total_q / total_k bound the tiled loads.
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream);
-// Two query tiles per item (one where p.tiles is 1), one block per SM; same tensor maps.
-int launch_prefill_pair(const PrefillParams& p, const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv,
-                        int64_t max_items, cudaStream_t stream);
 
 }  // namespace nvllm

@@ -595,10 +595,6 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   }
   // an upper bound of the work items known to the host: no more blocks than that
   const int64_t max_items = static_cast<int64_t>((p.max_seqlen_q + bmt - 1) / bmt) * (p.hq / pack) * p.batch;
-  if (const char* e = std::getenv("NVLLM_PREFILL_IMPL"); e && e[0] == 'p') {
-    p.tiles = max_items <= num_sms() ? 1 : 2;
-    return launch_prefill_pair(p, mq, mk, mv, max_items, stream);
-  }
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
   if (max_items < grid) grid = static_cast<int>(max_items);
