@@ -123,8 +123,9 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   // their end, and the packed heads share every K/V tile.
   const int pack = p.pack, BMT = BM / pack;
 
-  pdl_trigger();
+  if (!p.store_follows) pdl_trigger();
   if (!p.lengths_early) pdl_wait();
+  if (p.store_follows) pdl_trigger();
   // Rank the sequences by key length, longest first (ties by index): rank = how many come before.
   if (p.batch <= SORT_BATCH) {
     for (int b = tid; b < p.batch; b += NTHREADS_P) prefix[b] = p.cu_k[b + 1] - p.cu_k[b];  // lengths, for a moment
