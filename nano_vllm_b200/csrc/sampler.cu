@@ -58,7 +58,8 @@ struct SampleParams {
   const float* temperatures;
   const float* noise;  // nullable
   int64_t noise_stride;
-  uint64_t seed, step;
+  uint64_t step;
+  uint2 key[10];            // the generator's keys of its ten rounds, from the seed
   int64_t* tokens;          // token ids, or packed candidates when `candidates` is set
   int vocab;                // elements in a row of `logits`
   int64_t offset;           // global vocabulary index of element 0 of a row
@@ -83,30 +84,27 @@ __device__ __forceinline__ long long pack_candidate(float score, int idx) {
 // one product of round 1 and one of round 2 do not depend on it and are made once.  High and low
 // words are separate multiplications on purpose: the 64-bit product is one instruction but slower
 // (64 us against 56 for the whole kernel at batch 256).
+// The round keys come with the kernel's parameters, where an instruction can read them in place.
 struct Philox {
-  static constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u, W0 = 0x9E3779B9u, W1 = 0xBB67AE85u;
-  uint2 key;
+  static constexpr uint32_t M0 = 0xD2511F53u, M1 = 0xCD9E8D57u;
+  const uint2 (&key)[10];
   uint32_t a, b, c, d;  // key and counter words that are the same for every c0
-  __device__ __forceinline__ Philox(uint64_t seed, uint32_t row, uint64_t step) {
-    key = make_uint2(static_cast<uint32_t>(seed), static_cast<uint32_t>(seed >> 32));
+  __device__ __forceinline__ Philox(const uint2 (&keys)[10], uint32_t row, uint64_t step) : key(keys) {
     const uint32_t lo = static_cast<uint32_t>(step), hi = static_cast<uint32_t>(step >> 32);
-    a = hi ^ key.y;                            // round 1: z = hi(M0 c0) ^ a, w = lo(M0 c0)
-    const uint32_t x1 = __umulhi(M1, lo) ^ row ^ key.x;
-    b = (M1 * lo) ^ (key.x + W0);              // round 2: x = hi(M1 z) ^ b, y = lo(M1 z)
-    c = __umulhi(M0, x1) ^ (key.y + W1);       //          z = w ^ c
+    a = hi ^ key[0].y;                            // round 1: z = hi(M0 c0) ^ a, w = lo(M0 c0)
+    const uint32_t x1 = __umulhi(M1, lo) ^ row ^ key[0].x;
+    b = (M1 * lo) ^ key[1].x;              // round 2: x = hi(M1 z) ^ b, y = lo(M1 z)
+    c = __umulhi(M0, x1) ^ key[1].y;       //          z = w ^ c
     d = M0 * x1;                               //          w = d
   }
   __device__ __forceinline__ uint4 operator()(uint32_t c0) const {
     const uint32_t z1 = __umulhi(M0, c0) ^ a, w1 = M0 * c0;
     uint4 s = make_uint4(__umulhi(M1, z1) ^ b, M1 * z1, w1 ^ c, d);
-    uint32_t k0 = key.x + W0, k1 = key.y + W1;
 #pragma unroll
     for (int r = 2; r < 10; ++r) {
-      k0 += W0;
-      k1 += W1;
       const uint32_t hi0 = __umulhi(M0, s.x), lo0 = M0 * s.x;
       const uint32_t hi1 = __umulhi(M1, s.z), lo1 = M1 * s.z;
-      s = make_uint4(hi1 ^ s.y ^ k0, lo1, hi0 ^ s.w ^ k1, lo0);
+      s = make_uint4(hi1 ^ s.y ^ key[r].x, lo1, hi0 ^ s.w ^ key[r].y, lo0);
     }
     return s;
   }
@@ -206,31 +204,38 @@ __device__ __forceinline__ uint4 shift_pair(const uint4& a, const uint4& b, int 
 #define NVLLM_SAMPLER_MINBLOCKS 4
 #endif
 
-// Calls f(pieces, first group, stride between the pieces' groups) for this thread's share of the
+// Calls f(pieces, first group, stride between the pieces' groups, full) for this thread's share of the
 // `n_groups` groups of a row that start at `first`, C pieces at a time; the next C are loaded before
-// the current ones are looked at.  All lanes of a warp make the same calls; pieces of groups past
-// the end are zero.
+// the current ones are looked at.  All lanes of a warp make the same calls.  full is a constant: true
+// where every piece of every lane of the warp is a group, else pieces past the end are zero.
 template <bool ALIGNED, int C, typename T, class F>
 __device__ __forceinline__ void for_groups(const T* first, int n_groups, int tid, int nthreads, F&& f) {
   const int lane = tid & 31;
   const int shift = ALIGNED ? 0 : static_cast<int>(reinterpret_cast<uintptr_t>(first) & 15u);
   const uint4* base = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(first) - shift);
-  auto load = [&](uint4 (&raw)[C], int g) {
+  auto load = [&](uint4 (&raw)[C], int g, auto full) {
 #pragma unroll
     for (int c = 0; c < C; ++c, g += nthreads) {
-      const bool live = g < n_groups;
+      const bool live = decltype(full)::value || g < n_groups;
       raw[c] = live ? __ldg(base + g) : make_uint4(0, 0, 0, 0);
       if constexpr (!ALIGNED) raw[c] = shift_pair<sizeof(T)>(raw[c], live ? __ldg(base + g + 1) : make_uint4(0, 0, 0, 0), shift);
     }
   };
+  const int step = C * nthreads;
   uint4 raw[C], next[C];
-  int g0 = tid - lane;
-  load(next, g0 + lane);
-  for (; g0 < n_groups; g0 += C * nthreads) {
+  int g = tid;
+  const int n_full = n_groups - (C - 1) * nthreads - (31 - lane);  // g below this: a full call (the same for all lanes)
+  if (g < n_full) load(next, g, std::true_type{});
+  while (g < n_full) {
 #pragma unroll
     for (int c = 0; c < C; ++c) raw[c] = next[c];
-    load(next, g0 + C * nthreads + lane);
-    f(raw, g0 + lane, nthreads);
+    if (g + step < n_full) load(next, g + step, std::true_type{});
+    f(raw, g, nthreads, std::true_type{});
+    g += step;
+  }
+  for (; g - lane < n_groups; g += step) {
+    load(raw, g, std::false_type{});
+    f(raw, g, nthreads, std::false_type{});
   }
 }
 
@@ -249,7 +254,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
   const float t = p.temperatures[row];
   const bool greedy = !(t > 0.f) && !(t < 0.f);  // T == 0 (or NaN): plain argmax, as torch.where(T == 0, ...)
   const float inv_t = greedy ? 1.f : 1.f / t;
-  const Philox draw4(p.seed, static_cast<uint32_t>(row), p.step);  // unique per element and call
+  const Philox draw4(p.key, static_cast<uint32_t>(row), p.step);  // unique per element and call
   __shared__ int s_best;  // best score of the block so far, ordered()
   if (threadIdx.x == 0) s_best = ordered(-INFINITY);
   __syncthreads();
@@ -264,10 +269,10 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
   auto scan = [&](auto aligned) {
     constexpr bool A = decltype(aligned)::value;
     if (greedy) {
-      for_groups<A, 4>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[4], int g, int stride) {
+      for_groups<A, 4>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[4], int g, int stride, auto full) {
 #pragma unroll
         for (int c = 0; c < 4; ++c, g += stride) {
-          if (g >= n_groups || !(G::max(raw[c]) > best.score)) continue;
+          if ((!decltype(full)::value && g >= n_groups) || !(G::max(raw[c]) > best.score)) continue;
           float e[N];
           G::unpack(raw[c], e);
 #pragma unroll
@@ -275,8 +280,8 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
         }
       });
     } else if (nz) {
-      for_groups<A, 1>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[1], int g, int) {
-        if (g >= n_groups) return;
+      for_groups<A, 1>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[1], int g, int, auto full) {
+        if (!decltype(full)::value && g >= n_groups) return;
         float e[N];
         G::unpack(raw[0], e);
         const float* z = nz + lead + g * N;
@@ -287,14 +292,15 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
       // log2 of 2^32 times the largest v with which x reaches a score b: x log2(e) / T - bar_of(b).  The slack
       // covers the rounding of the scores, of the exponential and of v.
       const float x_scale = inv_t * 1.4426950408889634f;
-      auto bar_of = [](float b) { return fmaf(b, 1.4426950408889634f, -32.01f - 1e-6f * fabsf(b)); };
+      auto bar_of = [&](float b) { return t < 0.f ? -INFINITY : fmaf(b, 1.4426950408889634f, -32.01f - 1e-6f * fabsf(b)); };
       // draws up to this can win; NaN (nothing seen yet, infinities) and T < 0 let everything pass
-      auto limit_of = [&](const uint4& raw, float bar) { return t < 0.f ? INFINITY : fast_exp2(fmaf(G::max(raw), x_scale, -bar)); };
+      auto limit_of = [&](const uint4& raw, float bar) { return fast_exp2(fmaf(G::max(raw), x_scale, -bar)); };
       // two pieces at a time, so that the chains of their generator calls overlap
       constexpr int C = 2;
       float bar = bar_of(-INFINITY);
       int seen = ordered(-INFINITY);
-      for_groups<A, C>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[C], int g, int stride) {
+      for_groups<A, C>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[C], int g, int stride, auto full) {
+        auto live = [&](int c) { return decltype(full)::value || g + c * stride < n_groups; };
         const int now = *static_cast<volatile int*>(&s_best);
         if (now != seen) {
           seen = now;
@@ -305,7 +311,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
 #pragma unroll
         for (int c = 0; c < C; ++c) {
           limit[c] = limit_of(raw[c], bar);
-          any |= g + c * stride < n_groups && !(limit[c] < 0.25f);
+          any |= live(c) && !(limit[c] < 0.25f);
         }
         if (!__any_sync(0xffffffffu, any)) return;
         uint32_t bits[C][N];
@@ -331,7 +337,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
               const float log2v = fmaf(static_cast<float>(__float_as_int(static_cast<float>(bits[c][k]) + 0.5f)),
                                        1.1920928955078125e-07f, -159.f);
               const float s = fmaf(log2v + 0.1f, -0.69314718f, fmaf(e[k], inv_t, -0.33f));
-              if (bits[c][k] < 0x80000000u && g + c * stride < n_groups) reach = fmaxf(reach, s);
+              if (bits[c][k] < 0x80000000u && live(c)) reach = fmaxf(reach, s);
             }
           }
           const int reached = __reduce_max_sync(0xffffffffu, ordered(reach));
@@ -346,7 +352,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
           below[c] = limit[c] < 4.2e9f ? __float2uint_ru(limit[c]) : 0xffffffffu;  // NaN: everything passes
           uint32_t least = min(min(bits[c][0], bits[c][1]), min(bits[c][2], bits[c][3]));
           if constexpr (N == 8) least = min(least, min(min(bits[c][4], bits[c][5]), min(bits[c][6], bits[c][7])));
-          pass |= g + c * stride < n_groups && least <= below[c];
+          pass |= live(c) && least <= below[c];
         }
         if (!__any_sync(0xffffffffu, pass)) return;
 #pragma unroll
@@ -355,7 +361,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
           G::unpack(raw[c], e);
 #pragma unroll
           for (int k = 0; k < N; ++k)
-            if (bits[c][k] <= below[c] && g + c * stride < n_groups)
+            if (bits[c][k] <= below[c] && live(c))
               take_next(best, e[k] * inv_t - ln_exponential(bits[c][k]), off + lead + (g + c * stride) * N + k);
         }
         const int warp_best = __reduce_max_sync(0xffffffffu, ordered(best.score));
@@ -496,7 +502,8 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   p.temperatures = temperatures;
   p.noise = exponential_noise;
   p.noise_stride = noise_row_stride;
-  p.seed = seed;
+  for (int r = 0; r < 10; ++r)
+    p.key[r] = make_uint2(static_cast<uint32_t>(seed) + r * 0x9E3779B9u, static_cast<uint32_t>(seed >> 32) + r * 0xBB67AE85u);
   p.step = step;
   p.tokens = tokens;
   p.vocab = vocab;
