@@ -111,6 +111,7 @@ def host():
     global _host
     if _host is None:
         load()
+        import torch  # noqa: F401  (the extension links against torch's libraries)
         try:
             from . import _host as module
         except ImportError as e:

@@ -104,10 +104,10 @@ def test_recorded_reference_modules(cuda, name):
 
 
 @pytest.mark.parametrize("hq,hkv,d,n,norm", [(16, 8, 128, 2401, True), (3, 1, 128, 16001, True), (5, 5, 64, 10243, True),
-                                             (14, 2, 64, 9003, False)])
-def test_launches_of_four_heads_per_lane_group_equal_those_of_one(cuda, hq, hkv, d, n, norm):
-    """A large launch gives each lane group four heads, a small one gives it one: the same bits, at head
-    counts that put q, k and v heads (or fewer than four) into one group."""
+                                             (14, 2, 64, 9003, False), (48, 8, 128, 777, True)])
+def test_launches_by_rows_equal_those_by_heads(cuda, hq, hkv, d, n, norm):
+    """A large launch moves token rows through shared memory, a small one takes a head per lane group: the
+    same bits, at head counts that do not divide over a block's lane groups."""
     g = torch.Generator(device=cuda).manual_seed(n)
     qkv = (torch.randn(n, (hq + 2 * hkv) * d, generator=g, device=cuda) * 3).bfloat16()
     positions = torch.randint(0, 512, (n,), generator=g, device=cuda)
@@ -117,7 +117,7 @@ def test_launches_of_four_heads_per_lane_group_equal_those_of_one(cuda, hq, hkv,
     slots = torch.randperm(blocks * 256, generator=g, device=cuda)[:n].to(torch.int32)
     slots[1::7] = -1
     results = []
-    for step in (n, 997):
+    for step in (n, 331):
         x, kv = qkv.clone(), torch.zeros(2, blocks, 256, hkv, d, dtype=torch.bfloat16, device=cuda)
         for a in range(0, n, step):
             A.qk_norm_rope_store(x[a:a + step], positions[a:a + step], qw, kw, cache, 1e-6, slots[a:a + step], kv[0], kv[1],
