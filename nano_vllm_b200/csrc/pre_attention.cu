@@ -253,11 +253,12 @@ __global__ void __launch_bounds__(kRowWarps * 32) pre_attention_rows_kernel(cons
     wq = load_weights(p.q_weight + sub * 8, true);
     wk = load_weights(p.k_weight + sub * 8, true);
   }
+  bool ok = true;
   for (int i = 0; i < n_mine; ++i) {
     const int st = i % kRowStages;
     const uint32_t table = base + st * stage_bytes, row = table + TABLE_BYTES;
-    // A copy never fails; bounded like every wait.  All threads carry on to the barrier either way.
-    if (!mbar_wait(bar(st), (i / kRowStages) & 1)) atomicOr(p.status, NVLLM_STATUS_TIMEOUT);
+    // A copy never fails; bounded like every wait, after which nothing is waited for any more.
+    if (ok && !(ok = mbar_wait(bar(st), (i / kRowStages) & 1))) atomicOr(p.status, NVLLM_STATUS_TIMEOUT);
     uint64_t c[4], s[4];
     const uint32_t mine = table + (sub % (LANES / 2)) * 32;
     auto pairs_of = [](const uint4& v, uint64_t& a, uint64_t& b) {

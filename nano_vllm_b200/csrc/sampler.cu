@@ -16,15 +16,15 @@
 // counted by (row, position in the row, step); no state is kept between calls, the same
 // (seed, step) reproduces the same tokens.
 //
-// A row is read by one thread-block cluster of 1, 2, 4 or 8 blocks of 256 threads (the fewer
+// A row is read by one thread-block cluster of 1, 2, 4, 8 or 16 blocks of 256 threads (the fewer
 // the rows, the more blocks each gets, so that a decode batch of any size spreads over the 148
 // SMs).  A thread takes groups of 16 bytes (8 bf16 or 4 fp32 logits), loaded one step ahead.  Each
-// block reduces to one candidate, block 0 of the cluster collects the others' candidates from
-// their shared memory.  Ties go to the lowest index.
+// warp reduces to one candidate and puts it into the shared memory of the cluster's first block, where
+// the largest is taken.  Ties go to the lowest index.
 //
 // What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
 // per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
-// (now 53, of which the rounds are most; greedy rows 32 -> 20).  The logarithms are only needed for elements that can still win: since e >= v, where v is the uniform
+// (now 48; greedy rows 32 -> 17; batch 1, 12.7 -> 7.4).  The logarithms are only needed for elements that can still win: since e >= v, where v is the uniform
 // draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
 // the group's largest x and the smallest of its draws decide that for the whole group, against the
 // best score that any warp of the block has seen; only groups that pass (a few per warp and row)
@@ -47,6 +47,7 @@
 #include <cooperative_groups.h>
 
 #include <type_traits>
+#include <utility>
 
 #include "common.cuh"
 
@@ -77,6 +78,11 @@ __device__ __forceinline__ float from_ordered(int i) { return __int_as_float(i >
 __device__ __forceinline__ long long pack_candidate(float score, int idx) {
   const int s = ordered(score);
   return (static_cast<long long>(s) << 32) | static_cast<long long>(0xffffffffu - static_cast<unsigned int>(idx));
+}
+
+__device__ __forceinline__ int64_t candidate_index(long long packed) {
+  const unsigned int idx = 0xffffffffu - static_cast<unsigned int>(packed & 0xffffffffll);
+  return idx == 0x7fffffffu ? 0 : static_cast<int64_t>(idx);
 }
 
 // Philox4x32 with 10 rounds (Salmon et al., "Parallel random numbers: as easy as 1, 2, 3", SC'11),
@@ -239,12 +245,16 @@ __device__ __forceinline__ void for_groups(const T* first, int n_groups, int tid
   }
 }
 
+constexpr int kMaxCluster = 16;
+
 template <typename T>
 __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(const SampleParams p) {
   using G = Group<T>;
   constexpr int N = G::N;
   namespace cg = cooperative_groups;
+  pdl_prologue();
   cg::cluster_group cluster = cg::this_cluster();
+  auto started = cluster.barrier_arrive();  // waited for before another block's shared memory is written
   const int csize = static_cast<int>(cluster.num_blocks()), crank = static_cast<int>(cluster.block_rank());
   const int row = blockIdx.x / csize;
   const int tid = crank * blockDim.x + threadIdx.x;  // thread index within the row's cluster
@@ -256,6 +266,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
   const float inv_t = greedy ? 1.f : 1.f / t;
   const Philox draw4(p.key, static_cast<uint32_t>(row), p.step);  // unique per element and call
   __shared__ int s_best;  // best score of the block so far, ordered()
+  __shared__ long long s_candidates[kMaxCluster * 8];  // block 0 of the cluster: one per warp of the row
   if (threadIdx.x == 0) s_best = ordered(-INFINITY);
   __syncthreads();
 
@@ -389,60 +400,33 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
     take(best, s, off + i);
   }
 
-  // block argmax: shuffle inside a warp, shared memory across the warps; then across the cluster
-  auto warp_reduce = [&]() {
+  // Argmax of the row: by shuffle inside a warp, then every warp of the cluster puts its candidate into
+  // block 0's shared memory, and one warp there takes the largest.
 #pragma unroll
-    for (int sh = 16; sh > 0; sh >>= 1) {
-      const float s = __shfl_xor_sync(0xffffffffu, best.score, sh);
-      const int i = __shfl_xor_sync(0xffffffffu, best.idx, sh);
-      take(best, s, i);
-    }
-  };
-  warp_reduce();
-  __shared__ float w_score[8];
-  __shared__ int w_idx[8];
-  __shared__ float blk_score;
-  __shared__ int blk_idx;
-  const int lt = threadIdx.x;
-  if ((lt & 31) == 0) {
-    w_score[lt >> 5] = best.score;
-    w_idx[lt >> 5] = best.idx;
+  for (int sh = 16; sh > 0; sh >>= 1) {
+    const float s = __shfl_xor_sync(0xffffffffu, best.score, sh);
+    const int i = __shfl_xor_sync(0xffffffffu, best.idx, sh);
+    take(best, s, i);
   }
-  __syncthreads();
-  if (lt < 32) {
-    const int nw = (blockDim.x + 31) >> 5;
-    best.score = lt < nw ? w_score[lt] : -INFINITY;
-    best.idx = lt < nw ? w_idx[lt] : 0x7fffffff;
-    warp_reduce();
-    if (lt == 0) {
-      blk_score = best.score;
-      blk_idx = best.idx;
-    }
-  }
-  cluster.sync();  // every block's candidate is in its shared memory
-  if (crank == 0 && lt < 32) {
-    best.score = -INFINITY;
-    best.idx = 0x7fffffff;
-    if (lt < csize) {
-      best.score = *cluster.map_shared_rank(&blk_score, lt);
-      best.idx = *cluster.map_shared_rank(&blk_idx, lt);
-    }
-    warp_reduce();
-    // a row of NaN / -inf only: token 0, like an argmax over equal values (after the merge, for
-    // candidates: the sentinel index loses against any real candidate of another rank)
-    if (lt == 0) {
-      if (p.candidates) p.tokens[row] = pack_candidate(best.score, best.idx);
-      else p.tokens[row] = best.idx == 0x7fffffff ? 0 : best.idx;
-    }
-  }
-  cluster.sync();  // no block leaves while its shared memory may still be read
+  cluster.barrier_wait(std::move(started));
+  const int lt = threadIdx.x, warps = static_cast<int>(blockDim.x) >> 5;
+  if ((lt & 31) == 0)
+    cluster.map_shared_rank(s_candidates, 0)[crank * warps + (lt >> 5)] = pack_candidate(best.score == 0.f ? 0.f : best.score, best.idx);
+  cluster.sync();
+  if (crank != 0 || lt >= 32) return;
+  long long top = s_candidates[0];
+  for (int k = lt; k < csize * warps; k += 32) top = max(top, s_candidates[k]);
+#pragma unroll
+  for (int sh = 16; sh > 0; sh >>= 1) top = max(top, __shfl_xor_sync(0xffffffffu, top, sh));
+  // a row of NaN / -inf only: token 0, like an argmax over equal values (after the merge, for
+  // candidates: the sentinel index loses against any real candidate of another rank)
+  if (lt == 0) p.tokens[row] = p.candidates ? top : candidate_index(top);
 }
 
 __global__ void sample_unpack_kernel(const long long* packed, int64_t* tokens, int batch) {
   const int b = blockIdx.x * blockDim.x + threadIdx.x;
   if (b >= batch) return;
-  const unsigned int idx = 0xffffffffu - static_cast<unsigned int>(packed[b] & 0xffffffffll);
-  tokens[b] = idx == 0x7fffffffu ? 0 : static_cast<int64_t>(idx);
+  tokens[b] = candidate_index(packed[b]);
 }
 
 static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t row_stride, const float* temperatures,
@@ -513,23 +497,44 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: no CUDA device is usable");
   // Blocks per row: as few (1, 2, 4, 8) as give every SM three blocks, since every block pays its start
   // and its merge; more would only help the balance, fewer leave the SMs short of warps (measured at
-  // batch 8 to 512).  No more than the row has work for.
+  // batch 1 to 512).  Sixteen where that is still no more than one block per SM (batch 1: 8.7 us, 10.8 with
+  // eight; beyond, clusters of sixteen crowd on a part of the chip: 19.0 for 14.5 at batch 32).  No
+  // more than the row has work for.
   int csize = 1;
-  while (csize < 8 && static_cast<int64_t>(batch) * csize < 3ll * sms && vocab >= csize * 2 * 256 * 8) csize *= 2;
+  auto fits = [&](int c, int64_t most) { return vocab >= c * 256 * 8 && static_cast<int64_t>(batch) * c <= most; };
+  while (csize < 8 && static_cast<int64_t>(batch) * csize < 3ll * sms && fits(2 * csize, INT64_MAX)) csize *= 2;
+  if (csize == 8 && fits(16, sms)) csize = 16;
+  const int64_t blocks = static_cast<int64_t>(batch) * csize;
+  // Launched under the end of the kernel before (1.5 us less), except for grids of about one or two blocks
+  // per SM, which then land unevenly on the SMs that happen to be free (17.8 us for 14.5 at batch 32).
+  const bool early = 2 * blocks <= sms || blocks >= 3ll * sms;
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(static_cast<unsigned>(batch) * csize, 1, 1);
+  cfg.gridDim = dim3(static_cast<unsigned>(blocks), 1, 1);
   cfg.blockDim = dim3(256, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = static_cast<cudaStream_t>(stream);
-  cudaLaunchAttribute attr[1];
+  auto kernel = logits_are_fp32 ? sample_kernel<float> : sample_kernel<__nv_bfloat16>;
+  if (csize > 8) {  // more than the portable cluster size has to be asked for, once per device and kernel
+    static bool allowed[2][64] = {};
+    int dev = 0;
+    cudaGetDevice(&dev);
+    if (dev < 0 || dev >= 64) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: device index %d out of range", dev);
+    if (!allowed[logits_are_fp32 ? 1 : 0][dev]) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "sample_tokens: set-up failed: %s", cudaGetErrorString(e));
+      allowed[logits_are_fp32 ? 1 : 0][dev] = true;
+    }
+  }
+  cudaLaunchAttribute attr[2];
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = csize;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = logits_are_fp32 ? cudaLaunchKernelEx(&cfg, sample_kernel<float>, p)
-                                  : cudaLaunchKernelEx(&cfg, sample_kernel<__nv_bfloat16>, p);
+  cfg.numAttrs = early ? 2 : 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return fail(NVLLM_E_CUDA, "sample_tokens launch: %s", cudaGetErrorString(e));
