@@ -24,7 +24,8 @@
 //
 // What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
 // per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
-// (now 48; greedy rows 32 -> 17; batch 1, 12.7 -> 7.4).  The logarithms are only needed for elements that can still win: since e >= v, where v is the uniform
+// (now 48; greedy rows 32 -> 17; batch 1, 12.7 -> 7.4).  The logarithms are only needed for elements that
+// can still win: since e >= v, where v is the uniform
 // draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
 // the group's largest x and the smallest of its draws decide that for the whole group, against the
 // best score that any warp of the block has seen; only groups that pass (a few per warp and row)
