@@ -24,7 +24,7 @@
 //
 // What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
 // per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
-// (now 48; greedy rows 32 -> 17; batch 1, 12.7 -> 7.4).  The logarithms are only needed for elements that
+// (now 47; greedy rows 32 -> 16; batch 1, 12.7 -> 6.5).  The logarithms are only needed for elements that
 // can still win: since e >= v, where v is the uniform
 // draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
 // the group's largest x and the smallest of its draws decide that for the whole group, against the
@@ -307,74 +307,56 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
       auto bar_of = [&](float b) { return t < 0.f ? -INFINITY : fmaf(b, 1.4426950408889634f, -32.01f - 1e-6f * fabsf(b)); };
       // draws up to this can win; NaN (nothing seen yet, infinities) and T < 0 let everything pass
       auto limit_of = [&](const uint4& raw, float bar) { return fast_exp2(fmaf(G::max(raw), x_scale, -bar)); };
-      // two pieces at a time, so that the chains of their generator calls overlap
-      constexpr int C = 2;
       float bar = bar_of(-INFINITY);
       int seen = ordered(-INFINITY);
-      for_groups<A, C>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[C], int g, int stride, auto full) {
-        auto live = [&](int c) { return decltype(full)::value || g + c * stride < n_groups; };
+      // One group at a time: two, with twice as many generator chains in flight, are slower below some 400
+      // rows (17.4 / 19.7 us at batch 64), and so are fewer registers and more warps.
+      for_groups<A, 1>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[1], int g, int, auto full) {
+        const bool live = decltype(full)::value || g < n_groups;
         const int now = *static_cast<volatile int*>(&s_best);
         if (now != seen) {
           seen = now;
           bar = bar_of(from_ordered(now));
         }
-        float limit[C];
-        bool any = false;
+        float limit = limit_of(raw[0], bar);
+        if (!__any_sync(0xffffffffu, live && !(limit < 0.25f))) return;
+        const int pos = off + lead + g * N;
+        uint32_t bits[N];
 #pragma unroll
-        for (int c = 0; c < C; ++c) {
-          limit[c] = limit_of(raw[c], bar);
-          any |= live(c) && !(limit[c] < 0.25f);
+        for (int h = 0; h < N / 4; ++h) {
+          const uint4 r = draw4(static_cast<uint32_t>(pos >> 2) + h);
+          bits[4 * h] = r.x; bits[4 * h + 1] = r.y; bits[4 * h + 2] = r.z; bits[4 * h + 3] = r.w;
         }
-        if (!__any_sync(0xffffffffu, any)) return;
-        uint32_t bits[C][N];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-#pragma unroll
-          for (int h = 0; h < N / 4; ++h) {
-            const uint4 r = draw4(static_cast<uint32_t>((off + lead + (g + c * stride) * N) >> 2) + h);
-            bits[c][4 * h] = r.x; bits[c][4 * h + 1] = r.y; bits[c][4 * h + 2] = r.z; bits[c][4 * h + 3] = r.w;
-          }
-        }
+        float e[N];
         if (seen == ordered(-INFINITY)) {
           // Nothing is known of the row yet: take a bar from these elements.  -ln(e) >= -ln(v) - 0.33 for
           // v < 1/2 (e <= 1.39 v), and the exponent and mantissa bits of v read as a number give log2(v)
           // to within 0.09, so this is a score that some element reaches, found without logarithms.
           float reach = -INFINITY;
-#pragma unroll
-          for (int c = 0; c < C; ++c) {
-            float e[N];
-            G::unpack(raw[c], e);
+          if (live) {
+            G::unpack(raw[0], e);
 #pragma unroll
             for (int k = 0; k < N; ++k) {
-              const float log2v = fmaf(static_cast<float>(__float_as_int(static_cast<float>(bits[c][k]) + 0.5f)),
+              const float log2v = fmaf(static_cast<float>(__float_as_int(static_cast<float>(bits[k]) + 0.5f)),
                                        1.1920928955078125e-07f, -159.f);
               const float s = fmaf(log2v + 0.1f, -0.69314718f, fmaf(e[k], inv_t, -0.33f));
-              if (bits[c][k] < 0x80000000u && live(c)) reach = fmaxf(reach, s);
+              if (bits[k] < 0x80000000u) reach = fmaxf(reach, s);
             }
           }
           const int reached = __reduce_max_sync(0xffffffffu, ordered(reach));
           if ((threadIdx.x & 31) == 0) atomicMax(&s_best, reached);
-#pragma unroll
-          for (int c = 0; c < C; ++c) limit[c] = limit_of(raw[c], bar_of(from_ordered(reached)));
+          limit = limit_of(raw[0], bar_of(from_ordered(reached)));
         }
-        bool pass = false;
-        uint32_t below[C];
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          below[c] = limit[c] < 4.2e9f ? __float2uint_ru(limit[c]) : 0xffffffffu;  // NaN: everything passes
-          uint32_t least = min(min(bits[c][0], bits[c][1]), min(bits[c][2], bits[c][3]));
-          if constexpr (N == 8) least = min(least, min(min(bits[c][4], bits[c][5]), min(bits[c][6], bits[c][7])));
-          pass |= live(c) && least <= below[c];
-        }
+        const uint32_t below = limit < 4.2e9f ? __float2uint_ru(limit) : 0xffffffffu;  // NaN: everything passes
+        uint32_t least = min(min(bits[0], bits[1]), min(bits[2], bits[3]));
+        if constexpr (N == 8) least = min(least, min(min(bits[4], bits[5]), min(bits[6], bits[7])));
+        const bool pass = live && least <= below;
         if (!__any_sync(0xffffffffu, pass)) return;
-#pragma unroll
-        for (int c = 0; c < C; ++c) {
-          float e[N];
-          G::unpack(raw[c], e);
+        if (pass) {
+          G::unpack(raw[0], e);
 #pragma unroll
           for (int k = 0; k < N; ++k)
-            if (bits[c][k] <= below[c] && live(c))
-              take_next(best, e[k] * inv_t - ln_exponential(bits[c][k]), off + lead + (g + c * stride) * N + k);
+            if (bits[k] <= below) take_next(best, e[k] * inv_t - ln_exponential(bits[k]), pos + k);
         }
         const int warp_best = __reduce_max_sync(0xffffffffu, ordered(best.score));
         if ((threadIdx.x & 31) == 0 && warp_best > now) atomicMax(&s_best, warp_best);
