@@ -56,7 +56,12 @@ store_kvcache_kernel(const uint4* __restrict__ key, int64_t key_stride16,      /
       v_cache[dst[u]] = vreg[u];
     }
   }
-  if constexpr (BESIDE) pdl_wait();  // the next kernel may take this one's end for the end of both
+  if constexpr (BESIDE) {
+    // The next kernel may take this one's end for the end of both.  One block is enough for that, the last:
+    // a block that waits keeps the place of those that still have rows to copy
+    // (all of them waiting: four 4096-token prompts 302 us instead of 295).
+    if (blockIdx.x == gridDim.x - 1) pdl_wait();
+  }
 }
 
 // launch == false: argument checks only.
