@@ -36,7 +36,7 @@ int num_sms();
 // (launch_kernel), so that their blocks may become resident while the predecessor in the stream
 // drains: about 1 us of every launch in a chain.  Each of them passes pdl_wait(), which returns when
 // the previous kernel has completed and its writes are visible, before it touches anything that
-// another kernel may have written, and so completion stays transitive along the stream.
+// another kernel may have written (a guess that is verified afterwards excepted), and so completion stays transitive along the stream.
 // pdl_trigger() lets the next kernel in the stream start launching once every block has reached
 // it (kernels that were not launched with the attribute are unaffected).
 // A kernel whose predecessor was issued by the same entry point, and calls pdl_wait() before

@@ -129,7 +129,10 @@ struct Cut {
 // 32000 in the head_dim 64 geometry: 16.1 us, 26.1 without a limit).
 constexpr float kSplitBalance = 8.f;
 
-template <class C>
+// GUESS: the first split of the batch and the loads that follow from it are made on lengths that the previous
+// kernel may yet change (see where it branches).  In a chain of decode layers of 16 sequences, of which each
+// streams 7 us, that takes the trips for lengths, sums and first rows off the path: 17.4 -> 15.6 us a layer.
+template <class C, bool GUESS>
 __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const DecodeParams p) {
   constexpr int D = C::D, TT = C::TT, NST = C::NST, NW = C::NW, UNIT = C::UNIT, NT = NW * 32;
   constexpr int QUADS = D / 4, GROUPS = NT / QUADS;  // lanes that hold a head four columns each; such groups in a block
@@ -139,88 +142,22 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   __shared__ int s_last_arrival[2];
 
   pdl_trigger();
-  if (!p.lengths_early) pdl_wait();
+  if (!GUESS && !p.lengths_early) pdl_wait();
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int gid = lane >> 2, tig = lane & 3;
   const int kvh = blockIdx.x % p.hkv;
   const int range = blockIdx.x / p.hkv;
   const int ctx_cap = p.max_blocks * kBlockSize;
-  auto length_of = [&](int b) {
-    const int c = p.ctx_lens[b];
-    return c < 0 ? 0 : (c > ctx_cap ? ctx_cap : c);
-  };
+  auto capped = [&](int c) { return c < 0 ? 0 : (c > ctx_cap ? ctx_cap : c); };
+  auto length_of = [&](int b) { return capped(p.ctx_lens[b]); };
   auto units_of = [](int ctx) { return (ctx + UNIT - 1) / UNIT; };
-
-  // ---- 1. units per sequence, block-wide scan, this block's range of the unit list ------
-  const int per_thread = (p.batch + NT - 1) / NT;
-  const int b_lo = min(tid * per_thread, p.batch), b_hi = min(b_lo + per_thread, p.batch);
-  // The first table line of every sequence on its way to this SM while the lengths are summed: the
-  // block does not know yet whose it needs (beyond this batch the stream hides the trip).
-  if (p.batch <= NT && tid < p.batch)
-    asm volatile("prefetch.global.L1 [%0];" ::"l"(p.block_tables + tid * p.bt_stride));
-  int local = 0, len_lo = 0;
-  for (int b = b_lo; b < b_hi; ++b) {
-    const int c = length_of(b);
-    if (b == b_lo) len_lo = c;
-    local += units_of(c);
-    if (c == 0 && b % p.n_ranges == range) {  // empty context: defined output (zeros), no cache access
-      uint4* dst = reinterpret_cast<uint4*>(p.out + b * p.out_stride + static_cast<int64_t>(kvh * p.g) * D);
-      for (int i = 0; i < p.g * D / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
-    }
-  }
-  int incl = local;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int v = __shfl_up_sync(0xffffffffu, incl, d);
-    if (lane >= d) incl += v;
-  }
-  if (lane == 31) s_scan[warp] = incl;
-  __syncthreads();
-  int before = 0, total = 0;
-#pragma unroll
-  for (int w = 0; w < NW; ++w) {
-    if (w < warp) before += s_scan[w];
-    total += s_scan[w];
-  }
-  const int excl = before + incl - local;
-  // No more ranges than units, so that every range in use holds at least one unit and the ranges
-  // that share a sequence are consecutive.  And where sequences are few, no more than balance the
-  // two costs of a cut: a range streams total / n units and a sequence's merge reads n / batch
-  // partials, so that the sum is least at n = sqrt(c total batch).
-  const int n_ranges = max(1, min(min(p.n_ranges, total), static_cast<int>(sqrtf(kSplitBalance * total * p.batch))));
-  if (range >= n_ranges || total == 0) return;  // block-uniform (also when the whole batch is empty)
-  // the first `longer` ranges hold one unit more than the others
-  const int per_range = total / n_ranges, longer = total - per_range * n_ranges;
-  const int u0 = range * per_range + min(range, longer);
-  const int u1 = u0 + per_range + (range < longer ? 1 : 0);
-  if (local > 0 && excl <= u0 && u0 < excl + local) {  // the one thread whose sequences hold unit u0
-    int first = excl;
-    for (int b = b_lo;; ++b) {
-      const int len = b == b_lo ? len_lo : length_of(b), n = units_of(len);
-      if (u0 < first + n) {
-        s_start[0] = b;
-        s_start[1] = first;
-        s_start[2] = len;
-        break;
-      }
-      first += n;
-    }
-  }
-  __syncthreads();
-  // the range that holds global unit u
-  auto range_of = [&](int u) {
-    const int split = longer * (per_range + 1);
-    return u < split ? u / (per_range + 1) : longer + (u - split) / per_range;
+  auto write_zeros = [&](int b) {  // empty context: defined output, no cache access
+    if (b % p.n_ranges != range) return;
+    uint4* dst = reinterpret_cast<uint4*>(p.out + b * p.out_stride + static_cast<int64_t>(kvh * p.g) * D);
+    for (int i = 0; i < p.g * D / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
   };
 
   auto slot_of = [&](int b) { return p.k_new != nullptr ? p.slot_mapping[b] : -1; };
-  SeqCursor cc;  // compute side
-  cc.b = s_start[0];
-  cc.first = s_start[1];
-  cc.ctx = s_start[2];
-  cc.units = units_of(cc.ctx);
-  cc.slot = slot_of(cc.b);
-  SeqCursor pc = cc;  // load side, NST-1 units ahead
   auto seek = [&](SeqCursor& c, int u) {  // u < total, so c.b stays inside the batch
     if (u < c.first + c.units) return;
     do {
@@ -228,11 +165,9 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       ++c.b;
       c.ctx = length_of(c.b);
       c.units = units_of(c.ctx);
-    } while (u >= c.first + c.units);
+    } while (u >= c.first + c.units && (!GUESS || c.b < p.batch - 1));  // a guess may count on more units than there are
     c.slot = slot_of(c.b);
   };
-
-  if (p.lengths_early) pdl_wait();  // from here on the cache is read
 
   // Q^T as the B operand: lane (gid, tig) holds q[head gid][16*ks + 2*tig .. +1] and [.. + 8].
   auto load_q = [&](uint32_t (&dst)[C::KS][2], int b) {
@@ -248,14 +183,11 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       }
     }
   };
-  uint32_t qb[C::KS][2], qn[C::KS][2];  // this sequence's fragments; the next sequence's, fetched early
-  load_q(qb, cc.b);
-  int qn_b = min(cc.b + 1, p.batch - 1);
-  load_q(qn, qn_b);
 
   const uint32_t warp_smem = smem_u32(smem) + warp * C::WARP_BYTES;
   const int64_t row_elems = static_cast<int64_t>(p.hkv) * D;
 
+  int bad = 0;
   unsigned fresh = 0;  // step variant: stages whose tile holds the new token's row
   auto load_tile = [&](const SeqCursor& c, int u, int stage) {
     fresh &= ~(1u << stage);
@@ -264,7 +196,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     int64_t blk = p.block_tables[c.b * p.bt_stride + t0 / kBlockSize];
     const bool blk_ok = blk >= 0 && blk < p.num_blocks;
     if (!blk_ok) {
-      if (lane == 0) atomicOr(p.status, NVLLM_STATUS_BAD_BLOCK);
+      bad = NVLLM_STATUS_BAD_BLOCK;  // reported at the end: a guess may load for nothing
       blk = 0;
     }
     const int64_t slot0 = blk * kBlockSize + (t0 % kBlockSize);
@@ -297,6 +229,142 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       cp_async16(dst, ksrc, bytes);
       cp_async16(dst + C::TILE_BYTES, vsrc, bytes);
     }
+  };
+
+  // ---- 1. units per sequence, block-wide scan, this block's range of the unit list ------
+  const int per_thread = GUESS ? 1 : (p.batch + NT - 1) / NT;
+  const int b_lo = min(tid * per_thread, p.batch), b_hi = min(b_lo + per_thread, p.batch);
+  // The first table line of every sequence on its way to this SM while the lengths are summed: the
+  // block does not know yet whose it needs (beyond this batch the stream hides the trip).
+  auto prefetch_table = [&]() {
+    if (p.batch <= NT && tid < p.batch)
+      asm volatile("prefetch.global.L1 [%0];" ::"l"(p.block_tables + tid * p.bt_stride));
+  };
+  int total, n_ranges, per_range, longer, u0, u1, len_lo;
+  auto split = [&](bool ahead) {
+    if (!ahead) prefetch_table();
+    int local = 0;
+    len_lo = 0;
+    for (int b = b_lo; b < b_hi; ++b) {
+      const int c = ahead ? capped(__ldcg(p.ctx_lens + b)) : length_of(b);
+      if (b == b_lo) len_lo = c;
+      local += units_of(c);
+      if (!GUESS && c == 0) write_zeros(b);
+    }
+    int incl = local;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += v;
+    }
+    if (lane == 31) s_scan[warp] = incl;
+    __syncthreads();
+    int before = 0;
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < NW; ++w) {
+      if (w < warp) before += s_scan[w];
+      total += s_scan[w];
+    }
+    const int excl = before + incl - local;
+    // No more ranges than units, so that every range in use holds at least one unit and the ranges
+    // that share a sequence are consecutive.  And where sequences are few, no more than balance the
+    // two costs of a cut: a range streams total / n units and a sequence's merge reads n / batch
+    // partials, so that the sum is least at n = sqrt(c total batch).
+    n_ranges = max(1, min(min(p.n_ranges, total), static_cast<int>(sqrtf(kSplitBalance * total * p.batch))));
+    if (range >= n_ranges || total == 0) return false;  // block-uniform (also when the whole batch is empty)
+    // the first `longer` ranges hold one unit more than the others
+    per_range = total / n_ranges, longer = total - per_range * n_ranges;
+    u0 = range * per_range + min(range, longer);
+    u1 = u0 + per_range + (range < longer ? 1 : 0);
+    if (local > 0 && excl <= u0 && u0 < excl + local) {  // the one thread whose sequences hold unit u0
+      int first = excl;
+      for (int b = b_lo;; ++b) {
+        const int len = b == b_lo ? len_lo : length_of(b), n = units_of(len);
+        if (u0 < first + n) {
+          s_start[0] = b;
+          s_start[1] = first;
+          s_start[2] = len;
+          break;
+        }
+        first += n;
+      }
+    }
+    __syncthreads();
+    return true;
+  };
+
+  SeqCursor cc, pc;  // compute side; load side, NST-1 units ahead
+  uint32_t qb[C::KS][2], qn[C::KS][2];  // this sequence's fragments; the next sequence's, fetched early
+  int qn_b, n_units;
+  auto start = [&]() {
+    cc.b = s_start[0];
+    cc.first = s_start[1];
+    cc.ctx = s_start[2];
+    cc.units = units_of(cc.ctx);
+    cc.slot = slot_of(cc.b);
+    pc = cc;
+    if (!GUESS && p.lengths_early) pdl_wait();  // from here on the cache is read
+    load_q(qb, cc.b);
+    qn_b = min(cc.b + 1, p.batch - 1);
+    load_q(qn, qn_b);
+    n_units = u1 - u0;
+#pragma unroll
+    for (int j = 0; j < NST - 1; ++j) {
+      if (j < n_units) {
+        seek(pc, u0 + j);
+        load_tile(pc, u0 + j, j);
+      }
+      cp_async_commit();
+    }
+  };
+
+  if constexpr (GUESS) {
+    // The range is cut by what the lengths are now and its first tiles are brought to L2.  When the previous
+    // kernel is done those tiles are loaded while the lengths are read again, and if one has changed the
+    // range is cut anew.  What is read before the wait goes round L1, is held to the bounds of the table
+    // and the cache, and serves the guess alone.
+    bool mine = split(true);
+    if (mine) {
+      const int b = s_start[0], first = s_start[1], ctx = s_start[2];
+      const int u_end = min(min(u1, first + units_of(ctx)), u0 + NST - 1);
+      for (int u = u0; u < u_end; ++u) {
+        const int t0 = (u - first) * UNIT + warp * TT;
+        if (t0 >= ctx) break;
+        const int64_t blk = __ldcg(p.block_tables + b * p.bt_stride + t0 / kBlockSize);
+        if (blk < 0 || blk >= p.num_blocks) break;
+        constexpr int LINES = C::ROW_BYTES / 128;
+#pragma unroll
+        for (int it = 0; it < TT * LINES / 32; ++it) {
+          const int r = (it * 32 + lane) / LINES, part = (it * 32 + lane) % LINES;
+          const int64_t off = (blk * kBlockSize + t0 % kBlockSize + r) * row_elems + kvh * D + part * 64;
+          if (t0 + r < ctx) {
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.k_cache + off));
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v_cache + off));
+          }
+        }
+      }
+    }
+    pdl_wait();
+    const int now = tid < p.batch ? length_of(tid) : 0;
+    if (mine) start();
+    if (__syncthreads_or(now != len_lo)) {
+      cp_async_wait<0>();
+      __syncthreads();
+      bad = 0;
+      mine = split(false);
+      if (mine) start();
+    }
+    if (tid < p.batch && len_lo == 0) write_zeros(tid);
+    if (!mine) return;
+  } else {
+    if (!split(false)) return;
+    start();
+  }
+  // the range that holds global unit u
+  auto range_of = [&](int u) {
+    const int split = longer * (per_range + 1);
+    return u < split ? u / (per_range + 1) : longer + (u - split) / per_range;
   };
 
   float o[C::DT][4];
@@ -468,16 +536,6 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   };
 
   // ---- 2. stream the range ------------------------------------------------------------------
-  const int n_units = u1 - u0;
-#pragma unroll
-  for (int j = 0; j < NST - 1; ++j) {
-    if (j < n_units) {
-      seek(pc, u0 + j);
-      load_tile(pc, u0 + j, j);
-    }
-    cp_async_commit();
-  }
-
   for (int i = 0;; ++i) {
     const int u = u0 + i;
     if (i == n_units || u >= cc.first + cc.units) {  // block-uniform: the range leaves sequence cc.b
@@ -595,6 +653,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     }
   }
   cp_async_wait<0>();
+  if (bad && lane == 0) atomicOr(p.status, bad);
   if (n_cut == 0) return;  // block-uniform
   __syncthreads();         // every thread's partials are written
   if (tid < n_cut) {
@@ -655,19 +714,27 @@ static int64_t workspace_bytes_for(int batch, int hq, int hkv, int d) {
   return kCounterBytes + rows * d * 4 + rows * 2 * 4;
 }
 
-template <class C>
+template <class C, bool GUESS>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(decode_paged_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+    cudaError_t e = cudaFuncSetAttribute(decode_paged_kernel<C, GUESS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
     if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
     attr_set[dev] = true;
   }
   const int grid = p.n_ranges * p.hkv;
-  return launch_kernel("decode_paged", decode_paged_kernel<C>, dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream,
-                       p);
+  return launch_kernel("decode_paged", decode_paged_kernel<C, GUESS>, dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM,
+                       stream, p);
+}
+
+// A guess for plain launches with a sequence per thread at most.  Larger batches stream long enough for
+// the trips at the start not to matter, and the step kernel's predecessor in a chain is itself.
+template <class C>
+static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
+  const bool ahead = !p.lengths_early && !p.k_new && p.batch <= C::NW * 32;
+  return ahead ? launch_decode<C, true>(p, stream) : launch_decode<C, false>(p, stream);
 }
 
 // Shared body of nvllm_decode_paged and nvllm_decode_step.

@@ -220,6 +220,43 @@ def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
     assert torch.equal(got.view_as(dev.q), A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, dev.scale))
 
 
+@pytest.mark.parametrize("batch", [1, 31, 128, 129])
+def test_lengths_written_by_the_kernel_just_before(cuda, batch):
+    """The lengths are the rows of a cache that the launch in front stores to: the decode, which may
+    start on the lengths of the time before, must use the new ones, longer, shorter or none, and
+    report nothing about table entries that only the old ones reach."""
+    g = torch.Generator().manual_seed(batch)
+    longest = torch.randint(1, 3000, (batch,), generator=g)
+    case = W.make_decode_case(31, batch, 1, 1, 16, 8, 128, context_lens=longest.tolist())
+    dev = case.to(cuda)
+    plane = torch.zeros(2, 256, 1, 256, dtype=torch.bfloat16, device=cuda)  # rows of 128 int32
+    lens = plane[1].view(-1).view(torch.int32)[:batch]
+    slots = torch.arange(511, -1, -1, dtype=torch.int32, device=cuda)  # the rows that hold the lengths last
+    scratch = torch.zeros_like(plane)
+    steps = []
+    for i in range(6):
+        now = [longest, longest // 2, torch.zeros_like(longest), longest * (torch.arange(batch) % 2), longest // 9, longest][i]
+        table = case.block_tables.clone()
+        for b in range(batch):
+            table[b, (int(now[b]) + 255) // 256:] = -1
+        rows = torch.zeros(512, 128, dtype=torch.int32)
+        flat = torch.zeros(256 * 128, dtype=torch.int32)
+        flat[:batch] = now.int()
+        rows[:256] = flat.view(256, 128).flip(0)
+        key = rows.to(cuda).view(torch.bfloat16).view(512, 1, 256)
+        steps.append((now.int(), table.to(cuda), key))
+    outs = []
+    torch.cuda.synchronize()
+    for now, table, key in steps:
+        A.store_kvcache(key, key, plane, scratch, slots)
+        outs.append(A.decode_paged(dev.q, dev.k_cache, dev.v_cache, lens, table, case.scale))
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+    for (now, table, _), out in zip(steps, outs):
+        ref = R.decode_ref(case.q, case.k_cache, case.v_cache, now, case.block_tables, case.scale)
+        assert_close_to_oracle(out, ref, f"batch {batch}, lengths to {int(now.max())}")
+
+
 @pytest.mark.parametrize("tp", [2, 4, 8])
 def test_head_sharded_ranks_reassemble_the_unsharded_result(cuda, tp):
     """Tensor parallelism: rank r holds query heads [r*Hq/tp, ...) and KV heads [r*Hkv/tp, ...) of
