@@ -714,27 +714,24 @@ static int64_t workspace_bytes_for(int batch, int hq, int hkv, int d) {
   return kCounterBytes + rows * d * 4 + rows * 2 * 4;
 }
 
-template <class C, bool GUESS>
+template <class C>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(decode_paged_kernel<C, GUESS>, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
-    if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {  // both variants, so that the other's first launch may be captured
+    for (auto kernel : {decode_paged_kernel<C, false>, decode_paged_kernel<C, true>}) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
+    }
     attr_set[dev] = true;
   }
+  // A guess for plain launches with a sequence per thread at most.  Larger batches stream long enough for
+  // the trips at the start not to matter, and the step kernel's predecessor in a chain is itself.
+  const bool guess = !p.lengths_early && !p.k_new && p.batch <= C::NW * 32;
   const int grid = p.n_ranges * p.hkv;
-  return launch_kernel("decode_paged", decode_paged_kernel<C, GUESS>, dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM,
-                       stream, p);
-}
-
-// A guess for plain launches with a sequence per thread at most.  Larger batches stream long enough for
-// the trips at the start not to matter, and the step kernel's predecessor in a chain is itself.
-template <class C>
-static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
-  const bool ahead = !p.lengths_early && !p.k_new && p.batch <= C::NW * 32;
-  return ahead ? launch_decode<C, true>(p, stream) : launch_decode<C, false>(p, stream);
+  return launch_kernel("decode_paged", guess ? decode_paged_kernel<C, true> : decode_paged_kernel<C, false>,
+                       dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream, p);
 }
 
 // Shared body of nvllm_decode_paged and nvllm_decode_step.

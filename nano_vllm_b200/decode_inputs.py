@@ -1,4 +1,4 @@
-"""Decode-step inputs in one copy and one launch.
+"""Decode-step inputs in one launch.
 
 Host mirror of what nano-vllm's ``ModelRunner`` does before it can replay a decode graph:
 ``prepare_decode`` / ``prepare_block_tables`` / ``prepare_sample``
