@@ -43,6 +43,8 @@
 // 35.3 -> 32.7; 256 sequences of 2048-8192 tokens (32 / 8 heads, step variant) 795 -> 747.
 #include <cstdlib>
 
+#include <type_traits>
+
 #include "common.cuh"
 
 // Pipeline shape of the head_dim-128 kernel: tokens per warp tile, ring stages per warp, warps per
@@ -80,12 +82,13 @@ struct DecodeParams {
   int batch, hq, hkv, g;
   float scale_log2e;
   int64_t num_blocks;
-  // step variant: the new token's rows; k_new == nullptr for plain decode
+  // step and layer variant: the new tokens' rows
   const __nv_bfloat16* k_new;
   int64_t k_new_stride;
   const __nv_bfloat16* v_new;
   int64_t v_new_stride;
   const int32_t* slot_mapping;
+  int n_new;               // layer variant: new rows, one to a lane, stored to slot_mapping[row]
   int n_ranges;
   bool lengths_early;      // lengths and tables were complete before the previous kernel in the stream let this one start
   unsigned int* counters;  // [batch * hkv], zero between launches
@@ -129,11 +132,17 @@ struct Cut {
 // 32000 in the head_dim 64 geometry: 16.1 us, 26.1 without a limit).
 constexpr float kSplitBalance = 8.f;
 
-// GUESS: the first split of the batch and the loads that follow from it are made on lengths that the previous
-// kernel may yet change (see where it branches).  In a chain of decode layers of 16 sequences, of which each
-// streams 7 us, that takes the trips for lengths, sums and first rows off the path: 17.4 -> 15.6 us a layer.
-template <class C, bool GUESS>
+// The four kernels.  Step and Layer also store the new tokens' rows: Step where the row's slot is that of its
+// position, Layer to any slot.
+// Guess and Layer make the first split of the batch, and the loads that follow from it, on lengths that the
+// previous kernel may yet change (see where they branch).  In a chain of decode layers of 16 sequences, of
+// which each streams 7 us, that takes the trips for lengths, sums and first rows off the path, and with
+// nothing of Step in it the kernel starts its loads sooner: 17.4 -> 14.9 us a layer.
+enum class Variant { Plain, Step, Guess, Layer };
+
+template <class C, Variant V>
 __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const DecodeParams p) {
+  constexpr bool STEP = V == Variant::Step, LAYER = V == Variant::Layer, GUESS = V == Variant::Guess || LAYER;
   constexpr int D = C::D, TT = C::TT, NST = C::NST, NW = C::NW, UNIT = C::UNIT, NT = NW * 32;
   constexpr int QUADS = D / 4, GROUPS = NT / QUADS;  // lanes that hold a head four columns each; such groups in a block
   extern __shared__ __align__(128) unsigned char smem[];
@@ -157,7 +166,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     for (int i = 0; i < p.g * D / 8; ++i) dst[i] = make_uint4(0u, 0u, 0u, 0u);
   };
 
-  auto slot_of = [&](int b) { return p.k_new != nullptr ? p.slot_mapping[b] : -1; };
+  auto slot_of = [&](int b) { return STEP ? p.slot_mapping[b] : -1; };
   auto seek = [&](SeqCursor& c, int u) {  // u < total, so c.b stays inside the batch
     if (u < c.first + c.units) return;
     do {
@@ -188,6 +197,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   const int64_t row_elems = static_cast<int64_t>(p.hkv) * D;
 
   int bad = 0;
+  int new_slot = -1;   // layer variant, lane l: slot of the l-th new row
   unsigned fresh = 0;  // step variant: stages whose tile holds the new token's row
   auto load_tile = [&](const SeqCursor& c, int u, int stage) {
     fresh &= ~(1u << stage);
@@ -204,7 +214,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     // provided slot_mapping agrees with the block table, and goes to the cache when the tile is used.
     const int last = c.ctx - 1;
     int new_row = -1;
-    if (p.k_new != nullptr && last < t0 + TT && c.slot >= 0) {  // last >= t0 holds because t0 < ctx
+    if (STEP && last < t0 + TT && c.slot >= 0) {  // last >= t0 holds because t0 < ctx
       if (blk_ok && c.slot == slot0 + (last - t0)) {
         new_row = last - t0;
         fresh |= 1u << stage;
@@ -212,23 +222,40 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
         atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
       }
     }
+    // Layer variant: whatever row of whatever sequence lies in a slot that this launch stores to is the new
+    // one, as it would be behind a launch that stores.
+    unsigned stored = 0;
+    if (LAYER && blk_ok) stored = __ballot_sync(0xffffffffu, new_slot >= slot0 && new_slot < slot0 + TT);
     const uint32_t kdst = warp_smem + stage * C::STAGE_BYTES;
+    auto copy = [&](auto patch) {
 #pragma unroll
-    for (int it = 0; it < TT * C::CPR / 32; ++it) {
-      const int idx = it * 32 + lane;
-      const int r = idx / C::CPR, col = idx % C::CPR;
-      const int bytes = (blk_ok && t0 + r < c.ctx) ? 16 : 0;
-      const int64_t off = bytes ? (slot0 + r) * row_elems + kvh * D + col * 8 : 0;
-      const __nv_bfloat16 *ksrc = p.k_cache + off, *vsrc = p.v_cache + off;
-      if (r == new_row) {
-        const int64_t in_row = static_cast<int64_t>(kvh) * D + col * 8;
-        ksrc = p.k_new + c.b * p.k_new_stride + in_row;
-        vsrc = p.v_new + c.b * p.v_new_stride + in_row;
+      for (int it = 0; it < TT * C::CPR / 32; ++it) {
+        const int idx = it * 32 + lane;
+        const int r = idx / C::CPR, col = idx % C::CPR;
+        const int bytes = (blk_ok && t0 + r < c.ctx) ? 16 : 0;
+        const int64_t off = bytes ? (slot0 + r) * row_elems + kvh * D + col * 8 : 0;
+        const __nv_bfloat16 *ksrc = p.k_cache + off, *vsrc = p.v_cache + off;
+        if (STEP && r == new_row) {
+          const int64_t in_row = static_cast<int64_t>(kvh) * D + col * 8;
+          ksrc = p.k_new + c.b * p.k_new_stride + in_row;
+          vsrc = p.v_new + c.b * p.v_new_stride + in_row;
+        }
+        if constexpr (decltype(patch)::value) {
+          for (unsigned left = stored; left; left &= left - 1) {
+            const int i = __ffs(left) - 1;
+            if (__shfl_sync(0xffffffffu, new_slot, i) == slot0 + r) {
+              ksrc = p.k_new + i * p.k_new_stride + kvh * D + col * 8;
+              vsrc = p.v_new + i * p.v_new_stride + kvh * D + col * 8;
+            }
+          }
+        }
+        const uint32_t dst = kdst + r * C::ROW_BYTES + ((col ^ (r & 7)) << 4);
+        cp_async16(dst, ksrc, bytes);
+        cp_async16(dst + C::TILE_BYTES, vsrc, bytes);
       }
-      const uint32_t dst = kdst + r * C::ROW_BYTES + ((col ^ (r & 7)) << 4);
-      cp_async16(dst, ksrc, bytes);
-      cp_async16(dst + C::TILE_BYTES, vsrc, bytes);
-    }
+    };
+    if (LAYER && stored) copy(std::true_type{});
+    else copy(std::false_type{});
   };
 
   // ---- 1. units per sequence, block-wide scan, this block's range of the unit list ------
@@ -324,6 +351,9 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     // kernel is done those tiles are loaded while the lengths are read again, and if one has changed the
     // range is cut anew.  What is read before the wait goes round L1, is held to the bounds of the table
     // and the cache, and serves the guess alone.
+    const int64_t n_slots = p.num_blocks * kBlockSize;
+    auto in_cache = [&](int slot) { return slot >= 0 && slot < n_slots ? slot : -1; };
+    if (LAYER && lane < p.n_new) new_slot = in_cache(__ldcg(p.slot_mapping + lane));
     bool mine = split(true);
     if (mine) {
       const int b = s_start[0], first = s_start[1], ctx = s_start[2];
@@ -347,15 +377,30 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     }
     pdl_wait();
     const int now = tid < p.batch ? length_of(tid) : 0;
+    const int slot_now = LAYER && lane < p.n_new ? p.slot_mapping[lane] : -1;
     if (mine) start();
-    if (__syncthreads_or(now != len_lo)) {
+    if (__syncthreads_or(now != len_lo || (LAYER && in_cache(slot_now) != new_slot))) {
       cp_async_wait<0>();
       __syncthreads();
       bad = 0;
+      new_slot = in_cache(slot_now);
       mine = split(false);
       if (mine) start();
     }
     if (tid < p.batch && len_lo == 0) write_zeros(tid);
+    if (LAYER && warp == NW - 1) {
+      for (int i = range; i < p.n_new; i += p.n_ranges) {
+        const int64_t slot = __shfl_sync(0xffffffffu, new_slot, i);
+        if (slot < 0) continue;
+        for (int k = lane; k < 2 * C::CPR; k += 32) {  // K pieces, then V pieces (for head_dim 128 one per lane)
+          const bool is_k = k < C::CPR;
+          const int64_t col = kvh * D + k % C::CPR * 8;
+          *reinterpret_cast<uint4*>((is_k ? p.k_cache : p.v_cache) + slot * row_elems + col) =
+              *reinterpret_cast<const uint4*>(is_k ? p.k_new + i * p.k_new_stride + col : p.v_new + i * p.v_new_stride + col);
+        }
+      }
+      if (blockIdx.x == 0 && slot_now >= n_slots) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
+    }
     if (!mine) return;
   } else {
     if (!split(false)) return;
@@ -719,18 +764,22 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {  // both variants, so that the other's first launch may be captured
-    for (auto kernel : {decode_paged_kernel<C, false>, decode_paged_kernel<C, true>}) {
+  if (dev >= 0 && dev < 64 && !attr_set[dev]) {  // all variants, so that the others' first launch may be captured
+    for (auto kernel : {decode_paged_kernel<C, Variant::Plain>, decode_paged_kernel<C, Variant::Step>, decode_paged_kernel<C, Variant::Guess>,
+                        decode_paged_kernel<C, Variant::Layer>}) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
       if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
     }
     attr_set[dev] = true;
   }
-  // A guess for plain launches with a sequence per thread at most.  Larger batches stream long enough for
-  // the trips at the start not to matter, and the step kernel's predecessor in a chain is itself.
-  const bool guess = !p.lengths_early && !p.k_new && p.batch <= C::NW * 32;
+  // A guess for launches with a sequence per thread at most.  Larger batches stream long enough for the trips
+  // at the start not to matter, and the step kernel's predecessor in a chain is itself.
+  auto kernel = p.n_new > 0                                           ? decode_paged_kernel<C, Variant::Layer>
+                : p.k_new                                             ? decode_paged_kernel<C, Variant::Step>
+                : !p.lengths_early && p.batch <= C::NW * 32           ? decode_paged_kernel<C, Variant::Guess>
+                                                                      : decode_paged_kernel<C, Variant::Plain>;
   const int grid = p.n_ranges * p.hkv;
-  return launch_kernel("decode_paged", guess ? decode_paged_kernel<C, true> : decode_paged_kernel<C, false>,
+  return launch_kernel("decode_paged", kernel,
                        dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream, p);
 }
 
@@ -740,7 +789,7 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
                          void* v_cache, const int32_t* context_lens, const int32_t* block_tables, int64_t bt_row_stride,
                          int32_t max_blocks, void* out, int64_t out_row_stride, int32_t batch, int32_t num_q_heads,
                          int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks, void* workspace,
-                         int64_t workspace_bytes, void* stream, bool with_store, bool lengths_early) {
+                         int64_t workspace_bytes, void* stream, bool with_store, bool lengths_early, int n_new = 0) {
   int rc = check_decode_geometry(who, batch, max_blocks, num_q_heads, num_kv_heads, head_dim);
   if (rc) return rc;
   if (batch == 0) return NVLLM_OK;
@@ -790,6 +839,7 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
   p.v_new = with_store ? static_cast<const __nv_bfloat16*>(v_new) : nullptr;
   p.v_new_stride = v_new_row_stride;
   p.slot_mapping = slot_mapping;
+  p.n_new = n_new;
   p.lengths_early = lengths_early;
   p.n_ranges = ranges_for(decode_ctas(), num_kv_heads);
   const int64_t rows = (static_cast<int64_t>(ranges_for(kMaxDecodeCtas, num_kv_heads)) + batch) * num_q_heads;
@@ -851,12 +901,18 @@ extern "C" int nvllm_attention_decode(const void* q, int64_t q_row_stride, const
                                       int64_t bt_row_stride, int32_t max_blocks, void* out, int64_t out_row_stride,
                                       int32_t batch, int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim, float scale,
                                       int64_t num_blocks, void* workspace, int64_t workspace_bytes, void* stream) {
-  const int rc = nvllm_store_kvcache(key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_new,
-                                     num_kv_heads * head_dim, num_blocks * nvllm::kBlockSize, stream);
+  using namespace nvllm;
+  // Few sequences: one launch, in which a block that meets a slot stored to takes the new row instead (one
+  // sequence of 317 tokens 9.3 -> 7.0 us, eight of 100 to 1024 11.1 -> 10.0); a lane holds a slot, hence
+  // the 32.  More: the copy first, under which the decode reads its lengths.
+  const bool one_launch = n_new > 0 && n_new <= 32 && batch > 0 && batch <= 32;
+  const int rc = store_kvcache(!one_launch, false, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_new,
+                               num_kv_heads * head_dim, num_blocks * kBlockSize, stream);
   if (rc) return rc;
-  return nvllm::decode_common("attention_decode", q, q_row_stride, nullptr, 0, nullptr, 0, nullptr, k_cache, v_cache, context_lens,
-                              block_tables, bt_row_stride, max_blocks, out, out_row_stride, batch, num_q_heads, num_kv_heads,
-                              head_dim, scale, num_blocks, workspace, workspace_bytes, stream, false, n_new > 0);
+  return decode_common("attention_decode", q, q_row_stride, key, key_row_stride, value, value_row_stride, slot_mapping, k_cache,
+                       v_cache, context_lens, block_tables, bt_row_stride, max_blocks, out, out_row_stride, batch, num_q_heads,
+                       num_kv_heads, head_dim, scale, num_blocks, workspace, workspace_bytes, stream, one_launch,
+                       n_new > 0 && !one_launch, one_launch ? static_cast<int>(n_new) : 0);
 }
 
 // ---- decode without a caller-provided workspace ---------------------------------------------

@@ -28,12 +28,6 @@ struct PrefillParams {
   bool store_follows;  // a kernel that may run under this one comes next: let it start, but not before pdl_wait()
 };
 
-// nvllm_store_kvcache's body.  `launch` false: checks only.  `beside`: the launch before it in the stream is
-// a prefill with store_follows set, under which the copy may run.
-int store_kvcache(bool launch, bool beside, const void* key, int64_t key_row_stride, const void* value, int64_t value_row_stride,
-                  void* k_cache, void* v_cache, const int32_t* slot_mapping, int64_t n_tokens, int32_t row_elems,
-                  int64_t num_slots, void* stream);
-
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).
 // The engine schedules at most 512 sequences per step (nanovllm/config.py:10).
 constexpr int kPrefillMaxBatch = 1024;

@@ -220,6 +220,49 @@ def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
     assert torch.equal(got.view_as(dev.q), A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, dev.scale))
 
 
+@pytest.mark.parametrize("batch", [1, 2, 31, 32, 33])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
+def test_layer_equals_store_then_decode_wherever_the_slots_lie(cuda, batch, hq, hkv, d):
+    """One launch for few sequences: rows stored at their position, elsewhere in the same sequence, in
+    another sequence's context, at a padding row's slot 0, twice to one slot, and nowhere."""
+    g = torch.Generator().manual_seed(batch)
+    lens = torch.randint(1, 1500, (batch,), generator=g)
+    case = W.make_decode_case(37, batch, 1, 1, hq, hkv, d, context_lens=lens.tolist())
+    slots = case.slot_mapping.clone()
+    ctx = case.context_lens.clone()
+    first = case.block_tables[:, 0].long() * 256
+    slots[0] = first[0] + int(lens[0]) // 2 % 256  # in the middle of its own context
+    if batch > 2:
+        slots[1] = first[2]  # the first row of its neighbour
+        ctx[3], slots[3] = 0, 0  # graph padding
+        slots[4] = -1
+        slots[5] = slots[6]
+        case.k_new[5], case.v_new[5] = case.k_new[6], case.v_new[6]
+        slots[batch - 1] = first[batch - 2] + 1
+    dev = case.to(cuda)
+    slots, ctx = slots.to(cuda), ctx.to(cuda)
+    k2, v2 = dev.k_cache.clone(), dev.v_cache.clone()
+    layer = A.Attention(hq, d, dev.scale, hkv)
+    layer.k_cache, layer.v_cache = dev.k_cache, dev.v_cache
+    for _ in range(2):
+        C.set_context(False, slot_mapping=slots, context_lens=ctx, block_tables=dev.block_tables)
+        got = layer(dev.q.view(batch, -1), dev.k_new.view(batch, -1), dev.v_new.view(batch, -1))
+        C.reset_context()
+        A.store_kvcache(dev.k_new, dev.v_new, k2, v2, slots)
+        want = A.decode_paged(dev.q, k2, v2, ctx, dev.block_tables, dev.scale)
+        assert torch.equal(got.view_as(want), want)
+        assert torch.equal(dev.k_cache, k2) and torch.equal(dev.v_cache, v2)
+        dev.k_new, dev.v_new = dev.k_new.flip(-1).contiguous(), dev.v_new.flip(-1).contiguous()
+        slots = torch.where(slots >= 0, (slots // 256) * 256 + (slots + 77) % 256, slots)  # other rows of those blocks
+    assert _lib.read_status() == 0
+    slots[0] = dev.k_cache.shape[0] * 256
+    C.set_context(False, slot_mapping=slots, context_lens=ctx, block_tables=dev.block_tables)
+    layer(dev.q.view(batch, -1), dev.k_new.view(batch, -1), dev.v_new.view(batch, -1))
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 1  # NVLLM_STATUS_BAD_SLOT
+
+
 @pytest.mark.parametrize("batch", [1, 31, 128, 129])
 def test_lengths_written_by_the_kernel_just_before(cuda, batch):
     """The lengths are the rows of a cache that the launch in front stores to: the decode, which may
