@@ -29,9 +29,8 @@ constexpr int kBlockSize = NVLLM_BLOCK_SIZE;
 // constant of one chip.
 int num_sms();
 
-// nvllm_store_kvcache's body.  `launch` false: checks only.  `beside`: the launch before it in the stream is
-// a prefill with store_follows set, under which the copy may run.
-int store_kvcache(bool launch, bool beside, const void* key, int64_t key_row_stride, const void* value, int64_t value_row_stride,
+// nvllm_store_kvcache's body.  `launch` false: checks only.
+int store_kvcache(bool launch, const void* key, int64_t key_row_stride, const void* value, int64_t value_row_stride,
                   void* k_cache, void* v_cache, const int32_t* slot_mapping, int64_t n_tokens, int32_t row_elems,
                   int64_t num_slots, void* stream);
 

@@ -906,7 +906,7 @@ extern "C" int nvllm_attention_decode(const void* q, int64_t q_row_stride, const
   // sequence of 317 tokens 9.3 -> 7.0 us, eight of 100 to 1024 11.1 -> 10.0); a lane holds a slot, hence
   // the 32.  More: the copy first, under which the decode reads its lengths.
   const bool one_launch = n_new > 0 && n_new <= 32 && batch > 0 && batch <= 32;
-  const int rc = store_kvcache(!one_launch, false, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_new,
+  const int rc = store_kvcache(!one_launch, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_new,
                                num_kv_heads * head_dim, num_blocks * kBlockSize, stream);
   if (rc) return rc;
   return decode_common("attention_decode", q, q_row_stride, key, key_row_stride, value, value_row_stride, slot_mapping, k_cache,

@@ -6,12 +6,20 @@
 
 namespace nvllm {
 
+// The persistent tcgen05 kernel is the product.  NVLLM_PREFILL_IMPL=mma (read on every call)
+// selects the warp-level mma.sync kernel instead: the cross-check of the tests and the A/B
+// baseline of measurements, never chosen by the library itself.
+static bool forced_mma() {
+  const char* forced = std::getenv("NVLLM_PREFILL_IMPL");
+  return forced && forced[0] == 'm';
+}
+
 static int prefill_common(const void* q, int64_t q_row_stride, const void* k, int64_t k_row_stride, const void* v,
                           int64_t v_row_stride, const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks, void* out,
                           int64_t out_row_stride, const int32_t* cu_seqlens_q, const int32_t* cu_seqlens_k, int64_t total_q,
                           int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads,
                           int32_t num_kv_heads, int32_t head_dim, float scale, int64_t num_blocks, void* stream,
-                          bool lengths_early, bool store_follows) {
+                          bool lengths_early, const int32_t* slots, void* k_store, void* v_store) {
   if (head_dim != 64 && head_dim != 128)
     return fail(NVLLM_E_GEOMETRY, "prefill_varlen: head_dim=%d unsupported (64 or 128)", head_dim);
   if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads)
@@ -39,12 +47,8 @@ static int prefill_common(const void* q, int64_t q_row_stride, const void* k, in
     if (k_row_stride % 8 || v_row_stride % 8)
       return fail(NVLLM_E_ALIGN, "prefill_varlen: k/v row strides must be multiples of 8 elements");
   }
-  // The persistent tcgen05 kernel is the product.  NVLLM_PREFILL_IMPL=mma (read on every call)
-  // selects the warp-level mma.sync kernel instead: the cross-check of the tests and the A/B
-  // baseline of measurements, never chosen by the library itself.
-  const char* forced = std::getenv("NVLLM_PREFILL_IMPL");
   const bool has_rows = block_tables || total_k > 0;
-  const bool use_mma = (forced && forced[0] == 'm') || !has_rows;
+  const bool use_mma = forced_mma() || !has_rows;
   if (!use_mma && batch > kPrefillMaxBatch)
     return fail(NVLLM_E_GEOMETRY, "prefill_varlen: batch=%d exceeds the %d sequences of one launch", batch, kPrefillMaxBatch);
   if (batch > 65535) return fail(NVLLM_E_GEOMETRY, "prefill_varlen: batch=%d outside the launch limits", batch);
@@ -75,7 +79,10 @@ static int prefill_common(const void* q, int64_t q_row_stride, const void* k, in
   p.scale_log2e = scale * 1.4426950408889634f;
   p.num_blocks = num_blocks;
   p.lengths_early = lengths_early;
-  p.store_follows = store_follows;
+  p.slots = slots;
+  p.k_store = static_cast<__nv_bfloat16*>(k_store);
+  p.v_store = static_cast<__nv_bfloat16*>(v_store);
+  p.n_new = slots ? total_k : 0;
   if (use_mma) return launch_prefill_mma(p, static_cast<cudaStream_t>(stream));
   return launch_prefill_tcp(p, total_q, total_k, static_cast<cudaStream_t>(stream));
 }
@@ -91,7 +98,7 @@ extern "C" int nvllm_prefill_varlen(const void* q, int64_t q_row_stride, const v
                                     void* stream) {
   return nvllm::prefill_common(q, q_row_stride, k, k_row_stride, v, v_row_stride, block_tables, bt_row_stride, max_blocks, out,
                                out_row_stride, cu_seqlens_q, cu_seqlens_k, total_q, total_k, batch, max_seqlen_q, max_seqlen_k,
-                               num_q_heads, num_kv_heads, head_dim, scale, num_blocks, stream, false, false);
+                               num_q_heads, num_kv_heads, head_dim, scale, num_blocks, stream, false, nullptr, nullptr, nullptr);
 }
 
 extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
@@ -102,19 +109,15 @@ extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, cons
                                        int32_t max_seqlen_q, int32_t max_seqlen_k, int32_t num_q_heads, int32_t num_kv_heads,
                                        int32_t head_dim, float scale, int64_t num_blocks, void* stream) {
   using namespace nvllm;
-  // Packed keys do not depend on the cache: the prefill goes first and the copy runs under it, in the
-  // registers its blocks leave free (four 4096-token prompts: 18 us of 256).  Through the table the
-  // copy has to be complete first; the lengths are then ranked under it.
-  const bool beside = !block_tables && batch > 0 && max_seqlen_q > 0 && total_q > 0 && total_k > 0;
-  auto store = [&](bool launch) {
-    return store_kvcache(launch, beside, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, total_k,
-                         num_kv_heads * head_dim, num_blocks * kBlockSize, stream);
-  };
-  int rc = store(!beside);
+  // Packed keys do not depend on the cache: warps of the prefill that have nothing else to do copy them
+  // there.  Through the table the copy has to be complete first; the lengths are then ranked under it.
+  const bool inside = !block_tables && batch > 0 && max_seqlen_q > 0 && total_q > 0 && total_k > 0 && !forced_mma() &&
+                      total_k * num_kv_heads * head_dim / 8 < (1ll << 30);  // indexed with 32 bits
+  const int rc = store_kvcache(!inside, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, total_k,
+                               num_kv_heads * head_dim, num_blocks * kBlockSize, stream);
   if (rc) return rc;
-  rc = prefill_common(q, q_row_stride, block_tables ? k_cache : key, key_row_stride, block_tables ? v_cache : value,
-                      value_row_stride, block_tables, bt_row_stride, max_blocks, out, out_row_stride, cu_seqlens_q, cu_seqlens_k,
-                      total_q, total_k, batch, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads, head_dim, scale, num_blocks,
-                      stream, !beside && total_k > 0, beside);
-  return rc || !beside ? rc : store(true);
+  return prefill_common(q, q_row_stride, block_tables ? k_cache : key, key_row_stride, block_tables ? v_cache : value,
+                        value_row_stride, block_tables, bt_row_stride, max_blocks, out, out_row_stride, cu_seqlens_q, cu_seqlens_k,
+                        total_q, total_k, batch, max_seqlen_q, max_seqlen_k, num_q_heads, num_kv_heads, head_dim, scale, num_blocks,
+                        stream, !inside && total_k > 0, inside ? slot_mapping : nullptr, k_cache, v_cache);
 }

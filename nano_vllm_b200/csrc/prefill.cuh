@@ -25,7 +25,11 @@ struct PrefillParams {
   int64_t num_blocks;
   int* status;
   bool lengths_early;  // cu_q / cu_k were complete before the previous kernel in the stream let this one start
-  bool store_follows;  // a kernel that may run under this one comes next: let it start, but not before pdl_wait()
+  // Packed rows that are also to be stored in the cache (slots nullptr: none): row i at slots[i].
+  const int32_t* slots;
+  __nv_bfloat16* k_store;
+  __nv_bfloat16* v_store;
+  int64_t n_new;
 };
 
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).

@@ -36,6 +36,7 @@
 // warp owns the same 32 rows in TMEM and in the output, and passes them 32 columns at a time
 // through a private 2 KB patch of shared memory to turn row-per-lane registers into 64-byte row
 // segments.
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 
@@ -123,9 +124,8 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   // their end, and the packed heads share every K/V tile.
   const int pack = p.pack, BMT = BM / pack;
 
-  if (!p.store_follows) pdl_trigger();
+  pdl_trigger();
   if (!p.lengths_early) pdl_wait();
-  if (p.store_follows) pdl_trigger();
   // Rank the sequences by key length, longest first (ties by index): rank = how many come before.
   if (p.batch <= SORT_BATCH) {
     for (int b = tid; b < p.batch; b += NTHREADS_P) prefix[b] = p.cu_k[b + 1] - p.cu_k[b];  // lengths, for a moment
@@ -358,6 +358,37 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       if (!ok) {  // make sure nothing is still running on TMEM before it is freed
         umma_commit(bar(DRAIN));
         (void)mbar_wait(bar(DRAIN), 0);
+      }
+    }
+   } else if (p.slots) {
+    // -------------------------------------------------- two warps left: the packed K/V rows to the cache
+    // A piece of 16 bytes of a K and a V row per lane, two such at a time: 8 KB in flight per SM move four
+    // prompts of 4096 tokens (134 MB) under the products (a copy kernel beside this one: 288 us, now 284), and
+    // a prompt of 200 tokens needs no second launch (10.5 -> 9.5).
+    const uint32_t per_row = p.hkv * D / 8, total = static_cast<uint32_t>(p.n_new) * per_row, step = gridDim.x * 64;
+    const int64_t n_slots = p.num_blocks * kBlockSize;
+    for (uint32_t i0 = blockIdx.x * 64 + (tid - 320); i0 < total; i0 += 2 * step) {
+      uint4 kreg[2], vreg[2];
+      int64_t dst[2];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const uint32_t i = i0 + u * step, tok = i / per_row, piece = i - tok * per_row;
+        dst[u] = -1;
+        if (i >= total) continue;
+        const int64_t slot = p.slots[tok];
+        if (slot >= n_slots) {
+          if (piece == 0) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
+        } else if (slot >= 0) {
+          dst[u] = slot * per_row + piece;
+        }
+        kreg[u] = __ldg(reinterpret_cast<const uint4*>(p.k + tok * p.k_stride) + piece);
+        vreg[u] = __ldg(reinterpret_cast<const uint4*>(p.v + tok * p.v_stride) + piece);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        if (dst[u] < 0) continue;
+        reinterpret_cast<uint4*>(p.k_store)[dst[u]] = kreg[u];
+        reinterpret_cast<uint4*>(p.v_store)[dst[u]] = vreg[u];
       }
     }
    }
@@ -598,7 +629,9 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   const int64_t max_items = static_cast<int64_t>((p.max_seqlen_q + bmt - 1) / bmt) * (p.hq / pack) * p.batch;
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
-  if (max_items < grid) grid = static_cast<int>(max_items);
+  // and, where rows are to be stored, enough of them to do that in a few trips
+  const int64_t store_blocks = (p.n_new * p.hkv * (D / 8) + 255) / 256;
+  grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, store_blocks)));
   // the two head_dim instantiations share the counter array: give each its own half
   const int slot = static_cast<int>(launch_seq.fetch_add(1) % (tcp::NUM_SLOTS / 2)) + (D == 64 ? tcp::NUM_SLOTS / 2 : 0);
   return launch_kernel("prefill (tcgen05, persistent)", prefill_tcp_kernel<D>, dim3(grid), dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq,

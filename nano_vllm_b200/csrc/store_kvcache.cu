@@ -8,25 +8,16 @@ namespace nvllm {
 
 constexpr int kStoreThreads = 256;
 constexpr int kStoreUnroll = 2;  // 16-byte pieces per thread per tensor
-// Beside the prefill kernel, whose two blocks leave an SM 4096 registers: blocks of 128 threads with 32
-// registers, one piece per tensor.
-constexpr int kBesideThreads = 128;
-constexpr int kBesideUnroll = 1;
 
-// BESIDE: the previous kernel in the stream neither writes what is read here nor touches the cache, and
-// let this one start only after its own pdl_wait(): the copy runs under it.
-template <bool BESIDE>
-__global__ void __launch_bounds__(BESIDE ? kBesideThreads : kStoreThreads, BESIDE ? 16 : 1)
+__global__ void __launch_bounds__(kStoreThreads)
 store_kvcache_kernel(const uint4* __restrict__ key, int64_t key_stride16,      // row strides in 16-byte units
                      const uint4* __restrict__ value, int64_t value_stride16,
                      uint4* __restrict__ k_cache, uint4* __restrict__ v_cache,
                      const int32_t* __restrict__ slot_mapping,
                      int64_t n_tokens, int pieces_per_row, int64_t num_slots, int* __restrict__ status) {
-  constexpr int THREADS = BESIDE ? kBesideThreads : kStoreThreads, UNROLL = BESIDE ? kBesideUnroll : kStoreUnroll;
-  if constexpr (!BESIDE) {
-    pdl_wait();
-    pdl_trigger();  // after the wait: the attention kernel that follows may read its metadata early
-  }
+  constexpr int THREADS = kStoreThreads, UNROLL = kStoreUnroll;
+  pdl_wait();
+  pdl_trigger();  // after the wait: the attention kernel that follows may read its metadata early
   const int64_t total = n_tokens * pieces_per_row;
   const int64_t base = (static_cast<int64_t>(blockIdx.x) * THREADS) * UNROLL + threadIdx.x;
 
@@ -56,16 +47,10 @@ store_kvcache_kernel(const uint4* __restrict__ key, int64_t key_stride16,      /
       v_cache[dst[u]] = vreg[u];
     }
   }
-  if constexpr (BESIDE) {
-    // The next kernel may take this one's end for the end of both.  One block is enough for that, the last:
-    // a block that waits keeps the place of those that still have rows to copy
-    // (all of them waiting: four 4096-token prompts 302 us instead of 295).
-    if (blockIdx.x == gridDim.x - 1) pdl_wait();
-  }
 }
 
 // launch == false: argument checks only.
-int store_kvcache(bool launch, bool beside, const void* key, int64_t key_row_stride, const void* value, int64_t value_row_stride,
+int store_kvcache(bool launch, const void* key, int64_t key_row_stride, const void* value, int64_t value_row_stride,
                   void* k_cache, void* v_cache, const int32_t* slot_mapping, int64_t n_tokens, int32_t row_elems,
                   int64_t num_slots, void* stream) {
   if (n_tokens < 0) return fail(NVLLM_E_GEOMETRY, "store_kvcache: n_tokens=%lld < 0", (long long)n_tokens);
@@ -88,13 +73,11 @@ int store_kvcache(bool launch, bool beside, const void* key, int64_t key_row_str
 
   const int pieces = row_elems / 8;
   const int64_t total = n_tokens * pieces;
-  const int threads = beside ? kBesideThreads : kStoreThreads;
-  const int64_t per_block = static_cast<int64_t>(threads) * (beside ? kBesideUnroll : kStoreUnroll);
+  const int64_t per_block = kStoreThreads * kStoreUnroll;
   const int64_t blocks = (total + per_block - 1) / per_block;
   if (blocks > 0x7fffffffLL) return fail(NVLLM_E_GEOMETRY, "store_kvcache: too many tokens for one launch");
   if (!launch) return NVLLM_OK;
-  return launch_kernel("store_kvcache", beside ? store_kvcache_kernel<true> : store_kvcache_kernel<false>,
-                       dim3(static_cast<unsigned>(blocks)), dim3(threads), 0, static_cast<cudaStream_t>(stream),
+  return launch_kernel("store_kvcache", store_kvcache_kernel, dim3(static_cast<unsigned>(blocks)), dim3(kStoreThreads), 0, static_cast<cudaStream_t>(stream),
                        static_cast<const uint4*>(key), key_row_stride / 8, static_cast<const uint4*>(value), value_row_stride / 8,
                        static_cast<uint4*>(k_cache), static_cast<uint4*>(v_cache), slot_mapping, n_tokens, pieces, num_slots,
                        status);
@@ -107,6 +90,6 @@ extern "C" int nvllm_store_kvcache(const void* key, int64_t key_row_stride,
                                    void* k_cache, void* v_cache,
                                    const int32_t* slot_mapping, int64_t n_tokens,
                                    int32_t row_elems, int64_t num_slots, void* stream) {
-  return nvllm::store_kvcache(true, false, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_tokens,
+  return nvllm::store_kvcache(true, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, n_tokens,
                               row_elems, num_slots, stream);
 }

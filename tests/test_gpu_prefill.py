@@ -3,7 +3,7 @@ import pytest
 import torch
 
 from conftest import assert_close_to_oracle
-from nano_vllm_b200 import _lib, attention as A, workloads as W
+from nano_vllm_b200 import _lib, attention as A, context as C, workloads as W
 from oracle import paged_attention_ref as R
 
 pytestmark = pytest.mark.gpu
@@ -97,6 +97,36 @@ def test_every_prefill_kernel_on_the_same_case(cuda, monkeypatch, impl, d):
     _check(cuda, case, f"{impl} d{d} prefix")
     case = W.make_prefill_case(27, 5, 1, 1, 8, 8, d, share_every=0, lengths=[257, 2, 900, 128, 64])
     _check(cuda, case, f"{impl} d{d} packed")
+
+
+@pytest.mark.parametrize("impl", ["", "mma"])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64), (3, 3, 64)])
+@pytest.mark.parametrize("lengths", [[1], [63, 1, 130], [3000, 2500]])
+def test_layer_stores_packed_rows_as_the_store_does(cuda, monkeypatch, impl, hq, hkv, d, lengths):
+    """The prefill's own copy of the rows into the cache: fewer rows than lanes, several trips, K and V of
+    different strides, rows without a slot, a slot past the cache."""
+    monkeypatch.setenv("NVLLM_PREFILL_IMPL", impl)
+    dev = W.make_prefill_case(41, len(lengths), 1, 1, hq, hkv, d, lengths=lengths, share_every=0).to(cuda)
+    n = dev.q.shape[0]
+    qkv = torch.cat([dev.q.view(n, -1), dev.k.view(n, -1), dev.v.view(n, -1)], dim=1)
+    q, k, v = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+    v = v.contiguous()
+    slots = dev.slot_mapping.clone()
+    slots[n // 3::7] = -1
+    layer = A.Attention(hq, d, dev.scale, hkv)
+    layer.k_cache, layer.v_cache = dev.k_cache.clone(), dev.v_cache.clone()
+    k2, v2 = dev.k_cache.clone(), dev.v_cache.clone()
+    for status in (0, 1):
+        C.set_context(True, dev.cu_seqlens_q, dev.cu_seqlens_k, dev.max_seqlen_q, dev.max_seqlen_k, slots, None, None)
+        got = layer(q, k, v)
+        C.reset_context()
+        A.store_kvcache(dev.k, dev.v, k2, v2, torch.where(slots < k2.shape[0] * 256, slots, -1))
+        want = A.prefill_varlen(dev.q, dev.k, dev.v, dev.cu_seqlens_q, dev.cu_seqlens_k, dev.max_seqlen_q, dev.max_seqlen_k, dev.scale)
+        torch.cuda.synchronize()
+        assert torch.equal(got.view_as(want), want)
+        assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+        assert _lib.read_status() == status
+        slots[n - 1] = k2.shape[0] * 256  # NVLLM_STATUS_BAD_SLOT the second time
 
 
 def test_many_sequences_through_the_persistent_kernel(cuda):
