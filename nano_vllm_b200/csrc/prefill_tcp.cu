@@ -55,7 +55,7 @@ constexpr int SORT_BATCH = 256;  // batches up to this size are ranked by length
 enum PBar {
   ITEM_FULL0 = tc::NUM_BARS, ITEM_FULL1, ITEM_FREE0, ITEM_FREE1, O_FREE, EPI_FULL0, EPI_FULL1, P_NUM_BARS
 };
-// Twelve warps in three groups of four: softmax, epilogue, and (TMA producer, MMA issuer, two idle).
+// Twelve warps in three groups of four: softmax, epilogue, and (TMA producer, MMA issuer, two that copy rows).
 // Registers are handed over between the groups at start-up (setmaxnreg): two blocks of 384 threads
 // per SM leave 80 per thread at launch; the softmax rows need about twice that, the other groups
 // a fraction.  128 x (RS + RE + RX) = 384 x 80.
