@@ -216,8 +216,9 @@ NVLLM_API int nvllm_prefill_varlen(const void* q, int64_t q_row_stride,
 /*
  * nvllm_store_kvcache followed by nvllm_decode_paged / nvllm_prefill_varlen, as the attention layer
  * does for every step (nanovllm/layers/attention.py:65-77), with the same arguments and results.
- * Two launches; the attention kernel sums its lengths while the store is still running, which the
- * two separate calls may not do because they do not know what ran before them.  n_new / total_k:
+ * One launch for a decode of up to 32 sequences and for a prefill of packed rows; else two, of which the
+ * second reads its lengths while the first still runs, which two separate calls may not do because
+ * they do not know what ran before them.  n_new / total_k:
  * rows of key / value and entries of slot_mapping (all of them are stored, as by
  * nvllm_store_kvcache: num_slots = 256 * num_blocks).  Prefill reads key / value where
  * block_tables is NULL, and the cache through the table otherwise.

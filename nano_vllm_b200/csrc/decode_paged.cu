@@ -33,7 +33,7 @@
 //     The counters are returned to zero by that block.
 //   * Step variant: the block that streams token ctx-1 of a sequence takes that row from the
 //     new K/V activation instead of the cache (with the same asynchronous copies) and writes it to
-//     its cache slot when the tile is used.
+//     its cache slot when the tile is used.  Layer variant: the same for any slot_mapping, a few rows.
 //
 // Small batches are bound by a chain of trips to memory: lengths, block table, K/V, then for cut
 // sequences partials out, arrival, partials in.  Table lines are fetched under the lengths, the
@@ -42,7 +42,6 @@
 // 6.2 us, one of 4096 20.0 -> 10.7, 8 of 100-1024 16.3 -> 11.9, 16 of them 18.1 -> 14.9, 64 of them
 // 35.3 -> 32.7; 256 sequences of 2048-8192 tokens (32 / 8 heads, step variant) 795 -> 747.
 #include <cstdlib>
-
 #include <type_traits>
 
 #include "common.cuh"

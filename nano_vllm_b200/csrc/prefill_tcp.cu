@@ -9,7 +9,7 @@
 // (128-byte swizzle, no multicast) into a two-stage ring; one tcgen05.commit per MMA group.
 // Twelve warps: 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
 // item's last P V product is done they normalise O and store it while the softmax warps are
-// already in the next item's first tile), warp 8 lane 0 = TMA producer, warp 9 lane 0 = MMA issuer;
+// already in the next item's first tile), warp 8 = TMA producer, warp 9 = MMA issuer (one elected lane each);
 // the three warp groups trade registers at start-up (setmaxnreg) so that two such blocks fit an
 // SM.  A thread block does not end with its query tile: two blocks per SM stay resident
 // for the whole launch, keep their TMEM allocation and barriers, and pull work items (sequence,
