@@ -402,7 +402,10 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     }
     if (!mine) return;
   } else {
-    if (!split(false)) return;
+    if (!split(false)) {
+      if (p.lengths_early) pdl_wait();  // every block waits: where all contexts are empty, none gets to start()
+      return;
+    }
     start();
   }
   // the range that holds global unit u

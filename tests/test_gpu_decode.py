@@ -300,6 +300,41 @@ def test_lengths_written_by_the_kernel_just_before(cuda, batch):
         assert_close_to_oracle(out, ref, f"batch {batch}, lengths to {int(now.max())}")
 
 
+@pytest.mark.parametrize("batch", [33, 129])
+def test_a_batch_of_empty_sequences_completes_after_its_store(cuda, batch):
+    """The layer call of more than 32 sequences that are all empty has no tile to stream.  The launch
+    behind it takes its completion for that of the store as well, here one of 48 MB whose last rows
+    are read: they must be there."""
+    hq, hkv, d = 16, 8, 128
+    case = W.make_decode_case(43, 4, 1, 1, hq, hkv, d, context_lens=[1, 255, 256, 257])
+    dev = case.to(cuda)
+    n_new = 12000
+    slots = torch.full((n_new,), -1, dtype=torch.int32, device=cuda)  # the last rows are tokens of the batch read afterwards
+    slots[-4:] = dev.slot_mapping
+    kv = torch.randn(2, n_new, hkv, d, generator=torch.Generator().manual_seed(batch)).bfloat16().to(cuda)
+    spare = torch.arange(256, dtype=torch.int32, device=cuda) + 256 * dev.k_cache.shape[0]
+    slots[:-4] = spare.repeat(n_new // 256 + 1)[:n_new - 4]
+    kv[:, :-4] = 0  # rows that go to the same slot are the same
+    pad = torch.zeros(1, 256, hkv, d, dtype=torch.bfloat16, device=cuda)
+    layer = A.Attention(hq, d, dev.scale, hkv)
+    layer.k_cache, layer.v_cache = torch.cat([dev.k_cache, pad]), torch.cat([dev.v_cache, pad])
+    zeros = torch.zeros(batch, dtype=torch.int32, device=cuda)
+    q, table = torch.randn(batch, hq * d, device=cuda).bfloat16(), torch.zeros(batch, 16, dtype=torch.int32, device=cuda)
+    for _ in range(3):
+        torch.cuda.synchronize()
+        C.set_context(False, slot_mapping=slots, context_lens=zeros, block_tables=table)
+        empty = layer(q, kv[0].view(n_new, -1), kv[1].view(n_new, -1))
+        C.reset_context()
+        got = A.decode_paged(dev.q, layer.k_cache, layer.v_cache, dev.context_lens, dev.block_tables, dev.scale)
+        torch.cuda.synchronize()
+        assert not empty.any()
+        R.store_kvcache_ref(kv[0, -4:].cpu(), kv[1, -4:].cpu(), case.k_cache, case.v_cache, case.slot_mapping)
+        ref = R.decode_ref(case.q, case.k_cache, case.v_cache, case.context_lens, case.block_tables, case.scale)
+        assert_close_to_oracle(got, ref, f"behind {batch} empty sequences")
+        kv[:, -4:] = -kv[:, -4:]
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("tp", [2, 4, 8])
 def test_head_sharded_ranks_reassemble_the_unsharded_result(cuda, tp):
     """Tensor parallelism: rank r holds query heads [r*Hq/tp, ...) and KV heads [r*Hkv/tp, ...) of
