@@ -590,6 +590,22 @@ void cuda_check(cudaError_t e) {
   if (e != cudaSuccess) raise(PyExc_RuntimeError, std::string("CUDA error: ") + cudaGetErrorString(e));
 }
 
+// Returns when the launch that last read block t is done.  Other threads run while it is still pending, and what
+// they did meanwhile is looked at again: one of them may have staged from the same block.
+void wait_until_read(const Stager& s, int t) {
+  while (s.used[t]) {
+    cudaError_t e = cudaEventQuery(s.read[t]);
+    if (e == cudaSuccess) return;
+    if (e == cudaErrorNotReady) {
+      (void)cudaGetLastError();
+      Py_BEGIN_ALLOW_THREADS
+      e = cudaEventSynchronize(s.read[t]);
+      Py_END_ALLOW_THREADS
+    }
+    cuda_check(e);
+  }
+}
+
 PyObject* make_stager(PyObject* const* a) {  // host block 0, host block 1, device temperatures, max_bs, table_width
   auto s = std::make_unique<Stager>();
   s->host[0] = tensor(a[0], "host block");
@@ -619,7 +635,7 @@ PyObject* stage(PyObject* const* a) {
   require(0 < n0 && n0 <= graph_bs && graph_bs <= s->max_bs, "0 < n <= graph_bs <= self.max_bs");
   const int t = s->turn;
   s->turn ^= 1;
-  if (s->used[t]) cuda_check(cudaEventSynchronize(s->read[t]));  // returns at once unless that launch is still pending
+  wait_until_read(*s, t);
   int64_t end, widest, n;
   pack_into(a[1], ptr<unsigned char>(s->host[t]), s->host[t].numel(), with, a[4], &end, &widest, &n);
   const at::Tensor &ids = tensor(a[5], "input_ids"), &pos = tensor(a[6], "positions"), &slots = tensor(a[7], "slot_mapping"),

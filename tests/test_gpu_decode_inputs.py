@@ -1,6 +1,8 @@
 """Decode-step inputs expanded on the GPU into a graph's static tensors, against the restated
 reference semantics (clear, then copy the first rows; block tables padded with -1)."""
 import random
+import threading
+import time
 
 import numpy as np
 import pytest
@@ -51,6 +53,46 @@ def test_steps_of_changing_batch_size(cuda, width, max_len):
         for k in gv:
             assert (gv[k][touched:] == 7).all(), f"{k}: rows beyond the graph's batch were written"
     assert _lib.read_status() == 0
+
+
+def _ticking(fn):
+    """Runs fn beside a thread that counts; returns fn's seconds and how often the thread ran meanwhile."""
+    count, stop = 0, threading.Event()
+
+    def tick():
+        nonlocal count
+        while not stop.is_set():
+            count += 1
+            time.sleep(1e-3)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        time.sleep(0.02)
+        before, t0 = count, time.perf_counter()
+        fn()
+        return time.perf_counter() - t0, count - before
+    finally:
+        stop.set()
+        thread.join()
+
+
+def test_other_threads_run_while_a_step_waits_for_its_block(cuda):
+    """A third step waits for the launch that reads the first one's block; the interpreter does not."""
+    gv = _graph_vars(cuda, 16, 16, 0)
+    stager = DI.DecodeInputStager(16, 16, cuda)
+    steps = [make_seqs(random.Random(i), 16, max_len=4096) for i in range(3)]
+    stager.stage(steps[0], 16, gv)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(600_000_000)  # a third of a second in front of the launches
+    stager.stage(steps[0], 16, gv)
+    stager.stage(steps[1], 16, gv)
+    seconds, ticks = _ticking(lambda: stager.stage(steps[2], 16, gv))
+    torch.cuda.synchronize()
+    assert seconds > 0.1, "the step did not have to wait"
+    assert ticks > 20 * seconds, f"another thread ran {ticks} times in {seconds:.2f} s"
+    for k, want in R.decode_inputs_ref(steps[2], 16, 16).items():
+        assert np.array_equal(gv[k].cpu().numpy(), want), k
 
 
 def test_bad_arguments_are_refused(cuda, lib):
