@@ -15,10 +15,14 @@
 //     the launch can be captured in a CUDA graph.  Every block derives the split from
 //     context_lens itself (a block-wide scan of the units per sequence), so blocks carry the
 //     same number of bytes whatever the lengths are: no tail of half-empty waves, one ramp-up.
-//   * A thread block has NW warps that do not synchronise with one another while streaming.
-//     Warp w owns the TT-token tile w of every unit and runs its own NST-stage cp.async ring
-//     (16-byte copies, XOR-swizzled rows so ldmatrix is conflict free).  The ring keeps running
-//     across sequence boundaries.  Rows past the end of a context are zero-filled, never read.
+//   * Warp w of a thread block owns the TT-token tile w of every unit and runs its own NST-stage
+//     cp.async ring (16-byte copies, XOR-swizzled rows so ldmatrix is conflict free).  The ring keeps
+//     running across sequence boundaries.  Rows past the end of a context are zero-filled, never read.
+//     The Plain variant has the warps meet at every unit, so that a block's reads stay within a stretch
+//     of memory instead of spreading over as many as it has warps: 256 sequences of 2048-8192 tokens
+//     (32 / 8 heads) 731 -> 717 us in a chain, 805 -> 777 alone behind a flush of L2, one of 8 ranks' shard
+//     of it 133 -> 127, 48 of 32768 (head_dim 64, layer) 126.3 -> 122.7, 512 of 100-1024 (16 / 8 heads) 175.9 ->
+//     176.6.  The Step variant loses by it (786 -> 793 in a chain, 820 -> 839 behind a flush).
 //   * Tensor cores do the dot products with the tokens on the M side so that G <= 8 query
 //     heads fit the N=8 side without padding M: S^T[16 tok x 8 heads] = K[16 x D] Q^T[D x 8]
 //     and O^T[D x 8] += V^T[D x 16] P^T[16 x 8] (mma.sync.m16n8k16, bf16 in / fp32 out).
@@ -603,7 +607,8 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       load_q(qn, qn_b);
     }
     cp_async_wait<NST - 2>();
-    __syncwarp();
+    if (V == Variant::Plain) __syncthreads();  // the warps' tiles of a unit are fetched together
+    else __syncwarp();
     if (i + NST - 1 < n_units) {
       seek(pc, u + NST - 1);
       load_tile(pc, u + NST - 1, (i + NST - 1) % NST);
