@@ -301,6 +301,11 @@ NVLLM_API int nvllm_sample_candidates(const void* logits, int32_t logits_are_fp3
                             int32_t batch, int32_t vocab, void* stream);
 NVLLM_API int nvllm_sample_unpack(const int64_t* candidates, int64_t* tokens, int32_t batch, void* stream);
 
+/* Thread blocks (one cluster) that read a row on a device with num_sms multiprocessors whose largest
+ * cluster is largest_cluster: 16 where the device grants it, never more than the portable 8 where it does
+ * not.  Host arithmetic, exposed for tests and reports. */
+NVLLM_API int nvllm_sample_plan(int32_t batch, int32_t vocab, int32_t num_sms, int32_t largest_cluster);
+
 /*
  * Decode-step inputs for a captured CUDA graph, in one launch.  `staged` is a device copy of
  * one host staging block holding, at the given BYTE offsets: tokens int64[batch] (last token of

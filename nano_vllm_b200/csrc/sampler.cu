@@ -47,6 +47,7 @@
 // index.  nvllm_sample_unpack turns the winning candidates into token ids.
 #include <cooperative_groups.h>
 
+#include <atomic>
 #include <type_traits>
 #include <utility>
 
@@ -412,11 +413,62 @@ __global__ void sample_unpack_kernel(const long long* packed, int64_t* tokens, i
   tokens[b] = candidate_index(packed[b]);
 }
 
+constexpr int kThreads = 256, kPortableCluster = 8;
+
+// Blocks per row: as few (1, 2, 4, 8) as give every SM three blocks, since every block pays its start
+// and its merge; more would only help the balance, fewer leave the SMs short of warps (measured at
+// batch 1 to 512).  Sixteen where that is still no more than one block per SM (batch 1: 8.7 us, 10.8 with
+// eight; beyond, clusters of sixteen crowd on a part of the chip: 19.0 for 14.5 at batch 32) and the device
+// can hold such a cluster.  No more than the row has work for.
+static int blocks_per_row(int batch, int vocab, int sms, int largest) {
+  int csize = 1;
+  auto fits = [&](int c, int64_t most) { return vocab >= c * kThreads * 8 && static_cast<int64_t>(batch) * c <= most; };
+  while (csize < kPortableCluster && static_cast<int64_t>(batch) * csize < 3ll * sms && fits(2 * csize, INT64_MAX)) csize *= 2;
+  if (csize == kPortableCluster && largest >= kMaxCluster && fits(kMaxCluster, sms)) csize = kMaxCluster;
+  return csize;
+}
+
+// The largest cluster the current device takes: more than the portable eight has to be allowed, and then be
+// possible with the SMs that this process has (asked once per device and kernel).
+template <typename T>
+static int largest_cluster() {
+  static std::atomic<int> known[64];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+    (void)cudaGetLastError();
+    return kPortableCluster;
+  }
+  int largest = known[dev].load(std::memory_order_acquire);
+  if (largest) return largest;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kMaxCluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(kMaxCluster, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int clusters = 0;
+  const bool possible = cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
+                        cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<T>, &cfg) == cudaSuccess && clusters > 0;
+  if (!possible) (void)cudaGetLastError();
+  largest = possible ? kMaxCluster : kPortableCluster;
+  known[dev].store(largest, std::memory_order_release);
+  return largest;
+}
+
 static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t row_stride, const float* temperatures,
                          const float* exponential_noise, int64_t noise_row_stride, uint64_t seed, uint64_t step,
                          int64_t vocab_offset, int candidates, int64_t* tokens, int32_t batch, int32_t vocab, void* stream);
 
 }  // namespace nvllm
+
+extern "C" int nvllm_sample_plan(int32_t batch, int32_t vocab, int32_t num_sms, int32_t largest_cluster) {
+  using namespace nvllm;
+  if (batch < 0 || vocab <= 0 || num_sms <= 0) return fail(NVLLM_E_GEOMETRY, "sample_plan: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
+  return blocks_per_row(batch, vocab, num_sms, largest_cluster);
+}
 
 extern "C" int nvllm_sample_tokens(const void* logits, int32_t logits_are_fp32, int64_t row_stride,
                                    const float* temperatures, const float* exponential_noise, int64_t noise_row_stride,
@@ -478,36 +530,17 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   p.candidates = candidates;
   const int sms = num_sms();
   if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: no CUDA device is usable");
-  // Blocks per row: as few (1, 2, 4, 8) as give every SM three blocks, since every block pays its start
-  // and its merge; more would only help the balance, fewer leave the SMs short of warps (measured at
-  // batch 1 to 512).  Sixteen where that is still no more than one block per SM (batch 1: 8.7 us, 10.8 with
-  // eight; beyond, clusters of sixteen crowd on a part of the chip: 19.0 for 14.5 at batch 32).  No
-  // more than the row has work for.
-  int csize = 1;
-  auto fits = [&](int c, int64_t most) { return vocab >= c * 256 * 8 && static_cast<int64_t>(batch) * c <= most; };
-  while (csize < 8 && static_cast<int64_t>(batch) * csize < 3ll * sms && fits(2 * csize, INT64_MAX)) csize *= 2;
-  if (csize == 8 && fits(16, sms)) csize = 16;
+  const int csize = blocks_per_row(batch, vocab, sms, logits_are_fp32 ? largest_cluster<float>() : largest_cluster<__nv_bfloat16>());
   const int64_t blocks = static_cast<int64_t>(batch) * csize;
   // Launched under the end of the kernel before (1.5 us less), except for grids of about one or two blocks
   // per SM, which then land unevenly on the SMs that happen to be free (17.8 us for 14.5 at batch 32).
   const bool early = 2 * blocks <= sms || blocks >= 3ll * sms;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(blocks), 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = static_cast<cudaStream_t>(stream);
   auto kernel = logits_are_fp32 ? sample_kernel<float> : sample_kernel<__nv_bfloat16>;
-  if (csize > 8) {  // more than the portable cluster size has to be asked for, once per device and kernel
-    static bool allowed[2][64] = {};
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (dev < 0 || dev >= 64) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: device index %d out of range", dev);
-    if (!allowed[logits_are_fp32 ? 1 : 0][dev]) {
-      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "sample_tokens: set-up failed: %s", cudaGetErrorString(e));
-      allowed[logits_are_fp32 ? 1 : 0][dev] = true;
-    }
-  }
   cudaLaunchAttribute attr[2];
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;

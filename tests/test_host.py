@@ -126,6 +126,17 @@ def test_all_reduce_protocol_choice_is_host_arithmetic(lib):
     assert protocol_for(2 << 20, 8, mb, forced=1) == "cells-two-shot"  # cells to every peer do not fit: 2 x 2 MiB x 8 > 8 MiB
 
 
+@pytest.mark.parametrize("sms", [148, 132, 20])
+def test_sampler_takes_no_larger_cluster_than_the_device_grants(lib, sms):
+    """Sixteen blocks to a row for the fewest rows where that is possible, else eight; the same plan
+    for larger batches and rows too short for it."""
+    for batch in (1, 2, 9, 10, 32, 64, 256, 512):
+        for vocab in (7, 2047, 4096, 16384, 32768, 151936):
+            wide, portable = lib.nvllm_sample_plan(batch, vocab, sms, 16), lib.nvllm_sample_plan(batch, vocab, sms, 8)
+            assert portable in (1, 2, 4, 8) and wide == (16 if batch * 16 <= sms and vocab >= 16 * 2048 else portable)
+    assert lib.nvllm_sample_plan(1, 151936, sms, 8) == 8 and lib.nvllm_sample_plan(1, 0, sms, 8) == -3
+
+
 def test_fused_projection_tile_choice_is_host_arithmetic(lib):
     """Tile width of the projection fused with its all-reduce: the narrowest of 32 / 64 / 128 columns
     that leaves one tile per thread block (128 blocks), 0 for shapes the kernel refuses."""
