@@ -579,9 +579,18 @@ struct Stager {
   bool used[2] = {false, false};
   int turn = 0;
   int64_t max_bs, width;
+  // A launch that is still pending reads its block, which goes back to the pinned allocator with this object.
   ~Stager() {
-    for (cudaEvent_t e : read)
-      if (e) cudaEventDestroy(e);
+    for (int t = 0; t < 2; ++t) {
+      if (!read[t]) continue;
+      if (used[t] && cudaEventQuery(read[t]) == cudaErrorNotReady) {
+        Py_BEGIN_ALLOW_THREADS
+        cudaEventSynchronize(read[t]);
+        Py_END_ALLOW_THREADS
+      }
+      cudaEventDestroy(read[t]);
+    }
+    (void)cudaGetLastError();
   }
 };
 constexpr const char* kStagerName = "nano_vllm_b200.stager";

@@ -95,6 +95,25 @@ def test_other_threads_run_while_a_step_waits_for_its_block(cuda):
         assert np.array_equal(gv[k].cpu().numpy(), want), k
 
 
+def test_a_step_outlives_its_stager(cuda):
+    """The launch reads the pinned block itself: dropped while it is pending, the block must not serve
+    another allocation before that."""
+    gv = _graph_vars(cuda, 512, 16, 0)
+    stager = DI.DecodeInputStager(512, 16, cuda)
+    seqs = make_seqs(random.Random(3), 512, max_len=4096)
+    stager.stage(seqs, 512, gv)
+    torch.cuda.synchronize()
+    nbytes = stager.host[0].numel()
+    torch.cuda._sleep(600_000_000)
+    stager.stage(seqs, 512, {k: v.zero_() for k, v in gv.items()})
+    del stager
+    others = [torch.zeros(nbytes, dtype=torch.uint8, pin_memory=True) for _ in range(4)]
+    torch.cuda.synchronize()
+    for k, want in R.decode_inputs_ref(seqs, 512, 16).items():
+        assert np.array_equal(gv[k].cpu().numpy(), want), k
+    assert not any(o.any() for o in others)
+
+
 def test_bad_arguments_are_refused(cuda, lib):
     gv = _graph_vars(cuda, 16, 16, 0)
     staged = torch.zeros(4096, dtype=torch.uint8, device=cuda)
