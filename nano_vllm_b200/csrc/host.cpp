@@ -115,6 +115,24 @@ void check(int64_t code) {
   if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "nvllm call failed");
   throw PyErrorSet{};
 }
+// What may wait for the device runs without the interpreter lock, as a ctypes call or a torch operation does: a
+// launch waits while the device's queue is full and an allocation may wait for all that is in front of it,
+// which other threads of the program may have to finish.
+template <class F>
+auto unlocked(F&& f) {
+  struct Unlock {
+    PyThreadState* state = PyEval_SaveThread();
+    ~Unlock() { PyEval_RestoreThread(state); }
+  } unlock;
+  return f();
+}
+template <class F>
+void launch(F&& f) {
+  check(unlocked(f));
+}
+at::Tensor new_tensor(at::IntArrayRef sizes, const at::TensorOptions& options) {
+  return unlocked([&] { return at::empty(sizes, options); });
+}
 template <class T>
 T* ptr(const at::Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
@@ -133,11 +151,15 @@ void workspace(const at::Tensor& like, int64_t nbytes, void** p, int64_t* size) 
   if (nbytes == 0) return;
   const size_t dev = static_cast<size_t>(like.device().index());
   if (g_workspaces.size() <= dev) g_workspaces.resize(dev + 1);
-  at::Tensor& ws = g_workspaces[dev];
-  if (!ws.defined() || ws.numel() < nbytes) {
-    if (ws.defined()) g_retired.push_back(ws);
-    ws = at::zeros({std::max<int64_t>(nbytes, 1 << 20)}, like.options().dtype(at::kByte));
+  auto enough = [&] { return g_workspaces[dev].defined() && g_workspaces[dev].numel() >= nbytes; };
+  if (!enough()) {
+    at::Tensor fresh = unlocked([&] { return at::zeros({std::max<int64_t>(nbytes, 1 << 20)}, like.options().dtype(at::kByte)); });
+    if (!enough()) {  // not grown by another thread meanwhile
+      if (g_workspaces[dev].defined()) g_retired.push_back(g_workspaces[dev]);
+      g_workspaces[dev] = std::move(fresh);
+    }
   }
+  const at::Tensor& ws = g_workspaces[dev];
   *p = ws.data_ptr();
   *size = ws.numel();
 }
@@ -162,8 +184,10 @@ void check_store(const Rows& k, int64_t row, const at::Tensor& k_cache, const at
 void store(const Rows& k, const Rows& v, int64_t row, const at::Tensor& k_cache, const at::Tensor& v_cache,
            const at::Tensor& slot_mapping) {
   check_store(k, row, k_cache, v_cache, slot_mapping);
-  check(api.store_kvcache(k.p, k.stride, v.p, v.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(slot_mapping), k.n,
-                          static_cast<int32_t>(row), k_cache.numel() / row, stream_of(k_cache)));
+  launch([&] {
+    return api.store_kvcache(k.p, k.stride, v.p, v.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(slot_mapping),
+                             k.n, static_cast<int32_t>(row), k_cache.numel() / row, stream_of(k_cache));
+  });
 }
 
 struct Step {  // the new tokens' rows, for a call that stores as well
@@ -195,18 +219,25 @@ void decode(const Rows& q, int64_t hq, int64_t d, const at::Tensor& k_cache, con
                 D = static_cast<int32_t>(d);
   void* st = stream_of(k_cache);
   if (step && !step->one_launch)
-    check(api.attention_decode(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots, step->k.n,
-                               k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens), ptr<int32_t>(block_tables),
-                               block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D, static_cast<float>(scale),
-                               num_blocks, ws, ws_size, st));
+    launch([&] {
+      return api.attention_decode(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots, step->k.n,
+                                  k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens),
+                                  ptr<int32_t>(block_tables), block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D,
+                                  static_cast<float>(scale), num_blocks, ws, ws_size, st);
+    });
   else if (step)
-    check(api.decode_step(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots, k_cache.data_ptr(),
-                          v_cache.data_ptr(), ptr<int32_t>(context_lens), ptr<int32_t>(block_tables), block_tables.stride(0),
-                          width, out.p, out.stride, B, HQ, HKV, D, static_cast<float>(scale), num_blocks, ws, ws_size, st));
+    launch([&] {
+      return api.decode_step(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots,
+                             k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens), ptr<int32_t>(block_tables),
+                             block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D, static_cast<float>(scale),
+                             num_blocks, ws, ws_size, st);
+    });
   else
-    check(api.decode_paged(q.p, q.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens),
-                           ptr<int32_t>(block_tables), block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D,
-                           static_cast<float>(scale), num_blocks, ws, ws_size, st));
+    launch([&] {
+      return api.decode_paged(q.p, q.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(context_lens),
+                              ptr<int32_t>(block_tables), block_tables.stride(0), width, out.p, out.stride, B, HQ, HKV, D,
+                              static_cast<float>(scale), num_blocks, ws, ws_size, st);
+    });
 }
 
 // K/V of a prefill: packed rows, or the cache planes with a block table.
@@ -235,22 +266,26 @@ void prefill(const Rows& q, int64_t hq, int64_t d, const KV& kv, const at::Tenso
   if (bt)
     require(bt->dim() == 2 && bt->size(0) == batch, "block_tables.dim() == 2 and block_tables.shape[0] == batch");
   if (step) {
-    check(api.attention_prefill(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots,
-                                k_cache->data_ptr(), v_cache->data_ptr(), bt ? ptr<int32_t>(*bt) : nullptr, bt ? bt->stride(0) : 0,
-                                bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride, ptr<int32_t>(cu_q),
-                                ptr<int32_t>(cu_k), q.n, step->k.n, static_cast<int32_t>(batch), static_cast<int32_t>(max_q),
-                                static_cast<int32_t>(max_k), static_cast<int32_t>(hq), static_cast<int32_t>(kv.hkv),
-                                static_cast<int32_t>(d), static_cast<float>(scale),
-                                k_cache->numel() / (NVLLM_BLOCK_SIZE * kv.hkv * d), stream));
+    launch([&] {
+      return api.attention_prefill(q.p, q.stride, step->k.p, step->k.stride, step->v.p, step->v.stride, step->slots,
+                                   k_cache->data_ptr(), v_cache->data_ptr(), bt ? ptr<int32_t>(*bt) : nullptr,
+                                   bt ? bt->stride(0) : 0, bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride,
+                                   ptr<int32_t>(cu_q), ptr<int32_t>(cu_k), q.n, step->k.n, static_cast<int32_t>(batch),
+                                   static_cast<int32_t>(max_q), static_cast<int32_t>(max_k), static_cast<int32_t>(hq),
+                                   static_cast<int32_t>(kv.hkv), static_cast<int32_t>(d), static_cast<float>(scale),
+                                   k_cache->numel() / (NVLLM_BLOCK_SIZE * kv.hkv * d), stream);
+    });
     return;
   }
   if (q.n == 0 || batch == 0) return;
-  check(api.prefill_varlen(q.p, q.stride, kv.k.p, kv.k.stride, kv.v.p, kv.v.stride, bt ? ptr<int32_t>(*bt) : nullptr,
-                           bt ? bt->stride(0) : 0, bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride,
-                           ptr<int32_t>(cu_q), ptr<int32_t>(cu_k), q.n, kv.k.n, static_cast<int32_t>(batch),
-                           static_cast<int32_t>(max_q), static_cast<int32_t>(max_k), static_cast<int32_t>(hq),
-                           static_cast<int32_t>(kv.hkv), static_cast<int32_t>(d), static_cast<float>(scale), kv.num_blocks,
-                           stream));
+  launch([&] {
+    return api.prefill_varlen(q.p, q.stride, kv.k.p, kv.k.stride, kv.v.p, kv.v.stride, bt ? ptr<int32_t>(*bt) : nullptr,
+                              bt ? bt->stride(0) : 0, bt ? static_cast<int32_t>(bt->size(1)) : 0, out.p, out.stride,
+                              ptr<int32_t>(cu_q), ptr<int32_t>(cu_k), q.n, kv.k.n, static_cast<int32_t>(batch),
+                              static_cast<int32_t>(max_q), static_cast<int32_t>(max_k), static_cast<int32_t>(hq),
+                              static_cast<int32_t>(kv.hkv), static_cast<int32_t>(d), static_cast<float>(scale), kv.num_blocks,
+                              stream);
+  });
 }
 
 // [n, heads, d] argument of a functional entry point.
@@ -260,7 +295,7 @@ Rows rows3(const at::Tensor& t, const char* what) {
 }
 
 at::Tensor output_for(PyObject* out, const at::Tensor& q, Rows* rows) {
-  at::Tensor o = out == Py_None ? at::empty(q.sizes(), q.options()) : tensor(out, "out");
+  at::Tensor o = out == Py_None ? new_tensor(q.sizes(), q.options()) : tensor(out, "out");
   require(o.dim() == 3 && o.stride(-1) == 1 && o.stride(1) == q.size(2), "out.stride(-1) == 1 and out.stride(1) == D");
   *rows = {o.data_ptr(), o.size(0), o.stride(0)};
   return o;
@@ -410,7 +445,7 @@ PyObject* attention_forward(PyObject* const* a) {
       store(kr, vr, hkv * d, k_cache, v_cache, sm);
     }
   }
-  at::Tensor out = at::empty({qr.n, hq * d}, q.options());
+  at::Tensor out = new_tensor({qr.n, hq * d}, q.options());
   const Rows o = {out.data_ptr(), qr.n, hq * d};
   if (prefill_phase) {
     Ref cq(PyObject_GetAttr(ctx, names.cu_seqlens_q)), ck(PyObject_GetAttr(ctx, names.cu_seqlens_k));
@@ -462,11 +497,14 @@ PyObject* qk_norm_rope_store(PyObject* const* a) {
       sm = ptr<int32_t>(*slots);
     }
   }
+  const float eps = static_cast<float>(as_double(a[5]));
   const c10::cuda::CUDAGuard guard(qkv.device());
-  check(api.qk_norm_rope_store(qkv.data_ptr(), qkv.stride(0), ptr<int64_t>(positions), qw ? qw->data_ptr() : nullptr,
-                               kw ? kw->data_ptr() : nullptr, ptr<float>(cs), cs.numel() / d, static_cast<float>(as_double(a[5])),
-                               sm, kc, vc, num_slots, qkv.size(0), static_cast<int32_t>(hq), static_cast<int32_t>(hkv),
-                               static_cast<int32_t>(d), stream_of(qkv)));
+  launch([&] {
+    return api.qk_norm_rope_store(qkv.data_ptr(), qkv.stride(0), ptr<int64_t>(positions), qw ? qw->data_ptr() : nullptr,
+                                  kw ? kw->data_ptr() : nullptr, ptr<float>(cs), cs.numel() / d, eps, sm, kc, vc, num_slots,
+                                  qkv.size(0), static_cast<int32_t>(hq), static_cast<int32_t>(hkv), static_cast<int32_t>(d),
+                                  stream_of(qkv));
+  });
   Py_RETURN_NONE;
 }
 
@@ -485,18 +523,23 @@ PyObject* sample(PyObject* const* a, bool candidates) {
     require(noise->is_cuda() && noise->scalar_type() == at::kFloat && noise->sizes() == logits.sizes() && noise->stride(-1) == 1,
             "noise must be CUDA float32 of the logits' shape");
   const c10::cuda::CUDAGuard guard(logits.device());
-  at::Tensor out = a[5] == Py_None ? at::empty({B}, logits.options().dtype(at::kLong)) : tensor(a[5], "out");
+  at::Tensor out = a[5] == Py_None ? new_tensor({B}, logits.options().dtype(at::kLong)) : tensor(a[5], "out");
   require(out.is_cuda() && out.scalar_type() == at::kLong && out.numel() == B && out.is_contiguous(),
           "out must be contiguous CUDA int64, one per row");
   const float* nz = noise ? ptr<float>(*noise) : nullptr;
   const int64_t nzs = noise ? noise->stride(0) : 0;
   const uint64_t seed = as_u64(a[3]), step = as_u64(a[4]);
+  const int64_t offset = candidates ? as_i64(a[6]) : 0;
   if (candidates)
-    check(api.sample_candidates(logits.data_ptr(), fp32, logits.stride(0), ptr<float>(temps), nz, nzs, seed, step, as_i64(a[6]),
-                                ptr<int64_t>(out), static_cast<int32_t>(B), static_cast<int32_t>(V), stream_of(logits)));
+    launch([&] {
+      return api.sample_candidates(logits.data_ptr(), fp32, logits.stride(0), ptr<float>(temps), nz, nzs, seed, step, offset,
+                                   ptr<int64_t>(out), static_cast<int32_t>(B), static_cast<int32_t>(V), stream_of(logits));
+    });
   else
-    check(api.sample_tokens(logits.data_ptr(), fp32, logits.stride(0), ptr<float>(temps), nz, nzs, seed, step, ptr<int64_t>(out),
-                            static_cast<int32_t>(B), static_cast<int32_t>(V), stream_of(logits)));
+    launch([&] {
+      return api.sample_tokens(logits.data_ptr(), fp32, logits.stride(0), ptr<float>(temps), nz, nzs, seed, step,
+                               ptr<int64_t>(out), static_cast<int32_t>(B), static_cast<int32_t>(V), stream_of(logits));
+    });
   return wrap(std::move(out));
 }
 PyObject* sample_tokens(PyObject* const* a) { return sample(a, false); }
@@ -655,11 +698,14 @@ PyObject* stage(PyObject* const* a) {
   const bool temps = with || a[4] != Py_None;
   const c10::cuda::CUDAGuard guard(s->temperatures.device());
   void* st = stream_of(s->temperatures);
-  check(api.decode_step_inputs_pinned(s->host[t].data_ptr(), off.tokens, off.lens, off.offsets, off.blocks, off.temperatures,
-                                      temps ? ptr<float>(s->temperatures) : nullptr, static_cast<int32_t>(n),
-                                      static_cast<int32_t>(graph_bs), static_cast<int32_t>(widest),
-                                      static_cast<int32_t>(s->width), ptr<int64_t>(ids), ptr<int64_t>(pos), ptr<int32_t>(slots),
-                                      ptr<int32_t>(lens), ptr<int32_t>(bt), bt.stride(0), st));
+  launch([&] {
+    return api.decode_step_inputs_pinned(s->host[t].data_ptr(), off.tokens, off.lens, off.offsets, off.blocks,
+                                         off.temperatures, temps ? ptr<float>(s->temperatures) : nullptr,
+                                         static_cast<int32_t>(n), static_cast<int32_t>(graph_bs),
+                                         static_cast<int32_t>(widest), static_cast<int32_t>(s->width), ptr<int64_t>(ids),
+                                         ptr<int64_t>(pos), ptr<int32_t>(slots), ptr<int32_t>(lens), ptr<int32_t>(bt),
+                                         bt.stride(0), st);
+  });
   cuda_check(cudaEventRecord(s->read[t], static_cast<cudaStream_t>(st)));
   s->used[t] = true;
   return wrap(s->temperatures.narrow(0, 0, n));

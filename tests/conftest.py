@@ -1,4 +1,6 @@
 import sys
+import threading
+import time
 from pathlib import Path
 
 import pytest
@@ -38,3 +40,25 @@ def assert_close_to_oracle(out_bf16, ref_fp32, what=""):
     assert not diff.isnan().any(), f"{what}: NaN in output"
     mx, mean = diff.max().item(), diff.mean().item()
     assert mx <= MAX_ABS_TOL and mean <= MEAN_ABS_TOL, f"{what}: max-abs {mx:.4g} mean-abs {mean:.4g}"
+
+
+def ticking(fn):
+    """Runs fn beside a thread that counts; returns fn's seconds and how often the thread ran meanwhile."""
+    count, stop = 0, threading.Event()
+
+    def tick():
+        nonlocal count
+        while not stop.is_set():
+            count += 1
+            time.sleep(1e-3)
+
+    thread = threading.Thread(target=tick)
+    thread.start()
+    try:
+        time.sleep(0.02)
+        before, t0 = count, time.perf_counter()
+        fn()
+        return time.perf_counter() - t0, count - before
+    finally:
+        stop.set()
+        thread.join()

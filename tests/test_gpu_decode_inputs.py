@@ -1,8 +1,6 @@
 """Decode-step inputs expanded on the GPU into a graph's static tensors, against the restated
 reference semantics (clear, then copy the first rows; block tables padded with -1)."""
 import random
-import threading
-import time
 
 import numpy as np
 import pytest
@@ -14,6 +12,7 @@ from pathlib import Path
 sys.path.insert(0, str(Path(__file__).resolve().parent / "golden"))
 import cases as C  # noqa: E402
 
+from conftest import ticking
 from nano_vllm_b200 import _lib, decode_inputs as DI
 from oracle import paged_attention_ref as R
 from test_decode_inputs_host import make_seqs
@@ -55,28 +54,6 @@ def test_steps_of_changing_batch_size(cuda, width, max_len):
     assert _lib.read_status() == 0
 
 
-def _ticking(fn):
-    """Runs fn beside a thread that counts; returns fn's seconds and how often the thread ran meanwhile."""
-    count, stop = 0, threading.Event()
-
-    def tick():
-        nonlocal count
-        while not stop.is_set():
-            count += 1
-            time.sleep(1e-3)
-
-    thread = threading.Thread(target=tick)
-    thread.start()
-    try:
-        time.sleep(0.02)
-        before, t0 = count, time.perf_counter()
-        fn()
-        return time.perf_counter() - t0, count - before
-    finally:
-        stop.set()
-        thread.join()
-
-
 def test_other_threads_run_while_a_step_waits_for_its_block(cuda):
     """A third step waits for the launch that reads the first one's block; the interpreter does not."""
     gv = _graph_vars(cuda, 16, 16, 0)
@@ -87,7 +64,7 @@ def test_other_threads_run_while_a_step_waits_for_its_block(cuda):
     torch.cuda._sleep(600_000_000)  # a third of a second in front of the launches
     stager.stage(steps[0], 16, gv)
     stager.stage(steps[1], 16, gv)
-    seconds, ticks = _ticking(lambda: stager.stage(steps[2], 16, gv))
+    seconds, ticks = ticking(lambda: stager.stage(steps[2], 16, gv))
     torch.cuda.synchronize()
     assert seconds > 0.1, "the step did not have to wait"
     assert ticks > 20 * seconds, f"another thread ran {ticks} times in {seconds:.2f} s"

@@ -3,7 +3,7 @@ restatement of the same control flow."""
 import pytest
 import torch
 
-from conftest import assert_close_to_oracle
+from conftest import assert_close_to_oracle, ticking
 from nano_vllm_b200 import attention as A, context as C, workloads as W
 from oracle import paged_attention_ref as R
 
@@ -52,3 +52,29 @@ def test_prefill_then_decode_through_the_layer(cuda):
     C.reset_context()
     assert_close_to_oracle(o1.view(B, hq, d), ref1, "layer decode")
     assert torch.equal(dev.k_cache.cpu().view(torch.int16), case.k_cache.view(torch.int16))
+
+
+def test_other_threads_run_while_launches_wait_for_the_queue(cuda):
+    """More calls than the device's queue takes while it is busy: the last ones wait, the interpreter does not."""
+    case = W.make_decode_case(33, 2, 1, 1, 16, 8, 128, context_lens=[300, 17])
+    dev = case.to(cuda)
+    layer = A.Attention(16, 128, case.scale, 8)
+    layer.k_cache, layer.v_cache = dev.k_cache, dev.v_cache
+    qkv = [t.view(2, -1) for t in (dev.q, dev.k_new, dev.v_new)]
+    C.set_context(False, slot_mapping=dev.slot_mapping, context_lens=dev.context_lens, block_tables=dev.block_tables)
+    first = layer(*qkv)
+    torch.cuda.synchronize()
+
+    def many():
+        torch.cuda._sleep(1_000_000_000)  # half a second
+        for _ in range(4000):
+            last = layer(*qkv)
+        return last
+
+    seconds, ticks = ticking(many)
+    torch.cuda.synchronize()
+    last = layer(*qkv)
+    C.reset_context()
+    assert seconds > 0.2, "the queue took every launch"
+    assert ticks > 40 * seconds, f"another thread ran {ticks} times in {seconds:.2f} s"
+    assert torch.equal(first, last)
