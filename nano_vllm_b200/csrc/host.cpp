@@ -136,6 +136,8 @@ at::Tensor new_tensor(at::IntArrayRef sizes, const at::TensorOptions& options) {
 template <class T>
 T* ptr(const at::Tensor& t) { return static_cast<T*>(t.data_ptr()); }
 void* stream_of(const at::Tensor& t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+// Rows of row_elems in a cache plane.  None of an empty one: the library refuses the shape that says so.
+int64_t rows_in(const at::Tensor& t, int64_t row_elems) { return row_elems > 0 ? t.numel() / row_elems : 0; }
 PyObject* wrap(at::Tensor t) { return THPVariable_Wrap(std::move(t)); }
 
 // ---- decode scratch ---------------------------------------------------------------------
@@ -186,7 +188,7 @@ void store(const Rows& k, const Rows& v, int64_t row, const at::Tensor& k_cache,
   check_store(k, row, k_cache, v_cache, slot_mapping);
   launch([&] {
     return api.store_kvcache(k.p, k.stride, v.p, v.stride, k_cache.data_ptr(), v_cache.data_ptr(), ptr<int32_t>(slot_mapping),
-                             k.n, static_cast<int32_t>(row), k_cache.numel() / row, stream_of(k_cache));
+                             k.n, static_cast<int32_t>(row), rows_in(k_cache, row), stream_of(k_cache));
   });
 }
 
@@ -208,7 +210,7 @@ void decode(const Rows& q, int64_t hq, int64_t d, const at::Tensor& k_cache, con
   if (q.n == 0) return;
   const int64_t hkv = k_cache.size(-2);
   const int32_t width = static_cast<int32_t>(block_tables.size(1));
-  const int64_t num_blocks = k_cache.numel() / (NVLLM_BLOCK_SIZE * hkv * d);
+  const int64_t num_blocks = rows_in(k_cache, NVLLM_BLOCK_SIZE * hkv * d);
   const int64_t need = api.decode_workspace_bytes(static_cast<int32_t>(q.n), width, static_cast<int32_t>(hq),
                                                   static_cast<int32_t>(hkv), static_cast<int32_t>(d));
   check(need);
@@ -273,7 +275,7 @@ void prefill(const Rows& q, int64_t hq, int64_t d, const KV& kv, const at::Tenso
                                    ptr<int32_t>(cu_q), ptr<int32_t>(cu_k), q.n, step->k.n, static_cast<int32_t>(batch),
                                    static_cast<int32_t>(max_q), static_cast<int32_t>(max_k), static_cast<int32_t>(hq),
                                    static_cast<int32_t>(kv.hkv), static_cast<int32_t>(d), static_cast<float>(scale),
-                                   k_cache->numel() / (NVLLM_BLOCK_SIZE * kv.hkv * d), stream);
+                                   rows_in(*k_cache, NVLLM_BLOCK_SIZE * kv.hkv * d), stream);
     });
     return;
   }
@@ -437,7 +439,8 @@ PyObject* attention_forward(PyObject* const* a) {
   const Step* with_store = nullptr;
   if (do_store) {
     const at::Tensor& sm = tensor(slots.o, "slot_mapping");
-    if (qr.n > 0 && k_cache.numel() % (NVLLM_BLOCK_SIZE * hkv * d) == 0) {
+    const int64_t block = NVLLM_BLOCK_SIZE * hkv * d;
+    if (qr.n > 0 && block > 0 && k_cache.numel() % block == 0) {
       check_store(kr, hkv * d, k_cache, v_cache, sm);
       step = {kr, vr, ptr<int32_t>(sm), false};
       with_store = &step;
@@ -493,7 +496,7 @@ PyObject* qk_norm_rope_store(PyObject* const* a) {
               "contiguous caches and one slot per token");
       kc = k_cache.data_ptr();
       vc = v_cache.data_ptr();
-      num_slots = k_cache.numel() / (hkv * d);
+      num_slots = rows_in(k_cache, hkv * d);
       sm = ptr<int32_t>(*slots);
     }
   }

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from conftest import assert_close_to_oracle, ticking
-from nano_vllm_b200 import attention as A, context as C, workloads as W
+from nano_vllm_b200 import _lib, attention as A, context as C, workloads as W
 from oracle import paged_attention_ref as R
 
 pytestmark = pytest.mark.gpu
@@ -78,3 +78,33 @@ def test_other_threads_run_while_launches_wait_for_the_queue(cuda):
     assert seconds > 0.2, "the queue took every launch"
     assert ticks > 40 * seconds, f"another thread ran {ticks} times in {seconds:.2f} s"
     assert torch.equal(first, last)
+
+
+def test_shapes_without_kv_heads_are_refused(cuda):
+    """No key heads, or a cache of none: an error from every entry point, as from any other shape the
+    kernels do not take."""
+    bf = dict(dtype=torch.bfloat16, device=cuda)
+    i32 = dict(dtype=torch.int32, device=cuda)
+    q, none = torch.zeros(2, 4, 128, **bf), torch.zeros(2, 0, 128, **bf)
+    cache, empty = torch.zeros(3, 256, 1, 128, **bf), torch.zeros(3, 256, 0, 128, **bf)
+    slots, lens, table = torch.zeros(2, **i32), torch.ones(2, **i32), torch.zeros(2, 1, **i32)
+    flat = torch.zeros(1, **bf).expand(3, 256, 1, 128)  # a plane whose tokens lie zero elements apart
+    with pytest.raises(RuntimeError):
+        A.store_kvcache(none, none, flat, flat, slots)
+    with pytest.raises(RuntimeError):
+        A.decode_paged(q, empty, empty, lens, table, 0.1)
+    with pytest.raises(RuntimeError):
+        A.decode_step(q, none, none, empty, empty, slots, lens, table, 0.1)
+    with pytest.raises(RuntimeError):
+        A.qk_norm_rope_store(torch.zeros(2, 512, **bf), torch.zeros(2, dtype=torch.int64, device=cuda), None, None,
+                             torch.zeros(8, 128, device=cuda), 1e-6, slots, cache, cache, 4, 0, 128)
+    layer = A.Attention(4, 128, 0.1, 0)
+    layer.k_cache = layer.v_cache = flat
+    for prefill in (False, True):
+        C.set_context(prefill, cu_seqlens_q=slots, cu_seqlens_k=slots, max_seqlen_q=1, max_seqlen_k=1, slot_mapping=slots,
+                      context_lens=lens, block_tables=None if prefill else table)
+        with pytest.raises((RuntimeError, AssertionError)):
+            layer(q.view(2, -1), none.view(2, 0), none.view(2, 0))
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
