@@ -205,10 +205,11 @@ def test_strided_q_and_cuda_graph_replay(cuda):
 
 
 @pytest.mark.parametrize("hq,hkv,d", [(1, 1, 128), (3, 1, 128), (16, 2, 128), (1, 1, 64), (5, 1, 64), (8, 1, 64), (28, 4, 64)])
-@pytest.mark.parametrize("lens", [[32000], [20000, 1, 0, 9001], [129, 65, 64, 63]])
+@pytest.mark.parametrize("lens", [[32000], [20000, 1, 0, 9001], [129, 65, 64, 63], [20000, 3000] + [0, 70] * 16])
 def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
     """Merges of two to a hundred and more partials, with lane groups to spare (parts split between
-    them), as many as heads, and fewer; also through the layer, where the lengths are read early."""
+    them), as many as heads, and fewer; also through the layer, which is one launch for the first three
+    and reads its lengths under the store for the last."""
     case = W.make_decode_case(29, len(lens), 1, 1, hq, hkv, d, context_lens=lens)
     _check(cuda, case, f"hq{hq} hkv{hkv} d{d} {lens}")
     dev = case.to(cuda)
@@ -223,8 +224,8 @@ def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
 @pytest.mark.parametrize("batch", [1, 2, 31, 32, 33])
 @pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
 def test_layer_equals_store_then_decode_wherever_the_slots_lie(cuda, batch, hq, hkv, d):
-    """One launch for few sequences: rows stored at their position, elsewhere in the same sequence, in
-    another sequence's context, at a padding row's slot 0, twice to one slot, and nowhere."""
+    """One launch for few sequences, a store in front for more than 32: rows stored at their position, elsewhere
+    in the same sequence, in another sequence's context, at a padding row's slot 0, twice to one slot, and nowhere."""
     g = torch.Generator().manual_seed(batch)
     lens = torch.randint(1, 1500, (batch,), generator=g)
     case = W.make_decode_case(37, batch, 1, 1, hq, hkv, d, context_lens=lens.tolist())

@@ -211,3 +211,18 @@ def test_rows_at_any_alignment_pick_the_same_tokens(cuda, dtype, vocab, peak):
     cand = torch.stack([A.sample_candidates(logits[:, a:b].to(cuda), temps, a, seed=11, step=5) for a, b in zip(cuts, cuts[1:])])
     assert torch.equal(A.sample_unpack(cand.max(0).values), want)
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_rows_do_not_depend_on_the_blocks_that_read_them(cuda, lib, dtype):
+    """The first rows of batches that give a row sixteen, eight, four, two and one block: the same tokens."""
+    vocab = 40000
+    g = torch.Generator(device=cuda).manual_seed(17)
+    logits = (torch.randn(500, vocab, generator=g, device=cuda) * 3).to(dtype)
+    temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.3], device=cuda).repeat(100)
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    batches = (5, 20, 200, 400, 500)
+    assert [lib.nvllm_sample_plan(b, vocab, sms, 16) for b in batches] == [16, 8, 4, 2, 1] or sms != 148
+    want = A.sample_tokens(logits, temps, seed=3, step=8)
+    for b in batches[:-1]:
+        assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=3, step=8), want[:b]), f"batch {b}"
