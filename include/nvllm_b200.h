@@ -276,8 +276,9 @@ NVLLM_API int nvllm_qk_norm_rope_store(void* qkv, int64_t row_stride, const int6
  * for the same draw); when NULL, e comes from a Philox4x32-10 generator keyed by `seed` and
  * counted by (row, position, `step`): stateless, the same (seed, step) gives the same tokens,
  * and the caller advances `step` once per call.  tokens is int64 [batch].  Ties go to the lowest
- * index; NaN logits are never chosen.  Rows that start on a 16-byte boundary are read with
- * 16-byte loads, others element by element (no alignment is required).
+ * index; NaN logits are never chosen.  No alignment beyond the element's is required: rows that do
+ * not start on a 16-byte boundary are shifted out of aligned 16-byte loads, which may read the
+ * rest of the 16-byte pieces that a row's first and last elements lie in.
  */
 NVLLM_API int nvllm_sample_tokens(const void* logits, int32_t logits_are_fp32, int64_t row_stride,
                         const float* temperatures, const float* exponential_noise, int64_t noise_row_stride,

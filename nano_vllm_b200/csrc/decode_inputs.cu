@@ -5,8 +5,8 @@
 // nanovllm/engine/model_runner.py:151-159, 218-258) and then, to replay a captured graph, clears
 // the graph's five static input tensors and copies the fresh ones into their first rows
 // (run_model, model_runner.py:271-282): about sixteen launches and copies before the graph can
-// start.  Here the host packs the step into ONE staging block (one copy) and this kernel expands
-// it into the static buffers, rows [0, graph_bs):
+// start.  Here the host packs the step into ONE staging block, which this kernel reads where it lies (in
+// pinned host memory, or a device copy of it) and expands into the static buffers, rows [0, graph_bs):
 //   row r <  bs: input_ids = last token, positions = context_lens = sequence length,
 //                slot_mapping = last block * 256 + offset of the newest token,
 //                block_tables = the sequence's blocks, -1 up to the widest table of the batch,

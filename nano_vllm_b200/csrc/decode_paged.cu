@@ -74,7 +74,7 @@ constexpr int kMaxDecodeCtas = 1024;  // the workspace is sized for at most this
 struct DecodeParams {
   const __nv_bfloat16* q;
   int64_t q_stride;
-  __nv_bfloat16* k_cache;  // written only by the step variant
+  __nv_bfloat16* k_cache;  // written by the step and layer variants
   __nv_bfloat16* v_cache;
   const int32_t* ctx_lens;
   const int32_t* block_tables;

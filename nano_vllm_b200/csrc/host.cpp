@@ -1,9 +1,9 @@
 // Host path of the Python entry points: argument checks, output allocation and the C-ABI call, as a
 // CPython extension over torch's C++ tensors.
 //
-// An eager decode step of one layer is two launches of a few microseconds each; written in Python
+// An eager decode step of one layer is one or two launches of a few microseconds each; written in Python
 // (shape and stride look-ups, torch.cuda.device, current_stream, a ctypes call with two dozen
-// conversions) the host side of the two calls took 41 us at batch 1, four times the kernels.  The
+// conversions) the host side of two calls took 41 us at batch 1, four times the kernels.  The
 // same checks on at::Tensor cost tens of nanoseconds each, so the launches are what is left.
 //
 // The extension holds no product code of its own: it resolves the C-ABI functions of

@@ -8,7 +8,8 @@ namespace nvllm {
 
 // The persistent tcgen05 kernel is the product.  NVLLM_PREFILL_IMPL=mma (read on every call)
 // selects the warp-level mma.sync kernel instead: the cross-check of the tests and the A/B
-// baseline of measurements, never chosen by the library itself.
+// baseline of measurements, chosen by the library itself only for packed keys of no rows, of which
+// no tensor map can be made.
 static bool forced_mma() {
   const char* forced = std::getenv("NVLLM_PREFILL_IMPL");
   return forced && forced[0] == 'm';

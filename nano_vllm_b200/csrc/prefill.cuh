@@ -36,8 +36,8 @@ struct PrefillParams {
 // The engine schedules at most 512 sequences per step (nanovllm/config.py:10).
 constexpr int kPrefillMaxBatch = 1024;
 
-// Warp-level mma.sync kernel: every supported geometry; cross-check and A/B baseline only
-// (batch <= 65535).
+// Warp-level mma.sync kernel: every supported geometry; cross-check, A/B baseline, and calls without a
+// packed key row (batch <= 65535).
 int launch_prefill_mma(const PrefillParams& p, cudaStream_t stream);
 // tcgen05 / TMEM / TMA kernel in persistent blocks that pull (sequence, query tile, head) items
 // from a global counter; batch <= kPrefillMaxBatch.  total_q / total_k bound the tiled loads.

@@ -4,8 +4,8 @@
 // (flash_attn_varlen_func, causal, optional block table): query row i of a sequence with
 // Lq new tokens and Lk total tokens attends keys j <= i + (Lk - Lq).
 //
-// This kernel is the portable path: it serves head_dim 64 and every shape the tcgen05
-// kernel declines.  One thread block = 128 query rows of one (sequence, query head), 8 warps
+// This kernel is the cross-check of the tcgen05 kernel and the baseline it is measured against; the library
+// itself takes it only where packed keys are given and there are none.  One thread block = 128 query rows of one (sequence, query head), 8 warps
 // of 16 rows; K/V tiles of 64 tokens are double-buffered with cp.async from either the
 // packed K/V activations or the paged cache; online softmax in fp32 registers.
 #include "common.cuh"

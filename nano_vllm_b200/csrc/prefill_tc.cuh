@@ -7,15 +7,8 @@
 namespace nvllm {
 
 namespace tc {
-constexpr int BM = 128, BN = 64, D = 128, KST = 2;
-constexpr int Q_BYTES = BM * D * 2;        // 32 KB: two [128 x 64] swizzled sub-tiles
-constexpr int Q_SUB = Q_BYTES / 2;
-constexpr int KV_BYTES = BN * D * 2;       // 16 KB: two [64 x 64] swizzled sub-tiles
-constexpr int KV_SUB = KV_BYTES / 2;
-constexpr int OFF_Q = 0, OFF_K = Q_BYTES, OFF_V = OFF_K + KST * KV_BYTES, OFF_BAR = OFF_V + KST * KV_BYTES;
-constexpr int SMEM = OFF_BAR + 256 + 1024;  // + barriers + alignment slack
+constexpr int BM = 128, BN = 64, KST = 2;
 constexpr int TMEM_COLS = 256;              // S/P buffers: [0,64) and [64,128); O: [128,256)
-constexpr int NTHREADS = 192;
 constexpr float kRescaleThreshold = 8.f;    // log2 units
 // One tcgen05.commit per MMA group: a commit that follows a group of a different kind costs the
 // tensor pipe a bubble (~100-200 cycles measured), so each completion is signalled once and

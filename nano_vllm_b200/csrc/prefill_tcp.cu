@@ -363,8 +363,9 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
    } else if (p.slots) {
     // -------------------------------------------------- two warps left: the packed K/V rows to the cache
     // A piece of 16 bytes of a K and a V row per lane, two such at a time: 8 KB in flight per SM move four
-    // prompts of 4096 tokens (134 MB) under the products (a copy kernel beside this one: 288 us, now 284), and
-    // a prompt of 200 tokens needs no second launch (10.5 -> 9.5).
+    // prompts of 4096 tokens (134 MB) under the products.  In cycles that costs nothing (281 us at 1391 MHz, 277 at
+    // 1417 without rows to store, under the power cap); a launch of its own in front would be 23 us.  A
+    // prompt of 200 tokens needs no second launch (10.5 -> 9.5).
     const uint32_t per_row = p.hkv * D / 8, total = static_cast<uint32_t>(p.n_new) * per_row, step = gridDim.x * 64;
     const int64_t n_slots = p.num_blocks * kBlockSize;
     for (uint32_t i0 = blockIdx.x * 64 + (tid - 320); i0 < total; i0 += 2 * step) {

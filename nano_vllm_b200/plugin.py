@@ -10,7 +10,7 @@ nanovllm/layers/attention.py:32-79) and makes the layer read nano-vllm's own per
 Optional steps after ``install()``, each replacing one method of the engine by a version that
 calls this package: ``fuse_pre_attention()`` (q/k norm + rotary + KV store in one launch),
 ``fuse_sampler()`` (one-pass token sampling), ``fuse_decode_inputs()`` (decode-step inputs in
-one copy and one launch) and, for tensor-parallel runs, ``fuse_all_reduce()`` (peer-memory sum
+one launch) and, for tensor-parallel runs, ``fuse_all_reduce()`` (peer-memory sum
 behind the row-parallel projections) and ``fuse_lm_head()`` (every rank samples its own slice of
 the vocabulary; 8 bytes per row travel instead of the logits).
 """
@@ -132,8 +132,8 @@ def _install_run() -> None:
 
 
 def fuse_decode_inputs() -> None:
-    """Optional step: decode steps that replay a CUDA graph get their inputs through one staged
-    copy and one launch (decode_inputs.DecodeInputStager) instead of ``prepare_decode`` /
+    """Optional step: decode steps that replay a CUDA graph get their inputs through one pinned block
+    and one launch that reads it (decode_inputs.DecodeInputStager) instead of ``prepare_decode`` /
     ``prepare_sample`` and the clear-and-copy in ``run_model``
     (nanovllm/engine/model_runner.py:218-258, 271-282).  Prefill steps, eager decode and batches
     beyond the captured sizes go through the stock ``ModelRunner.run``."""
