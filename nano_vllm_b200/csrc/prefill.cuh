@@ -4,6 +4,10 @@
 
 namespace nvllm {
 
+// Who stores packed rows: nobody, a warp that has nothing else to do, or the epilogue warps from the key tiles in
+// shared memory.
+enum class Store { None, Spare, Tiles };
+
 struct PrefillParams {
   const __nv_bfloat16* q;
   int64_t q_stride;
@@ -20,7 +24,8 @@ struct PrefillParams {
   const int32_t* cu_k;
   int batch, max_seqlen_q, max_seqlen_k;
   int hq, hkv, g, d;
-  int pack;  // persistent tcgen05 kernel only: query heads packed into one tile (1..8)
+  // persistent tcgen05 kernel only: query heads packed into one tile (1..8), its query tokens, 2^16 / heads
+  int pack, tile_tokens, inv_pack;
   float scale_log2e;
   int64_t num_blocks;
   int* status;
@@ -30,6 +35,7 @@ struct PrefillParams {
   __nv_bfloat16* k_store;
   __nv_bfloat16* v_store;
   int64_t n_new;
+  Store store;  // persistent tcgen05 kernel only
 };
 
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).

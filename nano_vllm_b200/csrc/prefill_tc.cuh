@@ -22,20 +22,17 @@ enum Bar {
 constexpr int TILE_BYTES = 128 * 128 * 2, SUB_BYTES = TILE_BYTES / 2;
 }  // namespace tc
 
-// Bounded wait that also gives up as soon as another role has aborted.
+// Bounded wait that also gives up as soon as another role has aborted.  Small on purpose: it is inlined some
+// twenty times into a kernel whose warps run different parts of the code at the same time.
 __device__ __forceinline__ bool wait_or_abort(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
   if (sm100::mbar_try_wait(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (true) {
+  const uint32_t t0 = static_cast<uint32_t>(clock());
 #pragma unroll 1
-    for (int i = 0; i < 128; ++i)
-      if (sm100::mbar_try_wait(bar, parity)) return true;
-    if (*abort_flag) return false;
-    if (clock64() - t0 > sm100::kWaitLimitCycles) {
-      *abort_flag = 1;
-      return false;
-    }
-  }
+  do {
+    if (sm100::mbar_try_wait(bar, parity)) return true;
+  } while (!*abort_flag && static_cast<uint32_t>(clock()) - t0 < static_cast<uint32_t>(sm100::kWaitLimitCycles));
+  *abort_flag = 1;
+  return false;
 }
 
 }  // namespace nvllm

@@ -9,8 +9,9 @@
 // (128-byte swizzle, no multicast) into a two-stage ring; one tcgen05.commit per MMA group.
 // Twelve warps: 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
 // item's last P V product is done they normalise O and store it while the softmax warps are
-// already in the next item's first tile), warp 8 = TMA producer, warp 9 = MMA issuer (one elected lane each);
-// the three warp groups trade registers at start-up (setmaxnreg) so that two such blocks fit an
+// already in the next item's first tile, and write packed K/V rows to the cache from the key tiles), warp 8 = TMA producer of
+// Q and K, warp 9 = MMA issuer, warp 10 = TMA producer of V (one elected lane each), warp 11 = a copy of rows that no
+// tile stores; the three warp groups trade registers at start-up (setmaxnreg) so that two such blocks fit an
 // SM.  A thread block does not end with its query tile: two blocks per SM stay resident
 // for the whole launch, keep their TMEM allocation and barriers, and pull work items (sequence,
 // query tile, head group) from a global counter.  Under grouped-query attention the 128 rows of a tile are
@@ -36,6 +37,12 @@
 // warp owns the same 32 rows in TMEM and in the output, and passes them 32 columns at a time
 // through a private 2 KB patch of shared memory to turn row-per-lane registers into 64-byte row
 // segments.
+//
+// Code size: the warps of a block run seven different loops at the same time, and what they have to fetch of them
+// is on the path of each: in a kernel of 84 KB (loops unrolled as the compiler likes, barrier waits of 25
+// instructions, barriers set up one after the other by one thread) every fifth cycle of a warp waited for
+// instructions.  Hence the loops that are kept rolled here, the short wait, and no division for a row's token: 57 KB;
+// one prompt of 201 tokens 9.5 -> 9.05 us, of 1000 19.1 -> 18.1, 64 of 100-1024 tokens 136 -> 123.
 #include <algorithm>
 #include <atomic>
 #include <cstdlib>
@@ -53,9 +60,10 @@ using namespace tc;
 constexpr int MAX_BATCH = kPrefillMaxBatch;  // prefix array of query tiles per sequence lives in shared memory
 constexpr int SORT_BATCH = 256;  // batches up to this size are ranked by length (B^2 / 192 compares per thread)
 enum PBar {
-  ITEM_FULL0 = tc::NUM_BARS, ITEM_FULL1, ITEM_FREE0, ITEM_FREE1, O_FREE, EPI_FULL0, EPI_FULL1, P_NUM_BARS
+  ITEM_FULL0 = tc::NUM_BARS, ITEM_FULL1, ITEM_FREE0, ITEM_FREE1, O_FREE, EPI_FULL0, EPI_FULL1,
+  K_DUE0, K_DUE1, V_DUE0, V_DUE1, K_STORED0, K_STORED1, V_STORED0, V_STORED1, P_NUM_BARS
 };
-// Twelve warps in three groups of four: softmax, epilogue, and (TMA producer, MMA issuer, two that copy rows).
+// Twelve warps in three groups of four: softmax, epilogue, and (producer of Q and K, MMA issuer, producer of V, copy).
 // Registers are handed over between the groups at start-up (setmaxnreg): two blocks of 384 threads
 // per SM leave 80 per thread at launch; the softmax rows need about twice that, the other groups
 // a fraction.  128 x (RS + RE + RX) = 384 x 80.
@@ -95,6 +103,17 @@ struct Item {
   int b, h, m0, q0, Lq, k0, Lk, n_kv;  // n_kv < 0: no more work
 };
 
+// Key tiles that the first `tokens` query tokens of a sequence see.
+__device__ __forceinline__ int key_tiles(int tokens, int Lq, int Lk) {
+  const int end = min(Lk, min(tokens, Lq) + (Lk - Lq));
+  return end > 0 ? (end + tc::BN - 1) / tc::BN : 0;
+}
+// Key tiles below this one are also seen by an item before this one in its sequence and are stored there;
+// of the items that share a KV head's tiles only the first group of query heads stores.
+__device__ __forceinline__ int first_stored(const Item& x, int g) {
+  return x.h % g == 0 ? (x.m0 > 0 ? key_tiles(x.m0, x.Lq, x.Lk) : 0) : x.n_kv;
+}
+
 template <int D>
 __global__ void __launch_bounds__(tcp::NTHREADS_P, 2)
 prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tmap_q,
@@ -122,13 +141,33 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   // (row = token * n + head; n = p.pack need not be a power of two: 7 heads x 18 tokens leave two
   // rows unused), so short and ragged sequences waste fewer rows above the diagonal and past
   // their end, and the packed heads share every K/V tile.
-  const int pack = p.pack, BMT = BM / pack;
+  const int pack = p.pack, BMT = p.tile_tokens;
+  auto token_of = [&](int row) { return row * p.inv_pack >> 16; };  // row / pack, row < 128
 
   pdl_trigger();
+  if (warp == 9 && lane < P_NUM_BARS) {  // a barrier per lane
+    // four softmax warps fill P and the normalisers; four epilogue warps free O and store rows; an item slot is
+    // free when the softmax warps, the epilogue warps, the MMA issuer and the V producer are done with it
+    static_assert(P_NUM_BARS <= 32, "a barrier per lane");
+    const bool by_four = lane == P_FULL0 || lane == P_FULL1 || lane == O_FREE || lane == EPI_FULL0 || lane == EPI_FULL1 || lane >= K_STORED0;
+    mbar_init(bar(lane), by_four ? 4u : lane == ITEM_FREE0 || lane == ITEM_FREE1 ? 10u : 1u);
+    if (lane == 0) {
+      *abort_flag = 0;
+      prefetch_tmap(&tmap_q);
+      prefetch_tmap(&tmap_k);
+      prefetch_tmap(&tmap_v);
+    }
+    mbar_fence_init();
+  }
   if (!p.lengths_early) pdl_wait();
+  int* seq_tiles = prefix + (MAX_BATCH + 1) - SORT_BATCH;  // for as long as the prefix sums are not there yet
   // Rank the sequences by key length, longest first (ties by index): rank = how many come before.
   if (p.batch <= SORT_BATCH) {
-    for (int b = tid; b < p.batch; b += NTHREADS_P) prefix[b] = p.cu_k[b + 1] - p.cu_k[b];  // lengths, for a moment
+#pragma unroll 1
+    for (int b = tid; b < p.batch; b += NTHREADS_P) {
+      prefix[b] = p.cu_k[b + 1] - p.cu_k[b];  // lengths, for a moment
+      seq_tiles[b] = (p.cu_q[b + 1] - p.cu_q[b] + BMT - 1) / BMT;
+    }
     __syncthreads();
     int my_rank[(SORT_BATCH + NTHREADS_P - 1) / NTHREADS_P];
 #pragma unroll
@@ -151,18 +190,20 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       if (b < p.batch) order[my_rank[k]] = static_cast<unsigned short>(b);
     }
   } else {
+#pragma unroll 1
     for (int b = tid; b < p.batch; b += NTHREADS_P) order[b] = static_cast<unsigned short>(b);
   }
   __syncthreads();
   if (warp == 8) {
     // query tiles per sequence, in that order -> exclusive prefix sum (warp scan, 32 at a time)
     int carry = 0;
+#pragma unroll 1
     for (int i0 = 0; i0 < p.batch; i0 += 32) {
       const int i = i0 + lane;
       int tiles = 0;
       if (i < p.batch) {
         const int b = order[i];
-        tiles = (p.cu_q[b + 1] - p.cu_q[b] + BMT - 1) / BMT;
+        tiles = p.batch <= SORT_BATCH ? seq_tiles[b] : (p.cu_q[b + 1] - p.cu_q[b] + BMT - 1) / BMT;
       }
       int incl = tiles;
 #pragma unroll
@@ -173,22 +214,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       if (i < p.batch) prefix[i] = carry + incl - tiles;
       carry += __shfl_sync(0xffffffffu, incl, 31);
     }
-    if (lane == 0) {
-      prefix[p.batch] = carry;
-      for (int i = 0; i < P_NUM_BARS; ++i) {
-        // four softmax warps fill P and the normalisers; four epilogue warps free O; an item slot is
-        // free when the softmax warps, the epilogue warps and the MMA issuer are done with it
-        const uint32_t count = (i == P_FULL0 || i == P_FULL1 || i == O_FREE || i == EPI_FULL0 || i == EPI_FULL1) ? 4u
-                               : (i == ITEM_FREE0 || i == ITEM_FREE1)                                               ? 9u
-                                                                                                                    : 1u;
-        mbar_init(bar(i), count);
-      }
-      *abort_flag = 0;
-      mbar_fence_init();
-      prefetch_tmap(&tmap_q);
-      prefetch_tmap(&tmap_k);
-      prefetch_tmap(&tmap_v);
-    }
+    if (lane == 0) prefix[p.batch] = carry;
   }
   if (warp == 9) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
   if (p.lengths_early) pdl_wait();  // from here on q, k and v are read
@@ -206,6 +232,31 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     return x;
   };
 
+  // First row of an item's key tile j: of the cache, through the table, or of the packed rows.
+  auto key_row = [&](const Item& x, int j) {
+    if (!p.block_tables) return x.k0 + j * BN;
+    int64_t blk = p.block_tables[x.b * p.bt_stride + (j * BN) / kBlockSize];
+    if (blk < 0 || blk >= p.num_blocks) {
+      atomicOr(p.status, NVLLM_STATUS_BAD_BLOCK);
+      blk = 0;
+    }
+    return static_cast<int>(blk * kBlockSize + (j * BN) % kBlockSize);
+  };
+  // A producer's record of the tiles that are stored from its stages: bit st, the tile in the stage is; bit 2 + st,
+  // the parity of the stage's next completed store.  Waits for that before the stage is used again.
+  auto stage_stored = [&](unsigned& stored, int st, int done) {
+    if (!(stored >> st & 1u)) return true;
+    const bool ok = wait_or_abort(bar(done + st), stored >> (2 + st) & 1u, abort_flag);
+    stored ^= 5u << st;
+    return ok;
+  };
+  const int64_t n_slots = p.num_blocks * kBlockSize;
+  auto slot_of = [&](int64_t r) {  // of packed row r, -1: none
+    const int64_t slot = p.slots[r];
+    if (slot >= n_slots) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
+    return slot >= 0 && slot < n_slots ? static_cast<int>(slot) : -1;
+  };
+
   float* inv_buf = reinterpret_cast<float*>(base_ptr + G::OFF_INV);
   // The register hand-over sits inside each group's own branch: the allocator bounds the code that
   // follows a setmaxnreg on its path, and paths that merged again would all get the smallest bound.
@@ -217,17 +268,19 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
       int T = 0;   // key tiles loaded so far in this block's life
-      int nq = 0;  // items with at least one key tile so far (Q_FULL phase)
+      unsigned stored = 0;
       // Item number -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
       // working side by side share K/V tiles in L2.
       auto decode_item = [&](unsigned idx) {
         Item x;
+#pragma unroll 1
         while (true) {
           x.n_kv = -1;
           if (idx >= static_cast<unsigned>(total_items)) break;
           const int pi = idx / hgroups;
           x.h = (idx - pi * hgroups) * pack;  // first of the packed heads
           int lo = 0, hi = p.batch;  // largest i with prefix[i] <= pi
+#pragma unroll 1
           while (hi - lo > 1) {
             const int mid = (lo + hi) >> 1;
             if (prefix[mid] <= pi) lo = mid; else hi = mid;
@@ -239,13 +292,14 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
           x.Lk = p.cu_k[x.b + 1] - x.k0;
           const int tiles = prefix[lo + 1] - prefix[lo];
           x.m0 = (tiles - 1 - (pi - prefix[lo])) * BMT;  // a sequence's long tiles first
-          const int kv_end = min(x.Lk, min(x.m0 + BMT, x.Lq) + (x.Lk - x.Lq));
-          x.n_kv = kv_end > 0 ? (kv_end + BN - 1) / BN : 0;
+          x.n_kv = key_tiles(x.m0 + BMT, x.Lq, x.Lk);
           if (x.n_kv > 0) break;
           // No visible key for the whole tile (only possible when Lk < Lq, which the engine
           // never produces): the rows are zero; written here, the other roles never see it.
+#pragma unroll 1
           for (int r = x.m0; r < min(x.m0 + BMT, x.Lq); ++r) {
             uint4* dst = reinterpret_cast<uint4*>(p.out + static_cast<int64_t>(x.q0 + r) * p.out_stride + x.h * D);
+#pragma unroll 1
             for (int c = 0; c < PIECES * pack; ++c) dst[c] = make_uint4(0, 0, 0, 0);  // the packed heads are adjacent
           }
           idx = atomicAdd(&g_item_counter[counter_slot], 1u);
@@ -258,6 +312,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       // reserved long before its block is free is an item that an idle block cannot take (measured:
       // reserving at the start of the current item cost 9 % on four 4096-token sequences).
       unsigned next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
+#pragma unroll 1
       for (int it = 0;; ++it) {
         const Item x = decode_item(next_idx);
         if (it >= 2 && !wait_or_abort(bar(ITEM_FREE0 + (it & 1)), ((it >> 1) - 1) & 1, abort_flag)) break;
@@ -273,34 +328,58 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         mbar_expect_tx(bar(Q_FULL), G::NSUB * pack * BMT * 128);  // the box holds pack x BMT rows per sub-tile
         tma_load_3d(base + OFF_Q, &tmap_q, bar(Q_FULL), 0, x.h, x.q0 + x.m0);
         if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_Q + Q_SUB, &tmap_q, bar(Q_FULL), 64, x.h, x.q0 + x.m0);
-        ++nq;
-        const int32_t* bt_row = p.block_tables ? p.block_tables + x.b * p.bt_stride : nullptr;
+        const int store_from = first_stored(x, p.g);
         bool ok = true;
+#pragma unroll 1
         for (int j = 0; j < x.n_kv; ++j) {
           if (j == max(0, x.n_kv - 3)) next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
           const int t = T + j, st = t & 1, use = t >> 1;
-          int row;
-          if (bt_row) {
-            int64_t blk = bt_row[(j * BN) / kBlockSize];
-            if (blk < 0 || blk >= p.num_blocks) {
-              atomicOr(p.status, NVLLM_STATUS_BAD_BLOCK);
-              blk = 0;
-            }
-            row = static_cast<int>(blk * kBlockSize + (j * BN) % kBlockSize);
-          } else {
-            row = x.k0 + j * BN;
-          }
+          const int row = key_row(x, j);
           if (use > 0 && !(ok = wait_or_abort(bar(QK_DONE0 + st), (use - 1) & 1, abort_flag))) break;
+          if (!(ok = stage_stored(stored, st, K_STORED0))) break;
           mbar_expect_tx(bar(K_FULL0 + st), KV_BYTES);
           tma_load_3d(base + OFF_K + st * KV_BYTES, &tmap_k, bar(K_FULL0 + st), 0, kvh, row);
           if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_K + st * KV_BYTES + KV_SUB, &tmap_k, bar(K_FULL0 + st), 64, kvh, row);
-          if (use > 0 && !(ok = wait_or_abort(bar(PV_DONE0 + st), (use - 1) & 1, abort_flag))) break;
-          mbar_expect_tx(bar(V_FULL0 + st), KV_BYTES);
-          tma_load_3d(base + OFF_V + st * KV_BYTES, &tmap_v, bar(V_FULL0 + st), 0, kvh, row);
-          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_V + st * KV_BYTES + KV_SUB, &tmap_v, bar(V_FULL0 + st), 64, kvh, row);
+          if (p.store == Store::Tiles && j >= store_from) {
+            stored |= 1u << st;
+            mbar_arrive(bar(K_DUE0 + st));
+          }
         }
         if (!ok) break;
         T += x.n_kv;
+      }
+    }
+   } else if (warp == 10) {
+    // ------------------------------------------------------------------ V producer
+    // A thread of its own: a V stage is free only after the tile's P V product, and a single producer that
+    // waits for that would hold back the K load of the next tile, whose stage is free much earlier.
+    if (elect_one()) {
+      int T = 0;
+      unsigned stored = 0;
+      bool ok = true;
+#pragma unroll 1
+      for (int it = 0; ok; ++it) {
+        if (!(ok = wait_or_abort(bar(ITEM_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
+        const Item x = read_item(it);
+        if (x.n_kv < 0) break;
+        const int kvh = x.h / p.g, store_from = first_stored(x, p.g);
+#pragma unroll 1
+        for (int j = 0; j < x.n_kv; ++j) {
+          const int t = T + j, st = t & 1, use = t >> 1;
+          const int row = key_row(x, j);
+          if (use > 0 && !(ok = wait_or_abort(bar(PV_DONE0 + st), (use - 1) & 1, abort_flag))) break;
+          if (!(ok = stage_stored(stored, st, V_STORED0))) break;
+          mbar_expect_tx(bar(V_FULL0 + st), KV_BYTES);
+          tma_load_3d(base + OFF_V + st * KV_BYTES, &tmap_v, bar(V_FULL0 + st), 0, kvh, row);
+          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_V + st * KV_BYTES + KV_SUB, &tmap_v, bar(V_FULL0 + st), 64, kvh, row);
+          if (p.store == Store::Tiles && j >= store_from) {
+            stored |= 1u << st;
+            mbar_arrive(bar(V_DUE0 + st));
+          }
+        }
+        if (!ok) break;
+        T += x.n_kv;
+        mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
       }
     }
    } else if (warp == 9) {
@@ -328,16 +407,18 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       };
       int T = 0, nq = 0;
       bool ok = true;
+#pragma unroll 1
       for (int it = 0; ok; ++it) {
         if (!(ok = wait_or_abort(bar(ITEM_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
         const Item x = read_item(it);
         if (x.n_kv < 0) break;
         if (!(ok = wait_or_abort(bar(Q_FULL), nq & 1, abort_flag))) break;
         ++nq;
-        if (!(ok = issue_qk(T))) break;
-        for (int j = 0; j < x.n_kv; ++j) {
+#pragma unroll 1
+        for (int j = -1; j < x.n_kv; ++j) {
           const int t = T + j, st = t & 1, ph = (t >> 1) & 1;
           if (j + 1 < x.n_kv && !(ok = issue_qk(t + 1))) break;  // next S runs under this tile's softmax
+          if (j < 0) continue;
           if (!(ok = wait_or_abort(bar(V_FULL0 + st), ph, abort_flag))) break;
           if (!(ok = wait_or_abort(bar(P_FULL0 + st), ph, abort_flag))) break;
           // the first product of an item overwrites O: the previous item's O must have been read
@@ -360,36 +441,50 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         (void)mbar_wait(bar(DRAIN), 0);
       }
     }
-   } else if (p.slots) {
-    // -------------------------------------------------- two warps left: the packed K/V rows to the cache
-    // A piece of 16 bytes of a K and a V row per lane, two such at a time: 8 KB in flight per SM move four
-    // prompts of 4096 tokens (134 MB) under the products.  In cycles that costs nothing (281 us at 1391 MHz, 277 at
-    // 1417 without rows to store, under the power cap); a launch of its own in front would be 23 us.  A
-    // prompt of 200 tokens needs no second launch (10.5 -> 9.5).
-    const uint32_t per_row = p.hkv * D / 8, total = static_cast<uint32_t>(p.n_new) * per_row, step = gridDim.x * 64;
-    const int64_t n_slots = p.num_blocks * kBlockSize;
-    for (uint32_t i0 = blockIdx.x * 64 + (tid - 320); i0 < total; i0 += 2 * step) {
-      uint4 kreg[2], vreg[2];
-      int64_t dst[2];
-#pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        const uint32_t i = i0 + u * step, tok = i / per_row, piece = i - tok * per_row;
-        dst[u] = -1;
-        if (i >= total) continue;
-        const int64_t slot = p.slots[tok];
-        if (slot >= n_slots) {
-          if (piece == 0) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
-        } else if (slot >= 0) {
-          dst[u] = slot * per_row + piece;
-        }
-        kreg[u] = __ldg(reinterpret_cast<const uint4*>(p.k + tok * p.k_stride) + piece);
-        vreg[u] = __ldg(reinterpret_cast<const uint4*>(p.v + tok * p.v_stride) + piece);
+   } else if (p.store != Store::None) {
+    // -------------------------------------------------- a warp left: packed rows to the cache
+    // All of them, or those that no item has a tile of: of sequences without a query row, in front of the first
+    // sequence and behind the last.  A 16-byte piece of a K and a V row per lane, two such at a time.
+    const uint32_t per_row = p.hkv * PIECES;
+    const bool all = p.store == Store::Spare;
+    int b = all ? p.batch : static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
+#pragma unroll 1
+    while (b <= p.batch) {
+      int64_t from = 0, to = p.n_new;
+      uint32_t first = blockIdx.x, step = gridDim.x;
+      if (all || b == p.batch) {
+        if (!all) from = p.cu_k[p.batch];
+        b = p.batch + 1;
+      } else if (b < 0) {
+        to = p.cu_k[0];
+        b += gridDim.x;
+        b = min(b, p.batch);
+      } else {
+        from = p.cu_k[b], to = p.cu_q[b + 1] == p.cu_q[b] ? p.cu_k[b + 1] : from;
+        first = 0, step = 1;
+        b = min(b + static_cast<int>(gridDim.x), p.batch);
       }
+      const uint32_t total = static_cast<uint32_t>(max(min(to, p.n_new) - from, static_cast<int64_t>(0)) * per_row);
+#pragma unroll 1
+      for (uint32_t i0 = first * 32 + lane; i0 < total; i0 += 2 * step * 32) {
+        uint4 kreg[2], vreg[2];
+        int64_t dst[2];
 #pragma unroll
-      for (int u = 0; u < 2; ++u) {
-        if (dst[u] < 0) continue;
-        reinterpret_cast<uint4*>(p.k_store)[dst[u]] = kreg[u];
-        reinterpret_cast<uint4*>(p.v_store)[dst[u]] = vreg[u];
+        for (int u = 0; u < 2; ++u) {
+          const uint32_t i = i0 + u * step * 32, row = i / per_row, piece = i - row * per_row;
+          dst[u] = -1;
+          if (i >= total) continue;
+          const int slot = slot_of(from + row);
+          if (slot >= 0) dst[u] = static_cast<int64_t>(slot) * per_row + piece;
+          kreg[u] = __ldg(reinterpret_cast<const uint4*>(p.k + (from + row) * p.k_stride) + piece);
+          vreg[u] = __ldg(reinterpret_cast<const uint4*>(p.v + (from + row) * p.v_stride) + piece);
+        }
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+          if (dst[u] < 0) continue;
+          reinterpret_cast<uint4*>(p.k_store)[dst[u]] = kreg[u];
+          reinterpret_cast<uint4*>(p.v_store)[dst[u]] = vreg[u];
+        }
       }
     }
    }
@@ -397,16 +492,18 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     // ------------------------------------------------------------------ softmax rows
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOFTMAX));
     const int r = warp * 32 + lane;
-    const int r_tok = r / pack;  // this row's token within the tile (== BMT for the unused rows of a 7-head tile)
+    const int r_tok = token_of(r);  // this row's token within the tile (== BMT for the unused rows of a 7-head tile)
     const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
     int T = 0;
     bool ok = true;
+#pragma unroll 1
     for (int it = 0; ok; ++it) {
       if (!(ok = wait_or_abort(bar(ITEM_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
       const Item x = read_item(it);
       if (x.n_kv < 0) break;
       const int qi = x.m0 + r_tok, off = x.Lk - x.Lq;
       float m_used = -INFINITY, l = 0.f;
+#pragma unroll 1
       for (int j = 0; j < x.n_kv; ++j) {
         const int t = T + j, st = t & 1, ph = (t >> 1) & 1;
         const uint32_t tmem_s = tmem + st * 64 + lane_addr;
@@ -446,7 +543,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
           if (j > 0) {  // O holds tiles 0..j-1 of this item once the previous P V product has finished
             if (!(ok = wait_or_abort(bar(PV_DONE0 + ((t - 1) & 1)), ((t - 1) >> 1) & 1, abort_flag))) break;
             tc_fence_after();
-#pragma unroll
+#pragma unroll 1
             for (int c = 0; c < OCH; ++c) {
               uint32_t o[32];
               tmem_ld32(tmem_o + lane_addr + c * 32, o);
@@ -482,6 +579,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
           if (!(ok = wait_or_abort(bar(V_FULL0 + st), ph, abort_flag))) break;
           const int first = x.Lk - j0;  // rows [first, 64) are dead
           unsigned char* vt = base_ptr + OFF_V + st * KV_BYTES;
+#pragma unroll 1
           for (int i = r; i < (BN - first) * PIECES; i += 128) {
             const int row = first + i / PIECES, piece = i % PIECES;
             *reinterpret_cast<uint4*>(vt + (piece >> 3) * KV_SUB + row * 128 + (piece & 7) * 16) = make_uint4(0, 0, 0, 0);
@@ -513,11 +611,48 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     const uint32_t lane_addr = static_cast<uint32_t>(ew * 32) << 16;
     unsigned char* stage = base_ptr + G::OFF_STAGE + ew * 2048;  // this warp's 32 rows x 64 B
     int T = 0;
+    unsigned due = 0;  // bit st: parity of stage st's next K_DUE and V_DUE
     bool ok = true;
+#pragma unroll 1
     for (int it = 0; ok; ++it) {
       if (!(ok = wait_or_abort(bar(ITEM_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
       const Item x = read_item(it);
       if (x.n_kv < 0) break;
+      if (p.store == Store::Tiles) {
+        // Packed rows to the cache: the first item of a sequence that loads a key tile writes its rows to their slots
+        // from shared memory, 16 of the 64 per warp, 512 bytes with an instruction.
+        constexpr int ROWS = 32 / PIECES;  // rows that a warp writes at a time
+        const int piece = lane % PIECES;
+        const int64_t row_elems = static_cast<int64_t>(p.hkv) * D;
+        const int64_t col = static_cast<int64_t>(x.h / p.g) * D + piece * 8;
+#pragma unroll 1
+        for (int j = first_stored(x, p.g); j < x.n_kv; ++j) {
+          const int t = T + j, st = t & 1, r_warp = ew * 16;
+          const int64_t row0 = x.k0 + j * BN, n_rows = min(static_cast<int64_t>(min(BN, x.Lk - j * BN)), p.n_new - row0);
+          const int slot = lane < 16 && r_warp + lane < n_rows ? slot_of(row0 + r_warp + lane) : -1;
+          // A stage's barrier tells its phase by parity only, and these warps do not wait for every tile: between
+          // the producer's word that the load is issued and theirs that it is stored it stays at this tile's.
+#pragma unroll 1
+          for (int kv = 0; ok && kv < 2; ++kv) {
+            if (!(ok = wait_or_abort(bar((kv ? V_DUE0 : K_DUE0) + st), due >> st & 1, abort_flag))) break;
+            if (!(ok = wait_or_abort(bar((kv ? V_FULL0 : K_FULL0) + st), (t >> 1) & 1, abort_flag))) break;
+            const uint32_t src = base + (kv ? OFF_V : OFF_K) + st * KV_BYTES + (piece >> 3) * KV_SUB + r_warp * 128;
+            __nv_bfloat16* cache = (kv ? p.v_store : p.k_store) + col;
+#pragma unroll 8
+            for (int r0 = 0; r0 < 16; r0 += ROWS) {
+              const int r = r0 + lane / PIECES;
+              const int to = __shfl_sync(0xffffffffu, slot, r);
+              if (to >= 0)
+                *reinterpret_cast<uint4*>(cache + to * row_elems) = ld_shared16(src + r * 128 + (((piece ^ r) & 7) << 4));
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar((kv ? V_STORED0 : K_STORED0) + st));
+          }
+          if (!ok) break;
+          due ^= 1u << st;
+        }
+        if (!ok) break;
+      }
       T += x.n_kv;
       if (!(ok = wait_or_abort(bar(EPI_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
       const float inv = inv_buf[(it & 1) * 128 + r];
@@ -528,7 +663,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       const int srow = lane >> 2, spiece = lane & 3;
       __nv_bfloat16* out_tile = p.out + static_cast<int64_t>(x.q0 + x.m0) * p.out_stride + x.h * D;
       const int toks_valid = min(BMT, x.Lq - x.m0);
-#pragma unroll
+#pragma unroll 4
       for (int c = 0; c < OCH; ++c) {
         uint32_t o[32];
         tmem_ld32(tmem_o + lane_addr + c * 32, o);
@@ -553,7 +688,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         for (int i = 0; i < 4; ++i) {
           const int lr = i * 8 + srow;       // row within the warp's 32
           const int row = ew * 32 + lr;      // row of the tile
-          const int tok = row / pack, hh = row - tok * pack;
+          const int tok = token_of(row), hh = row - tok * pack;
           const uint4 v = *reinterpret_cast<const uint4*>(stage + lr * 64 + ((spiece ^ ((lr >> 1) & 3)) << 4));
           if (tok < toks_valid)
             *reinterpret_cast<uint4*>(out_tile + static_cast<int64_t>(tok) * p.out_stride + hh * D + c * 32 + spiece * 8) = v;
@@ -615,6 +750,8 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   for (int n = 2; n <= 8 && n <= cap; ++n)
     if (p.g % n == 0) p.pack = n;
   const int pack = p.pack, bmt = tc::BM / pack;
+  p.tile_tokens = bmt;
+  p.inv_pack = 65536 / pack + 1;  // exact for rows of a tile
   CUtensorMap mq, mk, mv;
   if (!make_tmap_3d(&mq, p.q, D, p.hq, total_q, D, p.q_stride, bmt, pack)) return NVLLM_E_CUDA;
   if (p.block_tables) {
@@ -630,9 +767,16 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   const int64_t max_items = static_cast<int64_t>((p.max_seqlen_q + bmt - 1) / bmt) * (p.hq / pack) * p.batch;
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
-  // and, where rows are to be stored, enough of them to do that in a few trips
-  const int64_t store_blocks = (p.n_new * p.hkv * (D / 8) + 255) / 256;
-  grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, store_blocks)));
+  // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
+  // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
+  // rows, 4 KB in flight; 123 from the tiles; 111 with nothing to store).  Where a block has one item at most that
+  // would end it later (a prompt of 201 tokens 9.05 -> 9.5 us): there an idle warp of every block copies the rows, by
+  // as many blocks as that takes two trips of, as long as four of them are enough (6 prompts of 300 tokens: 15.8
+  // us from the tiles, 20.2 copied).
+  const int64_t pieces = p.n_new * p.hkv * (D / 8);
+  p.store = !p.slots ? Store::None : max_items > grid || pieces > 4ll * 64 * grid ? Store::Tiles : Store::Spare;
+  const int64_t copy_blocks = p.store == Store::Spare ? (pieces + 127) / 128 : 0;
+  grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, copy_blocks)));
   // the two head_dim instantiations share the counter array: give each its own half
   const int slot = static_cast<int>(launch_seq.fetch_add(1) % (tcp::NUM_SLOTS / 2)) + (D == 64 ? tcp::NUM_SLOTS / 2 : 0);
   return launch_kernel("prefill (tcgen05, persistent)", prefill_tcp_kernel<D>, dim3(grid), dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq,

@@ -129,6 +129,37 @@ def test_layer_stores_packed_rows_as_the_store_does(cuda, monkeypatch, impl, hq,
         slots[n - 1] = k2.shape[0] * 256  # NVLLM_STATUS_BAD_SLOT the second time
 
 
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (32, 8, 128), (14, 2, 64), (3, 3, 64)])
+def test_layer_stores_every_packed_row_from_the_key_tiles(cuda, hq, hkv, d):
+    """More items than blocks: rows are stored from the key tiles.  Sequences with more keys than queries, fewer, or
+    no query at all, rows in front of the first sequence and behind the last, ends around a tile's, scattered slots."""
+    lq = [1, 0, 63, 64, 65, 700, 0, 127, 129, 30, 1000, 300, 1, 40] * 3
+    lk = [1, 70, 63, 64, 200, 700, 1, 128, 100, 300, 1000, 310, 129, 40] * 3
+    front, behind = 3, 70
+    gen = torch.Generator(device=cuda).manual_seed(5)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    n_q, n_k = sum(lq), front + sum(lk) + behind
+    q, k, v = rand(n_q, hq * d), rand(n_k, hkv * d), rand(n_k, 2 * hkv * d)[:, : hkv * d]
+    cu_q = torch.tensor([0] + lq, device=cuda).cumsum(0).int()
+    cu_k = (torch.tensor([0] + lk, device=cuda).cumsum(0) + front).int()
+    blocks = n_k // 256 + 3
+    slots = torch.randperm(blocks * 256, generator=gen, device=cuda)[:n_k].int()
+    slots[::11] = -1
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+    k2, v2 = layer.k_cache.clone(), layer.v_cache.clone()
+    A.store_kvcache(k.view(n_k, hkv, d), v.unflatten(1, (hkv, d)), k2, v2, slots)
+    want = A.prefill_varlen(q.view(n_q, hq, d), k.view(n_k, hkv, d), v.unflatten(1, (hkv, d)), cu_q, cu_k, max(lq), max(lk), d ** -0.5)
+    C.set_context(True, cu_q, cu_k, max(lq), max(lk), slots, None, None)
+    for _ in range(2):
+        got = layer(q, k, v)
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert torch.equal(got.view_as(want), want)
+    assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+    assert _lib.read_status() == 0
+
+
 def test_many_sequences_through_the_persistent_kernel(cuda):
     """More work items than resident blocks, and more sequences than one warp scans at once."""
     case = W.make_prefill_case(28, 150, 1, 300, 4, 2, 128, share_every=0)
