@@ -8,6 +8,20 @@ namespace nvllm {
 // shared memory.
 enum class Store { None, Spare, Tiles };
 
+// Where the key tiles of new rows are, for a prefill through the block table (prefill_route.cu).  Every cache block that
+// new rows of a sequence lie in has a job: those of sequence b start at route_first_job(cu_q[b], b), in the order
+// of its blocks.
+struct RouteTables {
+  int* tile_row = nullptr;  // [job][4]: first packed row of the 64-token tile, -1: read it through the table
+  int* block = nullptr;     // [job]: its cache block, -1: none that is new as a whole
+  int* source = nullptr;    // [sequence][max_blocks]: job of a cached block; anything, unless block[] agrees
+  int jobs = 0;             // 0: no tables, everything is read in one place
+};
+constexpr int kRouteRagged = 1 << 30;  // in tile_row: the sequence ends inside the tile; rows for that sequence only
+constexpr int kRouteJobs = 2048, kRouteEntries = 16384;  // the tables' sizes
+__host__ __device__ __forceinline__ int route_first_job(int q0, int b) { return (q0 >> 8) + 2 * b; }
+inline int64_t route_jobs(int64_t n_new, int batch) { return (n_new >> 8) + 2 * static_cast<int64_t>(batch); }
+
 struct PrefillParams {
   const __nv_bfloat16* q;
   int64_t q_stride;
@@ -36,6 +50,12 @@ struct PrefillParams {
   __nv_bfloat16* v_store;
   int64_t n_new;
   Store store;  // persistent tcgen05 kernel only
+  // and with a route: key and value are the packed rows, k and v the cache
+  RouteTables route;
+  const __nv_bfloat16* key;
+  int64_t key_stride;
+  const __nv_bfloat16* value;
+  int64_t value_stride;
 };
 
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).
@@ -48,5 +68,9 @@ int launch_prefill_mma(const PrefillParams& p, cudaStream_t stream);
 // tcgen05 / TMEM / TMA kernel in persistent blocks that pull (sequence, query tile, head) items
 // from a global counter; batch <= kPrefillMaxBatch.  total_q / total_k bound the tiled loads.
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream);
+// Work items of such a launch at most.
+int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch);
+// Fills the tables for a prefill through the block table and copies the rows that cannot be read packed.
+int launch_prefill_route(const PrefillParams& p, RouteTables* tables, cudaStream_t stream);
 
 }  // namespace nvllm

@@ -114,10 +114,11 @@ __device__ __forceinline__ int first_stored(const Item& x, int g) {
   return x.h % g == 0 ? (x.m0 > 0 ? key_tiles(x.m0, x.Lq, x.Lk) : 0) : x.n_kv;
 }
 
-template <int D>
+template <int D, bool ROUTED>
 __global__ void __launch_bounds__(tcp::NTHREADS_P, 2)
 prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
+                   const __grid_constant__ CUtensorMap tmap_key, const __grid_constant__ CUtensorMap tmap_value,
                    const int counter_slot) {
   using namespace tcp;
   using G = Geo<D>;
@@ -141,6 +142,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   // (row = token * n + head; n = p.pack need not be a power of two: 7 heads x 18 tokens leave two
   // rows unused), so short and ragged sequences waste fewer rows above the diagonal and past
   // their end, and the packed heads share every K/V tile.
+  constexpr int TILES = kBlockSize / BN;  // key tiles of a cache block
   const int pack = p.pack, BMT = p.tile_tokens;
   auto token_of = [&](int row) { return row * p.inv_pack >> 16; };  // row / pack, row < 128
 
@@ -156,6 +158,10 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       prefetch_tmap(&tmap_q);
       prefetch_tmap(&tmap_k);
       prefetch_tmap(&tmap_v);
+      if (ROUTED) {
+        prefetch_tmap(&tmap_key);
+        prefetch_tmap(&tmap_value);
+      }
     }
     mbar_fence_init();
   }
@@ -232,10 +238,29 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     return x;
   };
 
-  // First row of an item's key tile j: of the cache, through the table, or of the packed rows.
-  auto key_row = [&](const Item& x, int j) {
-    if (!p.block_tables) return x.k0 + j * BN;
-    int64_t blk = p.block_tables[x.b * p.bt_stride + (j * BN) / kBlockSize];
+  // First packed row of an item's key tile j if it is one of this step's rows, to be read there; else -1.
+  auto packed_row = [&](const Item& x, int j) {
+    if (!ROUTED && !p.block_tables) return x.k0 + j * BN;
+    const int i = j / TILES, off = x.Lk - x.Lq;
+    if (!ROUTED || off < 0 || i * kBlockSize < off) return -1;
+    const int row = __ldcg(p.route.tile_row + (route_first_job(x.q0, x.b) + i - (off >> 8)) * TILES + j % TILES);
+    return row < 0 ? row : row & ~kRouteRagged;
+  };
+  // First row of any other key tile: packed too if it lies in a block that another sequence fills in this step, else in
+  // the cache, through the table.
+  auto cached_row = [&](const Item& x, int j, bool& packed) {
+    const int i = j / TILES;
+    int64_t blk = p.block_tables[x.b * p.bt_stride + i];
+    if (ROUTED && i < p.max_blocks) {
+      const unsigned job = __ldcg(p.route.source + x.b * p.max_blocks + i);
+      if (job < static_cast<unsigned>(p.route.jobs) && __ldcg(p.route.block + job) == blk && i * kBlockSize < x.Lk - x.Lq) {
+        const int row = __ldcg(p.route.tile_row + job * TILES + j % TILES);
+        if (row >= 0 && !(row & kRouteRagged)) {
+          packed = true;
+          return row;
+        }
+      }
+    }
     if (blk < 0 || blk >= p.num_blocks) {
       atomicOr(p.status, NVLLM_STATUS_BAD_BLOCK);
       blk = 0;
@@ -334,13 +359,17 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         for (int j = 0; j < x.n_kv; ++j) {
           if (j == max(0, x.n_kv - 3)) next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
           const int t = T + j, st = t & 1, use = t >> 1;
-          const int row = key_row(x, j);
+          int row = packed_row(x, j);
+          const bool own = row >= 0;
+          bool packed = own;
+          if (!own) row = cached_row(x, j, packed);
+          const CUtensorMap* map = ROUTED && packed ? &tmap_key : &tmap_k;
           if (use > 0 && !(ok = wait_or_abort(bar(QK_DONE0 + st), (use - 1) & 1, abort_flag))) break;
           if (!(ok = stage_stored(stored, st, K_STORED0))) break;
           mbar_expect_tx(bar(K_FULL0 + st), KV_BYTES);
-          tma_load_3d(base + OFF_K + st * KV_BYTES, &tmap_k, bar(K_FULL0 + st), 0, kvh, row);
-          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_K + st * KV_BYTES + KV_SUB, &tmap_k, bar(K_FULL0 + st), 64, kvh, row);
-          if (p.store == Store::Tiles && j >= store_from) {
+          tma_load_3d(base + OFF_K + st * KV_BYTES, map, bar(K_FULL0 + st), 0, kvh, row);
+          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_K + st * KV_BYTES + KV_SUB, map, bar(K_FULL0 + st), 64, kvh, row);
+          if (p.store == Store::Tiles && own && j >= store_from) {
             stored |= 1u << st;
             mbar_arrive(bar(K_DUE0 + st));
           }
@@ -366,13 +395,17 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
 #pragma unroll 1
         for (int j = 0; j < x.n_kv; ++j) {
           const int t = T + j, st = t & 1, use = t >> 1;
-          const int row = key_row(x, j);
+          int row = packed_row(x, j);
+          const bool own = row >= 0;
+          bool packed = own;
+          if (!own) row = cached_row(x, j, packed);
+          const CUtensorMap* map = ROUTED && packed ? &tmap_value : &tmap_v;
           if (use > 0 && !(ok = wait_or_abort(bar(PV_DONE0 + st), (use - 1) & 1, abort_flag))) break;
           if (!(ok = stage_stored(stored, st, V_STORED0))) break;
           mbar_expect_tx(bar(V_FULL0 + st), KV_BYTES);
-          tma_load_3d(base + OFF_V + st * KV_BYTES, &tmap_v, bar(V_FULL0 + st), 0, kvh, row);
-          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_V + st * KV_BYTES + KV_SUB, &tmap_v, bar(V_FULL0 + st), 64, kvh, row);
-          if (p.store == Store::Tiles && j >= store_from) {
+          tma_load_3d(base + OFF_V + st * KV_BYTES, map, bar(V_FULL0 + st), 0, kvh, row);
+          if constexpr (G::NSUB == 2) tma_load_3d(base + OFF_V + st * KV_BYTES + KV_SUB, map, bar(V_FULL0 + st), 64, kvh, row);
+          if (p.store == Store::Tiles && own && j >= store_from) {
             stored |= 1u << st;
             mbar_arrive(bar(V_DUE0 + st));
           }
@@ -441,7 +474,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         (void)mbar_wait(bar(DRAIN), 0);
       }
     }
-   } else if (p.store != Store::None) {
+   } else if (p.store != Store::None && !ROUTED) {
     // -------------------------------------------------- a warp left: packed rows to the cache
     // All of them, or those that no item has a tile of: of sequences without a query row, in front of the first
     // sequence and behind the last.  A 16-byte piece of a K and a V row per lane, two such at a time.
@@ -628,7 +661,9 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
 #pragma unroll 1
         for (int j = first_stored(x, p.g); j < x.n_kv; ++j) {
           const int t = T + j, st = t & 1, r_warp = ew * 16;
-          const int64_t row0 = x.k0 + j * BN, n_rows = min(static_cast<int64_t>(min(BN, x.Lk - j * BN)), p.n_new - row0);
+          const int64_t row0 = packed_row(x, j);
+          if (row0 < 0) continue;  // read through the table: stored already
+          const int64_t n_rows = min(static_cast<int64_t>(min(BN, x.Lk - j * BN)), p.n_new - row0);
           const int slot = lane < 16 && r_warp + lane < n_rows ? slot_of(row0 + r_warp + lane) : -1;
           // A stage's barrier tells its phase by parity only, and these warps do not wait for every tile: between
           // the producer's word that the load is issued and theirs that it is stored it stays at this tile's.
@@ -718,53 +753,73 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
 
 // ---- host side ---------------------------------------------------------------------------
 
+static std::atomic<unsigned> g_launch_seq{0};  // its launches take the counter slots in turn, whatever their kernel
+
+// Heads packed into a query tile: the largest divisor of the group size that is at most 8
+// (NVLLM_PREFILL_PACK = 1..8 caps it; measurement aid, read on every call).
+static int heads_per_tile(int g) {
+  int cap = 8, pack = 1;
+  if (const char* s = std::getenv("NVLLM_PREFILL_PACK")) cap = std::atoi(s);
+  for (int n = 2; n <= 8 && n <= cap; ++n)
+    if (g % n == 0) pack = n;
+  return pack;
+}
+
+int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch) {
+  const int pack = heads_per_tile(hq / hkv), bmt = tc::BM / pack;
+  return static_cast<int64_t>((max_seqlen_q + bmt - 1) / bmt) * (hq / pack) * batch;
+}
+
 template <int D>
 static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int64_t total_k, cudaStream_t stream) {
   using G = tcp::Geo<D>;
-  static bool attr_done[64] = {false};
-  static std::atomic<unsigned> launch_seq{0};
+  static bool attr_done[64] = {false};  // of this head_dim
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return fail(NVLLM_E_NO_DEVICE, "prefill: device index %d out of range", dev);
   if (p_in.out_stride > (1 << 23)) return fail(NVLLM_E_GEOMETRY, "prefill: out row stride %lld too large", (long long)p_in.out_stride);
   if (!attr_done[dev]) {
-    cudaError_t e = cudaFuncSetAttribute(prefill_tcp_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-    if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
-    // The warp groups trade registers inside the pool the block gets at launch (threads x the kernel's
-    // register count); a build whose count is below the assumed 80 could never satisfy the softmax
-    // group's request, and that request waits without a bound.
-    cudaFuncAttributes attr;
-    e = cudaFuncGetAttributes(&attr, prefill_tcp_kernel<D>);
-    if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
-    if (attr.numRegs * tcp::NTHREADS_P < 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER))
-      return fail(NVLLM_E_CUDA, "prefill (persistent): built with %d registers per thread, the warp groups' hand-over needs %d",
-                  attr.numRegs, 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER) / tcp::NTHREADS_P);
+    for (auto kernel : {prefill_tcp_kernel<D, false>, prefill_tcp_kernel<D, true>}) {  // both: the other's first launch may be captured
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
+      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
+      // The warp groups trade registers inside the pool the block gets at launch (threads x the kernel's
+      // register count); a build whose count is below the assumed 80 could never satisfy the softmax
+      // group's request, and that request waits without a bound.
+      cudaFuncAttributes attr;
+      e = cudaFuncGetAttributes(&attr, kernel);
+      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
+      if (attr.numRegs * tcp::NTHREADS_P < 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER))
+        return fail(NVLLM_E_CUDA, "prefill (persistent): built with %d registers per thread, the warp groups' hand-over needs %d",
+                    attr.numRegs, 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER) / tcp::NTHREADS_P);
+    }
     attr_done[dev] = true;
   }
-  // heads packed into a query tile: the largest divisor of the group size that is at most 8
-  // (NVLLM_PREFILL_PACK = 1..8 caps it; measurement aid, read on every call)
-  int cap = 8;
-  if (const char* s = std::getenv("NVLLM_PREFILL_PACK")) cap = std::atoi(s);
   PrefillParams p = p_in;
-  p.pack = 1;
-  for (int n = 2; n <= 8 && n <= cap; ++n)
-    if (p.g % n == 0) p.pack = n;
+  const bool routed = p.route.jobs > 0;
+  p.pack = heads_per_tile(p.g);
   const int pack = p.pack, bmt = tc::BM / pack;
   p.tile_tokens = bmt;
   p.inv_pack = 65536 / pack + 1;  // exact for rows of a tile
-  CUtensorMap mq, mk, mv;
+  CUtensorMap mq, mk, mv, mkey, mvalue;
   if (!make_tmap_3d(&mq, p.q, D, p.hq, total_q, D, p.q_stride, bmt, pack)) return NVLLM_E_CUDA;
   if (p.block_tables) {
     const uint64_t slots = static_cast<uint64_t>(p.num_blocks) * kBlockSize;
     const uint64_t row = static_cast<uint64_t>(p.hkv) * D;
     if (!make_tmap_3d(&mk, p.k, D, p.hkv, slots, D, row, tc::BN)) return NVLLM_E_CUDA;
     if (!make_tmap_3d(&mv, p.v, D, p.hkv, slots, D, row, tc::BN)) return NVLLM_E_CUDA;
+    if (routed) {
+      if (!make_tmap_3d(&mkey, p.key, D, p.hkv, p.n_new, D, p.key_stride, tc::BN)) return NVLLM_E_CUDA;
+      if (!make_tmap_3d(&mvalue, p.value, D, p.hkv, p.n_new, D, p.value_stride, tc::BN)) return NVLLM_E_CUDA;
+    } else {
+      mkey = mk, mvalue = mv;
+    }
   } else {
     if (!make_tmap_3d(&mk, p.k, D, p.hkv, total_k, D, p.k_stride, tc::BN)) return NVLLM_E_CUDA;
     if (!make_tmap_3d(&mv, p.v, D, p.hkv, total_k, D, p.v_stride, tc::BN)) return NVLLM_E_CUDA;
+    mkey = mk, mvalue = mv;
   }
   // an upper bound of the work items known to the host: no more blocks than that
-  const int64_t max_items = static_cast<int64_t>((p.max_seqlen_q + bmt - 1) / bmt) * (p.hq / pack) * p.batch;
+  const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
   // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
@@ -774,13 +829,13 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   // as many blocks as that takes two trips of, as long as four of them are enough (6 prompts of 300 tokens: 15.8
   // us from the tiles, 20.2 copied).
   const int64_t pieces = p.n_new * p.hkv * (D / 8);
-  p.store = !p.slots ? Store::None : max_items > grid || pieces > 4ll * 64 * grid ? Store::Tiles : Store::Spare;
+  p.store = !p.slots ? Store::None : routed || max_items > grid || pieces > 4ll * 64 * grid ? Store::Tiles : Store::Spare;
   const int64_t copy_blocks = p.store == Store::Spare ? (pieces + 127) / 128 : 0;
   grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, copy_blocks)));
-  // the two head_dim instantiations share the counter array: give each its own half
-  const int slot = static_cast<int>(launch_seq.fetch_add(1) % (tcp::NUM_SLOTS / 2)) + (D == 64 ? tcp::NUM_SLOTS / 2 : 0);
-  return launch_kernel("prefill (tcgen05, persistent)", prefill_tcp_kernel<D>, dim3(grid), dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq,
-                       mk, mv, slot);
+  static_assert(sizeof(g_launch_seq) == 4 && (1ull << 32) % tcp::NUM_SLOTS == 0, "the slots follow one another when the count wraps");
+  const int slot = static_cast<int>(g_launch_seq.fetch_add(1) % tcp::NUM_SLOTS);
+  return launch_kernel("prefill (tcgen05, persistent)", routed ? prefill_tcp_kernel<D, true> : prefill_tcp_kernel<D, false>, dim3(grid),
+                       dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq, mk, mv, mkey, mvalue, slot);
 }
 
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream) {

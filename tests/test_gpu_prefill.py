@@ -160,6 +160,65 @@ def test_layer_stores_every_packed_row_from_the_key_tiles(cuda, hq, hkv, d):
     assert _lib.read_status() == 0
 
 
+@pytest.mark.parametrize("odd", [False, True])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (32, 8, 128), (14, 2, 64), (4, 4, 64)])
+def test_layer_through_the_table_reads_and_stores_new_rows_as_store_then_prefill_does(cuda, hq, hkv, d, odd):
+    """Cached blocks that were there before, that another sequence fills in the same step, and that end ragged; with
+    ``odd`` also rows without a slot, slots that are not the table's, cached tokens that end inside a block or a
+    tile, one block in two tables as new, more queries than keys, rows behind the last sequence."""
+    lq = [1, 63, 64, 65, 255, 256, 257, 700, 1000, 2000, 130, 40, 512, 900, 300, 777] * 2
+    cached = [0, 256, 512, 0, 1024, 0, 256, 0, 512, 0, 256, 0, 0, 256, 0, 0] * 2
+    if odd:
+        cached[1], cached[4], cached[20], cached[11], cached[17] = 100, 64, 500, -20, 320
+    lk = [a + c for a, c in zip(lq, cached)]
+    behind = 30 if odd else 0
+    gen = torch.Generator(device=cuda).manual_seed(9)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    width = max(lk) // 256 + 3
+    counts = [(n + 255) // 256 for n in lk]
+    blocks = sum(counts) + 5
+    ids = torch.randperm(blocks, generator=gen, device=cuda).cpu().tolist()
+    tables, at = [], 0
+    for n in counts:
+        tables.append(ids[at:at + n] + [-1] * (width - n))
+        at += n
+    tables[6][0] = tables[5][0]     # full new blocks of another sequence
+    tables[8][:2] = tables[7][:2]
+    tables[13][0] = tables[3][0]    # a block that its sequence fills only in part
+    slots = []
+    for a, c, row in zip(lq, cached, tables):
+        slots += [row[p // 256] * 256 + p % 256 if p >= 0 else -1 for p in range(c, c + a)]
+    slots = torch.tensor(slots, dtype=torch.int32)
+    if odd:
+        starts = torch.tensor([0] + lq).cumsum(0)
+        slots[starts[7] + 100] = -1
+        slots[starts[9] + 70: starts[9] + 75] = -1
+        spare = ids[-1] * 256
+        slots[starts[12]: starts[12] + 64] = torch.arange(spare, spare + 64, dtype=torch.int32)
+        tables[15][1] = tables[14][1]  # both fill it: only one of them gives it slots
+        slots[starts[15] + 256: starts[15] + 512] = -1
+        slots = torch.cat([slots, torch.arange(spare + 100, spare + 100 + behind, dtype=torch.int32)])
+    slots = slots.to(cuda)
+    n_q, n_k = sum(lq), sum(lq) + behind
+    q, k, v = rand(n_q, hq * d), rand(n_k, hkv * d), rand(n_k, 2 * hkv * d)[:, : hkv * d]
+    cu = lambda x: torch.tensor([0] + x, device=cuda).cumsum(0).int()
+    bt = torch.tensor(tables, dtype=torch.int32, device=cuda)
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+    for again in range(2):
+        k2, v2 = layer.k_cache.clone(), layer.v_cache.clone()
+        A.store_kvcache(k.view(n_k, hkv, d), v.unflatten(1, (hkv, d)), k2, v2, slots)
+        want = A.prefill_varlen(q.view(n_q, hq, d), k2, v2, cu(lq), cu(lk), max(lq), max(lk), d ** -0.5, bt)
+        C.set_context(True, cu(lq), cu(lk), max(lq), max(lk), slots, None, bt)
+        got = layer(q, k, v)
+        C.reset_context()
+        torch.cuda.synchronize()
+        assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+        assert torch.equal(got.view_as(want), want)
+        assert _lib.read_status() == 0
+        k, v, bt = -k, -v, bt.clone()
+
+
 def test_many_sequences_through_the_persistent_kernel(cuda):
     """More work items than resident blocks, and more sequences than one warp scans at once."""
     case = W.make_prefill_case(28, 150, 1, 300, 4, 2, 128, share_every=0)
