@@ -42,6 +42,8 @@
 // Small batches are bound by a chain of trips to memory: lengths, block table, K/V, then for cut
 // sequences partials out, arrival, partials in.  Table lines are fetched under the lengths, the
 // arrivals wait for nothing in the middle of a range, and a merge takes one trip for eight parts.
+// Where parts are few they are written as marked cells (kMark), so that the report of a partial needs no fence and the
+// merge's reads go out with it.
 // One launch in a chain, from a graph (head_dim 128, 16 / 8 heads): one sequence of 317 tokens 8.7 ->
 // 6.2 us, one of 4096 20.0 -> 10.7, 8 of 100-1024 16.3 -> 11.9, 16 of them 18.1 -> 14.9, 64 of them
 // 35.3 -> 32.7; 256 sequences of 2048-8192 tokens (32 / 8 heads, step variant) 795 -> 747.
@@ -97,6 +99,7 @@ struct DecodeParams {
   unsigned int* counters;  // [batch * hkv], zero between launches
   float* ws_o;             // [n_ranges + batch][hq][D]
   float* ws_ml;            // [n_ranges + batch][hq][2] = (running max in log2 units, sum)
+  bool cells;              // partials as marked cells in ws_o: [n_ranges + batch][hq][D + 2] of 8 bytes, see kMark
   int* status;
 };
 
@@ -118,6 +121,29 @@ struct DecodeCfg {
   static_assert(TT % 16 == 0 && kBlockSize % TT == 0, "a warp tile must not straddle a cache block");
   static_assert((TT * CPR) % 32 == 0, "tile copy must divide evenly over a warp");
 };
+
+// Marked cells.  A word of a partial next to a mark, 8 bytes that are written and read as one: the block that merges
+// sees for each of them whether it is there yet, so that a block that reports a partial needs no fence
+// between the partial and its arrival, and one that may have been the last to arrive reads the others' while the
+// answer is on its way.  What is read is marked only if it belongs to this launch: the block that merges takes the
+// marks off again, and no other word in a workspace is ever this one (plain partials are results of arithmetic that
+// flushes subnormal numbers to zero, which this is one of, and a workspace starts as zeros).
+constexpr uint32_t kMark = 1u;
+constexpr int kMaxPolls = 1 << 20;  // the stores are on their way when a block polls for them: far more than it takes
+
+__device__ __forceinline__ uint64_t cell(float x) { return static_cast<uint64_t>(kMark) << 32 | __float_as_uint(x); }
+__device__ __forceinline__ bool marked(const ulonglong2& c) {
+  return static_cast<uint32_t>(c.x >> 32) == kMark && static_cast<uint32_t>(c.y >> 32) == kMark;
+}
+__device__ __forceinline__ float value_of(uint64_t c) { return __uint_as_float(static_cast<uint32_t>(c)); }
+__device__ __forceinline__ void store_cells(uint64_t* at, uint64_t a, uint64_t b) {
+  asm volatile("st.relaxed.gpu.global.v2.b64 [%0], {%1, %2};" ::"l"(at), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ ulonglong2 load_cells(const uint64_t* at) {
+  ulonglong2 c;
+  asm volatile("ld.relaxed.gpu.global.v2.b64 {%0, %1}, [%2];" : "=l"(c.x), "=l"(c.y) : "l"(at) : "memory");
+  return c;
+}
 
 // The sequence a block is working in: index, global index of its first unit, units, length.
 struct SeqCursor {
@@ -143,7 +169,7 @@ constexpr float kSplitBalance = 8.f;
 // nothing of Step in it the kernel starts its loads sooner: 17.4 -> 14.9 us a layer.
 enum class Variant { Plain, Step, Guess, Layer };
 
-template <class C, Variant V>
+template <class C, Variant V, bool CELLS>
 __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const DecodeParams p) {
   constexpr bool STEP = V == Variant::Step, LAYER = V == Variant::Layer, GUESS = V == Variant::Guess || LAYER;
   constexpr int D = C::D, TT = C::TT, NST = C::NST, NW = C::NW, UNIT = C::UNIT, NT = NW * 32;
@@ -445,6 +471,14 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
 
   Cut cut0{}, cut1{};  // this range's sequences that other ranges share
   int n_cut = 0;
+  // With cells every warp that writes some reports for itself.  Its first lane: how many had before it, at the last cut
+  // and the one before that.  The former is not touched until it is needed, so that nothing waits for it.
+  unsigned int arrived = 0, arrived0 = 0;
+  const int writers = min(NW, (p.g * QUADS + 31) / 32);
+  constexpr int HEAD_CELLS = D + 2;  // of a head's partial: D columns, maximum, sum
+  auto cells_of = [&](int64_t slot, int h) {
+    return reinterpret_cast<uint64_t*>(p.ws_o) + (slot * p.hq + kvh * p.g + h) * HEAD_CELLS;
+  };
 
   // Leaves sequence cc.b: merges the NW warps' states and writes the output row or a partial.
   auto flush = [&]() {
@@ -493,13 +527,26 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       } else {
         // partial slot range + b: strictly increasing along the (range, sequence) pieces of the list
         const int64_t row = static_cast<int64_t>(range + cc.b) * p.hq + kvh * p.g + h;
-        *reinterpret_cast<float4*>(p.ws_o + row * D + d4 * 4) = acc;
-        if (d4 == 0) *reinterpret_cast<float2*>(p.ws_ml + row * 2) = make_float2(mm, L);
+        if constexpr (CELLS) {
+          uint64_t* to = cells_of(range + cc.b, h);
+          store_cells(to + d4 * 4, cell(acc.x), cell(acc.y));
+          store_cells(to + d4 * 4 + 2, cell(acc.z), cell(acc.w));
+          if (d4 == 0) store_cells(to + D, cell(mm), cell(L));
+        } else {
+          *reinterpret_cast<float4*>(p.ws_o + row * D + d4 * 4) = acc;
+          if (d4 == 0) *reinterpret_cast<float2*>(p.ws_ml + row * 2) = make_float2(mm, L);
+        }
       }
     }
-    if (n_parts > 1) {  // block-uniform; reported at the end of the range
+    if (n_parts > 1) {  // block-uniform
       if (n_cut == 0) cut0 = {cc.b, r_first, n_parts};
       else cut1 = {cc.b, r_first, n_parts};
+      if (CELLS && warp < writers) {  // reported at once: the answer is looked at when the range is done
+        __syncwarp();  // the warp's cells are on their way
+        arrived0 = arrived;
+        if (lane == 0)
+          asm volatile("atom.relaxed.gpu.global.add.u32 %0, [%1], 1;" : "=r"(arrived) : "l"(p.counters + cc.b * p.hkv + kvh) : "memory");
+      }
       ++n_cut;
     }
   };
@@ -584,6 +631,116 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       if (active && split == 0) write_quad(c.b, head, gl, acc, L);
     }
     if (tid == 0) p.counters[c.b * p.hkv + kvh] = 0u;  // ready for the next launch
+  };
+
+  // The same from cells, of both cuts, the one reported last first: its first reads are issued before it is known whether
+  // this block was the last to arrive.  Rolled up: this is run once, and its instructions are on the way to the end.
+  auto merge_cells = [&]() {
+    constexpr int AHEAD = 8;
+    const int group = tid / QUADS, gl = tid % QUADS;
+    const int n_split = max(1, GROUPS / p.g);
+    const bool narrow = p.g < GROUPS;
+    const int split = narrow ? group / p.g : 0;
+    const int64_t next = static_cast<int64_t>(p.hq) * HEAD_CELLS * n_split;  // from a part to the next one of this group's
+    int polls = 0;
+    auto was_last = [&](unsigned int before, const Cut& c) { return lane == 0 && warp < writers && before == static_cast<unsigned int>(c.n * writers - 1); };
+    const bool first_to_merge = n_cut > 1 && __syncthreads_or(was_last(arrived0, cut0));
+#pragma unroll 1
+    for (int which = n_cut - 1; which >= 0; --which) {
+      const Cut c = which ? cut1 : cut0;
+      bool ask = which == n_cut - 1;
+      if (!ask && !first_to_merge) break;
+#pragma unroll 1
+      for (int h0 = 0; h0 < p.g; h0 += GROUPS) {
+        const int head = narrow ? group % p.g : min(h0 + group, p.g - 1);
+        const bool active = narrow ? split < n_split : h0 + group < p.g;
+        // the parts of a group: split, split + n_split and so on
+        const int parts = active && c.n > split ? (c.n - split + n_split - 1) / n_split : 0;
+        uint64_t* const from = cells_of(c.r_first + c.b, head) + split * static_cast<int64_t>(p.hq) * HEAD_CELLS;
+        float mm = -INFINITY, L = 0.f, f = 0.f;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        auto rebase = [&](float m_new) {
+          const float keep = mm == -INFINITY ? 0.f : fast_exp2(mm - m_new);
+          L *= keep;
+          acc.x *= keep;
+          acc.y *= keep;
+          acc.z *= keep;
+          acc.w *= keep;
+          mm = m_new;
+        };
+        const int rounds = (c.n + n_split - 1) / n_split;  // of the group with most parts
+#pragma unroll 1
+        for (int k0 = 0; k0 < rounds; k0 += AHEAD) {
+          // a lane holds the statistics of one of QUADS parts, and four columns of AHEAD of them
+          const bool fresh_ml = k0 % QUADS == 0, have = fresh_ml && k0 + gl < parts;
+          ulonglong2 ml = make_ulonglong2(0, 0), lo[AHEAD], hi[AHEAD];
+          uint64_t* const ml_at = from + (k0 + gl) * next + D;
+          uint64_t* const row_at = from + k0 * next + gl * 4;
+          bool there;
+          do {
+            there = true;
+            if (have) ml = load_cells(ml_at);
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k)
+              if (k0 + k < parts) {
+                lo[k] = load_cells(row_at + k * next);
+                hi[k] = load_cells(row_at + k * next + 2);
+              }
+            if (ask) {  // block-uniform
+              ask = false;
+              if (!__syncthreads_or(was_last(arrived, c))) goto next_cut;
+            }
+            if (have) there = marked(ml);
+#pragma unroll
+            for (int k = 0; k < AHEAD; ++k)
+              if (k0 + k < parts) there = there && marked(lo[k]) && marked(hi[k]);
+          } while (!there && ++polls < kMaxPolls);
+          if (fresh_ml) {
+            const float m_mine = have ? value_of(ml.x) : -INFINITY;
+            float m_new = fmaxf(mm, m_mine);
+#pragma unroll
+            for (int sh = QUADS / 2; sh > 0; sh >>= 1) m_new = fmaxf(m_new, __shfl_xor_sync(0xffffffffu, m_new, sh));
+            rebase(m_new);
+            f = m_mine == -INFINITY ? 0.f : fast_exp2(m_mine - m_new);
+            float sum = have ? value_of(ml.y) * f : 0.f;
+#pragma unroll
+            for (int sh = QUADS / 2; sh > 0; sh >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, sh);
+            L += sum;
+            if (have) store_cells(ml_at, 0, 0);
+          }
+#pragma unroll
+          for (int k = 0; k < AHEAD; ++k) {
+            const float fk = __shfl_sync(0xffffffffu, f, (k0 + k) % QUADS, QUADS);
+            if (k0 + k >= parts) continue;
+            add_scaled(acc, make_float4(value_of(lo[k].x), value_of(lo[k].y), value_of(hi[k].x), value_of(hi[k].y)), fk);
+            store_cells(row_at + k * next, 0, 0);
+            store_cells(row_at + k * next + 2, 0, 0);
+          }
+        }
+        if (n_split > 1) {  // block-uniform
+          float* patch = sm_o + group * (D + 4);
+          if (active && split > 0) {
+            *reinterpret_cast<float4*>(patch + gl * 4) = acc;
+            if (gl == 0) *reinterpret_cast<float2*>(patch + D) = make_float2(mm, L);
+          }
+          __syncthreads();
+          if (active && split == 0)
+            for (int k = 1; k < n_split; ++k) {
+              const float* other = sm_o + (group + k * p.g) * (D + 4);
+              const float2 ml = *reinterpret_cast<const float2*>(other + D);
+              rebase(fmaxf(mm, ml.x));
+              const float fo = ml.x == -INFINITY ? 0.f : fast_exp2(ml.x - mm);
+              L += ml.y * fo;
+              add_scaled(acc, *reinterpret_cast<const float4*>(other + gl * 4), fo);
+            }
+        }
+        if (active && split == 0) write_quad(c.b, head, gl, acc, L);
+      }
+      if (tid == 0) p.counters[c.b * p.hkv + kvh] = 0u;  // ready for the next launch
+    next_cut:
+      __syncthreads();  // the patch and the answer have been read
+    }
+    if (polls >= kMaxPolls) atomicOr(p.status, NVLLM_STATUS_TIMEOUT);
   };
 
   // ---- 2. stream the range ------------------------------------------------------------------
@@ -707,13 +864,17 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   cp_async_wait<0>();
   if (bad && lane == 0) atomicOr(p.status, bad);
   if (n_cut == 0) return;  // block-uniform
+  if constexpr (CELLS) {
+    merge_cells();
+    return;
+  }
   __syncthreads();         // every thread's partials are written
   if (tid < n_cut) {
     const Cut& c = tid == 0 ? cut0 : cut1;
-    unsigned int arrived;  // releases the block's partials (the barrier ordered them before), acquires the others'
+    unsigned int before;  // releases the block's partials (the barrier ordered them before), acquires the others'
     asm volatile("atom.acq_rel.gpu.global.add.u32 %0, [%1], 1;"
-                 : "=r"(arrived) : "l"(p.counters + c.b * p.hkv + kvh) : "memory");
-    s_last_arrival[tid] = arrived == static_cast<unsigned int>(c.n - 1);
+                 : "=r"(before) : "l"(p.counters + c.b * p.hkv + kvh) : "memory");
+    s_last_arrival[tid] = before == static_cast<unsigned int>(c.n - 1);
   }
   __syncthreads();
   if (s_last_arrival[0]) merge_cut(cut0);
@@ -768,12 +929,15 @@ static int64_t workspace_bytes_for(int batch, int hq, int hkv, int d) {
 
 template <class C>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
+  constexpr bool HAS_CELLS = C::D == 128;
   static bool attr_set[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev >= 0 && dev < 64 && !attr_set[dev]) {  // all variants, so that the others' first launch may be captured
-    for (auto kernel : {decode_paged_kernel<C, Variant::Plain>, decode_paged_kernel<C, Variant::Step>, decode_paged_kernel<C, Variant::Guess>,
-                        decode_paged_kernel<C, Variant::Layer>}) {
+    for (auto kernel : {decode_paged_kernel<C, Variant::Plain, false>, decode_paged_kernel<C, Variant::Step, false>,
+                        decode_paged_kernel<C, Variant::Guess, false>, decode_paged_kernel<C, Variant::Layer, false>,
+                        decode_paged_kernel<C, Variant::Plain, HAS_CELLS>, decode_paged_kernel<C, Variant::Step, HAS_CELLS>,
+                        decode_paged_kernel<C, Variant::Guess, HAS_CELLS>, decode_paged_kernel<C, Variant::Layer, HAS_CELLS>}) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
       if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
     }
@@ -781,10 +945,18 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   }
   // A guess for launches with a sequence per thread at most.  Larger batches stream long enough for the trips
   // at the start not to matter, and the step kernel's predecessor in a chain is itself.
-  auto kernel = p.n_new > 0                                           ? decode_paged_kernel<C, Variant::Layer>
-                : p.k_new                                             ? decode_paged_kernel<C, Variant::Step>
-                : !p.lengths_early && p.batch <= C::NW * 32           ? decode_paged_kernel<C, Variant::Guess>
-                                                                      : decode_paged_kernel<C, Variant::Plain>;
+  const Variant v = p.n_new > 0                                 ? Variant::Layer
+                    : p.k_new                                   ? Variant::Step
+                    : !p.lengths_early && p.batch <= C::NW * 32 ? Variant::Guess
+                                                                : Variant::Plain;
+  auto pick = [v](auto cells) {
+    constexpr bool K = decltype(cells)::value;
+    return v == Variant::Layer   ? decode_paged_kernel<C, Variant::Layer, K>
+           : v == Variant::Step  ? decode_paged_kernel<C, Variant::Step, K>
+           : v == Variant::Guess ? decode_paged_kernel<C, Variant::Guess, K>
+                                 : decode_paged_kernel<C, Variant::Plain, K>;
+  };
+  auto kernel = p.cells ? pick(std::bool_constant<HAS_CELLS>{}) : pick(std::false_type{});
   const int grid = p.n_ranges * p.hkv;
   return launch_kernel("decode_paged", kernel,
                        dim3(static_cast<unsigned>(grid)), dim3(C::NW * 32), C::SMEM, stream, p);
@@ -853,6 +1025,15 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
   p.counters = static_cast<unsigned int*>(workspace);
   p.ws_o = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kCounterBytes);
   p.ws_ml = p.ws_o + rows * head_dim;
+  // Marked cells, where a sequence is cut into few parts of few bytes: else the doubled bytes and the reads for nothing
+  // cost more than the fence.  28 captured layers, 16 / 8 heads (37 ranges), 100-1024 tokens: 16 sequences 419 -> 395 us,
+  // 32 548 -> 521, 48 693 -> 668; with 12-100, 64-512 and 375-3000 tokens 16 of them 213 -> 206, 349 -> 357, 667 -> 644.
+  // A layer with its store: 8 sequences 10.25 -> 11.4, 24 of 66-200 and 170-512 tokens 10.95 -> 11.5 and 13.4 -> 12.8, 32
+  // of 100-1024 20.0 -> 19.0.  36 captured layers of 16 with 32 / 8 heads 541 -> 547.  Cells take twice the room; the
+  // workspace is sized for more thread blocks than this device takes, so that those of up to 400 / Hkv sequences fit
+  // all the same.
+  p.cells = (n_new > 0 ? 4 * p.n_ranges <= 5 * batch : p.n_ranges <= 3 * batch) && p.g <= 2 && head_dim == 128 &&
+            (p.n_ranges + static_cast<int64_t>(batch)) * num_q_heads * 2 <= rows;
 
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   if (head_dim == 128) return launch_decode<DecodeCfg<128, NVLLM_DEC_TT, NVLLM_DEC_NST, NVLLM_DEC_NW>>(p, st);

@@ -221,6 +221,25 @@ def test_sequences_cut_into_many_parts(cuda, hq, hkv, d, lens):
     assert torch.equal(got.view_as(dev.q), A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, dev.scale))
 
 
+@pytest.mark.parametrize("batch", [12, 13, 14, 32, 53, 54, 55])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (8, 8, 128), (32, 8, 64)])
+def test_cut_sequences_around_the_sizes_of_marked_cells(cuda, batch, hq, hkv, d):
+    """Partials as marked cells and plain ones in turn in one workspace: nothing that one launch leaves is taken for a
+    partial of the next.  Many parts beside sequences of a few units and empty ones."""
+    lens = ([5000, 64, 0, 65, 129, 700, 1] * 8)[:batch]
+    case = W.make_decode_case(29, batch, 1, 1, hq, hkv, d, context_lens=lens)
+    few = W.make_decode_case(30, 2, 1, 1, hq, hkv, d, context_lens=[4000, 300]).to(cuda)
+    outs = [_check(cuda, case, f"batch {batch}", store_first=False)]
+    dev = case.to(cuda)
+    for _ in range(3):
+        A.decode_paged(few.q, few.k_cache, few.v_cache, few.context_lens, few.block_tables, few.scale)
+        outs.append(A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, case.scale))
+        outs.append(A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, case.scale))
+    torch.cuda.synchronize()
+    assert all(torch.equal(o, outs[0]) for o in outs[1:])
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("batch", [1, 2, 31, 32, 33])
 @pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
 def test_layer_equals_store_then_decode_wherever_the_slots_lie(cuda, batch, hq, hkv, d):
