@@ -673,12 +673,16 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
             if (!(ok = wait_or_abort(bar((kv ? V_FULL0 : K_FULL0) + st), (t >> 1) & 1, abort_flag))) break;
             const uint32_t src = base + (kv ? OFF_V : OFF_K) + st * KV_BYTES + (piece >> 3) * KV_SUB + r_warp * 128;
             __nv_bfloat16* cache = (kv ? p.v_store : p.k_store) + col;
-#pragma unroll 8
-            for (int r0 = 0; r0 < 16; r0 += ROWS) {
-              const int r = r0 + lane / PIECES;
-              const int to = __shfl_sync(0xffffffffu, slot, r);
-              if (to >= 0)
-                *reinterpret_cast<uint4*>(cache + to * row_elems) = ld_shared16(src + r * 128 + (((piece ^ r) & 7) << 4));
+            uint4 v[16 / ROWS];
+#pragma unroll
+            for (int i = 0; i < 16 / ROWS; ++i) {  // all in flight before the first is written: one after the other took 1700 cycles
+              const int r = i * ROWS + lane / PIECES;
+              v[i] = ld_shared16(src + r * 128 + (((piece ^ r) & 7) << 4));
+            }
+#pragma unroll
+            for (int i = 0; i < 16 / ROWS; ++i) {
+              const int to = __shfl_sync(0xffffffffu, slot, i * ROWS + lane / PIECES);
+              if (to >= 0) *reinterpret_cast<uint4*>(cache + to * row_elems) = v[i];
             }
             __syncwarp();
             if (lane == 0) mbar_arrive(bar((kv ? V_STORED0 : K_STORED0) + st));
