@@ -26,7 +26,8 @@
 // Order of the items: sequences longest first (ranked in shared memory by every block at start-up,
 // for batches of up to SORT_BATCH sequences), a sequence's long tiles first, head groups fastest.
 // The blocks that are still busy when the counter runs out are then working on the cheapest
-// items, so the launch ends without a tail of half-idle SMs.
+// items, so the launch ends without a tail of half-idle SMs.  Where there are no more items than blocks the
+// sequences' long tiles go first instead.
 //
 // Item hand-off: the producer lane decodes an item into one of two descriptor slots in shared
 // memory (ITEM_FULL / ITEM_FREE barriers).  All rings keep running across items: tile t of the
@@ -292,6 +293,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
+      const bool spread = p.batch > 1 && total_items <= static_cast<int>(gridDim.x);
       int T = 0;   // key tiles loaded so far in this block's life
       unsigned stored = 0;
       // Item number -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
@@ -339,6 +341,16 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       unsigned next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
 #pragma unroll 1
       for (int it = 0;; ++it) {
+        if (spread && next_idx < static_cast<unsigned>(total_items)) {
+          // No more items than blocks: every q-th of the list in turn, so that all sequences' long tiles come first, and
+          // the blocks that share an SM with them get short ones (6 prompts of 300 tokens 15.6 -> 14.0 us, 10 of 100 12.3 ->
+          // 11.6, 3 of 500 15.6 -> 15.1).
+          const int n_tiles = prefix[p.batch], pi = next_idx / hgroups, q = (n_tiles + p.batch - 1) / p.batch, full = n_tiles / q;
+          const int rest = n_tiles - full * q, split = rest * (full + 1);
+          const int col = pi < split ? pi / (full + 1) : rest + (pi - split) / full;
+          const int row = pi - (pi < split ? col * (full + 1) : split + (col - rest) * full);
+          next_idx += (row * q + col - pi) * hgroups;
+        }
         const Item x = decode_item(next_idx);
         if (it >= 2 && !wait_or_abort(bar(ITEM_FREE0 + (it & 1)), ((it >> 1) - 1) & 1, abort_flag)) break;
         volatile int* s = slots + (it & 1) * 8;

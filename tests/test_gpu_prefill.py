@@ -219,6 +219,14 @@ def test_layer_through_the_table_reads_and_stores_new_rows_as_store_then_prefill
         k, v, bt = -k, -v, bt.clone()
 
 
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64), (2, 2, 64)])
+@pytest.mark.parametrize("lengths", [[300] * 6, [1, 700], [129, 1, 64, 65, 257, 3, 2, 128], [64] * 18, [63] * 19])
+def test_every_item_of_a_launch_with_an_item_to_a_block(cuda, hq, hkv, d, lengths):
+    """The items of several short prompts go out in another order than the list's: none twice, none left out."""
+    case = W.make_prefill_case(47, len(lengths), 1, 1, hq, hkv, d, lengths=lengths, share_every=0)
+    _check(cuda, case, f"{lengths} hq{hq} d{d}")
+
+
 def test_many_sequences_through_the_persistent_kernel(cuda):
     """More work items than resident blocks, and more sequences than one warp scans at once."""
     case = W.make_prefill_case(28, 150, 1, 300, 4, 2, 128, share_every=0)
