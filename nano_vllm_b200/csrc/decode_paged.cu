@@ -930,18 +930,24 @@ static int64_t workspace_bytes_for(int batch, int hq, int hkv, int d) {
 template <class C>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   constexpr bool HAS_CELLS = C::D == 128;
-  static bool attr_set[64] = {false};
+  // All variants at once, so that the others' first launch may be captured; those with cells when the first of them is
+  // launched (loading a kernel costs the process about a millisecond).
+  static bool attr_set[2][64] = {{false}};
   int dev = 0;
   cudaGetDevice(&dev);
-  if (dev >= 0 && dev < 64 && !attr_set[dev]) {  // all variants, so that the others' first launch may be captured
-    for (auto kernel : {decode_paged_kernel<C, Variant::Plain, false>, decode_paged_kernel<C, Variant::Step, false>,
-                        decode_paged_kernel<C, Variant::Guess, false>, decode_paged_kernel<C, Variant::Layer, false>,
-                        decode_paged_kernel<C, Variant::Plain, HAS_CELLS>, decode_paged_kernel<C, Variant::Step, HAS_CELLS>,
-                        decode_paged_kernel<C, Variant::Guess, HAS_CELLS>, decode_paged_kernel<C, Variant::Layer, HAS_CELLS>}) {
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
+  auto reserve = [](auto cells) {
+    constexpr bool K = decltype(cells)::value;
+    for (auto kernel : {decode_paged_kernel<C, Variant::Plain, K>, decode_paged_kernel<C, Variant::Step, K>,
+                        decode_paged_kernel<C, Variant::Guess, K>, decode_paged_kernel<C, Variant::Layer, K>}) {
+      const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
       if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
     }
-    attr_set[dev] = true;
+    return NVLLM_OK;
+  };
+  if (dev >= 0 && dev < 64 && !attr_set[p.cells][dev]) {
+    const int rc = p.cells ? reserve(std::bool_constant<HAS_CELLS>{}) : reserve(std::false_type{});
+    if (rc) return rc;
+    attr_set[p.cells][dev] = true;
   }
   // A guess for launches with a sequence per thread at most.  Larger batches stream long enough for the trips
   // at the start not to matter, and the step kernel's predecessor in a chain is itself.
