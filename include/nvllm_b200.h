@@ -89,7 +89,8 @@ NVLLM_API int nvllm_store_kvcache(const void* key, int64_t key_row_stride,
  * thread block that delivers the last of them merges them (no second kernel).
  * `workspace`: nvllm_decode_workspace_bytes(...) bytes for the same (batch, Hq, Hkv, D),
  * 16-byte aligned.  Its first 64 KiB are arrival counters: ZERO-FILL THE WORKSPACE ONCE before
- * its first use; every completed call leaves the counters at zero again, so one workspace can
+ * its first use, and let nothing but these calls write to it; every completed call leaves the counters
+ * at zero again and the marks on its partials taken off, so one workspace can
  * serve all later calls, of any geometry, that do not overlap on the GPU.
  * Supported: D in {64,128}; Hq % Hkv == 0; G <= 8; batch * Hkv <= 16384.
  */
@@ -168,10 +169,10 @@ NVLLM_API int nvllm_decode_plan(int32_t batch, int32_t max_blocks, int32_t num_q
  *   - the first call on each device looks up the array's device address (with that device
  *     current); make that first call outside stream capture;
  *   - all calls on a device share the one array, which still holds whatever the previous
- *     call left there.  Only the arrival counters at its head have to start at zero: they do
- *     when the library is loaded, and the thread block that merges a sequence puts its counter
- *     back to zero, so a completed call leaves them cleared.  Partials are written before they
- *     are read within one call.  Two calls whose kernels may run at the same time on one GPU
+ *     call left there.  The arrival counters at its head have to start at zero and the rest without
+ *     a marked partial: it is all zeros when the library is loaded, and the thread block that merges a
+ *     sequence puts its counter back to zero and takes the marks off, so a completed call leaves it as it
+ *     has to be.  Partials are written before they are read within one call.  Two calls whose kernels may run at the same time on one GPU
  *     (different streams, or graphs replayed concurrently) would disturb each other's counters
  *     and partials — keep calls to this entry point ordered on a device.
  */
@@ -218,10 +219,12 @@ NVLLM_API int nvllm_prefill_varlen(const void* q, int64_t q_row_stride,
  * does for every step (nanovllm/layers/attention.py:65-77), with the same arguments and results.
  * One launch for a decode of up to 32 sequences and for a prefill of packed rows; else two, of which the
  * second reads its lengths while the first still runs, which two separate calls may not do because
- * they do not know what ran before them.  n_new / total_k:
+ * they do not know what ran before them.  The first of the two stores the rows, or, for a prefill through the
+ * table that keeps all SMs busy, works out which of them the second may read from key / value and
+ * store itself.  n_new / total_k:
  * rows of key / value and entries of slot_mapping (all of them are stored, as by
  * nvllm_store_kvcache: num_slots = 256 * num_blocks).  Prefill reads key / value where
- * block_tables is NULL, and the cache through the table otherwise.
+ * block_tables is NULL, and otherwise what the cache holds through the table once all rows are stored.
  */
 NVLLM_API int nvllm_attention_decode(const void* q, int64_t q_row_stride,
                       const void* key, int64_t key_row_stride,

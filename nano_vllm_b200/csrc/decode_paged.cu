@@ -127,8 +127,8 @@ struct DecodeCfg {
 // between the partial and its arrival, and one that may have been the last to arrive reads the others' while the
 // answer is on its way.  What is read is marked only if it belongs to this launch: the block that merges takes the
 // marks off again, and no other word in a workspace is ever this one (plain partials are results of arithmetic that
-// flushes subnormal numbers to zero, which this is one of, and a workspace starts as zeros).
-constexpr uint32_t kMark = 1u;
+// flushes subnormal numbers to zero, and a workspace starts as zeros).
+constexpr uint32_t kMark = 0x0059c3a7u;  // as a float subnormal
 constexpr int kMaxPolls = 1 << 20;  // the stores are on their way when a block polls for them: far more than it takes
 
 __device__ __forceinline__ uint64_t cell(float x) { return static_cast<uint64_t>(kMark) << 32 | __float_as_uint(x); }
@@ -1175,7 +1175,8 @@ extern "C" int nvllm_decode_paged_static(const void* q, int64_t q_row_stride, co
   // What must start at zero are the arrival counters at the head of the array.  They are zero
   // when the library is loaded, and the block that merges a sequence's partials puts its
   // counter back to zero, so every completed call leaves them cleared for the next one.  The
-  // partials themselves are always written before they are read within one call.
+  // partials themselves are always written before they are read within one call, and the marks of those that
+  // are marked cells are taken off by the block that reads them.
   return nvllm_decode_paged(q, q_row_stride, k_cache, v_cache, context_lens, block_tables, bt_row_stride, max_blocks,
                             out, out_row_stride, batch, num_q_heads, num_kv_heads, head_dim, scale, num_blocks,
                             scratch, kStaticScratchBytes, stream);

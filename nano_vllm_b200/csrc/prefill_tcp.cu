@@ -42,7 +42,7 @@
 // Code size: the warps of a block run seven different loops at the same time, and what they have to fetch of them
 // is on the path of each: in a kernel of 84 KB (loops unrolled as the compiler likes, barrier waits of 25
 // instructions, barriers set up one after the other by one thread) every fifth cycle of a warp waited for
-// instructions.  Hence the loops that are kept rolled here, the short wait, and no division for a row's token: 57 KB;
+// instructions.  Hence the loops that are kept rolled here, the short wait, and no division for a row's token: 57-59 KB;
 // one prompt of 201 tokens 9.5 -> 9.05 us, of 1000 19.1 -> 18.1, 64 of 100-1024 tokens 136 -> 123.
 #include <algorithm>
 #include <atomic>
@@ -840,7 +840,7 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
   // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
   // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
-  // rows, 4 KB in flight; 123 from the tiles; 111 with nothing to store).  Where a block has one item at most that
+  // rows, 4 KB in flight; 120 from the tiles; 110 with nothing to store).  Where a block has one item at most that
   // would end it later (a prompt of 201 tokens 9.05 -> 9.5 us): there an idle warp of every block copies the rows, by
   // as many blocks as that takes two trips of, as long as four of them are enough (6 prompts of 300 tokens: 15.8
   // us from the tiles, 20.2 copied).
