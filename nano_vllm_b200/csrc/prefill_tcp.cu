@@ -714,7 +714,9 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       const int srow = lane >> 2, spiece = lane & 3;
       __nv_bfloat16* out_tile = p.out + static_cast<int64_t>(x.q0 + x.m0) * p.out_stride + x.h * D;
       const int toks_valid = min(BMT, x.Lq - x.m0);
-#pragma unroll 4
+      // unrolled where a block has few items (a prompt of 201 tokens 9.0 us, 9.1 rolled up); through the route tables it
+      // has many, and the instructions count (64 prompts 121 -> 118.6)
+#pragma unroll (ROUTED ? 1 : 4)
       for (int c = 0; c < OCH; ++c) {
         uint32_t o[32];
         tmem_ld32(tmem_o + lane_addr + c * 32, o);

@@ -126,3 +126,36 @@ def test_launches_by_rows_equal_those_by_heads(cuda, hq, hkv, d, n, norm):
     assert torch.equal(results[0][0].view(torch.int16), results[1][0].view(torch.int16))
     assert torch.equal(results[0][1].view(torch.int16), results[1][1].view(torch.int16))
     assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("n", [63, 64, 300])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
+def test_positions_written_by_the_kernel_just_before(cuda, n, hq, hkv, d):
+    """The positions are rows of a cache that the launch in front stores to, the last of many: the step, which may
+    fetch its table rows by the positions of the time before, must use the new ones."""
+    max_pos, eps = 4096, 1e-6
+    gen = torch.Generator(device=cuda).manual_seed(n)
+    table = R.rotary_cache_ref(d, max_pos, 1e6).to(cuda)
+    plane = torch.zeros(2, 256, 1, 256, dtype=torch.bfloat16, device=cuda)  # rows of 64 int64
+    positions = plane[1].view(-1).view(torch.int64)[:n]
+    scratch = torch.zeros_like(plane)
+    slots = torch.arange(511, -1, -1, dtype=torch.int32, device=cuda)
+    x = torch.randn(n, (hq + 2 * hkv) * d, generator=gen, device=cuda).bfloat16()
+    steps = []
+    for i in range(5):
+        now = torch.randint(0, max_pos, (n,), generator=gen, device=cuda)
+        flat = torch.zeros(256 * 64, dtype=torch.int64, device=cuda)
+        flat[:n] = now
+        key = torch.zeros(512, 64, dtype=torch.int64, device=cuda)
+        key[:256] = flat.view(256, 64).flip(0)
+        steps.append((now, key.view(torch.bfloat16).view(512, 1, 256), x.clone()))
+    run = lambda qkv, at: A.qk_norm_rope_store(qkv, at, None, None, table, eps, None, torch.empty(0), torch.empty(0), hq, hkv, d)
+    torch.cuda.synchronize()
+    for now, key, got in steps:
+        A.store_kvcache(key, key, plane, scratch, slots)
+        run(got, positions)
+    torch.cuda.synchronize()
+    for now, _, got in steps:
+        want = x.clone()
+        run(want, now)
+        assert torch.equal(got, want)
