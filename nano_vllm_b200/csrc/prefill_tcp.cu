@@ -293,7 +293,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
-      const bool spread = p.batch > 1 && total_items <= static_cast<int>(gridDim.x);
+      const bool spread = D == 128 && p.batch > 1 && total_items <= static_cast<int>(gridDim.x);
       int T = 0;   // key tiles loaded so far in this block's life
       unsigned stored = 0;
       // Item number -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
@@ -344,7 +344,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         if (spread && next_idx < static_cast<unsigned>(total_items)) {
           // No more items than blocks: every q-th of the list in turn, so that all sequences' long tiles come first, and
           // the blocks that share an SM with them get short ones (6 prompts of 300 tokens 15.6 -> 14.0 us, 10 of 100 12.3 ->
-          // 11.6, 3 of 500 15.6 -> 15.1).
+          // 11.6, 3 of 500 15.6 -> 15.1; at head_dim 64, 14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05: not there).
           const int n_tiles = prefix[p.batch], pi = next_idx / hgroups, q = (n_tiles + p.batch - 1) / p.batch, full = n_tiles / q;
           const int rest = n_tiles - full * q, split = rest * (full + 1);
           const int col = pi < split ? pi / (full + 1) : rest + (pi - split) / full;
