@@ -214,6 +214,10 @@ NVLLM_API int nvllm_prefill_varlen(const void* q, int64_t q_row_stride,
                          int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim,
                          float scale, int64_t num_blocks, void* stream);
 
+/* Which item of the list (query tiles of all sequences, head groups fastest) the drawn-th draw stands for in a prefill
+ * launch whose items are dealt out long tiles first.  Host arithmetic, exposed for tests. */
+NVLLM_API int nvllm_prefill_item(int32_t drawn, int32_t query_tiles, int32_t batch, int32_t head_groups);
+
 /*
  * nvllm_store_kvcache followed by nvllm_decode_paged / nvllm_prefill_varlen, as the attention layer
  * does for every step (nanovllm/layers/attention.py:65-77), with the same arguments and results.

@@ -111,6 +111,13 @@ extern "C" int nvllm_prefill_varlen(const void* q, int64_t q_row_stride, const v
                                num_q_heads, num_kv_heads, head_dim, scale, num_blocks, stream, false, nullptr, nullptr, nullptr);
 }
 
+extern "C" int nvllm_prefill_item(int32_t drawn, int32_t query_tiles, int32_t batch, int32_t head_groups) {
+  using namespace nvllm;
+  if (batch <= 0 || query_tiles <= 0 || head_groups <= 0 || drawn < 0 || drawn >= static_cast<int64_t>(query_tiles) * head_groups)
+    return fail(NVLLM_E_GEOMETRY, "prefill_item: drawn=%d query_tiles=%d batch=%d head_groups=%d invalid", drawn, query_tiles, batch, head_groups);
+  return spread_item(drawn, query_tiles, batch, head_groups);
+}
+
 extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
                                        const void* value, int64_t value_row_stride, const int32_t* slot_mapping, void* k_cache,
                                        void* v_cache, const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks,

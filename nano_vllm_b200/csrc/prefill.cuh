@@ -58,6 +58,17 @@ struct PrefillParams {
   int64_t value_stride;
 };
 
+// Order of a launch with no more items than blocks: every q-th query tile of the list in turn, q the sequences' mean, so
+// that all sequences' long tiles come first.  The item that the n-th draw of such a launch stands for; each of its
+// items for one draw, which is what makes the launch complete whatever block draws when.
+__host__ __device__ __forceinline__ int spread_item(int drawn, int n_tiles, int batch, int hgroups) {
+  const int pi = drawn / hgroups, q = (n_tiles + batch - 1) / batch, full = n_tiles / q;
+  const int rest = n_tiles - full * q, split = rest * (full + 1);
+  const int col = pi < split ? pi / (full + 1) : rest + (pi - split) / full;
+  const int row = pi - (pi < split ? col * (full + 1) : split + (col - rest) * full);
+  return drawn + (row * q + col - pi) * hgroups;
+}
+
 // Sequences per launch of the persistent kernel (its per-sequence tables live in shared memory).
 // The engine schedules at most 512 sequences per step (nanovllm/config.py:10).
 constexpr int kPrefillMaxBatch = 1024;

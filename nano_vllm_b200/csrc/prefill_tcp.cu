@@ -293,17 +293,21 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
+      // With an item to a block the blocks that share an SM with those of long tiles get short ones by that (6 prompts of
+      // 300 tokens 15.6 -> 14.0 us, 10 of 100 12.3 -> 11.6, 3 of 500 15.6 -> 15.1; at head_dim 64, 14 / 2 heads, 6 of
+      // 100-300 tokens 9.65 -> 10.05: not there).
       const bool spread = D == 128 && p.batch > 1 && total_items <= static_cast<int>(gridDim.x);
       int T = 0;   // key tiles loaded so far in this block's life
       unsigned stored = 0;
-      // Item number -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
+      // Number drawn -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
       // working side by side share K/V tiles in L2.
-      auto decode_item = [&](unsigned idx) {
+      auto decode_item = [&](unsigned drawn) {
         Item x;
 #pragma unroll 1
         while (true) {
           x.n_kv = -1;
-          if (idx >= static_cast<unsigned>(total_items)) break;
+          if (drawn >= static_cast<unsigned>(total_items)) break;
+          const int idx = spread ? spread_item(drawn, prefix[p.batch], p.batch, hgroups) : static_cast<int>(drawn);
           const int pi = idx / hgroups;
           x.h = (idx - pi * hgroups) * pack;  // first of the packed heads
           int lo = 0, hi = p.batch;  // largest i with prefix[i] <= pi
@@ -329,7 +333,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
 #pragma unroll 1
             for (int c = 0; c < PIECES * pack; ++c) dst[c] = make_uint4(0, 0, 0, 0);  // the packed heads are adjacent
           }
-          idx = atomicAdd(&g_item_counter[counter_slot], 1u);
+          drawn = atomicAdd(&g_item_counter[counter_slot], 1u);
         }
         return x;
       };
@@ -338,20 +342,10 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       // the end of the current item instead of in front of the next one.  Not earlier: an item
       // reserved long before its block is free is an item that an idle block cannot take (measured:
       // reserving at the start of the current item cost 9 % on four 4096-token sequences).
-      unsigned next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
+      unsigned next_draw = atomicAdd(&g_item_counter[counter_slot], 1u);
 #pragma unroll 1
       for (int it = 0;; ++it) {
-        if (spread && next_idx < static_cast<unsigned>(total_items)) {
-          // No more items than blocks: every q-th of the list in turn, so that all sequences' long tiles come first, and
-          // the blocks that share an SM with them get short ones (6 prompts of 300 tokens 15.6 -> 14.0 us, 10 of 100 12.3 ->
-          // 11.6, 3 of 500 15.6 -> 15.1; at head_dim 64, 14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05: not there).
-          const int n_tiles = prefix[p.batch], pi = next_idx / hgroups, q = (n_tiles + p.batch - 1) / p.batch, full = n_tiles / q;
-          const int rest = n_tiles - full * q, split = rest * (full + 1);
-          const int col = pi < split ? pi / (full + 1) : rest + (pi - split) / full;
-          const int row = pi - (pi < split ? col * (full + 1) : split + (col - rest) * full);
-          next_idx += (row * q + col - pi) * hgroups;
-        }
-        const Item x = decode_item(next_idx);
+        const Item x = decode_item(next_draw);
         if (it >= 2 && !wait_or_abort(bar(ITEM_FREE0 + (it & 1)), ((it >> 1) - 1) & 1, abort_flag)) break;
         volatile int* s = slots + (it & 1) * 8;
         s[0] = x.b; s[1] = x.h; s[2] = x.m0; s[3] = x.q0;
@@ -369,7 +363,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         bool ok = true;
 #pragma unroll 1
         for (int j = 0; j < x.n_kv; ++j) {
-          if (j == max(0, x.n_kv - 3)) next_idx = atomicAdd(&g_item_counter[counter_slot], 1u);
+          if (j == max(0, x.n_kv - 3)) next_draw = atomicAdd(&g_item_counter[counter_slot], 1u);
           const int t = T + j, st = t & 1, use = t >> 1;
           int row = packed_row(x, j);
           const bool own = row >= 0;

@@ -227,6 +227,31 @@ def test_every_item_of_a_launch_with_an_item_to_a_block(cuda, hq, hkv, d, length
     _check(cuda, case, f"{lengths} hq{hq} d{d}")
 
 
+@pytest.mark.parametrize("repeat", range(4))
+def test_items_without_a_visible_key_where_blocks_start_late(cuda, repeat):
+    """An item to a block, some of them tiles in front of all keys (more queries than keys), for which a block draws again:
+    a launch on another stream keeps all SMs but one, so that its blocks draw twice before others have drawn at all."""
+    hq, hkv, d = 16, 8, 128
+    lq, lk = [300] * 5, [300, 50, 300, 50, 300][repeat % 2:] + [300] * (repeat % 2)
+    gen = torch.Generator().manual_seed(48 + repeat)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()
+    q, k, v = rand(sum(lq), hq, d), rand(sum(lk), hkv, d), rand(sum(lk), hkv, d)
+    cu = lambda x: torch.tensor([0] + x).cumsum(0).int()
+    other = torch.cuda.Stream()
+    rows = (128 * (torch.cuda.get_device_properties(cuda).multi_processor_count - 1), 65536, 65536)  # all blocks but two
+    longer = [torch.randn(n, 2, d, device=cuda).bfloat16() for n in rows]
+    ends = [torch.tensor([0, n], dtype=torch.int32, device=cuda) for n in rows[:2]]
+    args = [t.to(cuda) for t in (q, k, v, cu(lq), cu(lk))]
+    out = torch.full((sum(lq), hq, d), float("nan"), dtype=torch.bfloat16, device=cuda)
+    torch.cuda.synchronize()
+    with torch.cuda.stream(other):
+        A.prefill_varlen(*longer, *ends, *rows[:2], d ** -0.5)
+    A.prefill_varlen(*args, max(lq), max(lk), d ** -0.5, out=out)
+    torch.cuda.synchronize()
+    assert_close_to_oracle(out, R.prefill_ref(q, k, v, cu(lq), cu(lk), d ** -0.5), f"{lk}")
+    assert _lib.read_status() == 0
+
+
 def test_many_sequences_through_the_persistent_kernel(cuda):
     """More work items than resident blocks, and more sequences than one warp scans at once."""
     case = W.make_prefill_case(28, 150, 1, 300, 4, 2, 128, share_every=0)

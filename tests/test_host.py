@@ -137,6 +137,20 @@ def test_sampler_takes_no_larger_cluster_than_the_device_grants(lib, sms):
     assert lib.nvllm_sample_plan(1, 151936, sms, 8) == 8 and lib.nvllm_sample_plan(1, 0, sms, 8) == -3
 
 
+@pytest.mark.parametrize("batch,tiles", [(2, 10), (2, 3), (6, 30), (7, 7), (9, 5), (20, 21), (3, 296), (5, 37)])
+def test_every_item_is_drawn_once_whatever_block_draws_when(lib, batch, tiles):
+    """The order of a launch with an item to a block: a permutation of the list, so that blocks that draw again (for a
+    tile without a visible key) before others have drawn at all leave nothing out."""
+    groups = 296 // tiles
+    total = tiles * groups
+    items = [lib.nvllm_prefill_item(n, tiles, batch, groups) for n in range(total)]
+    assert sorted(items) == list(range(total))
+    assert [i % groups for i in items] == [n % groups for n in range(total)]  # head groups fastest, as in the list
+    stride = -(-tiles // batch)
+    assert [i // groups for i in items[:(tiles // stride) * groups:groups]] == list(range(0, tiles // stride * stride, stride))
+    assert lib.nvllm_prefill_item(total, tiles, batch, groups) == -3 and lib.nvllm_prefill_item(0, tiles, 0, groups) == -3
+
+
 def test_fused_projection_tile_choice_is_host_arithmetic(lib):
     """Tile width of the projection fused with its all-reduce: the narrowest of 32 / 64 / 128 columns
     that leaves one tile per thread block (128 blocks), 0 for shapes the kernel refuses."""
