@@ -56,10 +56,12 @@ __global__ void __launch_bounds__(256) prefill_route_kernel(const RouteParams p)
     if (slot >= n_slots) atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
     return slot >= 0 && slot < n_slots ? static_cast<int>(slot) : -1;
   };
-  // rows behind the last sequence
-  for (int64_t r = p.cu_q[p.batch] + job; r < p.n_new; r += gridDim.x) {
-    const int slot = slot_of(r);
-    for (int i = tid; slot >= 0 && i < p.per_row; i += 256) copy_row(r, slot, i);
+  // rows of no sequence: in front of the first and behind the last
+  const int64_t front = p.cu_q[0], in_sequences = p.cu_q[p.batch] - front;
+  for (int64_t r = job; r < p.n_new - in_sequences; r += gridDim.x) {
+    const int64_t row = r < front ? r : r + in_sequences;
+    const int slot = slot_of(row);
+    for (int i = tid; slot >= 0 && i < p.per_row; i += 256) copy_row(row, slot, i);
   }
 
   // the job's sequence: the last one whose first job is not behind this one

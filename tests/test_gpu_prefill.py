@@ -219,6 +219,45 @@ def test_layer_through_the_table_reads_and_stores_new_rows_as_store_then_prefill
         k, v, bt = -k, -v, bt.clone()
 
 
+@pytest.mark.parametrize("front", [1, 255, 256, 700])
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
+def test_layer_through_the_table_stores_rows_in_front_of_the_first_sequence(cuda, hq, hkv, d, front):
+    """More items than blocks and cu_seqlens_q[0] > 0: the rows in front belong to no sequence and are stored like those
+    behind the last."""
+    lq, cached, behind = [700, 300, 64, 1000, 513] * 4, [0, 256, 512, 0, 256] * 4, 3
+    lk = [a + c for a, c in zip(lq, cached)]
+    gen = torch.Generator(device=cuda).manual_seed(front)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    counts = [(n + 255) // 256 for n in lk]
+    blocks = sum(counts) + 8
+    ids = torch.randperm(blocks, generator=gen, device=cuda).cpu().tolist()
+    tables, slots, at = [], [], 0
+    for a, c, n in zip(lq, cached, counts):
+        tables.append(ids[at:at + n] + [-1] * (max(counts) - n))
+        slots += [tables[-1][p // 256] * 256 + p % 256 for p in range(c, c + a)]
+        at += n
+    spare = [b * 256 + i for b in ids[at:] for i in range(256)]
+    slots = torch.tensor(spare[:front] + slots + spare[front:front + behind], dtype=torch.int32, device=cuda)
+    slots[1 + front // 2] = -1
+    n = front + sum(lq) + behind
+    q, k, v = rand(n, hq * d), rand(n, hkv * d), rand(n, hkv * d)
+    cu_q = (torch.tensor([0] + lq, device=cuda).cumsum(0) + front).int()
+    cu_k = torch.tensor([0] + lk, device=cuda).cumsum(0).int()
+    bt = torch.tensor(tables, dtype=torch.int32, device=cuda)
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+    k2, v2 = layer.k_cache.clone(), layer.v_cache.clone()
+    A.store_kvcache(k.view(n, hkv, d), v.view(n, hkv, d), k2, v2, slots)
+    want = A.prefill_varlen(q.view(n, hq, d), k2, v2, cu_q, cu_k, max(lq), max(lk), d ** -0.5, bt)
+    C.set_context(True, cu_q, cu_k, max(lq), max(lk), slots, None, bt)
+    got = layer(q, k, v)
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+    assert torch.equal(got.view_as(want)[front:n - behind], want[front:n - behind])
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64), (2, 2, 64)])
 @pytest.mark.parametrize("lengths", [[300] * 6, [1, 700], [129, 1, 64, 65, 257, 3, 2, 128], [64] * 18, [63] * 19])
 def test_every_item_of_a_launch_with_an_item_to_a_block(cuda, hq, hkv, d, lengths):
