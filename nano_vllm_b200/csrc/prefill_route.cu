@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(256) prefill_route_kernel(const RouteParams p)
   __shared__ int s_slot[kBlockSize];
   __shared__ int s_match[kBlockSize / 32];
   __shared__ int s_shared, s_twice;
+  __shared__ int s_keys[kPrefillMaxBatch], s_cached[kPrefillMaxBatch];  // of every sequence
 
   auto copy_row = [&](int64_t row, int64_t slot, int piece) {
     p.k_cache[slot * p.per_row + piece] = __ldg(p.key + row * p.key_stride16 + piece);
@@ -68,12 +69,17 @@ __global__ void __launch_bounds__(256) prefill_route_kernel(const RouteParams p)
   int before = 0;
   for (int b0 = 0; b0 < p.batch; b0 += 256) {
     const int b = b0 + tid;
-    before += __syncthreads_count(b < p.batch && route_first_job(p.cu_q[b], b) <= job);
+    int q0 = 0;
+    if (b < p.batch) {
+      q0 = p.cu_q[b];
+      s_keys[b] = p.cu_k[b + 1] - p.cu_k[b];
+      s_cached[b] = s_keys[b] - (p.cu_q[b + 1] - q0);
+    }
+    before += __syncthreads_count(b < p.batch && route_first_job(q0, b) <= job);
   }
   int n = 0, x = -1, i = 0, q0 = 0, off = 0, lk = 0, b = before - 1;
   if (b >= 0) {
-    q0 = p.cu_q[b], lk = p.cu_k[b + 1] - p.cu_k[b];
-    off = lk - (p.cu_q[b + 1] - q0);
+    q0 = p.cu_q[b], lk = s_keys[b], off = s_cached[b];
     i = (off >> 8) + job - route_first_job(q0, b);  // block of the sequence; negative where there are more queries than keys
     n = min((i + 1) * kBlockSize, lk) - max(i * kBlockSize, off);
   }
@@ -97,15 +103,31 @@ __global__ void __launch_bounds__(256) prefill_route_kernel(const RouteParams p)
   __syncthreads();
   const bool whole = off >= 0 && i * kBlockSize >= off && x >= 0;  // no cached token in the block
   if (whole) {  // block-uniform
-    for (int e = tid; e < p.batch * p.max_blocks; e += 256) {
-      const int b2 = e / p.max_blocks, i2 = e - b2 * p.max_blocks;
-      if (p.block_tables[b2 * p.bt_stride + i2] != x || (b2 == b && i2 == i)) continue;
-      const int lk2 = p.cu_k[b2 + 1] - p.cu_k[b2];
-      if (i2 * kBlockSize < lk2 - (p.cu_q[b2 + 1] - p.cu_q[b2])) {
-        p.out.source[e] = job;
-        s_shared = 1;
-      } else if (i2 * kBlockSize < lk2) {
-        s_twice = 1;  // two sequences' new rows in one block: no telling whose rows it ends up with
+    // The table entries that are in use, of all sequences: eight lanes to a sequence, four sequences at a time.
+    // Padding is not looked at: with whole rows 64 prompts of 100-1024 tokens took 149 us through a table 160 wide and
+    // 140 through one 4 wide, 100 of 20-150 tokens 59 and 36; now 139 and 35.5 through either.
+    for (int b0 = tid >> 3; b0 < p.batch; b0 += 128) {
+      int used[4], most = 0;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        used[u] = b0 + 32 * u < p.batch ? min((s_keys[b0 + 32 * u] + kBlockSize - 1) / kBlockSize, p.max_blocks) : 0;
+        most = max(most, used[u]);
+      }
+      for (int i2 = tid & 7; i2 < most; i2 += 8) {
+        int entry[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) entry[u] = i2 < used[u] ? __ldg(p.block_tables + (b0 + 32 * u) * p.bt_stride + i2) : -1;
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int b2 = b0 + 32 * u;
+          if (entry[u] != x || (b2 == b && i2 == i)) continue;
+          if (i2 * kBlockSize < s_cached[b2]) {
+            p.out.source[b2 * p.max_blocks + i2] = job;
+            s_shared = 1;
+          } else {
+            s_twice = 1;  // two sequences' new rows in one block: no telling whose rows it ends up with
+          }
+        }
       }
     }
   }

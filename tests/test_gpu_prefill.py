@@ -1,4 +1,6 @@
 """Varlen causal GQA prefill on the GPU, through the C ABI, against the fp32 CPU oracle."""
+import random
+
 import pytest
 import torch
 
@@ -255,6 +257,51 @@ def test_layer_through_the_table_stores_rows_in_front_of_the_first_sequence(cuda
     torch.cuda.synchronize()
     assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
     assert torch.equal(got.view_as(want)[front:n - behind], want[front:n - behind])
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (4, 2, 128)])
+@pytest.mark.parametrize("batch,width", [(16, 1024), (33, 9), (129, 127), (300, 54), (300, 55)])
+def test_layer_through_wide_tables_finds_blocks_that_others_fill(cuda, hq, hkv, d, batch, width):
+    """Every third sequence has blocks of the one before it cached, up to ten of them and behind others of its own; tables
+    near and past the largest that are routed, and more sequences than one trip of the search takes."""
+    r = random.Random(batch)
+    lq = [r.choice([1, 64, 257, 300, 513, 700]) for _ in range(batch)]
+    lq[1], lq[7], lq[batch - 2] = 2300, 2560, 1024
+    cached, tables, fresh = [], [], 0
+    for i in range(batch):
+        own = list(range(fresh, fresh + (i % 4 == 2)))  # a block that was there before
+        fresh += len(own)
+        if i % 3 == 2:
+            own += tables[i - 1][cached[i - 1] // 256:][:min(lq[i - 1] // 256, width - 5)]
+        if len(own) + 4 > width or len(own) * 256 + lq[i] > width * 256:
+            own, lq[i] = own[:1], min(lq[i], 700)
+        cached.append(len(own) * 256)
+        n = (lq[i] + 255) // 256
+        tables.append(own + list(range(fresh, fresh + n)))
+        fresh += n
+    lk = [a + c for a, c in zip(lq, cached)]
+    gen = torch.Generator(device=cuda).manual_seed(batch)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    perm = torch.randperm(fresh + 2, generator=gen, device=cuda).cpu()
+    tables = [[int(perm[x]) for x in row] for row in tables]
+    slots = [row[p // 256] * 256 + p % 256 for a, c, row in zip(lq, cached, tables) for p in range(c, c + a)]
+    slots = torch.tensor(slots, dtype=torch.int32, device=cuda)
+    bt = torch.tensor([row + [-1] * (width - len(row)) for row in tables], dtype=torch.int32, device=cuda)
+    n = sum(lq)
+    q, k, v = rand(n, hq * d), rand(n, hkv * d), rand(n, hkv * d)
+    cu = lambda x: torch.tensor([0] + x, device=cuda).cumsum(0).int()
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = rand(fresh + 2, 256, hkv, d), rand(fresh + 2, 256, hkv, d)
+    k2, v2 = layer.k_cache.clone(), layer.v_cache.clone()
+    A.store_kvcache(k.view(n, hkv, d), v.view(n, hkv, d), k2, v2, slots)
+    want = A.prefill_varlen(q.view(n, hq, d), k2, v2, cu(lq), cu(lk), max(lq), max(lk), d ** -0.5, bt)
+    C.set_context(True, cu(lq), cu(lk), max(lq), max(lk), slots, None, bt)
+    got = layer(q, k, v)
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+    assert torch.equal(got.view_as(want), want)
     assert _lib.read_status() == 0
 
 
