@@ -132,12 +132,17 @@ extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, cons
                       total_k * num_kv_heads * head_dim / 8 < (1ll << 30);  // indexed with 32 bits
   // Or, where blocks work on several items one after the other, they read this step's rows packed too and store them on the
   // way, with the tables of prefill_route.cu: 64 prompts of 100-1024 tokens, some with cached prefixes, 16 / 8 heads
-  // 137 -> 120 us, 8 of 1500-2048 120 -> 113, 8 of 100-1024 29.5 -> 26.7; at 14 / 2 heads of 64 0.5 us in 76.  With an
-  // item to a block the copy is the shorter way (4 prompts of 300-400 tokens 15.6, 16.0 with the tables).
+  // 161 -> 140 us (chain of three inputs), 8 of 1500-2048 114 -> 105, 8 of 100-1024 27.1 -> 24.4, whatever the table's width.
+  // With an item to a block the copy is the shorter way (4 prompts of 300-400 tokens 15.6, 16.0 with the tables).  So it
+  // is where the tables' blocks have few bytes each to save: at 4 / 2 heads of 128, 100 prompts of 20-150 tokens (36 KB a
+  // block) gain 10 %, 200 of 30-100 (29) 1 %, 256 of 20-64 (19) lose 7 %, 400 of 10-40 (12) 9 %; at 14 / 2 heads of 64, 64 of
+  // 100-1024 (63) gain 0.4 %, 100 of 20-150 (18) lose 1 %, 200 of 30-100 (15) 6 %; at 7 / 1 and 8 / 1 heads the sign changes
+  // between 15 and 30 too.
   const bool routed = block_tables && batch > 0 && batch <= kPrefillMaxBatch && max_blocks > 0 && !forced_mma() && total_q > 0 &&
                       max_seqlen_q > 0 && total_k >= total_q && total_k < kRouteRagged && route_jobs(total_k, batch) <= kRouteJobs &&
                       static_cast<int64_t>(batch) * max_blocks <= kRouteEntries && num_kv_heads > 0 && num_q_heads > 0 &&
                       num_q_heads % num_kv_heads == 0 &&
+                      total_k * num_kv_heads * head_dim * 4 >= kRouteJobBytes * route_jobs(total_k, batch) &&
                       prefill_max_items(num_q_heads, num_kv_heads, max_seqlen_q, batch) > 2 * num_sms();
   const int rc = store_kvcache(!inside && !routed, key, key_row_stride, value, value_row_stride, k_cache, v_cache, slot_mapping, total_k,
                                num_kv_heads * head_dim, num_blocks * kBlockSize, stream);

@@ -19,6 +19,7 @@ struct RouteTables {
 };
 constexpr int kRouteRagged = 1 << 30;  // in tile_row: the sequence ends inside the tile; rows for that sequence only
 constexpr int kRouteJobs = 2048, kRouteEntries = 16384;  // the tables' sizes
+constexpr int64_t kRouteJobBytes = 24 << 10;  // new rows of K and V per job from which on the tables are worth their launch
 __host__ __device__ __forceinline__ int route_first_job(int q0, int b) { return (q0 >> 8) + 2 * b; }
 inline int64_t route_jobs(int64_t n_new, int batch) { return (n_new >> 8) + 2 * static_cast<int64_t>(batch); }
 
