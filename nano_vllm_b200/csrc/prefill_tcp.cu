@@ -26,8 +26,8 @@
 // Order of the items: sequences longest first (ranked in shared memory by every block at start-up,
 // for batches of up to SORT_BATCH sequences), a sequence's long tiles first, head groups fastest.
 // The blocks that are still busy when the counter runs out are then working on the cheapest
-// items, so the launch ends without a tail of half-idle SMs.  Where there are no more items than blocks the
-// sequences' long tiles go first instead.
+// items, so the launch ends without a tail of half-idle SMs.  Where there are no more items than blocks, of prompts of
+// about one length, all sequences' long tiles go first instead.
 //
 // Item hand-off: the producer lane decodes an item into one of two descriptor slots in shared
 // memory (ITEM_FULL / ITEM_FREE barriers).  All rings keep running across items: tile t of the
@@ -293,10 +293,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
-      // With an item to a block the blocks that share an SM with those of long tiles get short ones by that (6 prompts of
-      // 300 tokens 15.6 -> 14.0 us, 10 of 100 12.3 -> 11.6, 3 of 500 15.6 -> 15.1; at head_dim 64, 14 / 2 heads, 6 of
-      // 100-300 tokens 9.65 -> 10.05: not there).
-      const bool spread = D == 128 && p.batch > 1 && total_items <= static_cast<int>(gridDim.x);
+      const bool spread = D == 128 && total_items > p.spread_from && total_items <= static_cast<int>(gridDim.x);
       int T = 0;   // key tiles loaded so far in this block's life
       unsigned stored = 0;
       // Number drawn -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
@@ -834,6 +831,15 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
   int grid = 2 * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
+  // With an item to a block and more items than SMs, blocks that share an SM with those of long tiles get short ones by
+  // another order: 6 prompts of 300 tokens 15.1 -> 13.4 us, 10 of 100 11.4 -> 10.4, 3 of 500 14.6 -> 14.1.  Which blocks
+  // meet on an SM is the hardware's choice, so this is a matter of averages: of 448 launches of 2-40 prompts (eight
+  // pairs of head counts) the 346 that the rule takes are 6 % faster in the mean, twelve of them 1-10 % slower (22 of
+  // 381-420 tokens, 2 / 1 heads, 12.9 -> 14.4).  Not where an SM has one block (the divisions cost 0.3 us: 5 prompts of 60
+  // tokens 8.2 -> 8.5), where long and short prompts mix, whose tiles every q-th of the list does not line up (19 of
+  // 209-582 16.0 -> 17.3), nor at head_dim 64 (14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05).
+  const bool alike = p.max_seqlen_q <= 5 * bmt || 20ll * p.max_seqlen_q * p.batch <= 23 * total_q;
+  p.spread_from = p.batch > 1 && alike ? num_sms() : 1 << 30;
   // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
   // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
   // rows, 4 KB in flight; 120 from the tiles; 110 with nothing to store).  Where a block has one item at most that
