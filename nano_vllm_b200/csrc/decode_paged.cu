@@ -930,8 +930,8 @@ static int64_t workspace_bytes_for(int batch, int hq, int hkv, int d) {
 template <class C>
 static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   constexpr bool HAS_CELLS = C::D == 128;
-  // All variants at once, so that the others' first launch may be captured; those with cells when the first of them is
-  // launched (loading a kernel costs the process about a millisecond).
+  // All variants at once; those with cells when the first of them is launched (loading a kernel costs the process about a
+  // millisecond).  That may be inside a capture.
   static bool attr_set[2][64] = {{false}};
   int dev = 0;
   cudaGetDevice(&dev);

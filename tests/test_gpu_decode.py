@@ -1,4 +1,8 @@
 """Paged GQA decode on the GPU, through the C ABI, against the fp32 CPU oracle."""
+import subprocess
+import sys
+from pathlib import Path
+
 import pytest
 import torch
 
@@ -376,3 +380,63 @@ def test_head_sharded_ranks_reassemble_the_unsharded_result(cuda, tp):
     ref = R.decode_ref(case.q, case.k_cache, case.v_cache, case.context_lens, case.block_tables, case.scale)
     assert_close_to_oracle(torch.cat(parts, dim=1), ref, f"tp{tp}")
     assert (torch.cat(parts, dim=1).float() - full.float()).abs().max().item() <= 2e-2
+
+
+SMALL_THEN_CAPTURE = """
+import sys
+import torch
+from nano_vllm_b200 import _lib, attention as A, context as C, workloads as W
+dev = torch.device("cuda:0")
+
+
+def decode(batch, one_launch):
+    c = W.make_decode_case(50 + batch, batch, 1, 1, 16, 8, 128, context_lens=([700, 64, 1000, 129] * 8)[:batch], device=dev).to(dev)
+    if one_launch is None:
+        return lambda: A.decode_paged(c.q, c.k_cache, c.v_cache, c.context_lens, c.block_tables, c.scale)
+    if one_launch:
+        return lambda: A.decode_step(c.q, c.k_new, c.v_new, c.k_cache, c.v_cache, c.slot_mapping, c.context_lens, c.block_tables, c.scale)
+    layer = A.Attention(16, 128, c.scale, 8)
+    layer.k_cache, layer.v_cache = c.k_cache, c.v_cache
+
+    def run():
+        C.set_context(False, slot_mapping=c.slot_mapping, context_lens=c.context_lens, block_tables=c.block_tables)
+        return layer(c.q.view(batch, -1), c.k_new.view(batch, -1), c.v_new.view(batch, -1))
+    return run
+
+
+def prefill(batch):
+    c = W.make_prefill_case(60 + batch, batch, 1, 1, 16, 8, 128, lengths=([700, 300, 1000, 600] * 8)[:batch], device=dev).to(dev)
+    layer = A.Attention(16, 128, c.scale, 8)
+    layer.k_cache, layer.v_cache = c.k_cache, c.v_cache
+
+    def run():
+        C.set_context(True, c.cu_seqlens_q, c.cu_seqlens_k, c.max_seqlen_q, c.max_seqlen_k, c.slot_mapping, None, c.block_tables)
+        return layer(c.q.view(c.q.shape[0], -1), c.k.view(c.q.shape[0], -1), c.v.view(c.q.shape[0], -1))
+    return run
+
+
+kind = sys.argv[1]
+small, large = {"plain": (decode(2, None), decode(16, None)), "step": (decode(2, True), decode(16, True)),
+                "layer": (decode(2, False), decode(32, False)), "prefill": (prefill(2), prefill(16))}[kind]
+small()
+torch.cuda.synchronize()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    got = large()
+for _ in range(2):
+    graph.replay()
+torch.cuda.synchronize()
+replayed = got.clone()
+assert torch.equal(large(), replayed) and replayed.abs().max() > 0
+assert _lib.read_status() == 0
+print("captured")
+"""
+
+
+@pytest.mark.parametrize("kind", ["plain", "step", "layer", "prefill"])
+def test_a_larger_batch_may_be_captured_after_a_small_one_has_run(cuda, kind):
+    """The first call of a head_dim sets up whatever kernel a later one of it takes, so that this one may be the first inside
+    a capture: a process of its own, as every kernel has run here already."""
+    root = Path(__file__).resolve().parents[1]
+    done = subprocess.run([sys.executable, "-c", SMALL_THEN_CAPTURE, kind], cwd=root, capture_output=True, text=True, timeout=300)
+    assert done.returncode == 0 and "captured" in done.stdout, done.stderr[-2000:]
