@@ -126,9 +126,11 @@ struct DecodeCfg {
 // sees for each of them whether it is there yet, so that a block that reports a partial needs no fence
 // between the partial and its arrival, and one that may have been the last to arrive reads the others' while the
 // answer is on its way.  What is read is marked only if it belongs to this launch: the block that merges takes the
-// marks off again, and no other word in a workspace is ever this one (plain partials are results of arithmetic that
-// flushes subnormal numbers to zero, and a workspace starts as zeros).
-constexpr uint32_t kMark = 0x0059c3a7u;  // as a float subnormal
+// marks off again, and no other word in a workspace is ever this one: a workspace starts as zeros, and plain partials are
+// results of single-precision arithmetic, whose only NaN is 0x7fffffff, whatever becomes of subnormal numbers.
+constexpr uint32_t kMark = 0x7f99c3a7u;
+static_assert((kMark & 0x7f800000u) == 0x7f800000u && (kMark & 0x007fffffu) != 0 && (kMark & 0x00400000u) == 0,
+              "as a float a signalling NaN: no operation returns one");
 constexpr int kMaxPolls = 1 << 20;  // the stores are on their way when a block polls for them: far more than it takes
 
 __device__ __forceinline__ uint64_t cell(float x) { return static_cast<uint64_t>(kMark) << 32 | __float_as_uint(x); }

@@ -244,6 +244,24 @@ def test_cut_sequences_around_the_sizes_of_marked_cells(cuda, batch, hq, hkv, d)
     assert _lib.read_status() == 0
 
 
+@pytest.mark.parametrize("value", [float("nan"), float("inf"), 1e-38])
+def test_no_partial_of_another_launch_is_taken_for_a_marked_cell(cuda, value):
+    """Plain partials that are NaN, infinite or next to zero, over the whole area that the marked cells of the next launch
+    lie in."""
+    case = W.make_decode_case(44, 32, 1, 1, 16, 8, 128, context_lens=([700, 64, 0, 129, 1000, 300] * 6)[:32])
+    want = _check(cuda, case, "marked", store_first=False)
+    dev = case.to(cuda)
+    few = W.make_decode_case(45, 11, 1, 1, 16, 8, 128, context_lens=[3000] * 11).to(cuda)  # 37 ranges, 47 partials
+    few.v_cache.fill_(value)
+    for _ in range(3):
+        A.decode_paged(few.q, few.k_cache, few.v_cache, few.context_lens, few.block_tables, few.scale)
+        got = A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, dev.block_tables, case.scale)
+        torch.cuda.synchronize()
+        assert torch.equal(got, want)
+        few.k_cache.fill_(value)
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("batch", [1, 2, 31, 32, 33])
 @pytest.mark.parametrize("hq,hkv,d", [(16, 8, 128), (14, 2, 64)])
 def test_layer_equals_store_then_decode_wherever_the_slots_lie(cuda, batch, hq, hkv, d):
