@@ -60,7 +60,8 @@ extern "C" {
 /* bits of the device status word */
 #define NVLLM_STATUS_BAD_SLOT 1  /* store_kvcache saw slot >= num_slots (row skipped) */
 #define NVLLM_STATUS_BAD_BLOCK 2 /* a block_tables entry in use was outside [0,num_blocks) */
-#define NVLLM_STATUS_TIMEOUT 4   /* a bounded in-kernel wait expired; that launch's output is invalid */
+#define NVLLM_STATUS_TIMEOUT 4   /* a bounded in-kernel wait expired; that launch's output is invalid, and a
+                                  * decode workspace that it used has to be zero-filled again */
 
 /*
  * Scatter the new tokens' K and V rows into the paged cache.
@@ -91,7 +92,9 @@ NVLLM_API int nvllm_store_kvcache(const void* key, int64_t key_row_stride,
  * 16-byte aligned.  Its first 64 KiB are arrival counters: ZERO-FILL THE WORKSPACE ONCE before
  * its first use, and let nothing but these calls write to it; every completed call leaves the counters
  * at zero again and the marks on its partials taken off, so one workspace can
- * serve all later calls, of any geometry, that do not overlap on the GPU.
+ * serve all later calls, of any geometry, that do not overlap on the GPU.  A call that reports
+ * NVLLM_STATUS_TIMEOUT may leave marks behind, which a later call would take for its own partials:
+ * zero-fill the workspace again before the next call.
  * Supported: D in {64,128}; Hq % Hkv == 0; G <= 8; batch * Hkv <= 16384.
  */
 NVLLM_API int nvllm_decode_paged(const void* q, int64_t q_row_stride,
@@ -172,7 +175,8 @@ NVLLM_API int nvllm_decode_plan(int32_t batch, int32_t max_blocks, int32_t num_q
  *     call left there.  The arrival counters at its head have to start at zero and the rest without
  *     a marked partial: it is all zeros when the library is loaded, and the thread block that merges a
  *     sequence puts its counter back to zero and takes the marks off, so a completed call leaves it as it
- *     has to be.  Partials are written before they are read within one call.  Two calls whose kernels may run at the same time on one GPU
+ *     has to be.  (After NVLLM_STATUS_TIMEOUT nvllm_read_status zeroes the array when it reports it.)
+ *     Partials are written before they are read within one call.  Two calls whose kernels may run at the same time on one GPU
  *     (different streams, or graphs replayed concurrently) would disturb each other's counters
  *     and partials — keep calls to this entry point ordered on a device.
  */
@@ -444,7 +448,9 @@ NVLLM_API int nvllm_selftest_wait_expiry(int32_t* device_result, void* stream);
 NVLLM_API const char* nvllm_last_error(void);
 
 /* Copies the current device's status word to *host_out and clears it.  Synchronises the
- * device: call it between steps, never during stream capture.  Returns 0 or NVLLM_E_*.
+ * device: call it between steps, never during stream capture.  When it reports
+ * NVLLM_STATUS_TIMEOUT it also zeroes the scratch array of nvllm_decode_paged_static; workspaces
+ * that callers own are theirs to zero-fill.  Returns 0 or NVLLM_E_*.
  * No counterpart in the reference. */
 NVLLM_API int nvllm_read_status(int32_t* host_out);
 

@@ -134,9 +134,12 @@ def check(code: int) -> None:
 
 
 def read_status() -> int:
-    """Returns and clears the current device's status word (synchronises the device)."""
+    """Returns and clears the current device's status word (synchronises the device).  A wait that ran out (bit 4) may
+    have left half of a launch's partials in the decode scratch: it is zeroed, as when it was made."""
     out = c_int32(0)
     check(load().nvllm_read_status(ctypes.byref(out)))
+    if out.value & 4 and _host is not None:
+        _host.clear_workspaces()
     return out.value
 
 

@@ -83,6 +83,10 @@ int nvllm_read_status(int32_t* host_out) {
   int32_t v = 0;
   cudaError_t e = cudaMemcpy(&v, dev, sizeof(v), cudaMemcpyDeviceToHost);
   if (e == cudaSuccess) e = cudaMemset(dev, 0, sizeof(int));
+  if (e == cudaSuccess && (v & NVLLM_STATUS_TIMEOUT)) {
+    e = cudaDeviceSynchronize();
+    if (e == cudaSuccess) e = nvllm::clear_static_scratch();
+  }
   if (e != cudaSuccess) return nvllm::fail(NVLLM_E_CUDA, "nvllm_read_status: %s", cudaGetErrorString(e));
   *host_out = v;
   return NVLLM_OK;

@@ -15,6 +15,8 @@ namespace nvllm {
 int fail(int code, const char* fmt, ...);
 // Device address of this device's status word (one per device, created on first use).
 int* status_word();
+// Zeroes what nvllm_decode_paged_static keeps on the current device and waits for that.
+cudaError_t clear_static_scratch();
 // Adds n to the process-wide launch counter.
 void count_launch(int n = 1);
 // Wraps cudaGetLastError() after a launch.

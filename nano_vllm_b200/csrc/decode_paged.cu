@@ -1154,6 +1154,14 @@ static int static_scratch(void** out) {
   return NVLLM_OK;
 }
 
+cudaError_t clear_static_scratch() {
+  int dev = -1;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess || dev < 0 || dev >= 64 || !g_static_scratch_addr[dev]) return e;  // not in use on this device
+  e = cudaMemset(g_static_scratch_addr[dev], 0, kStaticScratchBytes);
+  return e == cudaSuccess ? cudaDeviceSynchronize() : e;
+}
+
 }  // namespace nvllm
 
 extern "C" int nvllm_decode_paged_static(const void* q, int64_t q_row_stride, const void* k_cache,

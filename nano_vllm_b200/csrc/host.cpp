@@ -166,6 +166,18 @@ void workspace(const at::Tensor& like, int64_t nbytes, void** p, int64_t* size) 
   *size = ws.numel();
 }
 
+// Zeroes the current device's buffers, outgrown ones too (after a launch whose waits ran out), and waits for that.
+PyObject* clear_workspaces(PyObject* const*) {
+  const c10::DeviceIndex dev = c10::cuda::current_device();
+  std::vector<at::Tensor> all = g_workspaces;
+  all.insert(all.end(), g_retired.begin(), g_retired.end());
+  for (const at::Tensor& ws : all)
+    if (ws.defined() && ws.device().index() == dev) ws.zero_();
+  const c10::cuda::CUDAStream st = c10::cuda::getCurrentCUDAStream(dev);
+  unlocked([&] { st.synchronize(); });
+  Py_RETURN_NONE;
+}
+
 // ---- the operations -----------------------------------------------------------------------
 
 // Rows of [n, heads, d] with unit inner stride and d between heads.
@@ -772,6 +784,7 @@ PyObject* call(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   {#name, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(&call<name, nargs>)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     METHOD(bind, 2),
+    METHOD(clear_workspaces, 0),
     METHOD(store_kvcache, 5),
     METHOD(decode_paged, 7),
     METHOD(decode_step, 10),

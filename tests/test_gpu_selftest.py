@@ -39,3 +39,28 @@ def test_bounded_wait_expires_with_a_status_not_a_hang(cuda, lib):
     # the context still works and the status word is clear again
     x = torch.ones(8, device=cuda)
     assert float(x.sum()) == 8.0 and _lib.read_status() == 0
+
+
+def test_decode_after_an_expired_wait(cuda, lib):
+    """Reading the expired wait zeroes the decode scratch, the library's own and that of the host path: calls, captured
+    ones too, go on as before."""
+    from nano_vllm_b200 import attention as A, workloads as W
+    case = W.make_decode_case(46, 16, 1, 1, 16, 8, 128, context_lens=[700, 64, 1000, 129] * 4).to(cuda)
+    args = (case.q, case.k_cache, case.v_cache, case.context_lens, case.block_tables, case.scale)
+    out = torch.empty_like(case.q)
+    want = A.decode_paged(*args)
+    A.decode_paged_static(*args, out=out)
+    assert torch.equal(out, want)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        captured = A.decode_paged(*args)
+    res = torch.zeros(2, dtype=torch.int32, device=cuda)
+    _lib.check(lib.nvllm_selftest_wait_expiry(res.data_ptr(), torch.cuda.current_stream().cuda_stream))
+    assert _lib.read_status() & 4
+    for _ in range(2):
+        graph.replay()
+        out.zero_()
+        A.decode_paged_static(*args, out=out)
+        assert torch.equal(A.decode_paged(*args), want) and torch.equal(out, want) and torch.equal(captured, want)
+    assert _lib.read_status() == 0

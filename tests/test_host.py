@@ -178,3 +178,30 @@ def test_oracle_row_parallel_projection_rounds_every_rank_once():
     whole = (torch.cat(xs, 1).float() @ torch.cat(ws, 1).float().t()).to(torch.bfloat16)
     assert got.shape == whole.shape and not torch.equal(got, whole)
     assert float((got.float() - whole.float()).abs().max()) <= 4 * 2.0 ** -8 * float(whole.float().abs().max())
+
+
+@pytest.mark.parametrize("status", range(8))
+def test_reading_an_expired_wait_zeroes_the_decode_scratch(monkeypatch, status):
+    """Marks that such a launch leaves would be taken for a later one's partials; other bits leave the scratch alone."""
+    import ctypes
+
+    from nano_vllm_b200 import _lib
+    cleared = []
+
+    class Library:
+        @staticmethod
+        def nvllm_read_status(out):
+            ctypes.cast(out, ctypes.POINTER(ctypes.c_int32))[0] = status
+            return 0
+
+    class Host:
+        @staticmethod
+        def clear_workspaces():
+            cleared.append(True)
+
+    monkeypatch.setattr(_lib, "_lib", Library)
+    monkeypatch.setattr(_lib, "_host", Host)
+    assert _lib.read_status() == status
+    assert len(cleared) == (status >= 4)
+    monkeypatch.setattr(_lib, "_host", None)  # no call has been made: there is nothing to clear
+    assert _lib.read_status() == status
