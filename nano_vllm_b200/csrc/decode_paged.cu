@@ -1034,12 +1034,20 @@ static int decode_common(const char* who, const void* q, int64_t q_row_stride, c
   p.ws_o = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + kCounterBytes);
   p.ws_ml = p.ws_o + rows * head_dim;
   // Marked cells, where a sequence is cut into few parts of few bytes: else the doubled bytes and the reads for nothing
-  // cost more than the fence.  28 captured layers, 16 / 8 heads (37 ranges), 100-1024 tokens: 16 sequences 419 -> 395 us,
-  // 32 548 -> 521, 48 693 -> 668; with 12-100, 64-512 and 375-3000 tokens 16 of them 213 -> 206, 349 -> 357, 667 -> 644.
-  // A layer with its store: 8 sequences 10.25 -> 11.4, 24 of 66-200 and 170-512 tokens 10.95 -> 11.5 and 13.4 -> 12.8, 32
-  // of 100-1024 20.0 -> 19.0.  36 captured layers of 16 with 32 / 8 heads 541 -> 547.  Cells take twice the room; the
-  // workspace is sized for more thread blocks than this device takes, so that those of up to 400 / Hkv sequences fit
-  // all the same.
+  // cost more than the fence.  How many parts there are depends on lengths that only the device has; where a range has two
+  // or three units of a chain of layers, cells lose 1-2 %, so that the line is one of averages.  us for 28 captured
+  // layers of 2 query heads to a KV head, without -> with, by KV heads (ranges), batch and tokens:
+  //   8 (37)    13 of 12-100 214 -> 205, of 64-512 315 -> 290, of 100-1024 382 -> 368, of 375-3000 566 -> 551; 16 214 -> 208, 348 ->
+  //             356, 416 -> 391, 667 -> 647; 24 221 -> 214, 372 -> 380, 488 -> 473; 54 311 -> 281, 517 -> 492
+  //   4 (74)    25 205 -> 199, 310 -> 301, 372 -> 370, 560 -> 549; 32 of 64-512 335 -> 341; 48 218 -> 210, 364 -> 366, 457 -> 445;
+  //             108 307 -> 285, 524 -> 497
+  //   2 (148)   50 208 -> 201, 307 -> 303, 361 -> 366, 543 -> 527; 96 215 -> 208, 360 -> 364, 465 -> 440; 216 344 -> 322, 566 -> 537
+  //   1 (296)   99 211 -> 203, 312 -> 303, 359 -> 367, 563 -> 543; 256 317 -> 297, 471 -> 453, 604 -> 581; 400 351 -> 328, 828 -> 793
+  // The step variant gains everywhere (1-10 %; 16 of 64-512, 8 KV heads, 11.1 -> 10.3 us, 50 of them, 2 KV heads, 10.1 -> 9.2).  A
+  // layer with its store: 8 sequences of 100-1024 10.25 -> 11.4, 24 of 66-200 10.95 -> 11.5; 30-32 of 12-100 7.4 -> 7.4, of
+  // 64-512 14.2 -> 13.5, of 100-1024 19.2 -> 18.3.  4 query heads to a KV head: 36 captured layers of 16 541 -> 547.  Cells take
+  // twice the room; the workspace is sized for more thread blocks than this device takes, so that those of up to
+  // 400 / Hkv sequences fit all the same.
   p.cells = (n_new > 0 ? 4 * p.n_ranges <= 5 * batch : p.n_ranges <= 3 * batch) && p.g <= 2 && head_dim == 128 &&
             (p.n_ranges + static_cast<int64_t>(batch)) * num_q_heads * 2 <= rows;
 
