@@ -228,7 +228,7 @@ NVLLM_API int nvllm_prefill_item(int32_t drawn, int32_t query_tiles, int32_t bat
  * One launch for a decode of up to 32 sequences and for a prefill of packed rows; else two, of which the
  * second reads its lengths while the first still runs, which two separate calls may not do because
  * they do not know what ran before them.  The first of the two stores the rows, or, for a prefill through the
- * table that keeps all SMs busy, works out which of them the second may read from key / value and
+ * table that keeps all SMs busy with rows enough to save, works out which of them the second may read from key / value and
  * store itself.  n_new / total_k:
  * rows of key / value and entries of slot_mapping (all of them are stored, as by
  * nvllm_store_kvcache: num_slots = 256 * num_blocks).  Prefill reads key / value where
