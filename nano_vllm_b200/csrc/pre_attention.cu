@@ -147,7 +147,6 @@ constexpr int64_t kAheadFromTokens = 64;
 template <int D, bool AHEAD>
 __global__ void __launch_bounds__(kPreThreads) pre_attention_kernel(const PreAttnParams p) {
   pdl_trigger();  // lets the attention kernel that follows get its blocks resident early
-  if (!AHEAD) pdl_wait();
   constexpr int LANES = D / 8;  // lanes of a head
   const int sub = threadIdx.x & (LANES - 1);
   const unsigned heads = p.hq + 2 * p.hkv;
@@ -157,6 +156,11 @@ __global__ void __launch_bounds__(kPreThreads) pre_attention_kernel(const PreAtt
   const unsigned tok = live ? unit / heads : 0;
   const int head = live ? static_cast<int>(unit - tok * heads) : 0;
   uint4* row = reinterpret_cast<uint4*>(p.qkv + tok * p.row_stride + static_cast<int64_t>(head) * D) + sub;
+  // The row on its way to L2 (where whatever is still written to it goes too): its trip after the wait is then one to L2
+  // even while the attention kernel behind brings its first tiles there (28 captured layers of 16 sequences 380 -> 375 us,
+  // 24 at 14 / 2 heads of 64 167 -> 162).
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(row));
+  if (!AHEAD) pdl_wait();
   int64_t guess = 0;
   if (AHEAD) {
     guess = clamp_position(__ldcg(reinterpret_cast<const long long*>(p.positions) + tok), p.max_position);  // goes round L1
