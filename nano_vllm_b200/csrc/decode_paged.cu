@@ -158,17 +158,18 @@ struct Cut {
   int b, r_first, n;
 };
 
-// Cost of a streamed unit over the cost of a merged partial: of 1, 2, 4, 8 and no limit, 8 was the best or
-// within 0.6 us of it at every size of one to eight sequences of 300 to 32000 tokens (one sequence of
-// 32000 in the head_dim 64 geometry: 16.1 us, 26.1 without a limit).
-constexpr float kSplitBalance = 8.f;
+// Cost of a streamed unit over the cost of a merged partial.  With merges of eight parts to a trip, us at 8 -> 16 -> 32: 36
+// captured layers (32 / 8 heads) of two sequences of 500-4000 tokens 411 -> 358 -> 358, of one of 1050 281 -> 279 -> 289, of
+// four of 100-1024 292.5 -> 294.5 -> 294.7; 28 (16 / 8 heads) of two of 500-4000 280 -> 264 -> 264; a layer of one of 4096 8.53 ->
+// 8.12 -> 8.24, of two of 30000-32000 (14 / 2 heads of 64) 17.0 -> 17.45 -> 18.6.
+constexpr float kSplitBalance = 16.f;
 
 // The four kernels.  Step and Layer also store the new tokens' rows: Step where the row's slot is that of its
 // position, Layer to any slot.
-// Guess and Layer make the first split of the batch, and the loads that follow from it, on lengths that the
-// previous kernel may yet change (see where they branch).  In a chain of decode layers of 16 sequences, of
-// which each streams 7 us, that takes the trips for lengths, sums and first rows off the path, and with
-// nothing of Step in it the kernel starts its loads sooner: 17.4 -> 14.9 us a layer.
+// Guess and Layer make the first split of the batch, and the loads that follow from it, on lengths and table entries
+// that the previous kernel may yet change (see where they branch).  In a chain of decode layers of 16 sequences, of
+// which each streams 7 us, that takes the trips for lengths, sums, table and first rows off the path, and with
+// nothing of Step in it the kernel starts its loads sooner: 17.4 -> 14.9 us a layer, 13.4 with the table and cells.
 enum class Variant { Plain, Step, Guess, Layer };
 
 template <class C, Variant V, bool CELLS>
@@ -230,11 +231,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   int bad = 0;
   int new_slot = -1;   // layer variant, lane l: slot of the l-th new row
   unsigned fresh = 0;  // step variant: stages whose tile holds the new token's row
-  auto load_tile = [&](const SeqCursor& c, int u, int stage) {
-    fresh &= ~(1u << stage);
-    const int t0 = (u - c.first) * UNIT + warp * TT;
-    if (t0 >= c.ctx) return;  // this warp has no token in the sequence's last unit
-    int64_t blk = p.block_tables[c.b * p.bt_stride + t0 / kBlockSize];
+  auto load_rows = [&](int b, int t0, int ctx, int slot, int64_t blk, int stage) {
     const bool blk_ok = blk >= 0 && blk < p.num_blocks;
     if (!blk_ok) {
       bad = NVLLM_STATUS_BAD_BLOCK;  // reported at the end: a guess may load for nothing
@@ -243,10 +240,10 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     const int64_t slot0 = blk * kBlockSize + (t0 % kBlockSize);
     // Step variant: token ctx-1 is the one being decoded.  Its row comes from the activation,
     // provided slot_mapping agrees with the block table, and goes to the cache when the tile is used.
-    const int last = c.ctx - 1;
+    const int last = ctx - 1;
     int new_row = -1;
-    if (STEP && last < t0 + TT && c.slot >= 0) {  // last >= t0 holds because t0 < ctx
-      if (blk_ok && c.slot == slot0 + (last - t0)) {
+    if (STEP && last < t0 + TT && slot >= 0) {  // last >= t0 holds because t0 < ctx
+      if (blk_ok && slot == slot0 + (last - t0)) {
         new_row = last - t0;
         fresh |= 1u << stage;
       } else if (lane == 0) {
@@ -263,13 +260,13 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       for (int it = 0; it < TT * C::CPR / 32; ++it) {
         const int idx = it * 32 + lane;
         const int r = idx / C::CPR, col = idx % C::CPR;
-        const int bytes = (blk_ok && t0 + r < c.ctx) ? 16 : 0;
+        const int bytes = (blk_ok && t0 + r < ctx) ? 16 : 0;
         const int64_t off = bytes ? (slot0 + r) * row_elems + kvh * D + col * 8 : 0;
         const __nv_bfloat16 *ksrc = p.k_cache + off, *vsrc = p.v_cache + off;
         if (STEP && r == new_row) {
           const int64_t in_row = static_cast<int64_t>(kvh) * D + col * 8;
-          ksrc = p.k_new + c.b * p.k_new_stride + in_row;
-          vsrc = p.v_new + c.b * p.v_new_stride + in_row;
+          ksrc = p.k_new + b * p.k_new_stride + in_row;
+          vsrc = p.v_new + b * p.v_new_stride + in_row;
         }
         if constexpr (decltype(patch)::value) {
           for (unsigned left = stored; left; left &= left - 1) {
@@ -288,7 +285,6 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     if (LAYER && stored) copy(std::true_type{});
     else copy(std::false_type{});
   };
-
   // ---- 1. units per sequence, block-wide scan, this block's range of the unit list ------
   const int per_thread = GUESS ? 1 : (p.batch + NT - 1) / NT;
   const int b_lo = min(tid * per_thread, p.batch), b_hi = min(b_lo + per_thread, p.batch);
@@ -299,8 +295,10 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       asm volatile("prefetch.global.L1 [%0];" ::"l"(p.block_tables + tid * p.bt_stride));
   };
   int total, n_ranges, per_range, longer, u0, u1, len_lo;
+  int2* seqs = reinterpret_cast<int2*>(smem + C::RING_BYTES);  // a guess: first unit and length of every sequence
+  static_assert(NT * 8 <= C::MERGE_BYTES, "room for them until the first merge");
   auto split = [&](bool ahead) {
-    if (!ahead) prefetch_table();
+    if (!GUESS) prefetch_table();
     int local = 0;
     len_lo = 0;
     for (int b = b_lo; b < b_hi; ++b) {
@@ -325,6 +323,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       total += s_scan[w];
     }
     const int excl = before + incl - local;
+    if (GUESS && ahead) seqs[tid] = make_int2(excl, len_lo);
     // No more ranges than units, so that every range in use holds at least one unit and the ranges
     // that share a sequence are consecutive.  And where sequences are few, no more than balance the
     // two costs of a cut: a range streams total / n units and a sequence's merge reads n / batch
@@ -355,6 +354,21 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   SeqCursor cc, pc;  // compute side; load side, NST-1 units ahead
   uint32_t qb[C::KS][2], qn[C::KS][2];  // this sequence's fragments; the next sequence's, fetched early
   int qn_b, n_units;
+  // A guess: this warp's tiles of the range's first 32 units, one to a lane, -1 where it has no token in the unit.
+  int n_listed = 0, listed_t0 = -1, listed_ctx = 0, listed_blk = 0;
+  auto load_unit = [&](int j) {  // the range's j-th unit, j < n_units, rising from call to call
+    const int stage = j % NST;
+    if (GUESS && j < n_listed) {
+      const int t0 = __shfl_sync(0xffffffffu, listed_t0, j), ctx = __shfl_sync(0xffffffffu, listed_ctx, j);
+      const int blk = __shfl_sync(0xffffffffu, listed_blk, j);
+      if (t0 >= 0) load_rows(0, t0, ctx, -1, blk, stage);
+      return;
+    }
+    seek(pc, u0 + j);
+    fresh &= ~(1u << stage);
+    const int t0 = (u0 + j - pc.first) * UNIT + warp * TT;
+    if (t0 < pc.ctx) load_rows(pc.b, t0, pc.ctx, pc.slot, p.block_tables[pc.b * p.bt_stride + t0 / kBlockSize], stage);
+  };
   auto start = [&]() {
     cc.b = s_start[0];
     cc.first = s_start[1];
@@ -367,56 +381,77 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     qn_b = min(cc.b + 1, p.batch - 1);
     load_q(qn, qn_b);
     n_units = u1 - u0;
-#pragma unroll
+#pragma unroll(GUESS ? 1 : NST - 1)
     for (int j = 0; j < NST - 1; ++j) {
-      if (j < n_units) {
-        seek(pc, u0 + j);
-        load_tile(pc, u0 + j, j);
-      }
+      if (j < n_units) load_unit(j);
       cp_async_commit();
     }
   };
 
   if constexpr (GUESS) {
-    // The range is cut by what the lengths are now and its first tiles are brought to L2.  When the previous
-    // kernel is done those tiles are loaded while the lengths are read again, and if one has changed the
-    // range is cut anew.  What is read before the wait goes round L1, is held to the bounds of the table
-    // and the cache, and serves the guess alone.
+    // The range is cut by what the lengths are now, its tiles are listed, one to a lane, with the table's entries as they
+    // are now, and the first two units are brought to L2.  When the previous kernel is done those are loaded while
+    // lengths and entries are read again, and if one has changed the range is cut anew.  What is read before the wait goes
+    // round L1, is held to the bounds of the table and the cache, and serves the guess alone.  With the list no load of a
+    // range waits for a length or a table entry (24 captured layers of 16 sequences, 14 / 2 heads of 64, 180 -> 166 us, a
+    // layer of one of 317 tokens 6.25 -> 5.95).  Two units: with three or all of them the requests stand in the way of
+    // the pre-attention step in front (28 layers of 16, 16 / 8 heads, 376 -> 393 and 415), with one the range starts
+    // later (382).  The code itself is in the way of a launch that streams for 3 us: one copy of it for the guess and the
+    // second attempt, rolled loops (36 layers of two sequences 509 -> 493).
     const int64_t n_slots = p.num_blocks * kBlockSize;
     auto in_cache = [&](int slot) { return slot >= 0 && slot < n_slots ? slot : -1; };
     if (LAYER && lane < p.n_new) new_slot = in_cache(__ldcg(p.slot_mapping + lane));
-    bool mine = split(true);
-    if (mine) {
-      const int b = s_start[0], first = s_start[1], ctx = s_start[2];
-      const int u_end = min(min(u1, first + units_of(ctx)), u0 + NST - 1);
-      for (int u = u0; u < u_end; ++u) {
-        const int t0 = (u - first) * UNIT + warp * TT;
-        if (t0 >= ctx) break;
-        const int64_t blk = __ldcg(p.block_tables + b * p.bt_stride + t0 / kBlockSize);
-        if (blk < 0 || blk >= p.num_blocks) break;
-        constexpr int LINES = C::ROW_BYTES / 128;
+    int slot_now = -1;
+    bool mine;
+#pragma unroll 1
+    for (bool ahead = true;; ahead = false) {
+      mine = split(ahead);
+      int now = 0, blk_now = 0;
+      if (ahead) {
+        const int32_t* listed_at = p.block_tables;
+        if (mine) {
+          n_listed = min(u1 - u0, 32);
+          if (lane < n_listed) {
+            const int u = u0 + lane;
+            int b = s_start[0];
+            while (b + 1 < p.batch && u >= seqs[b].x + units_of(seqs[b].y)) ++b;
+            const int t0 = (u - seqs[b].x) * UNIT + warp * TT;
+            listed_ctx = seqs[b].y;
+            if (t0 < listed_ctx) {
+              listed_t0 = t0;
+              listed_at += b * p.bt_stride + t0 / kBlockSize;
+              listed_blk = __ldcg(listed_at);
+            }
+          }
+#pragma unroll 1
+          for (int j = 0; j < min(n_listed, NST - 1); ++j) {
+            const int t0 = __shfl_sync(0xffffffffu, listed_t0, j), ctx = __shfl_sync(0xffffffffu, listed_ctx, j);
+            const int64_t blk = __shfl_sync(0xffffffffu, listed_blk, j);
+            if (t0 < 0 || blk < 0 || blk >= p.num_blocks) continue;
+            constexpr int LINES = C::ROW_BYTES / 128;
 #pragma unroll
-        for (int it = 0; it < TT * LINES / 32; ++it) {
-          const int r = (it * 32 + lane) / LINES, part = (it * 32 + lane) % LINES;
-          const int64_t off = (blk * kBlockSize + t0 % kBlockSize + r) * row_elems + kvh * D + part * 64;
-          if (t0 + r < ctx) {
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.k_cache + off));
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v_cache + off));
+            for (int it = 0; it < TT * LINES / 32; ++it) {
+              const int r = (it * 32 + lane) / LINES, part = (it * 32 + lane) % LINES;
+              const int64_t off = (blk * kBlockSize + t0 % kBlockSize + r) * row_elems + kvh * D + part * 64;
+              if (t0 + r < ctx) {
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.k_cache + off));
+                asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v_cache + off));
+              }
+            }
           }
         }
+        pdl_wait();
+        if (tid < p.batch) now = length_of(tid);
+        blk_now = listed_t0 >= 0 ? *listed_at : listed_blk;
+        if (LAYER && lane < p.n_new) slot_now = p.slot_mapping[lane];
       }
-    }
-    pdl_wait();
-    const int now = tid < p.batch ? length_of(tid) : 0;
-    const int slot_now = LAYER && lane < p.n_new ? p.slot_mapping[lane] : -1;
-    if (mine) start();
-    if (__syncthreads_or(now != len_lo || (LAYER && in_cache(slot_now) != new_slot))) {
+      if (mine) start();
+      if (!ahead || !__syncthreads_or(now != len_lo || blk_now != listed_blk || (LAYER && in_cache(slot_now) != new_slot))) break;
       cp_async_wait<0>();
       __syncthreads();
       bad = 0;
+      n_listed = 0;
       new_slot = in_cache(slot_now);
-      mine = split(false);
-      if (mine) start();
     }
     if (tid < p.batch && len_lo == 0) write_zeros(tid);
     if (LAYER && warp == NW - 1) {
@@ -556,7 +591,10 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   // Merges the partials of a cut sequence, all of which are in the workspace, and writes its rows.
   // QUADS lanes take a head (four columns each); lane l of them also holds the statistics of one
   // part of every chunk of QUADS parts, so that a chunk's statistics and its first rows are in
-  // flight together and the weights go round by shuffle: one trip to L2 for up to eight parts.
+  // flight together and the weights go round by shuffle: a trip to L2 for every eight parts (when those past
+  // the eighth were read one after the other, 17 parts of four heads took 7 us, and 36 captured layers of two sequences
+  // of 500-4000 tokens 493 instead of 412; one layer of two of 32000, 14 / 2 heads of 64, 20.8 instead of 17.1).  Not through
+  // shared memory by cp.async, all parts in one trip: 476 and 20.1, and one sequence of 350 tokens 193 -> 209.
   // Lane groups left over split the parts of a head between them.
   auto merge_cut = [&](const Cut& c) {
     constexpr int AHEAD = 8;
@@ -605,11 +643,18 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
           if (active && j0 + k * n_split + split < c.n) add_scaled(acc, rows[k], fk);
         }
         const int n_here = min(QUADS, (c.n - j0 + n_split - 1) / n_split);
-#pragma unroll 8
-        for (int k = AHEAD; k < n_here; ++k) {
-          const int j = j0 + k * n_split + split;
-          const float fk = __shfl_sync(0xffffffffu, f, k, QUADS);
-          if (active && j < c.n) add_scaled(acc, row_of(j), fk);
+#pragma unroll 1
+        for (int k0 = AHEAD; k0 < n_here; k0 += AHEAD) {
+#pragma unroll
+          for (int k = 0; k < AHEAD; ++k) {
+            const int j = j0 + (k0 + k) * n_split + split;
+            if (active && j < c.n) rows[k] = row_of(j);
+          }
+#pragma unroll
+          for (int k = 0; k < AHEAD; ++k) {
+            const float fk = __shfl_sync(0xffffffffu, f, k0 + k, QUADS);
+            if (active && j0 + (k0 + k) * n_split + split < c.n) add_scaled(acc, rows[k], fk);
+          }
         }
       }
       if (n_split > 1) {  // block-uniform
@@ -768,10 +813,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     cp_async_wait<NST - 2>();
     if (V == Variant::Plain) __syncthreads();  // the warps' tiles of a unit are fetched together
     else __syncwarp();
-    if (i + NST - 1 < n_units) {
-      seek(pc, u + NST - 1);
-      load_tile(pc, u + NST - 1, (i + NST - 1) % NST);
-    }
+    if (i + NST - 1 < n_units) load_unit(i + NST - 1);
     cp_async_commit();
 
     const int t0 = (u - cc.first) * UNIT + warp * TT;

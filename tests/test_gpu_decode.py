@@ -342,6 +342,40 @@ def test_lengths_written_by_the_kernel_just_before(cuda, batch):
         assert_close_to_oracle(out, ref, f"batch {batch}, lengths to {int(now.max())}")
 
 
+@pytest.mark.parametrize("hq,hkv,d,lens", [(16, 8, 128, list(range(100, 1024, 60))), (32, 32, 128, [3500] * 6), (14, 2, 64, [1, 0, 5000, 127, 129]),
+                                           (8, 8, 128, [64, 0, 65] * 42)])
+def test_tables_written_by_the_kernel_just_before(cuda, hq, hkv, d, lens):
+    """The block table is in the rows of a cache that the launch in front stores to: the decode, which may list its tiles
+    by the entries of the time before, must use the new ones.  In a thread block: a few units, more than a warp lists
+    (3500 tokens and 32 KV heads), sequences without a token, several sequences."""
+    case = W.make_decode_case(37, len(lens), 1, 1, hq, hkv, d, context_lens=lens)
+    dev = case.to(cuda)
+    g = torch.Generator().manual_seed(5)
+    width = case.block_tables.shape[1]
+    plane = torch.zeros(2, 256, 1, 256, dtype=torch.bfloat16, device=cuda)  # rows of 128 int32
+    table = plane[1].view(-1).view(torch.int32)[:len(lens) * width].view(len(lens), width)
+    slots = torch.arange(511, -1, -1, dtype=torch.int32, device=cuda)  # the rows that hold the table last
+    scratch = torch.zeros_like(plane)
+    steps = []
+    for i in range(4):
+        perm = torch.cat([torch.randperm(case.k_cache.shape[0], generator=g).int(), torch.tensor([-1], dtype=torch.int32)])
+        now = perm[case.block_tables.long()]  # -1 stays -1
+        flat = torch.zeros(256 * 128, dtype=torch.int32)
+        flat[:now.numel()] = now.flatten()
+        rows = torch.cat([flat.view(256, 128).flip(0), torch.zeros(256, 128, dtype=torch.int32)])
+        steps.append((now, rows.to(cuda).view(torch.bfloat16).view(512, 1, 256)))
+    outs = []
+    torch.cuda.synchronize()
+    for _, key in steps:
+        A.store_kvcache(key, key, plane, scratch, slots)
+        outs.append(A.decode_paged(dev.q, dev.k_cache, dev.v_cache, dev.context_lens, table, case.scale))
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+    for (now, _), out in zip(steps, outs):
+        ref = R.decode_ref(case.q, case.k_cache, case.v_cache, case.context_lens, now, case.scale)
+        assert_close_to_oracle(out, ref, f"{hq}/{hkv} heads of {d}, {len(lens)} sequences")
+
+
 @pytest.mark.parametrize("batch", [33, 129])
 def test_a_batch_of_empty_sequences_completes_after_its_store(cuda, batch):
     """The layer call of more than 32 sequences that are all empty has no tile to stream.  The launch
