@@ -16,15 +16,14 @@
 // counted by (row, position in the row, step); no state is kept between calls, the same
 // (seed, step) reproduces the same tokens.
 //
-// A row is read by one thread-block cluster of 1, 2, 4, 8 or 16 blocks of 256 threads (the fewer
-// the rows, the more blocks each gets, so that a decode batch of any size spreads over the 148
-// SMs).  A thread takes groups of 16 bytes (8 bf16 or 4 fp32 logits), loaded one step ahead.  Each
+// A row is read by one thread-block cluster of 1 to 8 or 16 blocks of 256 to 768 threads, so that a decode batch of any
+// size spreads evenly over the 148 SMs.  A thread takes groups of 16 bytes (8 bf16 or 4 fp32 logits), loaded one step ahead.  Each
 // warp reduces to one candidate and puts it into the shared memory of the cluster's first block, where
 // the largest is taken.  Ties go to the lowest index.
 //
 // What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
 // per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
-// (now 47; greedy rows 32 -> 16; batch 1, 12.7 -> 6.5).  The logarithms are only needed for elements that
+// (now 43.5; greedy rows 32 -> 16; batch 1, 12.7 -> 5.7).  The logarithms are only needed for elements that
 // can still win: since e >= v, where v is the uniform
 // draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
 // the group's largest x and the smallest of its draws decide that for the whole group, against the
@@ -47,7 +46,9 @@
 // index.  nvllm_sample_unpack turns the winning candidates into token ids.
 #include <cooperative_groups.h>
 
-#include <atomic>
+#include <algorithm>
+#include <cmath>
+#include <mutex>
 #include <type_traits>
 #include <utility>
 
@@ -207,11 +208,6 @@ __device__ __forceinline__ uint4 shift_pair(const uint4& a, const uint4& b, int 
   return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-// Build-time shape (measurement aid): resident blocks per SM the register budget is held to.
-#ifndef NVLLM_SAMPLER_MINBLOCKS
-#define NVLLM_SAMPLER_MINBLOCKS 4
-#endif
-
 // Calls f(pieces, first group, stride between the pieces' groups, full) for this thread's share of the
 // `n_groups` groups of a row that start at `first`, C pieces at a time; the next C are loaded before
 // the current ones are looked at.  All lanes of a warp make the same calls.  full is a constant: true
@@ -250,11 +246,11 @@ __device__ __forceinline__ void for_groups(const T* first, int n_groups, int tid
 constexpr int kMaxCluster = 16;
 
 template <typename T>
-__global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(const SampleParams p) {
+__global__ void __launch_bounds__(1024, 1) sample_kernel(const SampleParams p) {
   using G = Group<T>;
   constexpr int N = G::N;
   namespace cg = cooperative_groups;
-  pdl_prologue();
+  pdl_wait();
   cg::cluster_group cluster = cg::this_cluster();
   auto started = cluster.barrier_arrive();  // waited for before another block's shared memory is written
   const int csize = static_cast<int>(cluster.num_blocks()), crank = static_cast<int>(cluster.block_rank());
@@ -268,7 +264,7 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
   const float inv_t = greedy ? 1.f : 1.f / t;
   const Philox draw4(p.key, static_cast<uint32_t>(row), p.step);  // unique per element and call
   __shared__ int s_best;  // best score of the block so far, ordered()
-  __shared__ long long s_candidates[kMaxCluster * 8];  // block 0 of the cluster: one per warp of the row
+  __shared__ long long s_candidates[kMaxCluster * 32];  // block 0 of the cluster: one per warp of the row
   if (threadIdx.x == 0) s_best = ordered(-INFINITY);
   __syncthreads();
 
@@ -392,6 +388,9 @@ __global__ void __launch_bounds__(256, NVLLM_SAMPLER_MINBLOCKS) sample_kernel(co
     const int i = __shfl_xor_sync(0xffffffffu, best.idx, sh);
     take(best, s, i);
   }
+  // The next kernel's blocks start when the last block here gets to its merge: started any earlier they land on the SMs that
+  // happen to be free first, two on one and none on the next (32 rows 17.8 us instead of 12.9).
+  pdl_trigger();
   cluster.barrier_wait(std::move(started));
   const int lt = threadIdx.x, warps = static_cast<int>(blockDim.x) >> 5;
   if ((lt & 31) == 0)
@@ -415,11 +414,9 @@ __global__ void sample_unpack_kernel(const long long* packed, int64_t* tokens, i
 
 constexpr int kThreads = 256, kPortableCluster = 8;
 
-// Blocks per row: as few (1, 2, 4, 8) as give every SM three blocks, since every block pays its start
-// and its merge; more would only help the balance, fewer leave the SMs short of warps (measured at
-// batch 1 to 512).  Sixteen where that is still no more than one block per SM (batch 1: 8.7 us, 10.8 with
-// eight; beyond, clusters of sixteen crowd on a part of the chip: 19.0 for 14.5 at batch 32) and the device
-// can hold such a cluster.  No more than the row has work for.
+// Blocks per row where the device does not say how many clusters it holds at a time: as few (1, 2, 4, 8) of 256 threads as
+// give every SM three.  Sixteen where that is no more than one block per SM and the device can hold such a cluster.
+// No more than the row has work for.
 static int blocks_per_row(int batch, int vocab, int sms, int largest) {
   int csize = 1;
   auto fits = [&](int c, int64_t most) { return vocab >= c * kThreads * 8 && static_cast<int64_t>(batch) * c <= most; };
@@ -428,34 +425,99 @@ static int blocks_per_row(int batch, int vocab, int sms, int largest) {
   return csize;
 }
 
-// The largest cluster the current device takes: more than the portable eight has to be allowed, and then be
-// possible with the SMs that this process has (asked once per device and kernel).
+// How a launch is laid out.  The generator keeps an SM busy from some 24 warps on, so a launch takes as long as the SM with
+// most rows to read, in whole or in part, and what counts is to spread them evenly and at once.  Blocks of 768 threads
+// stand one to an SM, so that as many clusters as the device can hold of them are spread evenly by force; 384 stand two to
+// an SM, 256 four.  Clusters are counted as the device counts them: one lies within a group of SMs, and what is left of a
+// group is no use to it (of six blocks to an SM each, 148 SMs hold fewer than 24).  Blocks of 512 threads are spread evenly
+// only where a cluster has one or two; further waves of them follow as the first ones end.  All times are for 151936 logits and
+// T = 0.6, before (powers of two, 256 threads) -> now, us: 1 row 6.35 -> 5.65, 9 9.7 -> 7.3, 16 12.2 -> 8.4, 24 12.4 -> 8.9, 32 12.4
+// -> 10.1, 48 15.3 -> 13.1, 64 16.6 -> 14.7, 88 23.0 -> 18.6, 110 27.3 -> 23.7, 128 27.6 -> 25, 180 37.4 -> 34.4, 222 43.6 ->
+// 36.8, 256 47.4 -> 43.5, 512 84.9 -> 76; 150 rows of 32000 logits 13.0 -> 11.7.  In each case within 6 % of the best of all
+// pairs of one to eight and sixteen blocks and 192, 256, 320, 384, 512 and 768 threads.
+struct Shape {
+  int blocks, threads;  // to a row, to a block
+};
+struct Form {
+  int threads, per_sm, least, most;  // of a block; blocks of it on an SM; blocks to a row
+  double cost;                       // of a row, relative to 512 threads
+};
+constexpr Form kForms[] = {{768, 1, 1, 8, 1.05}, {512, 2, 1, 1, 1.0}, {512, 2, 2, 2, 1.07}, {384, 2, 3, 8, 1.07}, {256, 4, 3, 8, 1.17}, {256, 4, 1, 2, 1.05}};
+constexpr int kNumForms = sizeof(kForms) / sizeof(kForms[0]);
+constexpr int kSixteen = 0;              // clusters of sixteen are counted in this form, one block to an SM, and launched with
+constexpr int kSixteenThreads = 512;     // fewer threads: 5.65 us for one row, 5.9 with 768
+constexpr int kFull = 768;                // threads that keep an SM busy
+constexpr double kGroupsPerUs = 990, kWaveUs = 6;  // what an SM reads of a row in a microsecond; start and end of a second wave
+
+// Clusters of every size that the current device holds at a time (asked once per device and kernel); 0: it does not say.
+struct Rooms {
+  int of[kNumForms][kMaxCluster + 1];
+};
+
+static Shape shape_of(int batch, int64_t groups, int sms, const Rooms& rooms) {
+  Shape best{0, 0};
+  double least = 0;
+  // per_sm: blocks on the fullest SM; waves: of blocks, more than one where the device does not hold all
+  auto offer = [&](const Form& form, int c, int threads, double per_sm, double waves) {
+    if (form.per_sm == 1)  // no more threads than a short row has groups
+      threads = static_cast<int>(std::min<int64_t>(threads, std::max<int64_t>(kThreads, (groups + 32 * c - 1) / (32 * c) * 32)));
+    const double work = std::max<double>(static_cast<double>(groups), c * threads) / kGroupsPerUs * form.cost * per_sm / c;
+    const double us = work * (form.per_sm > 1 ? std::max(1.0, kFull / (per_sm * threads)) : 1.0) + kWaveUs * std::max(0.0, waves - 1);
+    if (!best.blocks || us < least) best = {c, threads}, least = us;
+  };
+  if (rooms.of[kSixteen][kMaxCluster] >= batch) offer(kForms[kSixteen], kMaxCluster, kSixteenThreads, 1, 1);
+  for (int f = 0; f < kNumForms; ++f) {
+    const Form& form = kForms[f];
+    for (int c = form.least; c <= form.most; ++c) {
+      const int64_t room = c == 1 ? static_cast<int64_t>(sms) * form.per_sm : rooms.of[f][c];
+      const double even = static_cast<double>(batch) * c / sms;
+      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * even)) : form.per_sm, 1);
+      else if (c <= 2 && room > 0 && form.per_sm > 1) offer(form, c, form.threads, std::ceil(even), static_cast<double>(batch) / room);
+    }
+  }
+  return best;
+}
+
 template <typename T>
-static int largest_cluster() {
-  static std::atomic<int> known[64];
+static const Rooms& rooms_of_device() {
+  static Rooms known[64];
+  static std::once_flag asked[64];
+  static const Rooms none{};
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
     (void)cudaGetLastError();
-    return kPortableCluster;
+    return none;
   }
-  int largest = known[dev].load(std::memory_order_acquire);
-  if (largest) return largest;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = kMaxCluster;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(kMaxCluster, 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int clusters = 0;
-  const bool possible = cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess &&
-                        cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<T>, &cfg) == cudaSuccess && clusters > 0;
-  if (!possible) (void)cudaGetLastError();
-  largest = possible ? kMaxCluster : kPortableCluster;
-  known[dev].store(largest, std::memory_order_release);
-  return largest;
+  std::call_once(asked[dev], [&] {
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    auto ask = [&](int f, int c) {
+      int clusters = 0;
+      attr[0].val.clusterDim.x = c;
+      cfg.gridDim = dim3(c, 1, 1);
+      cfg.blockDim = dim3(kForms[f].threads, 1, 1);
+      if (cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<T>, &cfg) != cudaSuccess) (void)cudaGetLastError();
+      else known[dev].of[f][c] = clusters;
+    };
+    for (int f = 0; f < kNumForms; ++f)
+      for (int c = std::max(2, kForms[f].least); c <= kForms[f].most; ++c) ask(f, c);
+    // more than the portable eight blocks have to be allowed
+    if (cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) ask(kSixteen, kMaxCluster);
+    else (void)cudaGetLastError();
+  });
+  return known[dev];
+}
+
+template <typename T>
+static Shape launch_shape(int batch, int vocab, int64_t vocab_offset, int sms) {
+  const Rooms& rooms = rooms_of_device<T>();
+  if (rooms.of[kSixteen][2] <= 0) return {blocks_per_row(batch, vocab, sms, kPortableCluster), kThreads};
+  const int64_t lead = (4 - (vocab_offset & 3)) & 3;
+  return shape_of(batch, std::max<int64_t>(0, (vocab - lead) / Group<T>::N), sms, rooms);
 }
 
 static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t row_stride, const float* temperatures,
@@ -530,14 +592,12 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   p.candidates = candidates;
   const int sms = num_sms();
   if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: no CUDA device is usable");
-  const int csize = blocks_per_row(batch, vocab, sms, logits_are_fp32 ? largest_cluster<float>() : largest_cluster<__nv_bfloat16>());
+  const Shape shape = logits_are_fp32 ? launch_shape<float>(batch, vocab, vocab_offset, sms) : launch_shape<__nv_bfloat16>(batch, vocab, vocab_offset, sms);
+  const int csize = shape.blocks;
   const int64_t blocks = static_cast<int64_t>(batch) * csize;
-  // Launched under the end of the kernel before (1.5 us less), except for grids of about one or two blocks
-  // per SM, which then land unevenly on the SMs that happen to be free (17.8 us for 14.5 at batch 32).
-  const bool early = 2 * blocks <= sms || blocks >= 3ll * sms;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(blocks), 1, 1);
-  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.blockDim = dim3(shape.threads, 1, 1);
   cfg.dynamicSmemBytes = 0;
   cfg.stream = static_cast<cudaStream_t>(stream);
   auto kernel = logits_are_fp32 ? sample_kernel<float> : sample_kernel<__nv_bfloat16>;
@@ -549,7 +609,7 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = early ? 2 : 1;
+  cfg.numAttrs = 2;
   const cudaError_t e = cudaLaunchKernelEx(&cfg, kernel, p);
   if (e != cudaSuccess) {
     (void)cudaGetLastError();

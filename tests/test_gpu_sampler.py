@@ -226,3 +226,15 @@ def test_rows_do_not_depend_on_the_blocks_that_read_them(cuda, lib, dtype):
     want = A.sample_tokens(logits, temps, seed=3, step=8)
     for b in batches[:-1]:
         assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=3, step=8), want[:b]), f"batch {b}"
+
+
+@pytest.mark.parametrize("dtype,vocab", [(torch.bfloat16, 40000), (torch.float32, 9973), (torch.bfloat16, 517)])
+def test_rows_do_not_depend_on_the_form_of_the_launch(cuda, dtype, vocab):
+    """The first rows of batches that are read by one to eight and sixteen blocks of every size, in one wave and more, by
+    rows with less than a group for every thread too: the same tokens."""
+    g = torch.Generator(device=cuda).manual_seed(23)
+    logits = (torch.randn(620, vocab, generator=g, device=cuda) * 3).to(dtype)
+    temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.3], device=cuda).repeat(124)
+    want = A.sample_tokens(logits, temps, seed=4, step=9)
+    for b in (1, 7, 12, 16, 20, 24, 28, 32, 36, 48, 64, 80, 100, 128, 150, 180, 200, 222, 256, 300, 450, 593):
+        assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=4, step=9), want[:b]), f"batch {b}"
