@@ -33,8 +33,8 @@
 // distribution ends.  Greedy rows compare the group's maximum with the thread's best, two packed bf16 at a time.
 //
 // Groups start at multiples of four global positions (the generator's counter).  Where such a
-// group does not start on a 16-byte boundary (rows of an odd vocabulary, slices), it is shifted
-// out of two aligned loads; the up to fifteen elements around the whole groups go one at a time.
+// group does not start on a 16-byte boundary (rows of an odd vocabulary, slices), it is put together
+// from words; the up to fifteen elements around the whole groups go one at a time.
 //
 // Tensor parallelism: nano-vllm's LM head leaves every rank with the logits of its own slice of
 // the vocabulary and then gathers all slices on rank 0 and concatenates them
@@ -188,57 +188,63 @@ struct Group<float> {
   }
 };
 
-// 16 bytes that start `shift` bytes (a multiple of the element size, 0..15, uniform over the block)
-// into the pair (a, b).
-template <int ELEM>
-__device__ __forceinline__ uint4 shift_pair(const uint4& a, const uint4& b, int shift) {
-  uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
-  if (shift & 8) {
-#pragma unroll
-    for (int i = 0; i < 6; ++i) w[i] = w[i + 2];
-  }
-  if (shift & 4) {
-#pragma unroll
-    for (int i = 0; i < 5; ++i) w[i] = w[i + 1];
-  }
-  if (ELEM == 2 && (shift & 2)) {
-#pragma unroll
-    for (int i = 0; i < 4; ++i) w[i] = __funnelshift_r(w[i], w[i + 1], 16);
-  }
-  return make_uint4(w[0], w[1], w[2], w[3]);
-}
-
 // Calls f(pieces, first group, stride between the pieces' groups, full) for this thread's share of the
 // `n_groups` groups of a row that start at `first`, C pieces at a time; the next C are loaded before
 // the current ones are looked at.  All lanes of a warp make the same calls.  full is a constant: true
 // where every piece of every lane of the warp is a group, else pieces past the end are zero.
+// Pieces of a row that does not start on a 16-byte boundary come as the words that hold them, and are shifted by half a word,
+// where that is needed, when their turn comes: shifted as they were loaded they held every step up for
+// its own load (256 rows of 151643 bf16 54.7 -> 48.5 us, 512 102 -> 85, 300 of 50257 28.4 -> 26.1).
+struct Words {
+  uint32_t u[5];
+};
+
 template <bool ALIGNED, int C, typename T, class F>
 __device__ __forceinline__ void for_groups(const T* first, int n_groups, int tid, int nthreads, F&& f) {
+  using Piece = std::conditional_t<ALIGNED, uint4, Words>;
   const int lane = tid & 31;
-  const int shift = ALIGNED ? 0 : static_cast<int>(reinterpret_cast<uintptr_t>(first) & 15u);
-  const uint4* base = reinterpret_cast<const uint4*>(reinterpret_cast<uintptr_t>(first) - shift);
-  auto load = [&](uint4 (&raw)[C], int g, auto full) {
+  const uint4* base = reinterpret_cast<const uint4*>(first);
+  const uint32_t* words = reinterpret_cast<const uint32_t*>(reinterpret_cast<uintptr_t>(first) & ~uintptr_t{3});
+  const bool across = sizeof(T) == 2 && (reinterpret_cast<uintptr_t>(first) & 2);  // elements lie across two words
+  auto load = [&](Piece (&piece)[C], int g, auto full) {
 #pragma unroll
     for (int c = 0; c < C; ++c, g += nthreads) {
       const bool live = decltype(full)::value || g < n_groups;
-      raw[c] = live ? __ldg(base + g) : make_uint4(0, 0, 0, 0);
-      if constexpr (!ALIGNED) raw[c] = shift_pair<sizeof(T)>(raw[c], live ? __ldg(base + g + 1) : make_uint4(0, 0, 0, 0), shift);
+      if constexpr (ALIGNED) {
+        piece[c] = live ? __ldg(base + g) : make_uint4(0, 0, 0, 0);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 5; ++i) piece[c].u[i] = live && (i < 4 || across) ? __ldg(words + 4 * static_cast<int64_t>(g) + i) : 0;
+      }
+    }
+  };
+  auto whole = [&](const Piece& p) {
+    if constexpr (ALIGNED) {
+      return p;
+    } else {
+      uint32_t u[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) u[i] = across ? __funnelshift_r(p.u[i], p.u[i + 1], 16) : p.u[i];
+      return make_uint4(u[0], u[1], u[2], u[3]);
     }
   };
   const int step = C * nthreads;
-  uint4 raw[C], next[C];
+  uint4 raw[C];
+  Piece next[C];
   int g = tid;
   const int n_full = n_groups - (C - 1) * nthreads - (31 - lane);  // g below this: a full call (the same for all lanes)
   if (g < n_full) load(next, g, std::true_type{});
   while (g < n_full) {
 #pragma unroll
-    for (int c = 0; c < C; ++c) raw[c] = next[c];
+    for (int c = 0; c < C; ++c) raw[c] = whole(next[c]);
     if (g + step < n_full) load(next, g + step, std::true_type{});
     f(raw, g, nthreads, std::true_type{});
     g += step;
   }
   for (; g - lane < n_groups; g += step) {
-    load(raw, g, std::false_type{});
+    load(next, g, std::false_type{});
+#pragma unroll
+    for (int c = 0; c < C; ++c) raw[c] = whole(next[c]);
     f(raw, g, nthreads, std::false_type{});
   }
 }
