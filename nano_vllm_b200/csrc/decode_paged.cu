@@ -164,17 +164,18 @@ struct Cut {
 // 8.12 -> 8.24, of two of 30000-32000 (14 / 2 heads of 64) 17.0 -> 17.45 -> 18.6.
 constexpr float kSplitBalance = 16.f;
 
-// The four kernels.  Step and Layer also store the new tokens' rows: Step where the row's slot is that of its
+// The kernels.  Step, StepGuess and Layer also store the new tokens' rows: the former two where the row's slot is that of its
 // position, Layer to any slot.
-// Guess and Layer make the first split of the batch, and the loads that follow from it, on lengths and table entries
+// Guess, StepGuess and Layer make the first split of the batch, and the loads that follow from it, on lengths and table entries
 // that the previous kernel may yet change (see where they branch).  In a chain of decode layers of 16 sequences, of
 // which each streams 7 us, that takes the trips for lengths, sums, table and first rows off the path, and with
 // nothing of Step in it the kernel starts its loads sooner: 17.4 -> 14.9 us a layer, 13.4 with the table and cells.
-enum class Variant { Plain, Step, Guess, Layer };
+enum class Variant { Plain, Step, StepGuess, Guess, Layer };
 
 template <class C, Variant V, bool CELLS>
 __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const DecodeParams p) {
-  constexpr bool STEP = V == Variant::Step, LAYER = V == Variant::Layer, GUESS = V == Variant::Guess || LAYER;
+  constexpr bool LAYER = V == Variant::Layer, STEP = V == Variant::Step || V == Variant::StepGuess;
+  constexpr bool GUESS = V == Variant::Guess || V == Variant::StepGuess || LAYER;
   constexpr int D = C::D, TT = C::TT, NST = C::NST, NW = C::NW, UNIT = C::UNIT, NT = NW * 32;
   constexpr int QUADS = D / 4, GROUPS = NT / QUADS;  // lanes that hold a head four columns each; such groups in a block
   extern __shared__ __align__(128) unsigned char smem[];
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   auto load_rows = [&](int b, int t0, int ctx, int slot, int64_t blk, int stage) {
     const bool blk_ok = blk >= 0 && blk < p.num_blocks;
     if (!blk_ok) {
-      bad = NVLLM_STATUS_BAD_BLOCK;  // reported at the end: a guess may load for nothing
+      bad |= NVLLM_STATUS_BAD_BLOCK;  // reported at the end: a guess may load for nothing
       blk = 0;
     }
     const int64_t slot0 = blk * kBlockSize + (t0 % kBlockSize);
@@ -246,8 +247,8 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
       if (blk_ok && slot == slot0 + (last - t0)) {
         new_row = last - t0;
         fresh |= 1u << stage;
-      } else if (lane == 0) {
-        atomicOr(p.status, NVLLM_STATUS_BAD_SLOT);
+      } else {
+        bad |= NVLLM_STATUS_BAD_SLOT;
       }
     }
     // Layer variant: whatever row of whatever sequence lies in a slot that this launch stores to is the new
@@ -354,14 +355,17 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
   SeqCursor cc, pc;  // compute side; load side, NST-1 units ahead
   uint32_t qb[C::KS][2], qn[C::KS][2];  // this sequence's fragments; the next sequence's, fetched early
   int qn_b, n_units;
-  // A guess: this warp's tiles of the range's first 32 units, one to a lane, -1 where it has no token in the unit.
-  int n_listed = 0, listed_t0 = -1, listed_ctx = 0, listed_blk = 0;
+  // A guess: this warp's tiles of the range's first 32 units, one to a lane, -1 where it has no token in the unit.  Loaded
+  // unrolled in a step only: its chain has no other kernel in it, and the code stays where it is (8 of 100-1024 11.4 rolled, 11.0).
+  int n_listed = 0, listed_t0 = -1, listed_ctx = 0, listed_blk = 0, listed_b = 0, listed_slot = -1;
   auto load_unit = [&](int j) {  // the range's j-th unit, j < n_units, rising from call to call
     const int stage = j % NST;
     if (GUESS && j < n_listed) {
       const int t0 = __shfl_sync(0xffffffffu, listed_t0, j), ctx = __shfl_sync(0xffffffffu, listed_ctx, j);
       const int blk = __shfl_sync(0xffffffffu, listed_blk, j);
-      if (t0 >= 0) load_rows(0, t0, ctx, -1, blk, stage);
+      const int b = STEP ? __shfl_sync(0xffffffffu, listed_b, j) : 0, slot = STEP ? __shfl_sync(0xffffffffu, listed_slot, j) : -1;
+      if (STEP) fresh &= ~(1u << stage);
+      if (t0 >= 0) load_rows(b, t0, ctx, slot, blk, stage);
       return;
     }
     seek(pc, u0 + j);
@@ -381,7 +385,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     qn_b = min(cc.b + 1, p.batch - 1);
     load_q(qn, qn_b);
     n_units = u1 - u0;
-#pragma unroll(GUESS ? 1 : NST - 1)
+#pragma unroll(GUESS && !STEP ? 1 : NST - 1)
     for (int j = 0; j < NST - 1; ++j) {
       if (j < n_units) load_unit(j);
       cp_async_commit();
@@ -406,7 +410,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
 #pragma unroll 1
     for (bool ahead = true;; ahead = false) {
       mine = split(ahead);
-      int now = 0, blk_now = 0;
+      int now = 0, blk_now = 0, listed_slot_now = -1;
       if (ahead) {
         const int32_t* listed_at = p.block_tables;
         if (mine) {
@@ -421,6 +425,7 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
               listed_t0 = t0;
               listed_at += b * p.bt_stride + t0 / kBlockSize;
               listed_blk = __ldcg(listed_at);
+              if (STEP) listed_b = b, listed_slot = __ldcg(p.slot_mapping + b);
             }
           }
 #pragma unroll 1
@@ -444,9 +449,10 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
         if (tid < p.batch) now = length_of(tid);
         blk_now = listed_t0 >= 0 ? *listed_at : listed_blk;
         if (LAYER && lane < p.n_new) slot_now = p.slot_mapping[lane];
+        if (STEP && listed_t0 >= 0) listed_slot_now = p.slot_mapping[listed_b];
       }
       if (mine) start();
-      if (!ahead || !__syncthreads_or(now != len_lo || blk_now != listed_blk || (LAYER && in_cache(slot_now) != new_slot))) break;
+      if (!ahead || !__syncthreads_or(now != len_lo || blk_now != listed_blk || (LAYER && in_cache(slot_now) != new_slot) || (STEP && listed_slot_now != listed_slot))) break;
       cp_async_wait<0>();
       __syncthreads();
       bad = 0;
@@ -981,7 +987,7 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
   cudaGetDevice(&dev);
   auto reserve = [](auto cells) {
     constexpr bool K = decltype(cells)::value;
-    for (auto kernel : {decode_paged_kernel<C, Variant::Plain, K>, decode_paged_kernel<C, Variant::Step, K>,
+    for (auto kernel : {decode_paged_kernel<C, Variant::Plain, K>, decode_paged_kernel<C, Variant::Step, K>, decode_paged_kernel<C, Variant::StepGuess, K>,
                         decode_paged_kernel<C, Variant::Guess, K>, decode_paged_kernel<C, Variant::Layer, K>}) {
       const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, C::SMEM);
       if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "decode_paged: cannot reserve %d bytes of shared memory: %s", C::SMEM, cudaGetErrorString(e));
@@ -994,8 +1000,11 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
     attr_set[p.cells][dev] = true;
   }
   // A guess for launches with a sequence per thread at most.  Larger batches stream long enough for the trips
-  // at the start not to matter, and the step kernel's predecessor in a chain is itself.
+  // at the start not to matter.  Steps without and with it, us: 16 / 8 heads, one sequence of 317 tokens 6.6 -> 6.2, 8 of 100-1024
+  // 11.2 -> 11.0, 32 19.9 -> 18.4, 100 43.4 -> 41.6, 128 53.1 -> 50.8; 32 / 8 heads, 6 of 205-405 7.15 -> 6.55, 54 of 587-1349 40.1 ->
+  // 38.9; 14 / 2 heads of 64, 16 of 100-1024 7.0 -> 6.3, 8 of 8000-32000 26.1 -> 22.6.
   const Variant v = p.n_new > 0                                 ? Variant::Layer
+                    : p.k_new && p.batch <= C::NW * 32            ? Variant::StepGuess
                     : p.k_new                                   ? Variant::Step
                     : !p.lengths_early && p.batch <= C::NW * 32 ? Variant::Guess
                                                                 : Variant::Plain;
@@ -1003,6 +1012,7 @@ static int launch_decode(const DecodeParams& p, cudaStream_t stream) {
     constexpr bool K = decltype(cells)::value;
     return v == Variant::Layer   ? decode_paged_kernel<C, Variant::Layer, K>
            : v == Variant::Step  ? decode_paged_kernel<C, Variant::Step, K>
+           : v == Variant::StepGuess ? decode_paged_kernel<C, Variant::StepGuess, K>
            : v == Variant::Guess ? decode_paged_kernel<C, Variant::Guess, K>
                                  : decode_paged_kernel<C, Variant::Plain, K>;
   };

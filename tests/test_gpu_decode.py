@@ -376,6 +376,42 @@ def test_tables_written_by_the_kernel_just_before(cuda, hq, hkv, d, lens):
         assert_close_to_oracle(out, ref, f"{hq}/{hkv} heads of {d}, {len(lens)} sequences")
 
 
+@pytest.mark.parametrize("hq,hkv,d,batch", [(16, 8, 128, 1), (16, 8, 128, 16), (8, 2, 128, 128), (14, 2, 64, 20), (2, 1, 64, 129)])
+def test_step_whose_inputs_the_kernel_just_before_writes(cuda, hq, hkv, d, batch):
+    """Lengths, table and slots are in the rows of a cache that the launch in front stores to: a step that has listed
+    its tiles by what was there before must store and read by what is there now, and report nothing."""
+    g = torch.Generator().manual_seed(batch)
+    case = W.make_decode_case(41, batch, 1, 1, hq, hkv, d, context_lens=torch.randint(200, 1500, (batch,), generator=g).tolist())
+    dev = case.to(cuda)
+    width = case.block_tables.shape[1]
+    plane = torch.zeros(2, 256, 1, 256, dtype=torch.bfloat16, device=cuda)  # rows of 128 int32
+    words = plane[1].view(-1).view(torch.int32)
+    lens, slots, table = words[:batch], words[batch:2 * batch], words[2 * batch:(2 + width) * batch].view(batch, width)
+    backwards = torch.arange(511, -1, -1, dtype=torch.int32, device=cuda)  # the rows that hold the words last
+    scratch = torch.zeros_like(plane)
+    steps = []
+    for _ in range(4):
+        perm = torch.cat([torch.randperm(case.k_cache.shape[0], generator=g).int(), torch.tensor([-1], dtype=torch.int32)])
+        now = (case.context_lens * torch.rand(batch, generator=g)).int() + 1
+        t = perm[case.block_tables.long()]
+        s = t[torch.arange(batch), ((now - 1) // 256).long()] * 256 + (now - 1) % 256
+        flat = torch.zeros(256 * 128, dtype=torch.int32)
+        flat[:(2 + width) * batch] = torch.cat([now, s, t.flatten()])
+        rows = torch.cat([flat.view(256, 128).flip(0), torch.zeros(256, 128, dtype=torch.int32)])
+        steps.append((now, s, t, rows.to(cuda).view(torch.bfloat16).view(512, 1, 256)))
+    outs = []
+    torch.cuda.synchronize()
+    for *_, key in steps:
+        A.store_kvcache(key, key, plane, scratch, backwards)
+        outs.append(A.decode_step(dev.q, dev.k_new, dev.v_new, dev.k_cache, dev.v_cache, slots, lens, table, case.scale))
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+    for (now, s, t, _), out in zip(steps, outs):
+        R.store_kvcache_ref(case.k_new, case.v_new, case.k_cache, case.v_cache, s)
+        assert_close_to_oracle(out, R.decode_ref(case.q, case.k_cache, case.v_cache, now, t, case.scale), f"batch {batch}")
+    assert torch.equal(dev.k_cache.cpu().view(torch.int16), case.k_cache.view(torch.int16))
+
+
 @pytest.mark.parametrize("batch", [33, 129])
 def test_a_batch_of_empty_sequences_completes_after_its_store(cuda, batch):
     """The layer call of more than 32 sequences that are all empty has no tile to stream.  The launch
