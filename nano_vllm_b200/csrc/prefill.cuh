@@ -41,7 +41,7 @@ struct PrefillParams {
   int hq, hkv, g, d;
   // persistent tcgen05 kernel only: query heads packed into one tile (1..8), its query tokens, 2^16 / heads
   int pack, tile_tokens, inv_pack;
-  int spread_from;  // items above which a launch with no more of them than blocks takes the order of spread_item
+  int spread_from;  // items above which a launch with no more of them than blocks, or of three blocks to an SM, takes the order of spread_item
   float scale_log2e;
   int64_t num_blocks;
   int* status;
@@ -60,7 +60,7 @@ struct PrefillParams {
   int64_t value_stride;
 };
 
-// Order of some launches with no more items than blocks: every q-th query tile of the list in turn, q the sequences' mean, so
+// Order of some launches: every q-th query tile of the list in turn, q the sequences' mean, so
 // that all sequences' long tiles come first.  The item that the n-th draw of such a launch stands for; each of its
 // items for one draw, which is what makes the launch complete whatever block draws when.
 __host__ __device__ __forceinline__ int spread_item(int drawn, int n_tiles, int batch, int hgroups) {

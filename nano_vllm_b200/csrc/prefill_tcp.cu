@@ -7,7 +7,7 @@
 // their row of S with tcgen05.ld, write P as packed bf16 over it with tcgen05.st; O += P V (TS
 // form: P from TMEM, V as an MN-major shared-memory operand); Q, K, V arrive by TMA tile loads
 // (128-byte swizzle, no multicast) into a two-stage ring; one tcgen05.commit per MMA group.
-// Twelve warps: 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
+// Twelve warps (eight in the form of three blocks to an SM, see Geo): 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
 // item's last P V product is done they normalise O and store it while the softmax warps are
 // already in the next item's first tile, and write packed K/V rows to the cache from the key tiles), warp 8 = TMA producer of
 // Q and K, warp 9 = MMA issuer, warp 10 = TMA producer of V (one elected lane each), warp 11 = a copy of rows that no
@@ -62,18 +62,13 @@ constexpr int MAX_BATCH = kPrefillMaxBatch;  // prefix array of query tiles per 
 constexpr int SORT_BATCH = 256;  // batches up to this size are ranked by length (B^2 / 192 compares per thread)
 enum PBar {
   ITEM_FULL0 = tc::NUM_BARS, ITEM_FULL1, ITEM_FREE0, ITEM_FREE1, O_FREE, EPI_FULL0, EPI_FULL1,
-  K_DUE0, K_DUE1, V_DUE0, V_DUE1, K_STORED0, K_STORED1, V_STORED0, V_STORED1, P_NUM_BARS
+  K_DUE0, K_DUE1, V_DUE0, V_DUE1, K_STORED0, K_STORED1, V_STORED0, V_STORED1, P_NUM_BARS,
+  S_FREE = O_FREE  // blocks of two groups have this one and not the other
 };
-// Twelve warps in three groups of four: softmax, epilogue, and (producer of Q and K, MMA issuer, producer of V, copy).
-// Registers are handed over between the groups at start-up (setmaxnreg): two blocks of 384 threads
-// per SM leave 80 per thread at launch; the softmax rows need about twice that, the other groups
-// a fraction.  128 x (RS + RE + RX) = 384 x 80.
-constexpr int NTHREADS_P = 384;
-constexpr int REGS_SOFTMAX = 136, REGS_EPILOGUE = 64, REGS_OTHER = 40;
-static_assert(128 * (REGS_SOFTMAX + REGS_EPILOGUE + REGS_OTHER) <= 384 * 80, "register pool of a block");
+constexpr int REGS_LAUNCH = 80;  // a thread's at launch, in every form: 768 threads an SM
 // Shared-memory layout and tile sizes for one head_dim (64 or 128).  A tile row is split into
 // 64-element (128-byte) sub-tiles, the unit of the 128-byte swizzle.
-template <int D_>
+template <int D_, bool TRIO_>
 struct Geo {
   static constexpr int D = D_;
   static constexpr int NSUB = D / 64;               // sub-tiles per tile row
@@ -91,6 +86,20 @@ struct Geo {
   static constexpr int OCH = D / 32;      // 32-column chunks of O
   static constexpr int ROWB = D * 2;      // bytes of one output row
   static constexpr int PIECES = D / 8;    // 16-byte pieces of one row
+  // A block's warps in groups of four: softmax, epilogue, and (producer of Q and K, MMA issuer, producer of V, copy).
+  // Registers are handed over between the groups at start-up (setmaxnreg): the softmax rows need about twice what a
+  // thread has at launch, the other groups a fraction.
+  // TRIO, at head_dim 64: no epilogue group, and three blocks to an SM instead of two.  A softmax warp takes 1650 cycles
+  // for a tile (300 of them waiting for S) whose exponentials are 512 of its scheduler's and whose products 300 of the
+  // tensor pipe: two of them keep a scheduler's exponentials busy for 66 % of the time, three for 70-80.  A block has 160
+  // columns of TMEM: S 64, O 64 and P 32 (two blocks: P over the scores, of which there are two).  Scores and P in places
+  // of their own in two blocks made them slower (4 prompts of 4096 tokens 180 -> 206 us), as did steps of two key tiles
+  // (197); rings of four stages, or the row maximum beside the exponentials instead of in front of them, nothing.
+  static constexpr bool TRIO = TRIO_;
+  static constexpr int BLOCKS = TRIO ? 3 : 2, NTHREADS = TRIO ? 256 : 384, FIRST_OTHER = TRIO ? 4 : 8;
+  static constexpr int REGS_SOFTMAX = TRIO ? 104 : 136, REGS_EPILOGUE = TRIO ? 0 : 64, REGS_OTHER = TRIO ? 56 : 40;
+  static_assert(128 * (REGS_SOFTMAX + REGS_EPILOGUE + REGS_OTHER) <= NTHREADS * REGS_LAUNCH, "register pool of a block");
+  static constexpr int TMEM_O = TRIO ? 64 : 128;  // column of O
 };
 constexpr int NUM_SLOTS = 64;                     // launches that may be in flight at once
 static_assert(P_NUM_BARS * 8 <= 256, "barrier area");
@@ -115,18 +124,19 @@ __device__ __forceinline__ int first_stored(const Item& x, int g) {
   return x.h % g == 0 ? (x.m0 > 0 ? key_tiles(x.m0, x.Lq, x.Lk) : 0) : x.n_kv;
 }
 
-template <int D, bool ROUTED>
-__global__ void __launch_bounds__(tcp::NTHREADS_P, 2)
+template <int D, bool ROUTED, bool TRIO>
+__global__ void __launch_bounds__(tcp::Geo<D, TRIO>::NTHREADS, tcp::Geo<D, TRIO>::BLOCKS)
 prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tmap_q,
                    const __grid_constant__ CUtensorMap tmap_k, const __grid_constant__ CUtensorMap tmap_v,
                    const __grid_constant__ CUtensorMap tmap_key, const __grid_constant__ CUtensorMap tmap_value,
                    const int counter_slot) {
   using namespace tcp;
-  using G = Geo<D>;
+  using G = Geo<D, TRIO>;
   constexpr int Q_SUB = G::Q_SUB, KV_BYTES = G::KV_BYTES, KV_SUB = G::KV_SUB;
   constexpr int OFF_Q = G::OFF_Q, OFF_K = G::OFF_K, OFF_V = G::OFF_V, OFF_CTRL = G::OFF_CTRL;
   constexpr int OFF_SLOTS = G::OFF_SLOTS, OFF_MISC = G::OFF_MISC, OFF_PREFIX = G::OFF_PREFIX, OFF_ORDER = G::OFF_ORDER;
-  constexpr int OCH = G::OCH, PIECES = G::PIECES;
+  constexpr int OCH = G::OCH, PIECES = G::PIECES, NTHREADS_P = G::NTHREADS;
+  constexpr int W_QK = G::FIRST_OTHER, W_MMA = W_QK + 1, W_V = W_QK + 2;
   extern __shared__ unsigned char smem_raw[];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
 
@@ -148,12 +158,18 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   auto token_of = [&](int row) { return row * p.inv_pack >> 16; };  // row / pack, row < 128
 
   pdl_trigger();
-  if (warp == 9 && lane < P_NUM_BARS) {  // a barrier per lane
+  if (warp == W_MMA && lane < P_NUM_BARS) {  // a barrier per lane
     // four softmax warps fill P and the normalisers; four epilogue warps free O and store rows; an item slot is
-    // free when the softmax warps, the epilogue warps, the MMA issuer and the V producer are done with it
+    // free when the softmax warps, the epilogue warps, the MMA issuer and the V producer are done with it.  Two groups:
+    // the softmax warps free S, the last warp stores rows and has to do with items only where it does.
     static_assert(P_NUM_BARS <= 32, "a barrier per lane");
     const bool by_four = lane == P_FULL0 || lane == P_FULL1 || lane == O_FREE || lane == EPI_FULL0 || lane == EPI_FULL1 || lane >= K_STORED0;
-    mbar_init(bar(lane), by_four ? 4u : lane == ITEM_FREE0 || lane == ITEM_FREE1 ? 10u : 1u);
+    if constexpr (TRIO) {
+      const unsigned of_item = p.store == Store::Tiles ? 7u : 6u;
+      mbar_init(bar(lane), lane >= K_STORED0 ? 1u : by_four ? 4u : lane == ITEM_FREE0 || lane == ITEM_FREE1 ? of_item : 1u);
+    } else {
+      mbar_init(bar(lane), by_four ? 4u : lane == ITEM_FREE0 || lane == ITEM_FREE1 ? 10u : 1u);
+    }
     if (lane == 0) {
       *abort_flag = 0;
       prefetch_tmap(&tmap_q);
@@ -201,7 +217,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     for (int b = tid; b < p.batch; b += NTHREADS_P) order[b] = static_cast<unsigned short>(b);
   }
   __syncthreads();
-  if (warp == 8) {
+  if (warp == W_QK) {
     // query tiles per sequence, in that order -> exclusive prefix sum (warp scan, 32 at a time)
     int carry = 0;
 #pragma unroll 1
@@ -223,13 +239,18 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
     }
     if (lane == 0) prefix[p.batch] = carry;
   }
-  if (warp == 9) tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+  if (warp == W_MMA) {
+    if (TRIO) tmem_alloc(smem_u32(tmem_slot), 128, smem_u32(tmem_slot + 1), 32);
+    else tmem_alloc(smem_u32(tmem_slot), TMEM_COLS);
+  }
   if (p.lengths_early) pdl_wait();  // from here on q, k and v are read
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t tmem_o = tmem + 128;
+  const uint32_t tmem_o = tmem + G::TMEM_O;
+  auto tmem_s = [&](int st) { return TRIO ? tmem : tmem + st * 64; };                // scores of a tile
+  auto tmem_p = [&](int st) { return TRIO ? tmem_slot[1] : tmem + st * 64; };  // its P
 
   auto read_item = [&](int it) {
     volatile int* s = slots + (it & 1) * 8;
@@ -286,14 +307,14 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
   float* inv_buf = reinterpret_cast<float*>(base_ptr + G::OFF_INV);
   // The register hand-over sits inside each group's own branch: the allocator bounds the code that
   // follows a setmaxnreg on its path, and paths that merged again would all get the smallest bound.
-  if (warp >= 8) {
-   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_OTHER));
-   if (warp == 8) {
+  if (warp >= W_QK) {
+   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_OTHER));
+   if (warp == W_QK) {
     // ------------------------------------------------------------------ producer lane
     if (elect_one()) {
       const int hgroups = p.hq / pack;
       const int total_items = prefix[p.batch] * hgroups;
-      const bool spread = D == 128 && total_items > p.spread_from && total_items <= static_cast<int>(gridDim.x);
+      const bool spread = (D == 128 || TRIO) && total_items > p.spread_from && (TRIO || total_items <= static_cast<int>(gridDim.x));
       int T = 0;   // key tiles loaded so far in this block's life
       unsigned stored = 0;
       // Number drawn -> item: (query tile of a sequence, head); heads vary fastest so that the blocks
@@ -381,7 +402,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         T += x.n_kv;
       }
     }
-   } else if (warp == 10) {
+   } else if (warp == W_V) {
     // ------------------------------------------------------------------ V producer
     // A thread of its own: a V stage is free only after the tile's P V product, and a single producer that
     // waits for that would hold back the K load of the next tile, whose stage is free much earlier.
@@ -418,7 +439,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
       }
     }
-   } else if (warp == 9) {
+   } else if (warp == W_MMA) {
     // ------------------------------------------------------------------ MMA issuer
     if (elect_one()) {
       constexpr uint32_t idesc_qk = umma_idesc(BM, BN, 0, 0);
@@ -429,9 +450,10 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       auto issue_qk = [&](int t) -> bool {
         const int st = t & 1;
         if (!wait_or_abort(bar(K_FULL0 + st), (t >> 1) & 1, abort_flag)) return false;
+        if (TRIO && t > 0 && !wait_or_abort(bar(S_FREE), (t - 1) & 1, abort_flag)) return false;
         tc_fence_after();
         const uint64_t kd = k_desc + static_cast<uint64_t>(st * (KV_BYTES >> 4));
-        const uint32_t d_tmem = tmem + st * 64;
+        const uint32_t d_tmem = tmem_s(st);
 #pragma unroll
         for (int ks = 0; ks < D / 16; ++ks) {
           const uint64_t qoff = ((ks >> 2) * Q_SUB + (ks & 3) * 32) >> 4;
@@ -457,11 +479,12 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
           if (j < 0) continue;
           if (!(ok = wait_or_abort(bar(V_FULL0 + st), ph, abort_flag))) break;
           if (!(ok = wait_or_abort(bar(P_FULL0 + st), ph, abort_flag))) break;
-          // the first product of an item overwrites O: the previous item's O must have been read
-          if (j == 0 && it > 0 && !(ok = wait_or_abort(bar(O_FREE), (it - 1) & 1, abort_flag))) break;
+          // the first product of an item overwrites O: the previous item's O must have been read (two groups: by the warps
+          // that have just filled P)
+          if (!TRIO && j == 0 && it > 0 && !(ok = wait_or_abort(bar(O_FREE), (it - 1) & 1, abort_flag))) break;
           tc_fence_after();
           const uint64_t vd = v_desc + static_cast<uint64_t>(st * (KV_BYTES >> 4));
-          const uint32_t p_tmem = tmem + st * 64;
+          const uint32_t p_tmem = tmem_p(st);
 #pragma unroll
           for (int ks = 0; ks < BN / 16; ++ks)
             umma_ts(tmem_o, p_tmem + ks * 8, vd + static_cast<uint64_t>((ks * 2048) >> 4), idesc_pv,
@@ -477,13 +500,66 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
         (void)mbar_wait(bar(DRAIN), 0);
       }
     }
-   } else if (p.store != Store::None && !ROUTED) {
+   } else if (p.store != Store::None && (TRIO || !ROUTED)) {
     // -------------------------------------------------- a warp left: packed rows to the cache
+    if constexpr (TRIO) {
+      // Those of key tiles, which the epilogue warps store where there are any: the same, by one warp.
+      constexpr int ROWS = 32 / PIECES;
+      const int piece = lane % PIECES;
+      const int64_t row_elems = static_cast<int64_t>(p.hkv) * D;
+      int T = 0;
+      unsigned due = 0;  // bit st: parity of stage st's next K_DUE and V_DUE
+      bool ok = p.store == Store::Tiles;
+#pragma unroll 1
+      for (int it = 0; ok; ++it) {
+        if (!(ok = wait_or_abort(bar(ITEM_FULL0 + (it & 1)), (it >> 1) & 1, abort_flag))) break;
+        const Item x = read_item(it);
+        if (x.n_kv < 0) break;
+        const int64_t col = static_cast<int64_t>(x.h / p.g) * D + piece * 8;
+#pragma unroll 1
+        for (int j = first_stored(x, p.g); ok && j < x.n_kv; ++j) {
+          const int t = T + j, st = t & 1;
+          const int64_t row0 = packed_row(x, j);
+          if (row0 < 0) continue;  // read through the table: stored already
+          const int n_rows = static_cast<int>(min(static_cast<int64_t>(min(BN, x.Lk - j * BN)), p.n_new - row0));
+          int slot[2];  // of rows lane and 32 + lane
+#pragma unroll
+          for (int i = 0; i < 2; ++i) slot[i] = i * 32 + lane < n_rows ? slot_of(row0 + i * 32 + lane) : -1;
+#pragma unroll 1
+          for (int kv = 0; kv < 2; ++kv) {
+            if (!(ok = wait_or_abort(bar((kv ? V_DUE0 : K_DUE0) + st), due >> st & 1, abort_flag))) break;
+            if (!(ok = wait_or_abort(bar((kv ? V_FULL0 : K_FULL0) + st), (t >> 1) & 1, abort_flag))) break;
+            const uint32_t src = base + (kv ? OFF_V : OFF_K) + st * KV_BYTES + (piece >> 3) * KV_SUB;
+            __nv_bfloat16* cache = (kv ? p.v_store : p.k_store) + col;
+#pragma unroll 1
+            for (int r0 = 0; r0 < BN; r0 += 16) {
+              uint4 v[16 / ROWS];
+#pragma unroll
+              for (int i = 0; i < 16 / ROWS; ++i) {
+                const int r = r0 + i * ROWS + lane / PIECES;
+                v[i] = ld_shared16(src + r * 128 + (((piece ^ r) & 7) << 4));
+              }
+#pragma unroll
+              for (int i = 0; i < 16 / ROWS; ++i) {
+                const int to = __shfl_sync(0xffffffffu, r0 < 32 ? slot[0] : slot[1], r0 % 32 + i * ROWS + lane / PIECES);
+                if (to >= 0) *reinterpret_cast<uint4*>(cache + to * row_elems) = v[i];
+              }
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(bar((kv ? V_STORED0 : K_STORED0) + st));
+          }
+          due ^= 1u << st;
+        }
+        T += x.n_kv;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
+      }
+    }
     // All of them, or those that no item has a tile of: of sequences without a query row, in front of the first
     // sequence and behind the last.  A 16-byte piece of a K and a V row per lane, two such at a time.
     const uint32_t per_row = p.hkv * PIECES;
     const bool all = p.store == Store::Spare;
-    int b = all ? p.batch : static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
+    int b = ROUTED ? p.batch + 1 : all ? p.batch : static_cast<int>(blockIdx.x) - static_cast<int>(gridDim.x);
 #pragma unroll 1
     while (b <= p.batch) {
       int64_t from = 0, to = p.n_new;
@@ -526,7 +602,7 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
    }
   } else if (warp < 4) {
     // ------------------------------------------------------------------ softmax rows
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(REGS_SOFTMAX));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(G::REGS_SOFTMAX));
     const int r = warp * 32 + lane;
     const int r_tok = token_of(r);  // this row's token within the tile (== BMT for the unused rows of a 7-head tile)
     const uint32_t lane_addr = static_cast<uint32_t>(warp * 32) << 16;
@@ -542,13 +618,18 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
 #pragma unroll 1
       for (int j = 0; j < x.n_kv; ++j) {
         const int t = T + j, st = t & 1, ph = (t >> 1) & 1;
-        const uint32_t tmem_s = tmem + st * 64 + lane_addr;
+        const uint32_t scores = tmem_s(st) + lane_addr;
         if (!(ok = wait_or_abort(bar(QK_DONE0 + st), ph, abort_flag))) break;
         tc_fence_after();
         uint32_t s[64];
-        tmem_ld32(tmem_s, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
-        tmem_ld32(tmem_s + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
+        tmem_ld32(scores, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        tmem_ld32(scores + 32, *reinterpret_cast<uint32_t(*)[32]>(&s[32]));
         tmem_wait_ld();
+        if (TRIO) {  // the next tile's scores may be written
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(bar(S_FREE));
+        }
 
         const int j0 = j * BN;
         if ((j0 + BN - 1 > x.m0 + off) || (j0 + BN > x.Lk)) {  // tile touches the diagonal or the end
@@ -622,7 +703,11 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
           }
           fence_proxy_async();
         }
-        tmem_st32(tmem_s, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
+        if (TRIO && j > 0) {  // P has one place: the product of the tile before must have read it
+          if (!(ok = wait_or_abort(bar(PV_DONE0 + ((t - 1) & 1)), ((t - 1) >> 1) & 1, abort_flag))) break;
+          tc_fence_after();
+        }
+        tmem_st32(TRIO ? tmem_p(st) + lane_addr : scores, *reinterpret_cast<uint32_t(*)[32]>(&s[0]));
         tmem_wait_st();
         tc_fence_before();
         __syncwarp();
@@ -631,17 +716,56 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       if (!ok) break;
       T += x.n_kv;
 
-      // the row's normaliser goes to the epilogue warps; this warp is done with the item
-      inv_buf[(it & 1) * 128 + r] = l > 0.f ? 1.f / l : 0.f;
-      __syncwarp();
-      if (lane == 0) {
-        mbar_arrive(bar(EPI_FULL0 + (it & 1)));
-        mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
+      const float inv = l > 0.f ? 1.f / l : 0.f;
+      if constexpr (TRIO) {
+        if (!(ok = wait_or_abort(bar(PV_DONE0 + ((T - 1) & 1)), ((T - 1) >> 1) & 1, abort_flag))) break;
+        tc_fence_after();
+        // O / l -> bf16, 32 columns at a time through this warp's patch of shared memory, as an epilogue warp does it
+        unsigned char* stage = base_ptr + G::OFF_STAGE + warp * 2048;
+        const int srow = lane >> 2, spiece = lane & 3;
+        __nv_bfloat16* out_tile = p.out + static_cast<int64_t>(x.q0 + x.m0) * p.out_stride + x.h * D;
+        const int toks_valid = min(BMT, x.Lq - x.m0);
+#pragma unroll (ROUTED ? 1 : OCH)
+        for (int c = 0; c < OCH; ++c) {
+          uint32_t o[32];
+          tmem_ld32(tmem_o + lane_addr + c * 32, o);
+          tmem_wait_ld();
+          uint4 v[4];
+#pragma unroll
+          for (int k = 0; k < 4; ++k) {
+            v[k].x = pack_bf16x2(__uint_as_float(o[8 * k]) * inv, __uint_as_float(o[8 * k + 1]) * inv);
+            v[k].y = pack_bf16x2(__uint_as_float(o[8 * k + 2]) * inv, __uint_as_float(o[8 * k + 3]) * inv);
+            v[k].z = pack_bf16x2(__uint_as_float(o[8 * k + 4]) * inv, __uint_as_float(o[8 * k + 5]) * inv);
+            v[k].w = pack_bf16x2(__uint_as_float(o[8 * k + 6]) * inv, __uint_as_float(o[8 * k + 7]) * inv);
+          }
+#pragma unroll
+          for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(stage + lane * 64 + ((k ^ ((lane >> 1) & 3)) << 4)) = v[k];
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const int lr = i * 8 + srow, row = warp * 32 + lr;  // of the warp's 32, of the tile
+            const int tok = token_of(row), hh = row - tok * pack;
+            const uint4 v = *reinterpret_cast<const uint4*>(stage + lr * 64 + ((spiece ^ ((lr >> 1) & 3)) << 4));
+            if (tok < toks_valid)
+              *reinterpret_cast<uint4*>(out_tile + static_cast<int64_t>(tok) * p.out_stride + hh * D + c * 32 + spiece * 8) = v;
+          }
+          __syncwarp();
+        }
+        tc_fence_before();
+        if (lane == 0) mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
+      } else {
+        // the row's normaliser goes to the epilogue warps; this warp is done with the item
+        inv_buf[(it & 1) * 128 + r] = inv;
+        __syncwarp();
+        if (lane == 0) {
+          mbar_arrive(bar(EPI_FULL0 + (it & 1)));
+          mbar_arrive(bar(ITEM_FREE0 + (it & 1)));
+        }
       }
     }
-  } else {
+  } else if constexpr (!TRIO) {
     // ------------------------------------------------------------------ epilogue rows
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(REGS_EPILOGUE));
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(G::REGS_EPILOGUE));
     // Same rows as softmax warp (warp - 4): a warp reaches the TMEM lanes 32 x (warp mod 4).
     const int ew = warp - 4, r = ew * 32 + lane;
     const uint32_t lane_addr = static_cast<uint32_t>(ew * 32) << 16;
@@ -754,9 +878,10 @@ prefill_tcp_kernel(const PrefillParams p, const __grid_constant__ CUtensorMap tm
       __threadfence();
     }
   }
-  if (warp == 9) {
+  if (warp == W_MMA) {
     tc_fence_after();
-    tmem_dealloc(tmem, TMEM_COLS);
+    tmem_dealloc(tmem, TRIO ? 128 : TMEM_COLS);
+    if (TRIO) tmem_dealloc(tmem_slot[1], 32);
   }
 }
 
@@ -779,29 +904,67 @@ int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch) {
   return static_cast<int64_t>((max_seqlen_q + bmt - 1) / bmt) * (hq / pack) * batch;
 }
 
-template <int D>
+// Prompts of less than three key tiles are the two-block form's: a block of three has no warps to write an item's results while
+// the next is begun (14 / 2 heads, two blocks -> three, us: 100 of 100-200 tokens 26.9 -> 27.4, 128 of 128 28.3 -> 28.6, 200 of 20-100
+// 24.8 -> 26.8, 256 of 64 28.1 -> 30.5; 64 of 256 32.4 -> 32.1).
+constexpr int kTrioTokens = 3 * tc::BN;
+
+// All prompts within 2 % of one length: in launches of three blocks to an SM their long tiles go first.  Sequence after
+// sequence the last ones' start late and run alone at the end.  Three blocks, without -> with that order, us: 4 of 4096
+// tokens 189 -> 166, 16 of 1024 62.4 -> 56.2, 8 of 512 19.6 -> 16.1, 64 of 256 32.2 -> 31.5; of other prompts 12 of 700-800 34.3 -> 35.0, 80
+// of 180-200 28.4 -> 29.3.  Not with two blocks, whose short launches the code for it costs 1-1.7 %, nor at head_dim 128 (4
+// of 4096 242 -> 247, 64 of 256 50 -> 61: what keeps memory busy there is the mix of long and short tiles).
+static bool prompts_of_one_length(const PrefillParams& p, int64_t total_q) {
+  return p.batch > 1 && 50ll * p.max_seqlen_q * p.batch <= 51 * total_q;
+}
+
+// Head_dim 64: three blocks to an SM, of eight warps, or two of twelve.  Three get up to 12 % more done where there is
+// enough for all of them: four times the key tiles of the longest item for every SM, since an item takes a block of three
+// longer.  14 / 2 heads, two blocks -> three, us (tiles of an SM over those of the longest item in brackets): 64 of 100-1024
+// tokens 74.4 -> 70.9 (8.3), 32 39.4 -> 38.2 (4.1), 16 22.7 -> 22.6 (2), 8 17.4 -> 18.8 (1), 8 of 1500-2048 82.4 -> 81.4 (4.8), 5 of 1000-3000
+// 70.2 -> 71.3 (2.6), 40 of 200-400 26.4 -> 26.2 (4.1), 2 of 2000-2500 38.2 -> 43.3 (1.7).  For prompts of one length several items to a
+// block are enough: 4 of 4096 180 -> 167, 16 of 1024 63.0 -> 56.4, 6 of 2000-2010 81.3 -> 71.4, 2 of 4000-4096 96.1 -> 94.8 (3.1), 8 of 512
+// 17.9 -> 16.2 (1.8).
+static bool three_blocks(const PrefillParams& p, int64_t total_q) {
+  const int sms = num_sms(), pack = heads_per_tile(p.g), bmt = tc::BM / pack;
+  const double mean = static_cast<double>(total_q) / p.batch;
+  const double items = static_cast<double>(total_q) / bmt * (p.hq / pack), tiles = items * (mean / 2 + tc::BN / 2) / tc::BN;
+  return mean >= kTrioTokens &&
+         (prompts_of_one_length(p, total_q) ? items > 2.0 * sms : tiles >= 4.0 * sms * p.max_seqlen_k / tc::BN);
+}
+
+// Makes the kernels of a form ready for their launches on a device.
+template <int D, bool TRIO>
+static int prepare_prefill_tcp() {
+  for (auto kernel : {prefill_tcp_kernel<D, false, TRIO>, prefill_tcp_kernel<D, true, TRIO>}) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tcp::Geo<D, TRIO>::SMEM);
+    if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
+    // The warp groups trade registers inside the pool the block gets at launch (threads x the kernel's
+    // register count); a build whose count is below the assumed 80 could never satisfy the softmax
+    // group's request, and that request waits without a bound.
+    cudaFuncAttributes attr;
+    e = cudaFuncGetAttributes(&attr, kernel);
+    if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
+    if (attr.numRegs < tcp::REGS_LAUNCH)
+      return fail(NVLLM_E_CUDA, "prefill (persistent): built with %d registers per thread, the warp groups' hand-over needs %d",
+                  attr.numRegs, tcp::REGS_LAUNCH);
+  }
+  return NVLLM_OK;
+}
+
+template <int D, bool TRIO>
 static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int64_t total_k, cudaStream_t stream) {
-  using G = tcp::Geo<D>;
-  static bool attr_done[64] = {false};  // of this head_dim
+  using G = tcp::Geo<D, TRIO>;
+  static bool ready[64] = {false};
   int dev = 0;
   cudaGetDevice(&dev);
   if (dev < 0 || dev >= 64) return fail(NVLLM_E_NO_DEVICE, "prefill: device index %d out of range", dev);
   if (p_in.out_stride > (1 << 23)) return fail(NVLLM_E_GEOMETRY, "prefill: out row stride %lld too large", (long long)p_in.out_stride);
-  if (!attr_done[dev]) {
-    for (auto kernel : {prefill_tcp_kernel<D, false>, prefill_tcp_kernel<D, true>}) {  // both: the other's first launch may be captured
-      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, G::SMEM);
-      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
-      // The warp groups trade registers inside the pool the block gets at launch (threads x the kernel's
-      // register count); a build whose count is below the assumed 80 could never satisfy the softmax
-      // group's request, and that request waits without a bound.
-      cudaFuncAttributes attr;
-      e = cudaFuncGetAttributes(&attr, kernel);
-      if (e != cudaSuccess) return fail(NVLLM_E_CUDA, "prefill (persistent): set-up failed: %s", cudaGetErrorString(e));
-      if (attr.numRegs * tcp::NTHREADS_P < 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER))
-        return fail(NVLLM_E_CUDA, "prefill (persistent): built with %d registers per thread, the warp groups' hand-over needs %d",
-                    attr.numRegs, 128 * (tcp::REGS_SOFTMAX + tcp::REGS_EPILOGUE + tcp::REGS_OTHER) / tcp::NTHREADS_P);
-    }
-    attr_done[dev] = true;
+  if (!ready[dev]) {  // all forms of this head_dim: another's first launch may be captured
+    int rc = prepare_prefill_tcp<D, false>();
+    if (D == 64 && rc == NVLLM_OK) rc = prepare_prefill_tcp<64, true>();
+    if (rc) return rc;
+    ready[dev] = true;
   }
   PrefillParams p = p_in;
   const bool routed = p.route.jobs > 0;
@@ -829,7 +992,7 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   }
   // an upper bound of the work items known to the host: no more blocks than that
   const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
-  int grid = 2 * num_sms();
+  int grid = G::BLOCKS * num_sms();
   if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
   // With an item to a block and more items than SMs, blocks that share an SM with those of long tiles get short ones by
   // another order: 6 prompts of 300 tokens 15.1 -> 13.4 us, 10 of 100 11.4 -> 10.4, 3 of 500 14.6 -> 14.1.  Which blocks
@@ -839,7 +1002,7 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   // tokens 8.2 -> 8.5), where long and short prompts mix, whose tiles every q-th of the list does not line up (19 of
   // 209-582 16.0 -> 17.3), nor at head_dim 64 (14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05).
   const bool alike = p.max_seqlen_q <= 5 * bmt || 20ll * p.max_seqlen_q * p.batch <= 23 * total_q;
-  p.spread_from = p.batch > 1 && alike ? num_sms() : 1 << 30;
+  p.spread_from = TRIO ? (prompts_of_one_length(p, total_q) ? 0 : 1 << 30) : p.batch > 1 && alike ? num_sms() : 1 << 30;
   // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
   // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
   // rows, 4 KB in flight; 120 from the tiles; 110 with nothing to store).  Where a block has one item at most that
@@ -852,13 +1015,14 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
   grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, copy_blocks)));
   static_assert(sizeof(g_launch_seq) == 4 && (1ull << 32) % tcp::NUM_SLOTS == 0, "the slots follow one another when the count wraps");
   const int slot = static_cast<int>(g_launch_seq.fetch_add(1) % tcp::NUM_SLOTS);
-  return launch_kernel("prefill (tcgen05, persistent)", routed ? prefill_tcp_kernel<D, true> : prefill_tcp_kernel<D, false>, dim3(grid),
-                       dim3(tcp::NTHREADS_P), G::SMEM, stream, p, mq, mk, mv, mkey, mvalue, slot);
+  return launch_kernel("prefill (tcgen05, persistent)", routed ? prefill_tcp_kernel<D, true, TRIO> : prefill_tcp_kernel<D, false, TRIO>, dim3(grid),
+                       dim3(G::NTHREADS), G::SMEM, stream, p, mq, mk, mv, mkey, mvalue, slot);
 }
 
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream) {
-  if (p.d == 128) return launch_prefill_tcp_t<128>(p, total_q, total_k, stream);
-  return launch_prefill_tcp_t<64>(p, total_q, total_k, stream);
+  if (p.d == 128) return launch_prefill_tcp_t<128, false>(p, total_q, total_k, stream);
+  return three_blocks(p, total_q) ? launch_prefill_tcp_t<64, true>(p, total_q, total_k, stream)
+                                  : launch_prefill_tcp_t<64, false>(p, total_q, total_k, stream);
 }
 
 }  // namespace nvllm

@@ -313,6 +313,51 @@ def test_every_item_of_a_launch_with_an_item_to_a_block(cuda, hq, hkv, d, length
     _check(cuda, case, f"{lengths} hq{hq} d{d}")
 
 
+@pytest.mark.parametrize("hq,hkv", [(14, 2), (7, 1), (4, 4)])
+@pytest.mark.parametrize("lengths,share", [([130] * 40, 0), ([257] * 40, 4), ([500] * 20 + [510] * 19, 0), ([511] * 40, 4), ([128] * 45, 0)])
+def test_several_items_a_block_of_prompts_of_one_length(cuda, hq, hkv, lengths, share):
+    """head_dim 64, more items than blocks: all prompts' long tiles go first, packed and through the table."""
+    case = W.make_prefill_case(53, len(lengths), 1, 1, hq, hkv, 64, lengths=lengths, share_every=share)
+    _check(cuda, case, f"{len(lengths)} of {lengths[0]} hq{hq}")
+
+
+@pytest.mark.parametrize("hq,hkv,batch", [(14, 2, 70), (7, 1, 140), (4, 4, 180)])
+@pytest.mark.parametrize("table", [False, True])
+def test_rows_are_stored_with_three_blocks_to_an_sm(cuda, hq, hkv, batch, table):
+    """head_dim 64, enough items for three blocks an SM: packed rows are stored by one warp of each.  Ends around a tile's,
+    sequences without a query, rows in front and behind, scattered slots; through the table with blocks that others fill."""
+    d, r = 64, random.Random(batch)
+    lens = [r.choice([320, 319, 320, 257, 256, 255, 193, 320] + [0] * (not table)) for _ in range(batch)]
+    gen = torch.Generator(device=cuda).manual_seed(batch)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    if table:
+        c = W.make_prefill_case(59, batch, 1, 1, hq, hkv, d, device=cuda, lengths=lens, shared_blocks=[(i % 4 == 3) * min(1, min(lens[i - 1], lens[i] - 1) // 256) for i in range(batch)]).to(cuda)
+        q, k, v, cu_q, cu_k, slots, bt = c.q, c.k, c.v, c.cu_seqlens_q, c.cu_seqlens_k, c.slot_mapping, c.block_tables
+        layer.k_cache, layer.v_cache = c.k_cache, c.v_cache
+        max_q, max_k = c.max_seqlen_q, c.max_seqlen_k
+    else:
+        front, behind = 3, 70
+        n, n_k = sum(lens), front + sum(lens) + behind
+        q, k, v = rand(n, hq, d), rand(n_k, hkv, d), rand(n_k, hkv, d)
+        cu_q = torch.tensor([0] + lens, device=cuda).cumsum(0).int()
+        cu_k, bt, max_q, max_k = cu_q + front, None, max(lens), max(lens)
+        slots = torch.randperm((n_k // 256 + 3) * 256, generator=gen, device=cuda)[:n_k].int()
+        slots[::11] = -1
+        layer.k_cache, layer.v_cache = rand(n_k // 256 + 3, 256, hkv, d), rand(n_k // 256 + 3, 256, hkv, d)
+    k2, v2 = layer.k_cache.clone(), layer.v_cache.clone()
+    A.store_kvcache(k, v, k2, v2, slots)
+    want = A.prefill_varlen(q, k2 if table else k, v2 if table else v, cu_q, cu_k, max_q, max_k, d ** -0.5, bt)
+    C.set_context(True, cu_q, cu_k, max_q, max_k, slots, None, bt)
+    for _ in range(3):
+        got = layer(q.flatten(1), k.flatten(1), v.flatten(1))
+    C.reset_context()
+    torch.cuda.synchronize()
+    assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
+    assert torch.equal(got.view_as(want), want)
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("repeat", range(4))
 def test_items_without_a_visible_key_where_blocks_start_late(cuda, repeat):
     """An item to a block, some of them tiles in front of all keys (more queries than keys), for which a block draws again:
