@@ -10,9 +10,7 @@ namespace tc {
 constexpr int BM = 128, BN = 64, KST = 2;
 constexpr int TMEM_COLS = 256;              // S/P buffers: [0,64) and [64,128); O: [128,256)
 constexpr float kRescaleThreshold = 8.f;    // log2 units
-// One tcgen05.commit per MMA group: a commit that follows a group of a different kind costs the
-// tensor pipe a bubble (~100-200 cycles measured), so each completion is signalled once and
-// shared by all its waiters.  QK_DONE[s]: S buffer s holds S_j (softmax) and K stage s is free
+// One tcgen05.commit per MMA group, each completion signalled once and shared by all its waiters.  QK_DONE[s]: S buffer s holds S_j (softmax) and K stage s is free
 // (producer).  PV_DONE[s]: V stage s is free (producer), O includes tile j (rescale, epilogue).
 enum Bar {
   Q_FULL = 0, K_FULL0, K_FULL1, V_FULL0, V_FULL1, QK_DONE0, QK_DONE1, PV_DONE0, PV_DONE1,

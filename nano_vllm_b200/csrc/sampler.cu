@@ -436,10 +436,13 @@ static int blocks_per_row(int batch, int vocab, int sms, int largest) {
 // stand one to an SM, so that as many clusters as the device can hold of them are spread evenly by force; 384 stand two to
 // an SM, 256 four.  Clusters are counted as the device counts them: one lies within a group of SMs, and what is left of a
 // group is no use to it (of six blocks to an SM each, 148 SMs hold fewer than 24).  Blocks of 512 threads are spread evenly
-// only where a cluster has one or two; further waves of them follow as the first ones end.  All times are for 151936 logits and
+// only where a cluster has one or two.  More than two rows to an SM go out in powers of two blocks of 256 threads as before
+// (one block to a row, which all fit: 300 rows 65 us instead of 57, 400 76 instead of 65; waves of blocks of 512 threads sample 512 rows in 76
+// instead of 85, but take 29.3 instead of 25.7 for 450 greedy ones, which the host cannot tell).  All times are for 151936 logits and
 // T = 0.6, before (powers of two, 256 threads) -> now, us: 1 row 6.35 -> 5.65, 9 9.7 -> 7.3, 16 12.2 -> 8.4, 24 12.4 -> 8.9, 32 12.4
 // -> 10.1, 48 15.3 -> 13.1, 64 16.6 -> 14.7, 88 23.0 -> 18.6, 110 27.3 -> 23.7, 128 27.6 -> 25, 180 37.4 -> 34.4, 222 43.6 ->
-// 36.8, 256 47.4 -> 43.5, 512 84.9 -> 76; 150 rows of 32000 logits 13.0 -> 11.7.  In each case within 6 % of the best of all
+// 36.8, 256 47.4 -> 43.5; 150 rows of 32000 logits 13.0 -> 11.7; greedy 16 6.2 -> 4.1, 100 12.5 -> 9.3, 256 15.9 -> 15.6 (of fp32
+// 150 23.6 -> 17.7, but 64 9.6 -> 10.0 and 200 25.4 -> 26.1).  In each case within 6 % of the best of all
 // pairs of one to eight and sixteen blocks and 192, 256, 320, 384, 512 and 768 threads.
 struct Shape {
   int blocks, threads;  // to a row, to a block
@@ -453,7 +456,7 @@ constexpr int kNumForms = sizeof(kForms) / sizeof(kForms[0]);
 constexpr int kSixteen = 0;              // clusters of sixteen are counted in this form, one block to an SM, and launched with
 constexpr int kSixteenThreads = 512;     // fewer threads: 5.65 us for one row, 5.9 with 768
 constexpr int kFull = 768;                // threads that keep an SM busy
-constexpr double kGroupsPerUs = 990, kWaveUs = 6;  // what an SM reads of a row in a microsecond; start and end of a second wave
+constexpr double kGroupsPerUs = 990;     // what an SM reads of a row in a microsecond
 
 // Clusters of every size that the current device holds at a time (asked once per device and kernel); 0: it does not say.
 struct Rooms {
@@ -463,22 +466,20 @@ struct Rooms {
 static Shape shape_of(int batch, int64_t groups, int sms, const Rooms& rooms) {
   Shape best{0, 0};
   double least = 0;
-  // per_sm: blocks on the fullest SM; waves: of blocks, more than one where the device does not hold all
-  auto offer = [&](const Form& form, int c, int threads, double per_sm, double waves) {
+  auto offer = [&](const Form& form, int c, int threads, double per_sm) {  // per_sm: blocks on the fullest SM
     if (form.per_sm == 1)  // no more threads than a short row has groups
       threads = static_cast<int>(std::min<int64_t>(threads, std::max<int64_t>(kThreads, (groups + 32 * c - 1) / (32 * c) * 32)));
     const double work = std::max<double>(static_cast<double>(groups), c * threads) / kGroupsPerUs * form.cost * per_sm / c;
-    const double us = work * (form.per_sm > 1 ? std::max(1.0, kFull / (per_sm * threads)) : 1.0) + kWaveUs * std::max(0.0, waves - 1);
+    const double us = work * (form.per_sm > 1 ? std::max(1.0, kFull / (per_sm * threads)) : 1.0);
     if (!best.blocks || us < least) best = {c, threads}, least = us;
   };
-  if (rooms.of[kSixteen][kMaxCluster] >= batch) offer(kForms[kSixteen], kMaxCluster, kSixteenThreads, 1, 1);
+  if (rooms.of[kSixteen][kMaxCluster] >= batch) offer(kForms[kSixteen], kMaxCluster, kSixteenThreads, 1);
   for (int f = 0; f < kNumForms; ++f) {
     const Form& form = kForms[f];
     for (int c = form.least; c <= form.most; ++c) {
       const int64_t room = c == 1 ? static_cast<int64_t>(sms) * form.per_sm : rooms.of[f][c];
       const double even = static_cast<double>(batch) * c / sms;
-      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * even)) : form.per_sm, 1);
-      else if (c <= 2 && room > 0 && form.per_sm > 1) offer(form, c, form.threads, std::ceil(even), static_cast<double>(batch) / room);
+      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * even)) : form.per_sm);
     }
   }
   return best;
@@ -521,7 +522,7 @@ static const Rooms& rooms_of_device() {
 template <typename T>
 static Shape launch_shape(int batch, int vocab, int64_t vocab_offset, int sms) {
   const Rooms& rooms = rooms_of_device<T>();
-  if (rooms.of[kSixteen][2] <= 0) return {blocks_per_row(batch, vocab, sms, kPortableCluster), kThreads};
+  if (rooms.of[kSixteen][2] <= 0 || batch > 2 * sms) return {blocks_per_row(batch, vocab, sms, kPortableCluster), kThreads};
   const int64_t lead = (4 - (vocab_offset & 3)) & 3;
   return shape_of(batch, std::max<int64_t>(0, (vocab - lead) / Group<T>::N), sms, rooms);
 }
