@@ -34,7 +34,7 @@
 //
 // Groups start at multiples of four global positions (the generator's counter).  Where such a
 // group does not start on a 16-byte boundary (rows of an odd vocabulary, slices), it is put together
-// from words; the up to fifteen elements around the whole groups go one at a time.
+// from words (greedy fp32 rows: starts on one); the up to fifteen elements around the whole groups go one at a time.
 //
 // Tensor parallelism: nano-vllm's LM head leaves every rank with the logits of its own slice of
 // the vocabulary and then gathers all slices on rank 0 and concatenates them
@@ -276,8 +276,11 @@ __global__ void __launch_bounds__(1024, 1) sample_kernel(const SampleParams p) {
 
   Best best{-INFINITY, 0x7fffffff};
   const int off = static_cast<int>(p.offset);
-  // whole groups of this row: they start at multiples of four global positions
-  const int lead = (4 - (off & 3)) & 3;
+  // Whole groups of this row: they start at multiples of four global positions, the generator's counter.  Where nothing is
+  // generated, fp32 ones start on 16-byte boundaries instead: put together from four words each they held the loads up
+  // (512 greedy rows of 151643 fp32 59.7 -> 49.1 us, 256 of 50257 11.7 -> 7.7).
+  int lead = (4 - (off & 3)) & 3;
+  if (sizeof(T) == 4 && greedy) lead = static_cast<int>((16u - (reinterpret_cast<uintptr_t>(x) & 15u)) & 15u) / static_cast<int>(sizeof(T));
   const int n_groups = p.vocab > lead ? (p.vocab - lead) / N : 0;
   const T* first = x + lead;
 

@@ -214,6 +214,26 @@ def test_rows_at_any_alignment_pick_the_same_tokens(cuda, dtype, vocab, peak):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("vocab,offset", [(2, 0), (5, 3), (6, 1), (1001, 2), (33333, 5)])
+def test_greedy_rows_at_any_alignment_take_the_first_of_equal_logits(cuda, dtype, vocab, offset):
+    """The largest logit twice, at every distance from the row's start and end within a group, rows at every element
+    offset within a 16-byte piece, slices that start off a group of four positions."""
+    spots = sorted({p for p in (*range(9), *range(vocab - 9, vocab), vocab // 2) if 0 <= p < vocab})
+    firsts = [p for p in spots if p < vocab - 1]
+    temps = torch.zeros(len(firsts), device=cuda)
+    for shift in range(16 // torch.empty(0, dtype=dtype).element_size()):
+        buf = torch.full((len(firsts), vocab + 8), 100.0, dtype=dtype, device=cuda)  # what lies around the row must not be seen
+        rows = buf[:, shift:shift + vocab]
+        rows.zero_()
+        for r, p in enumerate(firsts):
+            rows[r, p] = rows[r, max(q for q in spots if q > p)] = 7.0
+        assert A.sample_tokens(rows, temps).tolist() == firsts, f"shift {shift}"
+        assert A.sample_unpack(A.sample_candidates(rows, temps, offset)).tolist() == [offset + p for p in firsts], f"shift {shift}"
+        rows.zero_()
+        assert A.sample_tokens(rows, temps).tolist() == [0] * len(firsts)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_rows_do_not_depend_on_the_blocks_that_read_them(cuda, lib, dtype):
     """The first rows of batches that give a row sixteen, eight, four, two and one block: the same tokens."""
     vocab = 40000
