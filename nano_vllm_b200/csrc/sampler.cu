@@ -423,15 +423,16 @@ __global__ void sample_unpack_kernel(const long long* packed, int64_t* tokens, i
 
 constexpr int kThreads = 256, kPortableCluster = 8;
 
-// Blocks per row where the device does not say how many clusters it holds at a time: as few (1, 2, 4, 8) of 256 threads as
-// give every SM three.  Sixteen where that is no more than one block per SM and the device can hold such a cluster.
+struct Shape {
+  int blocks, threads;  // to a row, to a block
+};
+
+// Blocks of 256 threads to a row in powers of two: as few as give every SM three, in waves where that is more than it holds.
 // No more than the row has work for.
-static int blocks_per_row(int batch, int vocab, int sms, int largest) {
+static Shape in_waves(int batch, int vocab, int sms) {
   int csize = 1;
-  auto fits = [&](int c, int64_t most) { return vocab >= c * kThreads * 8 && static_cast<int64_t>(batch) * c <= most; };
-  while (csize < kPortableCluster && static_cast<int64_t>(batch) * csize < 3ll * sms && fits(2 * csize, INT64_MAX)) csize *= 2;
-  if (csize == kPortableCluster && largest >= kMaxCluster && fits(kMaxCluster, sms)) csize = kMaxCluster;
-  return csize;
+  while (csize < kPortableCluster && static_cast<int64_t>(batch) * csize < 3ll * sms && vocab >= 2 * csize * kThreads * 8) csize *= 2;
+  return {csize, kThreads};
 }
 
 // How a launch is laid out.  The generator keeps an SM busy from some 24 warps on, so a launch takes as long as the SM with
@@ -447,42 +448,40 @@ static int blocks_per_row(int batch, int vocab, int sms, int largest) {
 // 36.8, 256 47.4 -> 43.5; 150 rows of 32000 logits 13.0 -> 11.7; greedy 16 6.2 -> 4.1, 100 12.5 -> 9.3, 256 15.9 -> 15.6 (of fp32
 // 150 23.6 -> 17.7, but 64 9.6 -> 10.0 and 200 25.4 -> 26.1).  In each case within 6 % of the best of all
 // pairs of one to eight and sixteen blocks and 192, 256, 320, 384, 512 and 768 threads.
-struct Shape {
-  int blocks, threads;  // to a row, to a block
-};
 struct Form {
   int threads, per_sm, least, most;  // of a block; blocks of it on an SM; blocks to a row
   double cost;                       // of a row, relative to 512 threads
 };
 constexpr Form kForms[] = {{768, 1, 1, 8, 1.05}, {512, 2, 1, 1, 1.0}, {512, 2, 2, 2, 1.07}, {384, 2, 3, 8, 1.07}, {256, 4, 3, 8, 1.17}, {256, 4, 1, 2, 1.05}};
-constexpr int kNumForms = sizeof(kForms) / sizeof(kForms[0]);
+static_assert(sizeof(kForms) / sizeof(kForms[0]) == NVLLM_SAMPLE_FORMS, "as the header says");
 constexpr int kSixteen = 0;              // clusters of sixteen are counted in this form, one block to an SM, and launched with
 constexpr int kSixteenThreads = 512;     // fewer threads: 5.65 us for one row, 5.9 with 768
-constexpr int kFull = 768;                // threads that keep an SM busy
-constexpr double kGroupsPerUs = 990;     // what an SM reads of a row in a microsecond
+constexpr int kFull = 768;               // threads that keep an SM busy
 
-// Clusters of every size that the current device holds at a time (asked once per device and kernel); 0: it does not say.
+// Clusters of every size that a device holds at a time, in every form; 0: it does not say.
 struct Rooms {
-  int of[kNumForms][kMaxCluster + 1];
+  int of[NVLLM_SAMPLE_FORMS][kMaxCluster + 1];
 };
 
-static Shape shape_of(int batch, int64_t groups, int sms, const Rooms& rooms) {
+static Shape shape_of(int batch, int vocab, int64_t vocab_offset, bool fp32, int sms, const Rooms& rooms) {
+  const Shape waves = in_waves(batch, vocab, sms);
+  if (rooms.of[kSixteen][2] <= 0 || batch > 2 * sms) return waves;
+  const int64_t lead = (4 - (vocab_offset & 3)) & 3, groups = std::max<int64_t>(0, (vocab - lead) / (fp32 ? 4 : 8));
   Shape best{0, 0};
-  double least = 0;
+  double least = 0;  // of the groups that the fullest SM has to read
   auto offer = [&](const Form& form, int c, int threads, double per_sm) {  // per_sm: blocks on the fullest SM
     if (form.per_sm == 1)  // no more threads than a short row has groups
       threads = static_cast<int>(std::min<int64_t>(threads, std::max<int64_t>(kThreads, (groups + 32 * c - 1) / (32 * c) * 32)));
-    const double work = std::max<double>(static_cast<double>(groups), c * threads) / kGroupsPerUs * form.cost * per_sm / c;
-    const double us = work * (form.per_sm > 1 ? std::max(1.0, kFull / (per_sm * threads)) : 1.0);
-    if (!best.blocks || us < least) best = {c, threads}, least = us;
+    double work = std::max<double>(static_cast<double>(groups), c * threads) * form.cost * per_sm / c;
+    if (form.per_sm > 1) work *= std::max(1.0, kFull / (per_sm * threads));
+    if (!best.blocks || work < least) best = {c, threads}, least = work;
   };
   if (rooms.of[kSixteen][kMaxCluster] >= batch) offer(kForms[kSixteen], kMaxCluster, kSixteenThreads, 1);
-  for (int f = 0; f < kNumForms; ++f) {
+  for (int f = 0; f < NVLLM_SAMPLE_FORMS; ++f) {
     const Form& form = kForms[f];
     for (int c = form.least; c <= form.most; ++c) {
       const int64_t room = c == 1 ? static_cast<int64_t>(sms) * form.per_sm : rooms.of[f][c];
-      const double even = static_cast<double>(batch) * c / sms;
-      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * even)) : form.per_sm);
+      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * batch * c / sms)) : form.per_sm);
     }
   }
   return best;
@@ -513,7 +512,7 @@ static const Rooms& rooms_of_device() {
       if (cudaOccupancyMaxActiveClusters(&clusters, sample_kernel<T>, &cfg) != cudaSuccess) (void)cudaGetLastError();
       else known[dev].of[f][c] = clusters;
     };
-    for (int f = 0; f < kNumForms; ++f)
+    for (int f = 0; f < NVLLM_SAMPLE_FORMS; ++f)
       for (int c = std::max(2, kForms[f].least); c <= kForms[f].most; ++c) ask(f, c);
     // more than the portable eight blocks have to be allowed
     if (cudaFuncSetAttribute(sample_kernel<T>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess) ask(kSixteen, kMaxCluster);
@@ -522,24 +521,27 @@ static const Rooms& rooms_of_device() {
   return known[dev];
 }
 
-template <typename T>
-static Shape launch_shape(int batch, int vocab, int64_t vocab_offset, int sms) {
-  const Rooms& rooms = rooms_of_device<T>();
-  if (rooms.of[kSixteen][2] <= 0 || batch > 2 * sms) return {blocks_per_row(batch, vocab, sms, kPortableCluster), kThreads};
-  const int64_t lead = (4 - (vocab_offset & 3)) & 3;
-  return shape_of(batch, std::max<int64_t>(0, (vocab - lead) / Group<T>::N), sms, rooms);
-}
-
 static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t row_stride, const float* temperatures,
                          const float* exponential_noise, int64_t noise_row_stride, uint64_t seed, uint64_t step,
                          int64_t vocab_offset, int candidates, int64_t* tokens, int32_t batch, int32_t vocab, void* stream);
 
 }  // namespace nvllm
 
-extern "C" int nvllm_sample_plan(int32_t batch, int32_t vocab, int32_t num_sms, int32_t largest_cluster) {
+extern "C" int nvllm_sample_plan(int32_t batch, int32_t vocab, int64_t vocab_offset, int32_t logits_are_fp32, int32_t num_sms,
+                                 const int32_t* clusters, int32_t* blocks, int32_t* threads) {
   using namespace nvllm;
-  if (batch < 0 || vocab <= 0 || num_sms <= 0) return fail(NVLLM_E_GEOMETRY, "sample_plan: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
-  return blocks_per_row(batch, vocab, num_sms, largest_cluster);
+  if (batch < 0 || vocab <= 0 || vocab_offset < 0 || num_sms < 0 || (!num_sms && clusters))
+    return fail(NVLLM_E_GEOMETRY, "sample_plan: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
+  if (!blocks || !threads) return fail(NVLLM_E_NULL, "sample_plan: NULL pointer argument");
+  Rooms rooms{};
+  if (clusters) std::copy(clusters, clusters + NVLLM_SAMPLE_FORMS * (kMaxCluster + 1), &rooms.of[0][0]);
+  else if (!num_sms) rooms = logits_are_fp32 ? rooms_of_device<float>() : rooms_of_device<__nv_bfloat16>();
+  const int sms = num_sms ? num_sms : nvllm::num_sms();
+  if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_plan: no CUDA device is usable");
+  const Shape shape = shape_of(batch, vocab, vocab_offset, logits_are_fp32, sms, rooms);
+  *blocks = shape.blocks;
+  *threads = shape.threads;
+  return NVLLM_OK;
 }
 
 extern "C" int nvllm_sample_tokens(const void* logits, int32_t logits_are_fp32, int64_t row_stride,
@@ -602,7 +604,8 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
   p.candidates = candidates;
   const int sms = num_sms();
   if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_tokens: no CUDA device is usable");
-  const Shape shape = logits_are_fp32 ? launch_shape<float>(batch, vocab, vocab_offset, sms) : launch_shape<__nv_bfloat16>(batch, vocab, vocab_offset, sms);
+  const Rooms& rooms = logits_are_fp32 ? rooms_of_device<float>() : rooms_of_device<__nv_bfloat16>();
+  const Shape shape = shape_of(batch, vocab, vocab_offset, logits_are_fp32, sms, rooms);
   const int csize = shape.blocks;
   const int64_t blocks = static_cast<int64_t>(batch) * csize;
   cudaLaunchConfig_t cfg = {};
