@@ -439,15 +439,18 @@ static Shape in_waves(int batch, int vocab, int sms) {
 // most rows to read, in whole or in part, and what counts is to spread them evenly and at once.  Blocks of 768 threads
 // stand one to an SM, so that as many clusters as the device can hold of them are spread evenly by force; 384 stand two to
 // an SM, 256 four.  Clusters are counted as the device counts them: one lies within a group of SMs, and what is left of a
-// group is no use to it (of six blocks to an SM each, 148 SMs hold fewer than 24).  Blocks of 512 threads are spread evenly
-// only where a cluster has one or two.  More than two rows to an SM go out in powers of two blocks of 256 threads as before
-// (one block to a row, which all fit: 300 rows 65 us instead of 57, 400 76 instead of 65; waves of blocks of 512 threads sample 512 rows in 76
-// instead of 85, but take 29.3 instead of 25.7 for 450 greedy ones, which the host cannot tell).  All times are for 151936 logits and
-// T = 0.6, before (powers of two, 256 threads) -> now, us: 1 row 6.35 -> 5.65, 9 9.7 -> 7.3, 16 12.2 -> 8.4, 24 12.4 -> 8.9, 32 12.4
-// -> 10.1, 48 15.3 -> 13.1, 64 16.6 -> 14.7, 88 23.0 -> 18.6, 110 27.3 -> 23.7, 128 27.6 -> 25, 180 37.4 -> 34.4, 222 43.6 ->
-// 36.8, 256 47.4 -> 43.5; 150 rows of 32000 logits 13.0 -> 11.7; greedy 16 6.2 -> 4.1, 100 12.5 -> 9.3, 256 15.9 -> 15.6 (of fp32
-// 150 23.6 -> 17.7, but 64 9.6 -> 10.0 and 200 25.4 -> 26.1).  In each case within 6 % of the best of all
-// pairs of one to eight and sixteen blocks and 192, 256, 320, 384, 512 and 768 threads.
+// group is no use to it (of six blocks to an SM each, 148 SMs hold 22).  Blocks of 512 threads are spread evenly only where a
+// cluster has one or two, 256 where it has two and every thread something to read.  The cost of a form is what the fullest
+// SM's share of sampled bf16 rows of 151936 logits took in it, over that of 512 threads; fp32 and greedy rows go by the same,
+// as the host does not know the temperatures.  Where it leads to no form that is even, powers of two in waves (in_waves):
+// more than two rows to an SM (300 rows 57 us, 65 at once, 400 65 and 76; waves of blocks of 512 threads sample 512 in 76
+// instead of 85, but take 29.3 instead of 25.7 for 450 greedy ones), and long ones of which SMs would have one or two (200
+// 36.4, 41.7 at once; fp32 45.6, 50.5, though greedy 25.1, 22.4).  Rows shorter than kLongRow have too little for the merges of
+// four blocks of 256 threads and more (112 rows of 32000 10.2 -> 8.7 us, of 18992 greedy fp32 4.8 -> 4.0).
+// All for 151936 logits and T = 0.6 unless said, in waves -> now, us: 1 row 6.05 -> 5.4, 16 10.35 -> 8.15, 64 16.1 -> 14.4, 100 24.8 ->
+// 21.7, 148 30.6 -> 23.6, 180 35.6 -> 31.4, 256 43.9 -> 42.3.  Of 980 launches (1-512 rows of 1000-151936 logits of both types,
+// sampled and greedy) in a chain the mean is 11 % faster; 32 are 4 % slower or more, four of them by over 0.4 us (56 greedy
+// fp32 rows of 18992 and 32000, 150 and 180 sampled ones of 4096) and 222 greedy bf16 rows of 151936 (11.2 -> 12.5).
 struct Form {
   int threads, per_sm, least, most;  // of a block; blocks of it on an SM; blocks to a row
   double cost;                       // of a row, relative to 512 threads
@@ -457,6 +460,7 @@ static_assert(sizeof(kForms) / sizeof(kForms[0]) == NVLLM_SAMPLE_FORMS, "as the 
 constexpr int kSixteen = 0;              // clusters of sixteen are counted in this form, one block to an SM, and launched with
 constexpr int kSixteenThreads = 512;     // fewer threads: 5.65 us for one row, 5.9 with 768
 constexpr int kFull = 768;               // threads that keep an SM busy
+constexpr int64_t kLongRow = 8192;       // groups
 
 // Clusters of every size that a device holds at a time, in every form; 0: it does not say.
 struct Rooms {
@@ -480,9 +484,17 @@ static Shape shape_of(int batch, int vocab, int64_t vocab_offset, bool fp32, int
   for (int f = 0; f < NVLLM_SAMPLE_FORMS; ++f) {
     const Form& form = kForms[f];
     for (int c = form.least; c <= form.most; ++c) {
+      if (form.threads == kThreads && c > 3 && groups < kLongRow) continue;
       const int64_t room = c == 1 ? static_cast<int64_t>(sms) * form.per_sm : rooms.of[f][c];
-      if (room >= batch) offer(form, c, form.threads, c == 1 ? std::min<double>(form.per_sm, std::ceil(1.15 * batch * c / sms)) : form.per_sm);
+      const bool spread = c == 1 || (c * form.threads == 512 && groups >= 512);  // more evenly than an SM may hold of them
+      if (room >= batch) offer(form, c, form.threads, spread ? std::min<double>(form.per_sm, std::ceil(1.15 * batch * c / sms)) : form.per_sm);
     }
+  }
+  // Between one and two long rows to an SM, where every such form leaves SMs with two rows beside SMs with one: in waves
+  if (groups >= kLongRow && batch > sms) {
+    const double filled = static_cast<double>(batch) * waves.blocks / (4.0 * sms);  // of what the SMs hold at a time
+    const double rows = waves.blocks == 4 ? 1.575 + 0.882 * (filled - 1) : waves.blocks == 2 ? 2.19 - 0.8 * (1 - filled) : 4;
+    if (rows * static_cast<double>(groups) < least) return waves;
   }
   return best;
 }
