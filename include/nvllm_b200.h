@@ -313,13 +313,19 @@ NVLLM_API int nvllm_sample_candidates(const void* logits, int32_t logits_are_fp3
                             int32_t batch, int32_t vocab, void* stream);
 NVLLM_API int nvllm_sample_unpack(const int64_t* candidates, int64_t* tokens, int32_t batch, void* stream);
 
+/* Thread blocks (one cluster) of a row by powers of two, for three blocks of 256 threads to a multiprocessor: what a launch has
+ * (with largest_cluster = 8) where there are more than two rows to a multiprocessor or the device does not say how many
+ * clusters it holds; with largest_cluster >= 16 also sixteen, where that is no more than one to a multiprocessor.  Other
+ * launches are laid out otherwise: see nvllm_sample_layout.  Host arithmetic, exposed for tests and reports. */
+NVLLM_API int nvllm_sample_plan(int32_t batch, int32_t vocab, int32_t num_sms, int32_t largest_cluster);
+
 /* How nvllm_sample_tokens / nvllm_sample_candidates lay a launch out: thread blocks (one cluster) that read a row, and threads
  * of a block.  num_sms = 0: on the current device, whose clusters are counted as for a launch.  Else, as host arithmetic, on a
  * device of num_sms multiprocessors that holds clusters[form][blocks] clusters at a time (forms: blocks of 768, 512, 512, 384,
  * 256 and 256 threads; blocks 0 to 16; NULL: the device does not say).  Exposed for tests and reports. */
 #define NVLLM_SAMPLE_FORMS 6
-NVLLM_API int nvllm_sample_plan(int32_t batch, int32_t vocab, int64_t vocab_offset, int32_t logits_are_fp32, int32_t num_sms,
-                                const int32_t* clusters, int32_t* blocks, int32_t* threads);
+NVLLM_API int nvllm_sample_layout(int32_t batch, int32_t vocab, int64_t vocab_offset, int32_t logits_are_fp32, int32_t num_sms,
+                                  const int32_t* clusters, int32_t* blocks, int32_t* threads);
 
 /*
  * Decode-step inputs for a captured CUDA graph, in one launch.  `staged` is a device copy of

@@ -47,7 +47,8 @@ SIGNATURES = {
     "nvllm_sample_candidates": (c_int32, [c_void_p, c_int32, c_int64, c_void_p, c_void_p, c_int64, c_uint64, c_uint64,
                                           c_int64, c_void_p, c_int32, c_int32, c_void_p]),
     "nvllm_sample_unpack": (c_int32, [c_void_p, c_void_p, c_int32, c_void_p]),
-    "nvllm_sample_plan": (c_int32, [c_int32, c_int32, c_int64, c_int32, c_int32, POINTER(c_int32), POINTER(c_int32), POINTER(c_int32)]),
+    "nvllm_sample_plan": (c_int32, [c_int32, c_int32, c_int32, c_int32]),
+    "nvllm_sample_layout": (c_int32, [c_int32, c_int32, c_int64, c_int32, c_int32, POINTER(c_int32), POINTER(c_int32), POINTER(c_int32)]),
     "nvllm_decode_step_inputs": (c_int32, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, c_int32, c_int32,
                                            c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_void_p]),
     "nvllm_decode_step_inputs_pinned": (c_int32, [c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64, c_void_p, c_int32,

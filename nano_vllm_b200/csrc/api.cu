@@ -92,7 +92,7 @@ int nvllm_read_status(int32_t* host_out) {
   return NVLLM_OK;
 }
 
-int nvllm_abi_version(void) { return 3; }
+int nvllm_abi_version(void) { return 2; }
 
 int64_t nvllm_launch_count(void) { return nvllm::g_launches.load(std::memory_order_relaxed); }
 

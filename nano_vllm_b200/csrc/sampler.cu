@@ -539,17 +539,26 @@ static int sample_launch(const void* logits, int32_t logits_are_fp32, int64_t ro
 
 }  // namespace nvllm
 
-extern "C" int nvllm_sample_plan(int32_t batch, int32_t vocab, int64_t vocab_offset, int32_t logits_are_fp32, int32_t num_sms,
-                                 const int32_t* clusters, int32_t* blocks, int32_t* threads) {
+extern "C" int nvllm_sample_plan(int32_t batch, int32_t vocab, int32_t num_sms, int32_t largest_cluster) {
+  using namespace nvllm;
+  if (batch < 0 || vocab <= 0 || num_sms <= 0) return fail(NVLLM_E_GEOMETRY, "sample_plan: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
+  const int c = in_waves(batch, vocab, num_sms).blocks;
+  const bool sixteen = c == kPortableCluster && largest_cluster >= kMaxCluster && vocab >= kMaxCluster * kThreads * 8 &&
+                       static_cast<int64_t>(batch) * kMaxCluster <= num_sms;
+  return sixteen ? kMaxCluster : c;
+}
+
+extern "C" int nvllm_sample_layout(int32_t batch, int32_t vocab, int64_t vocab_offset, int32_t logits_are_fp32, int32_t num_sms,
+                                   const int32_t* clusters, int32_t* blocks, int32_t* threads) {
   using namespace nvllm;
   if (batch < 0 || vocab <= 0 || vocab_offset < 0 || num_sms < 0 || (!num_sms && clusters))
-    return fail(NVLLM_E_GEOMETRY, "sample_plan: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
-  if (!blocks || !threads) return fail(NVLLM_E_NULL, "sample_plan: NULL pointer argument");
+    return fail(NVLLM_E_GEOMETRY, "sample_layout: batch=%d vocab=%d num_sms=%d invalid", batch, vocab, num_sms);
+  if (!blocks || !threads) return fail(NVLLM_E_NULL, "sample_layout: NULL pointer argument");
   Rooms rooms{};
   if (clusters) std::copy(clusters, clusters + NVLLM_SAMPLE_FORMS * (kMaxCluster + 1), &rooms.of[0][0]);
   else if (!num_sms) rooms = logits_are_fp32 ? rooms_of_device<float>() : rooms_of_device<__nv_bfloat16>();
   const int sms = num_sms ? num_sms : nvllm::num_sms();
-  if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_plan: no CUDA device is usable");
+  if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "sample_layout: no CUDA device is usable");
   const Shape shape = shape_of(batch, vocab, vocab_offset, logits_are_fp32, sms, rooms);
   *blocks = shape.blocks;
   *threads = shape.threads;

@@ -22,7 +22,7 @@ def test_every_declared_symbol_is_exported_and_bound(lib):
     for name in names:
         assert hasattr(lib, name), f"{name} declared in the header but not exported"
     assert sorted(names) == sorted(_lib.SIGNATURES), "ctypes table and header disagree"
-    assert lib.nvllm_abi_version() == 3
+    assert lib.nvllm_abi_version() == 2
 
 
 def test_decode_plan_and_workspace_are_pure_host_arithmetic(lib):

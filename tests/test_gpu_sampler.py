@@ -234,41 +234,51 @@ def test_greedy_rows_at_any_alignment_take_the_first_of_equal_logits(cuda, dtype
         assert A.sample_tokens(rows, temps).tolist() == [0] * len(firsts)
 
 
-def _form(lib, batch, vocab, dtype):
-    """(blocks to a row, threads of a block) of a launch on this device."""
-    c, n = ctypes.c_int32(), ctypes.c_int32()
-    assert lib.nvllm_sample_plan(batch, vocab, 0, int(dtype == torch.float32), 0, None, ctypes.byref(c), ctypes.byref(n)) == 0
-    return c.value, n.value
-
-
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
 def test_rows_do_not_depend_on_the_blocks_that_read_them(cuda, lib, dtype):
-    """The first rows of batches in waves of two blocks to a row and of one, and of one that is read at once: the same
-    tokens."""
+    """The first rows of batches that give a row sixteen, eight, four, two and one block: the same tokens."""
     vocab = 40000
     g = torch.Generator(device=cuda).manual_seed(17)
     logits = (torch.randn(500, vocab, generator=g, device=cuda) * 3).to(dtype)
     temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.3], device=cuda).repeat(100)
     sms = torch.cuda.get_device_properties(cuda).multi_processor_count
-    batches = (20, 400, 500)
-    assert [_form(lib, b, vocab, dtype) for b in batches[1:]] == [(2, 256), (1, 256)] or sms != 148
+    batches = (5, 20, 200, 400, 500)
+    assert [lib.nvllm_sample_plan(b, vocab, sms, 16) for b in batches] == [16, 8, 4, 2, 1] or sms != 148
     want = A.sample_tokens(logits, temps, seed=3, step=8)
     for b in batches[:-1]:
         assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=3, step=8), want[:b]), f"batch {b}"
 
 
-@pytest.mark.parametrize("dtype,vocab", [(torch.bfloat16, 40000), (torch.float32, 9973), (torch.bfloat16, 517), (torch.bfloat16, 151936), (torch.float32, 151643)])
-def test_rows_do_not_depend_on_the_form_of_the_launch(cuda, lib, dtype, vocab):
+@pytest.mark.parametrize("dtype,vocab", [(torch.bfloat16, 40000), (torch.float32, 9973), (torch.bfloat16, 517)])
+def test_rows_do_not_depend_on_the_form_of_the_launch(cuda, dtype, vocab):
     """The first rows of batches that are read by one to eight and sixteen blocks of every size, in one wave and more, by
     rows with less than a group for every thread too: the same tokens."""
     g = torch.Generator(device=cuda).manual_seed(23)
     logits = (torch.randn(620, vocab, generator=g, device=cuda) * 3).to(dtype)
     temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.3], device=cuda).repeat(124)
     want = A.sample_tokens(logits, temps, seed=4, step=9)
-    forms = {620: _form(lib, 620, vocab, dtype)}
     for b in (1, 7, 12, 16, 20, 24, 28, 32, 36, 48, 64, 80, 100, 128, 150, 180, 200, 222, 256, 300, 450, 593):
-        forms[b] = _form(lib, b, vocab, dtype)
         assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=4, step=9), want[:b]), f"batch {b}"
-    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148 and vocab > 100000:
-        assert {c for c, _ in forms.values()} >= {1, 2, 3, 4, 5, 6, 8, 16}, forms
-        assert {n for _, n in forms.values()} == {256, 384, 512, 768}, forms
+
+
+def _layout(lib, batch, vocab, dtype):
+    """(blocks to a row, threads of a block) of a launch on this device."""
+    c, n = ctypes.c_int32(), ctypes.c_int32()
+    assert lib.nvllm_sample_layout(batch, vocab, 0, int(dtype == torch.float32), 0, None, ctypes.byref(c), ctypes.byref(n)) == 0
+    return c.value, n.value
+
+
+@pytest.mark.parametrize("dtype,vocab", [(torch.bfloat16, 151936), (torch.float32, 151643)])
+def test_batches_of_every_layout_pick_the_same_tokens(cuda, lib, dtype, vocab):
+    """Long rows read by one to six, eight and sixteen blocks of 256 to 768 threads, in one wave and in several."""
+    g = torch.Generator(device=cuda).manual_seed(29)
+    logits = (torch.randn(620, vocab, generator=g, device=cuda) * 3).to(dtype)
+    temps = torch.tensor([0.6, 1.0, 0.0, 2.5, 0.3], device=cuda).repeat(124)
+    want = A.sample_tokens(logits, temps, seed=5, step=2)
+    layouts = {_layout(lib, 620, vocab, dtype)}
+    for b in (1, 7, 12, 16, 20, 24, 28, 32, 36, 48, 64, 80, 100, 128, 150, 180, 200, 222, 256, 300, 450, 593):
+        layouts.add(_layout(lib, b, vocab, dtype))
+        assert torch.equal(A.sample_tokens(logits[:b], temps[:b], seed=5, step=2), want[:b]), f"batch {b}"
+    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148:
+        assert {c for c, _ in layouts} >= {1, 2, 3, 4, 5, 6, 8, 16}, layouts
+        assert {n for _, n in layouts} == {256, 384, 512, 768}, layouts

@@ -129,6 +129,17 @@ def test_all_reduce_protocol_choice_is_host_arithmetic(lib):
 
 
 @pytest.mark.parametrize("sms", [148, 132, 20])
+def test_sampler_takes_no_larger_cluster_than_the_device_grants(lib, sms):
+    """Sixteen blocks to a row for the fewest rows where that is possible, else eight; the same plan
+    for larger batches and rows too short for it."""
+    for batch in (1, 2, 9, 10, 32, 64, 256, 512):
+        for vocab in (7, 2047, 4096, 16384, 32768, 151936):
+            wide, portable = lib.nvllm_sample_plan(batch, vocab, sms, 16), lib.nvllm_sample_plan(batch, vocab, sms, 8)
+            assert portable in (1, 2, 4, 8) and wide == (16 if batch * 16 <= sms and vocab >= 16 * 2048 else portable)
+    assert lib.nvllm_sample_plan(1, 151936, sms, 8) == 8 and lib.nvllm_sample_plan(1, 0, sms, 8) == -3
+
+
+@pytest.mark.parametrize("sms", [148, 132, 20])
 @pytest.mark.parametrize("device", ["full", "gaps", "no sixteen", "silent"])
 def test_sampler_lays_launches_out_for_what_the_device_holds(lib, sms, device):
     """One wave of clusters that the device holds at a time, or blocks of 256 threads in powers of two: more than two
@@ -146,7 +157,7 @@ def test_sampler_lays_launches_out_for_what_the_device_holds(lib, sms, device):
     for batch in (*range(1, 64), 74, 100, 148, 180, 222, 2 * sms, 2 * sms + 1, 512):
         for fp32 in (0, 1):
             for vocab in (7, 1000, 2047, 4096, 18992, 32768, 50257, 151936):
-                assert lib.nvllm_sample_plan(batch, vocab, 0, fp32, sms, table, ctypes.byref(blocks), ctypes.byref(threads)) == 0
+                assert lib.nvllm_sample_layout(batch, vocab, 0, fp32, sms, table, ctypes.byref(blocks), ctypes.byref(threads)) == 0
                 c, n = blocks.value, threads.value
                 assert 256 <= n <= 768 and n % 32 == 0
                 waves = 1
@@ -159,8 +170,8 @@ def test_sampler_lays_launches_out_for_what_the_device_holds(lib, sms, device):
                 seen.add((c, n))
     assert (16 in {c for c, _ in seen}) == (device == "full" and sms > 16)
     args = (0, 0, sms, table, ctypes.byref(blocks), ctypes.byref(threads))
-    assert lib.nvllm_sample_plan(1, 0, *args) == -3 and lib.nvllm_sample_plan(-1, 5, *args) == -3
-    assert lib.nvllm_sample_plan(1, 5, 0, 0, sms, table, None, ctypes.byref(threads)) == -1
+    assert lib.nvllm_sample_layout(1, 0, *args) == -3 and lib.nvllm_sample_layout(-1, 5, *args) == -3
+    assert lib.nvllm_sample_layout(1, 5, 0, 0, sms, table, None, ctypes.byref(threads)) == -1
 
 
 @pytest.mark.parametrize("batch,tiles", [(2, 10), (2, 3), (6, 30), (7, 7), (9, 5), (20, 21), (3, 296), (5, 37)])
