@@ -222,6 +222,15 @@ NVLLM_API int nvllm_prefill_varlen(const void* q, int64_t q_row_stride,
  * launch whose items are dealt out long tiles first.  Host arithmetic, exposed for tests. */
 NVLLM_API int nvllm_prefill_item(int32_t drawn, int32_t query_tiles, int32_t batch, int32_t head_groups);
 
+/* How a prefill is laid out on a device of num_sms multiprocessors: thread blocks that stand on one (three or two), the number of
+ * items above which they are dealt out long tiles first, and who stores new rows (0 nobody, 1 a spare warp of every block,
+ * 2 from the key tiles in shared memory).  rows: 0 packed K/V rows, nothing to store; 1 packed rows that the prefill stores
+ * itself; 2 through the block table, this step's rows read packed and stored on the way; 3 through the block table, nothing to
+ * store.  Host arithmetic, exposed for tests and reports. */
+NVLLM_API int nvllm_prefill_plan(int64_t total_q, int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k,
+                                 int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim, int32_t rows, int32_t num_sms,
+                                 int32_t* blocks_per_sm, int32_t* reordered_from, int32_t* store);
+
 /*
  * nvllm_store_kvcache followed by nvllm_decode_paged / nvllm_prefill_varlen, as the attention layer
  * does for every step (nanovllm/layers/attention.py:65-77), with the same arguments and results.

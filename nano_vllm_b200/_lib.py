@@ -33,6 +33,8 @@ SIGNATURES = {
                                        c_int32, c_void_p, c_int64, c_void_p, c_void_p, c_int64, c_int64, c_int32,
                                        c_int32, c_int32, c_int32, c_int32, c_int32, c_float, c_int64, c_void_p]),
     "nvllm_prefill_item": (c_int32, [c_int32, c_int32, c_int32, c_int32]),
+    "nvllm_prefill_plan": (c_int32, [c_int64, c_int64, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32, c_int32,
+                                     POINTER(c_int32), POINTER(c_int32), POINTER(c_int32)]),
     "nvllm_attention_decode": (c_int32, [c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p, c_int64, c_void_p,
                                          c_void_p, c_void_p, c_void_p, c_int64, c_int32, c_void_p, c_int64, c_int32, c_int32,
                                          c_int32, c_int32, c_float, c_int64, c_void_p, c_int64, c_void_p]),

@@ -118,6 +118,36 @@ extern "C" int nvllm_prefill_item(int32_t drawn, int32_t query_tiles, int32_t ba
   return spread_item(drawn, query_tiles, batch, head_groups);
 }
 
+extern "C" int nvllm_prefill_plan(int64_t total_q, int64_t total_k, int32_t batch, int32_t max_seqlen_q, int32_t max_seqlen_k,
+                                  int32_t num_q_heads, int32_t num_kv_heads, int32_t head_dim, int32_t rows, int32_t num_sms,
+                                  int32_t* blocks_per_sm, int32_t* reordered_from, int32_t* store) {
+  using namespace nvllm;
+  if (head_dim != 64 && head_dim != 128) return fail(NVLLM_E_GEOMETRY, "prefill_plan: head_dim=%d unsupported (64 or 128)", head_dim);
+  if (num_q_heads <= 0 || num_kv_heads <= 0 || num_q_heads % num_kv_heads || batch <= 0 || total_q <= 0 || total_k < 0 ||
+      max_seqlen_q <= 0 || max_seqlen_k < 0 || rows < 0 || rows > 3 || num_sms <= 0)
+    return fail(NVLLM_E_GEOMETRY, "prefill_plan: Hq=%d Hkv=%d batch=%d total_q=%lld rows=%d num_sms=%d invalid", num_q_heads, num_kv_heads,
+                batch, (long long)total_q, rows, num_sms);
+  if (!blocks_per_sm || !reordered_from || !store) return fail(NVLLM_E_NULL, "prefill_plan: NULL pointer argument");
+  PrefillParams p{};
+  p.batch = batch;
+  p.max_seqlen_q = max_seqlen_q;
+  p.max_seqlen_k = max_seqlen_k;
+  p.hq = num_q_heads;
+  p.hkv = num_kv_heads;
+  p.g = num_q_heads / num_kv_heads;
+  p.d = head_dim;
+  const bool stored = rows == 1 || rows == 2;
+  p.slots = stored ? store : nullptr;  // these two are only asked for whether there are any
+  p.block_tables = rows >= 2 ? store : nullptr;
+  p.n_new = stored ? total_k : 0;
+  p.route.jobs = rows == 2;
+  const PrefillPlan plan = prefill_plan(p, total_q, num_sms);
+  *blocks_per_sm = plan.blocks;
+  *reordered_from = plan.spread_from;
+  *store = static_cast<int32_t>(plan.store);
+  return NVLLM_OK;
+}
+
 extern "C" int nvllm_attention_prefill(const void* q, int64_t q_row_stride, const void* key, int64_t key_row_stride,
                                        const void* value, int64_t value_row_stride, const int32_t* slot_mapping, void* k_cache,
                                        void* v_cache, const int32_t* block_tables, int64_t bt_row_stride, int32_t max_blocks,

@@ -81,6 +81,14 @@ int launch_prefill_mma(const PrefillParams& p, cudaStream_t stream);
 // tcgen05 / TMEM / TMA kernel in persistent blocks that pull (sequence, query tile, head) items
 // from a global counter; batch <= kPrefillMaxBatch.  total_q / total_k bound the tiled loads.
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream);
+// How it is laid out on a device of `sms` multiprocessors: by the launch's sizes, whether there are rows to store (slots,
+// n_new) and whether through the block table, with the route's tables or without (block_tables, route.jobs).
+struct PrefillPlan {
+  int blocks, grid;  // to an SM (three at head_dim 64 only), of the launch
+  int spread_from;   // see PrefillParams
+  Store store;
+};
+PrefillPlan prefill_plan(const PrefillParams& p, int64_t total_q, int sms);
 // Work items of such a launch at most.
 int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch);
 // Fills the tables for a prefill through the block table and copies the rows that cannot be read packed.

@@ -904,33 +904,74 @@ int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch) {
   return static_cast<int64_t>((max_seqlen_q + bmt - 1) / bmt) * (hq / pack) * batch;
 }
 
-// Prompts of less than three key tiles are the two-block form's: a block of three has no warps to write an item's results while
-// the next is begun (14 / 2 heads, two blocks -> three, us: 100 of 100-200 tokens 26.9 -> 27.4, 128 of 128 28.3 -> 28.6, 200 of 20-100
-// 24.8 -> 26.8, 256 of 64 28.1 -> 30.5; 64 of 256 32.4 -> 32.1).
-constexpr int kTrioTokens = 3 * tc::BN;
+// Prompts of less than four key tiles are the two-block form's: a block of three has no warps to write an item's results while
+// the next is begun (24 prompts of 192 tokens, 14 / 2 heads, two blocks -> three 14.1 -> 15.0 us, 100 of 100-200 26.9 -> 27.4; of 256 20.7 -> 19.8).
+constexpr int kTrioTokens = 4 * tc::BN;
 
-// All prompts within 2 % of one length: in launches of three blocks to an SM their long tiles go first.  Sequence after
-// sequence the last ones' start late and run alone at the end.  Three blocks, without -> with that order, us: 4 of 4096
-// tokens 189 -> 166, 16 of 1024 62.4 -> 56.2, 8 of 512 19.6 -> 16.1, 64 of 256 32.2 -> 31.5; of other prompts 12 of 700-800 34.3 -> 35.0, 80
-// of 180-200 28.4 -> 29.3.  Not with two blocks, whose short launches the code for it costs 1-1.7 %, nor at head_dim 128 (4
-// of 4096 242 -> 247, 64 of 256 50 -> 61: what keeps memory busy there is the mix of long and short tiles).
-static bool prompts_of_one_length(const PrefillParams& p, int64_t total_q) {
-  return p.batch > 1 && 50ll * p.max_seqlen_q * p.batch <= 51 * total_q;
+// All prompts have the same number of query tiles, as far as their sum and the longest tell (through a table, where one prompt with
+// a cached block may take all that is missing, for sure; else if they are spread evenly up to the longest): in launches of three
+// blocks to an SM their long tiles go first.  Sequence after sequence the last ones' start late and run alone at the end.  Three
+// blocks, 14 / 2 heads, without -> with that order, us: 4 of 4096 tokens 189 -> 166, 16 of 1024 62.4 -> 56.2, 8 of 512 19.8 -> 15.9.
+// Where a prompt has a tile more than others the turns do not line up (two blocks -> three with the order: 6 of 500-510 tokens, 28
+// or 29 tiles, 15.1 -> 18.3, 12 of 250-255 12.8 -> 14.4; 16 / 16 heads, 5 of 2048 of which one has a cached block 80.4 -> 96.1).  Not with two
+// blocks, whose short launches the code for it costs 1-1.7 %, nor at head_dim 128 (4 of 4096 242 -> 247, 64 of 256 50 -> 61: what
+// keeps memory busy there is the mix of long and short tiles).
+static bool same_tiles(const PrefillParams& p, int64_t total_q, int bmt) {
+  const int64_t missing = static_cast<int64_t>(p.max_seqlen_q) * p.batch - total_q;  // to prompts that are all as long as the longest
+  const int in_last = (p.max_seqlen_q - 1) % bmt + 1;                               // tokens of that one's last tile
+  return p.batch > 1 && (p.block_tables ? missing < in_last : 2 * missing < static_cast<int64_t>(in_last) * p.batch);
 }
 
-// Head_dim 64: three blocks to an SM, of eight warps, or two of twelve.  Three get up to 12 % more done where there is
-// enough for all of them: four times the key tiles of the longest item for every SM, since an item takes a block of three
-// longer.  14 / 2 heads, two blocks -> three, us (tiles of an SM over those of the longest item in brackets): 64 of 100-1024
-// tokens 74.4 -> 70.9 (8.3), 32 39.4 -> 38.2 (4.1), 16 22.7 -> 22.6 (2), 8 17.4 -> 18.8 (1), 8 of 1500-2048 82.4 -> 81.4 (4.8), 5 of 1000-3000
-// 70.2 -> 71.3 (2.6), 40 of 200-400 26.4 -> 26.2 (4.1), 2 of 2000-2500 38.2 -> 43.3 (1.7).  For prompts of one length several items to a
-// block are enough: 4 of 4096 180 -> 167, 16 of 1024 63.0 -> 56.4, 6 of 2000-2010 81.3 -> 71.4, 2 of 4000-4096 96.1 -> 94.8 (3.1), 8 of 512
-// 17.9 -> 16.2 (1.8).
-static bool three_blocks(const PrefillParams& p, int64_t total_q) {
-  const int sms = num_sms(), pack = heads_per_tile(p.g), bmt = tc::BM / pack;
+// Head_dim 64: three blocks to an SM, of eight warps, or two of twelve.  Three get up to 20 % more done where there is enough
+// for all of them, since an item takes a block of three longer.
+// Prompts of the same number of tiles: more than two items to an SM, and eight query tiles to a prompt, since the rows of a key
+// tile are stored by one warp instead of four, the oftener the fewer query tiles read it.  Two blocks -> three, us: 4 of 4096
+// tokens, 14 / 2 heads 180 -> 165, 16 of 1024 62.9 -> 56.2, 4 of 1024 24.8 -> 21.4, 10 of 300 13.3 -> 13.1; 7 / 1 heads, 5 of 2048 46.6 -> 35.6;
+// 32 / 8, 8 of 512 27.3 -> 25.3; 16 / 16, 8 of 2048 123 -> 111.  On the other side 16 / 16 heads, 48 of 256 (two tiles) 34.9 -> 42.9, 32 of 512
+// (four) 52.4 -> 58.3.
+// Other prompts, several heads to a tile: eight times the longest item's key tiles for every SM, or four times from twelve
+// prompts of different lengths on: 64 of 100-1024 tokens, 14 / 2 heads, 73.9 -> 71.2, 48 of 200-800 63.1 -> 60.6.  On the other side 5 of
+// 2000-4096 (4.4 times) 108 -> 114, 16 of 1000-1024 (6.4 times) 62.7 -> 66.1; one head to a tile, 48 of 200-400 (8 times) 46.8 -> 51.3.
+// Of 237 launches that the rule takes (six pairs of heads, 256 to 4096 tokens) the mean is 6 % faster; 21 are slower, six of them
+// by 3-8 % (32 / 8 heads, 7 of 256 13.1 -> 14.1; 16 / 16, 3 of 1024 22.0 -> 23.0).
+static bool three_blocks(const PrefillParams& p, int64_t total_q, int sms) {
+  const int pack = heads_per_tile(p.g), bmt = tc::BM / pack;
   const double mean = static_cast<double>(total_q) / p.batch;
   const double items = static_cast<double>(total_q) / bmt * (p.hq / pack), tiles = items * (mean / 2 + tc::BN / 2) / tc::BN;
-  return mean >= kTrioTokens &&
-         (prompts_of_one_length(p, total_q) ? items > 2.0 * sms : tiles >= 4.0 * sms * p.max_seqlen_k / tc::BN);
+  if (mean < kTrioTokens) return false;
+  if (same_tiles(p, total_q, bmt)) return mean > 7 * bmt && items > 2.0 * sms;
+  const double times = tiles * tc::BN / (static_cast<double>(sms) * p.max_seqlen_k);
+  return pack > 1 && (times >= 8 || (times >= 4 && p.batch >= 12 && p.max_seqlen_q >= 1.03 * mean));
+}
+
+PrefillPlan prefill_plan(const PrefillParams& p, int64_t total_q, int sms) {
+  const int bmt = tc::BM / heads_per_tile(p.g);
+  const bool routed = p.route.jobs > 0;
+  PrefillPlan plan;
+  plan.blocks = p.d == 64 && three_blocks(p, total_q, sms) ? 3 : 2;
+  // an upper bound of the work items known to the host: no more blocks than that
+  const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
+  plan.grid = plan.blocks * sms;
+  // With an item to a block and more items than SMs, blocks that share an SM with those of long tiles get short ones by
+  // another order: 6 prompts of 300 tokens 15.1 -> 13.4 us, 10 of 100 11.4 -> 10.4, 3 of 500 14.6 -> 14.1.  Which blocks
+  // meet on an SM is the hardware's choice, so this is a matter of averages: of 448 launches of 2-40 prompts (eight
+  // pairs of head counts) the 346 that the rule takes are 6 % faster in the mean, twelve of them 1-10 % slower (22 of
+  // 381-420 tokens, 2 / 1 heads, 12.9 -> 14.4).  Not where an SM has one block (the divisions cost 0.3 us: 5 prompts of 60
+  // tokens 8.2 -> 8.5), where long and short prompts mix, whose tiles every q-th of the list does not line up (19 of
+  // 209-582 16.0 -> 17.3), nor at head_dim 64 (14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05).
+  const bool alike = p.max_seqlen_q <= 5 * bmt || 20ll * p.max_seqlen_q * p.batch <= 23 * total_q;
+  plan.spread_from = plan.blocks == 3 ? (same_tiles(p, total_q, bmt) ? 0 : 1 << 30) : p.d == 128 && p.batch > 1 && alike ? sms : 1 << 30;
+  // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
+  // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
+  // rows, 4 KB in flight; 120 from the tiles; 110 with nothing to store).  Where a block has one item at most that
+  // would end it later (a prompt of 201 tokens 9.05 -> 9.5 us): there an idle warp of every block copies the rows, by
+  // as many blocks as that takes two trips of, as long as four of them are enough (6 prompts of 300 tokens: 15.8
+  // us from the tiles, 20.2 copied).
+  const int64_t pieces = p.n_new * p.hkv * (p.d / 8);
+  plan.store = !p.slots ? Store::None : routed || max_items > plan.grid || pieces > 4ll * 64 * plan.grid ? Store::Tiles : Store::Spare;
+  const int64_t copy_blocks = plan.store == Store::Spare ? (pieces + 127) / 128 : 0;
+  plan.grid = static_cast<int>(std::min<int64_t>(plan.grid, std::max(max_items, copy_blocks)));
+  return plan;
 }
 
 // Makes the kernels of a form ready for their launches on a device.
@@ -953,7 +994,7 @@ static int prepare_prefill_tcp() {
 }
 
 template <int D, bool TRIO>
-static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int64_t total_k, cudaStream_t stream) {
+static int launch_prefill_tcp_t(const PrefillParams& p_in, const PrefillPlan& plan, int64_t total_q, int64_t total_k, cudaStream_t stream) {
   using G = tcp::Geo<D, TRIO>;
   static bool ready[64] = {false};
   int dev = 0;
@@ -990,39 +1031,21 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, int64_t total_q, int6
     if (!make_tmap_3d(&mv, p.v, D, p.hkv, total_k, D, p.v_stride, tc::BN)) return NVLLM_E_CUDA;
     mkey = mk, mvalue = mv;
   }
-  // an upper bound of the work items known to the host: no more blocks than that
-  const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
-  int grid = G::BLOCKS * num_sms();
-  if (grid <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
-  // With an item to a block and more items than SMs, blocks that share an SM with those of long tiles get short ones by
-  // another order: 6 prompts of 300 tokens 15.1 -> 13.4 us, 10 of 100 11.4 -> 10.4, 3 of 500 14.6 -> 14.1.  Which blocks
-  // meet on an SM is the hardware's choice, so this is a matter of averages: of 448 launches of 2-40 prompts (eight
-  // pairs of head counts) the 346 that the rule takes are 6 % faster in the mean, twelve of them 1-10 % slower (22 of
-  // 381-420 tokens, 2 / 1 heads, 12.9 -> 14.4).  Not where an SM has one block (the divisions cost 0.3 us: 5 prompts of 60
-  // tokens 8.2 -> 8.5), where long and short prompts mix, whose tiles every q-th of the list does not line up (19 of
-  // 209-582 16.0 -> 17.3), nor at head_dim 64 (14 / 2 heads, 6 of 100-300 tokens 9.65 -> 10.05).
-  const bool alike = p.max_seqlen_q <= 5 * bmt || 20ll * p.max_seqlen_q * p.batch <= 23 * total_q;
-  p.spread_from = TRIO ? (prompts_of_one_length(p, total_q) ? 0 : 1 << 30) : p.batch > 1 && alike ? num_sms() : 1 << 30;
-  // Rows to be stored.  Where blocks work on several items one after the other, from the key tiles that pass through
-  // shared memory (64 prompts of 100-1024 tokens, 16 / 8 heads: 200 us when two idle warps of every block copied all
-  // rows, 4 KB in flight; 120 from the tiles; 110 with nothing to store).  Where a block has one item at most that
-  // would end it later (a prompt of 201 tokens 9.05 -> 9.5 us): there an idle warp of every block copies the rows, by
-  // as many blocks as that takes two trips of, as long as four of them are enough (6 prompts of 300 tokens: 15.8
-  // us from the tiles, 20.2 copied).
-  const int64_t pieces = p.n_new * p.hkv * (D / 8);
-  p.store = !p.slots ? Store::None : routed || max_items > grid || pieces > 4ll * 64 * grid ? Store::Tiles : Store::Spare;
-  const int64_t copy_blocks = p.store == Store::Spare ? (pieces + 127) / 128 : 0;
-  grid = static_cast<int>(std::min<int64_t>(grid, std::max(max_items, copy_blocks)));
+  p.spread_from = plan.spread_from;
+  p.store = plan.store;
   static_assert(sizeof(g_launch_seq) == 4 && (1ull << 32) % tcp::NUM_SLOTS == 0, "the slots follow one another when the count wraps");
   const int slot = static_cast<int>(g_launch_seq.fetch_add(1) % tcp::NUM_SLOTS);
-  return launch_kernel("prefill (tcgen05, persistent)", routed ? prefill_tcp_kernel<D, true, TRIO> : prefill_tcp_kernel<D, false, TRIO>, dim3(grid),
+  return launch_kernel("prefill (tcgen05, persistent)", routed ? prefill_tcp_kernel<D, true, TRIO> : prefill_tcp_kernel<D, false, TRIO>, dim3(plan.grid),
                        dim3(G::NTHREADS), G::SMEM, stream, p, mq, mk, mv, mkey, mvalue, slot);
 }
 
 int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k, cudaStream_t stream) {
-  if (p.d == 128) return launch_prefill_tcp_t<128, false>(p, total_q, total_k, stream);
-  return three_blocks(p, total_q) ? launch_prefill_tcp_t<64, true>(p, total_q, total_k, stream)
-                                  : launch_prefill_tcp_t<64, false>(p, total_q, total_k, stream);
+  const int sms = num_sms();
+  if (sms <= 0) return fail(NVLLM_E_NO_DEVICE, "prefill: no CUDA device is usable");
+  const PrefillPlan plan = prefill_plan(p, total_q, sms);
+  if (p.d == 128) return launch_prefill_tcp_t<128, false>(p, plan, total_q, total_k, stream);
+  return plan.blocks == 3 ? launch_prefill_tcp_t<64, true>(p, plan, total_q, total_k, stream)
+                          : launch_prefill_tcp_t<64, false>(p, plan, total_q, total_k, stream);
 }
 
 }  // namespace nvllm

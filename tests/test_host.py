@@ -242,3 +242,49 @@ def test_reading_an_expired_wait_zeroes_the_decode_scratch(monkeypatch, status):
     assert len(cleared) == (status >= 4)
     monkeypatch.setattr(_lib, "_host", None)  # no call has been made: there is nothing to clear
     assert _lib.read_status() == status
+
+
+def _prefill_plan(lib, lens, hq, hkv, d, rows=0, sms=148, max_k=None):
+    out = [ctypes.c_int32() for _ in range(3)]
+    args = (sum(lens), sum(lens), len(lens), max(lens), max_k or max(lens), hq, hkv, d, rows, sms)
+    rc = lib.nvllm_prefill_plan(*args, *(ctypes.byref(x) for x in out))
+    return rc if rc else tuple(x.value for x in out)
+
+
+def test_prefill_layout_is_host_arithmetic(lib):
+    never, none, spare, tiles = 1 << 30, 0, 1, 2
+    # head_dim 64: prompts of the same number of query tiles, more than two items to a multiprocessor; a spare warp stores rows while there are few
+    assert _prefill_plan(lib, [512] * 7, 14, 2, 64) == (3, 0, none)
+    assert _prefill_plan(lib, [512] * 7, 14, 2, 64, rows=1) == (3, 0, spare)
+    assert _prefill_plan(lib, [512] * 7, 14, 2, 64, rows=2) == (3, 0, tiles)
+    assert _prefill_plan(lib, [512] * 16, 14, 2, 64, rows=1) == (3, 0, tiles)
+    assert _prefill_plan(lib, [512] * 5, 14, 2, 64) == (2, never, none)                 # 285 items
+    assert _prefill_plan(lib, [512] * 7, 14, 2, 64, sms=300) == (2, never, none)
+    assert _prefill_plan(lib, [255] * 60, 14, 2, 64) == (2, never, none)                # less than four key tiles
+    assert _prefill_plan(lib, [256] * 60, 14, 2, 64) == (3, 0, none)
+    assert _prefill_plan(lib, [896] * 60, 16, 16, 64) == (2, never, none)               # seven query tiles to a prompt
+    assert _prefill_plan(lib, [897] * 60, 16, 16, 64) == (3, 0, none)
+    # 29 tiles of 18 tokens, 8 in the last: lengths spread evenly over 505-512 have it, over 500-512 not
+    assert _prefill_plan(lib, [512, 505, 512, 505] * 3, 14, 2, 64) == (3, 0, none)
+    assert _prefill_plan(lib, [512, 500, 512, 500] * 3, 14, 2, 64) == (2, never, none)
+    # through the table one prompt may take all that is missing
+    assert _prefill_plan(lib, [512] * 11 + [505], 14, 2, 64, rows=3) == (3, 0, none)
+    assert _prefill_plan(lib, [512] * 11 + [504], 14, 2, 64, rows=3) == (2, never, none)
+    assert _prefill_plan(lib, [2048] * 4 + [1792], 16, 16, 64, rows=2) == (2, never, tiles)
+    # other prompts: eight times the longest item's key tiles to a multiprocessor, cached ones among them, or four times and
+    # twelve prompts of different lengths; in the list's order
+    mixed = [1024, 300, 700, 400]
+    assert _prefill_plan(lib, mixed * 8, 14, 2, 64) == (3, never, none)
+    assert _prefill_plan(lib, mixed * 8, 14, 2, 64, rows=2) == (3, never, tiles)
+    assert _prefill_plan(lib, mixed * 6, 14, 2, 64) == (2, never, none)                 # 3.9 times
+    assert _prefill_plan(lib, mixed * 8, 14, 2, 64, max_k=2048) == (2, never, none)
+    assert _prefill_plan(lib, mixed * 16, 14, 14, 64) == (2, never, none)               # one head to a tile
+    assert _prefill_plan(lib, [1022, 1001] * 8, 14, 2, 64) == (2, never, none)          # 6.4 times, of about one length
+    assert _prefill_plan(lib, [4096, 3000] * 3, 14, 2, 64) == (2, never, none)          # 6 times, six prompts
+    assert _prefill_plan(lib, [16384], 14, 2, 64) == (2, never, none) and _prefill_plan(lib, [32768], 14, 2, 64) == (3, never, none)
+    # head_dim 128: two blocks
+    for lens in ([512] * 40, mixed, [4096] * 4):
+        assert _prefill_plan(lib, lens, 16, 8, 128)[0] == 2
+    assert _prefill_plan(lib, [300] * 6, 16, 8, 128) == (2, 148, none)
+    assert _prefill_plan(lib, [512], 14, 2, 96) == -3 and _prefill_plan(lib, [512], 14, 3, 64) == -3
+    assert _prefill_plan(lib, [512], 14, 2, 64, rows=4) == -3 and _prefill_plan(lib, [512], 14, 2, 64, sms=0) == -3
