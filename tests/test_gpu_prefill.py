@@ -1,4 +1,5 @@
 """Varlen causal GQA prefill on the GPU, through the C ABI, against the fp32 CPU oracle."""
+import ctypes
 import random
 
 import pytest
@@ -355,6 +356,166 @@ def test_rows_are_stored_with_three_blocks_to_an_sm(cuda, hq, hkv, batch, table)
     torch.cuda.synchronize()
     assert torch.equal(layer.k_cache, k2) and torch.equal(layer.v_cache, v2)
     assert torch.equal(got.view_as(want), want)
+    assert _lib.read_status() == 0
+
+
+# ---- head_dim 64 with three blocks to an SM ------------------------------------------------------
+
+FORM_64 = [(14, 2), (7, 1), (16, 4)]
+NONE, SPARE, TILES = range(3)
+
+
+def _takes(cuda, lib, max_q, max_k, total_q, batch, hq, hkv, even, store, total_k=0, table=False):
+    """That a launch of head_dim 64 has three blocks to an SM, deals its items out long tiles first where the prompts have the
+    same number of them, and stores rows as named."""
+    out = [ctypes.c_int32() for _ in range(3)]
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    assert lib.nvllm_prefill_plan(total_q, total_k, batch, max_q, max_k, hq, hkv, 64, 3 if table else 1 if store else 0, sms, *(ctypes.byref(x) for x in out)) == 0
+    assert [x.value for x in out] == [3, 0 if even else 1 << 30, store] or sms != 148
+
+
+@pytest.mark.parametrize("hq,hkv,lens,shared,even", [(*heads, *x) for heads in FORM_64 for x in [
+    ([257] * 60, 0, True), ([320] * 40, 0, True), ([511, 512, 512, 510] * 6, 0, True), ([1024] * 15, 0, True), ([576] + [832] * 23, 1, True),
+    ([257] + [513] * 59, 1, True), ([700, 320, 1023, 300] * 32, 0, False), ([700, 964, 1023, 556] * 32, 1, False)]] + [
+    (4, 4, [1024] * 15, 0, True), (4, 4, [1024] + [1280] * 14, 1, True)])
+def test_three_blocks_to_an_sm(cuda, lib, hq, hkv, lens, shared, even):
+    """Prompts of the same number of query tiles, whose long tiles go first, and others; packed and through the table, where
+    all but the first begin with a cached block."""
+    case = W.make_prefill_case(71, len(lens), 1, 1, hq, hkv, 64, lengths=lens, shared_blocks=[shared * (i > 0) for i in range(len(lens))])
+    _takes(cuda, lib, case.max_seqlen_q, case.max_seqlen_k, case.q.shape[0], len(lens), hq, hkv, even, NONE, table=bool(shared))
+    _check(cuda, case, f"{len(lens)} of {lens[0]} hq{hq}")
+
+
+@pytest.mark.parametrize("d_heads,batch", [((14, 2), 7), ((7, 1), 14), ((8, 1), 12), ((16, 2), 6)])
+@pytest.mark.parametrize("low", [510, 512])
+def test_three_blocks_to_an_sm_whose_spare_warps_store_rows(cuda, lib, d_heads, batch, low):
+    """Few rows for many items: copied by a warp that no item has to do with.  Rows without a slot, in front of the first
+    sequence and behind the last, scattered slots; cache and output against the reference."""
+    (hq, hkv), d, r = d_heads, 64, random.Random(low)
+    lens = [r.randint(low, 512) for _ in range(batch - 1)] + [512]
+    front, behind = 3, 70
+    n, n_k = sum(lens), front + sum(lens) + behind
+    _takes(cuda, lib, 512, 512, n, batch, hq, hkv, True, SPARE, total_k=n_k)
+    gen = torch.Generator().manual_seed(batch)
+    rand = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()
+    q, k, v = rand(n, hq, d), rand(n_k, hkv, d), rand(n_k, hkv, d)
+    cu_q = torch.tensor([0] + lens).cumsum(0).int()
+    cu_k = cu_q + front
+    blocks = n_k // 256 + 3
+    slots = torch.randperm(blocks * 256, generator=gen)[:n_k].int()
+    slots[::11] = -1
+    k_cache, v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = k_cache.to(cuda), v_cache.to(cuda)
+    C.set_context(True, cu_q.to(cuda), cu_k.to(cuda), 512, 512, slots.to(cuda), None, None)
+    for _ in range(3):
+        got = layer(q.to(cuda).flatten(1), k.to(cuda).flatten(1), v.to(cuda).flatten(1))
+    C.reset_context()
+    torch.cuda.synchronize()
+    R.store_kvcache_ref(k, v, k_cache, v_cache, slots)
+    assert torch.equal(layer.k_cache.cpu().view(torch.int16), k_cache.view(torch.int16))
+    assert torch.equal(layer.v_cache.cpu().view(torch.int16), v_cache.view(torch.int16))
+    assert_close_to_oracle(got.view(n, hq, d), R.prefill_ref(q, k, v, cu_q, cu_k, d ** -0.5), f"{lens} hq{hq}")
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("hq,hkv", FORM_64)
+@pytest.mark.parametrize("table", [False, True])
+def test_three_blocks_to_an_sm_see_nothing_behind_a_sequence(cuda, lib, hq, hkv, table):
+    """NaN and infinities behind the sequences: in the rest of their last blocks, and in the rows behind the last packed one."""
+    lens = [300] + [556 if table else 300] * 47
+    case = W.make_prefill_case(73, 48, 1, 1, hq, hkv, 64, lengths=lens, shared_blocks=[int(table and i > 0) for i in range(48)])
+    _takes(cuda, lib, 300, max(lens), 300 * 48, 48, hq, hkv, True, NONE, table=table)
+    if table:
+        case.k_cache[:], case.v_cache[:] = float("nan"), float("inf")
+        return _check(cuda, case, "stale rows of the cache")
+    k = torch.cat([case.k, torch.full_like(case.k[:64], float("nan"))])
+    v = torch.cat([case.v, torch.full_like(case.v[:64], float("inf"))])
+    out = A.prefill_varlen(case.q.to(cuda), k.to(cuda), v.to(cuda), case.cu_seqlens_q.to(cuda), case.cu_seqlens_k.to(cuda), 300, 300, case.scale)
+    ref = R.prefill_ref(case.q, case.k, case.v, case.cu_seqlens_q, case.cu_seqlens_k, case.scale)
+    assert_close_to_oracle(out, ref, "rows behind the last")
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("hq,hkv", FORM_64)
+@pytest.mark.parametrize("lq", [[320] * 60, [320, 200, 319, 250] * 40])
+def test_three_blocks_to_an_sm_with_tiles_without_a_visible_key(cuda, lib, hq, hkv, lq):
+    """More queries than keys in every other sequence: blocks write zeros and draw again, in both orders of the items."""
+    lk = [n if i % 2 == 0 else (50, 128, 1)[i // 2 % 3] for i, n in enumerate(lq)]
+    _takes(cuda, lib, 320, 320, sum(lq), len(lq), hq, hkv, len(set(lq)) == 1, NONE)
+    gen = torch.Generator().manual_seed(len(lq))
+    rand = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()
+    q, k, v = rand(sum(lq), hq, 64), rand(sum(lk), hkv, 64), rand(sum(lk), hkv, 64)
+    cu = lambda x: torch.tensor([0] + x).cumsum(0).int()
+    args = [t.to(cuda) for t in (q, k, v, cu(lq), cu(lk))]
+    ref = R.prefill_ref(q, k, v, cu(lq), cu(lk), 0.125)
+    for _ in range(3):
+        out = torch.full((sum(lq), hq, 64), float("nan"), dtype=torch.bfloat16, device=cuda)
+        A.prefill_varlen(*args, 320, 320, 0.125, out=out)
+        assert_close_to_oracle(out, ref, f"hq{hq}")
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("hq,hkv", FORM_64)
+def test_three_blocks_to_an_sm_from_slices_in_graphs_and_on_two_streams(cuda, lib, hq, hkv):
+    """q, k and v as slices of one activation, v of another width; layers captured with their stores and replayed at the same
+    time on two streams, one of them beside launches of two blocks to an SM."""
+    d, lens, short = 64, [384] * 36, [100] * 30
+    _takes(cuda, lib, 384, 384, sum(lens), len(lens), hq, hkv, True, TILES, total_k=sum(lens))
+    gen = torch.Generator(device=cuda).manual_seed(83)
+    rand = lambda *shape: torch.randn(*shape, generator=gen, device=cuda).bfloat16()
+    runs = []
+    for seqs in ([lens], [lens, short]):
+        parts = []
+        for ls in seqs:
+            n = sum(ls)
+            qkv = rand(n, (hq + 2 * hkv) * d)
+            q, k, _ = qkv.split([hq * d, hkv * d, hkv * d], dim=1)
+            v = rand(n, 2 * hkv * d)[:, hkv * d:]
+            blocks = n // 256 + 3
+            layer = A.Attention(hq, d, d ** -0.5, hkv)
+            layer.k_cache, layer.v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+            slots = torch.randperm(blocks * 256, generator=gen, device=cuda)[:n].int()
+            parts.append((layer, q, k, v, torch.tensor([0] + ls, device=cuda).cumsum(0).int(), max(ls), slots))
+        runs.append(parts)
+
+    def go(parts):
+        outs = []
+        for layer, q, k, v, cu, longest, slots in parts:
+            C.set_context(True, cu, cu, longest, longest, slots, None, None)
+            outs.append(layer(q, k, v))
+        C.reset_context()
+        return outs
+
+    q, k, v, cu = (x.cpu() for x in runs[0][0][1:5])
+    ref = R.prefill_ref(q.unflatten(1, (hq, d)), k.unflatten(1, (hkv, d)), v.unflatten(1, (hkv, d)), cu, cu, d ** -0.5)
+    assert_close_to_oracle(go(runs[0])[0].view(-1, hq, d), ref, "slices")
+    want = [go(parts) for parts in runs]
+    planes = [[(p[0].k_cache.clone(), p[0].v_cache.clone()) for p in parts] for parts in runs]
+    torch.cuda.synchronize()
+    streams, graphs, outs = [torch.cuda.Stream() for _ in runs], [], []
+    for parts in runs:
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            outs.append(go(parts))
+    for _ in range(5):
+        for parts in runs:
+            for p in parts:
+                p[0].k_cache.zero_(), p[0].v_cache.zero_()
+        for got in outs:
+            for o in got:
+                o.fill_(float("nan"))
+        torch.cuda.synchronize()
+        for stream, graph in zip(streams, graphs):
+            with torch.cuda.stream(stream):
+                graph.replay()
+        torch.cuda.synchronize()
+        for parts, got, exp, kept in zip(runs, outs, want, planes):
+            for p, o, e, (kc, vc) in zip(parts, got, exp, kept):
+                stored = p[6].long()
+                assert torch.equal(o, e)
+                assert torch.equal(p[0].k_cache.flatten(0, 1)[stored], kc.flatten(0, 1)[stored])
+                assert torch.equal(p[0].v_cache.flatten(0, 1)[stored], vc.flatten(0, 1)[stored])
     assert _lib.read_status() == 0
 
 
