@@ -412,6 +412,75 @@ def test_step_whose_inputs_the_kernel_just_before_writes(cuda, hq, hkv, d, batch
     assert torch.equal(dev.k_cache.cpu().view(torch.int16), case.k_cache.view(torch.int16))
 
 
+def _units_to_a_range(cuda, lens, hq, hkv, d):
+    """Ranges that a KV head's units are cut into, and the units."""
+    unit, blocks = _lib.decode_plan(len(lens), 32, hq, hkv, d)
+    return blocks // hkv, sum(-(-n // unit) for n in lens)
+
+
+@pytest.mark.parametrize("hq,hkv,d,lens", [(32, 32, 128, [3500] * 6), (32, 32, 128, [2100, 5, 4000, 70, 3333, 1, 6000, 4321, 0]), (64, 64, 64, [3000] * 7)])
+def test_step_with_more_units_in_a_range_than_a_warp_lists(cuda, hq, hkv, d, lens):
+    """Over 32 units to a thread block, of a batch small enough to be listed ahead: new tokens on both sides of the 32nd."""
+    ranges, units = _units_to_a_range(cuda, lens, hq, hkv, d)
+    assert units > 32 * ranges or torch.cuda.get_device_properties(cuda).multi_processor_count != 148
+    case = W.make_decode_case(61, len(lens), 1, 1, hq, hkv, d, context_lens=lens)
+    sep, fus = case.to(cuda), case.to(cuda)
+    A.store_kvcache(sep.k_new, sep.v_new, sep.k_cache, sep.v_cache, sep.slot_mapping)
+    expected = A.decode_paged(sep.q, sep.k_cache, sep.v_cache, sep.context_lens, sep.block_tables, case.scale)
+    for _ in range(2):
+        got = A.decode_step(fus.q, fus.k_new, fus.v_new, fus.k_cache, fus.v_cache, fus.slot_mapping, fus.context_lens, fus.block_tables,
+                            case.scale)
+    torch.cuda.synchronize()
+    assert torch.equal(fus.k_cache, sep.k_cache) and torch.equal(fus.v_cache, sep.v_cache)
+    assert torch.equal(got, expected)
+    R.store_kvcache_ref(case.k_new, case.v_new, case.k_cache, case.v_cache, case.slot_mapping)
+    assert_close_to_oracle(got, R.decode_ref(case.q, case.k_cache, case.v_cache, case.context_lens, case.block_tables, case.scale), f"{lens}")
+    assert _lib.read_status() == 0
+
+
+@pytest.mark.parametrize("entries", [[(0, 8)], [(1, 13)], [(0, 8), (1, 13)]])
+def test_step_whose_only_change_lies_beyond_the_list(cuda, entries):
+    """Six sequences of 3500 tokens, 32 KV heads: ranges of 37 units, the first 32 of them listed.  The launch in front
+    changes only table entries of units past the 32nd of a range (and the slot of the new token in the second one's)."""
+    hq, hkv, d, lens = 32, 32, 128, [3500] * 6
+    ranges, units = _units_to_a_range(cuda, lens, hq, hkv, d)
+    if torch.cuda.get_device_properties(cuda).multi_processor_count == 148:
+        assert (ranges, units) == (9, 330)
+        for b, i in entries:  # 55 units a sequence, four to a block; the first six ranges have 37
+            spots = [b * 55 + u for u in range(4 * i, min(4 * i + 4, 55))]
+            assert all(s < 6 * 37 and s % 37 >= 32 for s in spots)
+    case = W.make_decode_case(67, 6, 1, 1, hq, hkv, d, context_lens=lens)
+    dev = case.to(cuda)
+    width, used = case.block_tables.shape[1], set(case.block_tables.flatten().tolist())
+    spare = [x for x in range(case.k_cache.shape[0]) if x not in used]
+    plane = torch.zeros(2, 256, 1, 256, dtype=torch.bfloat16, device=cuda)  # rows of 128 int32
+    words = plane[1].view(-1).view(torch.int32)
+    slots, table = words[:6], words[6:6 + 6 * width].view(6, width)
+    backwards = torch.arange(511, -1, -1, dtype=torch.int32, device=cuda)  # the rows that hold the words last
+    scratch = torch.zeros_like(plane)
+    steps = []
+    for i in range(4):
+        t = case.block_tables.clone()
+        for k, (b, e) in enumerate(entries):
+            t[b, e] = spare[2 * k + i % 2] if i else t[b, e]
+        s = t[:, 13] * 256 + 3499 % 256
+        flat = torch.zeros(256 * 128, dtype=torch.int32)
+        flat[:6 + 6 * width] = torch.cat([s, t.flatten()])
+        rows = torch.cat([flat.view(256, 128).flip(0), torch.zeros(256, 128, dtype=torch.int32)])
+        steps.append((s, t, rows.to(cuda).view(torch.bfloat16).view(512, 1, 256)))
+    outs = []
+    torch.cuda.synchronize()
+    for *_, key in steps:
+        A.store_kvcache(key, key, plane, scratch, backwards)
+        outs.append(A.decode_step(dev.q, dev.k_new, dev.v_new, dev.k_cache, dev.v_cache, slots, dev.context_lens, table, case.scale))
+    torch.cuda.synchronize()
+    assert _lib.read_status() == 0
+    for (s, t, _), out in zip(steps, outs):
+        R.store_kvcache_ref(case.k_new, case.v_new, case.k_cache, case.v_cache, s)
+        assert_close_to_oracle(out, R.decode_ref(case.q, case.k_cache, case.v_cache, case.context_lens, t, case.scale), f"{entries}")
+    assert torch.equal(dev.k_cache.cpu().view(torch.int16), case.k_cache.view(torch.int16))
+
+
 @pytest.mark.parametrize("batch", [33, 129])
 def test_a_batch_of_empty_sequences_completes_after_its_store(cuda, batch):
     """The layer call of more than 32 sequences that are all empty has no tile to stream.  The launch
