@@ -161,8 +161,10 @@ struct Cut {
 // Cost of a streamed unit over the cost of a merged partial.  With merges of eight parts to a trip, us at 8 -> 16 -> 32: 36
 // captured layers (32 / 8 heads) of two sequences of 500-4000 tokens 411 -> 358 -> 358, of one of 1050 281 -> 279 -> 289, of
 // four of 100-1024 292.5 -> 294.5 -> 294.7; 28 (16 / 8 heads) of two of 500-4000 280 -> 264 -> 264; a layer of one of 4096 8.53 ->
-// 8.12 -> 8.24, of two of 30000-32000 (14 / 2 heads of 64) 17.0 -> 17.45 -> 18.6.
-constexpr float kSplitBalance = 16.f;
+// 8.12 -> 8.24.  At head_dim 64, where a merge has the statistics of 16 parts in a trip, 8 where 16 would cut a sequence into more
+// than 32 parts (14 / 2 heads, layer of two of 20000-32000 tokens 57 parts 17.0, 41 parts 11.8; 7 / 1, six of 8000-16000 15.8, 12.3).
+constexpr float kSplitBalance = 16.f, kSplitBalanceLong = 8.f;
+constexpr int kSplitLong = 64;  // units of a sequence that make 32 parts at a balance of 16
 
 // The kernels.  Step, StepGuess and Layer also store the new tokens' rows: the former two where the row's slot is that of its
 // position, Layer to any slot.
@@ -329,7 +331,8 @@ __global__ void __launch_bounds__(C::NW * 32, 2) decode_paged_kernel(const Decod
     // that share a sequence are consecutive.  And where sequences are few, no more than balance the
     // two costs of a cut: a range streams total / n units and a sequence's merge reads n / batch
     // partials, so that the sum is least at n = sqrt(c total batch).
-    n_ranges = max(1, min(min(p.n_ranges, total), static_cast<int>(sqrtf(kSplitBalance * total * p.batch))));
+    const float balance = D == 64 && total > kSplitLong * p.batch ? kSplitBalanceLong : kSplitBalance;
+    n_ranges = max(1, min(min(p.n_ranges, total), static_cast<int>(sqrtf(balance * total * p.batch))));
     if (range >= n_ranges || total == 0) return false;  // block-uniform (also when the whole batch is empty)
     // the first `longer` ranges hold one unit more than the others
     per_range = total / n_ranges, longer = total - per_range * n_ranges;
