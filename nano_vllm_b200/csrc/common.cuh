@@ -39,9 +39,8 @@ int store_kvcache(bool launch, const void* key, int64_t key_row_stride, const vo
 // ---- device side -----------------------------------------------------------------------
 #ifdef __CUDACC__
 
-// Programmatic dependent launch.  The attention kernels and the pre-attention step are launched with the
-// attribute (launch_kernel), the sampler where its grid gains by it, so that their blocks may become
-// resident while the predecessor in the stream drains: about 1 us of every launch in a chain.  Each of their
+// Programmatic dependent launch.  The attention kernels, the pre-attention step (launch_kernel) and the sampler are
+// launched with the attribute, so that their blocks may become resident while the predecessor in the stream drains: about 1 us of every launch in a chain.  Each of their
 // blocks passes pdl_wait(), which returns when the previous kernel has completed and its writes are
 // visible, before it touches anything that another kernel may have written (a guess that is verified
 // afterwards excepted), and before it ends even where it has nothing to do: so completion stays

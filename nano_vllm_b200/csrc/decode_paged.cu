@@ -44,9 +44,9 @@
 // arrivals wait for nothing in the middle of a range, and a merge takes one trip for eight parts.
 // Where parts are few they are written as marked cells (kMark), so that the report of a partial needs no fence and the
 // merge's reads go out with it.
-// One launch in a chain, from a graph (head_dim 128, 16 / 8 heads): one sequence of 317 tokens 8.7 ->
-// 6.2 us, one of 4096 20.0 -> 10.7, 8 of 100-1024 16.3 -> 11.9, 16 of them 18.1 -> 14.9, 64 of them
-// 35.3 -> 32.7; 256 sequences of 2048-8192 tokens (32 / 8 heads, step variant) 795 -> 747.
+// One launch in a chain that stores the new rows too, from a graph (head_dim 128, 16 / 8 heads): one sequence of 300-600
+// tokens 6.0 us, one of 4096 7.9, 8 of 100-1024 9.6, 16 of them 11.1, 64 of them 30.1; 256 sequences of 2048-8192
+// tokens (32 / 8 heads) 745-755.
 #include <cstdlib>
 #include <type_traits>
 

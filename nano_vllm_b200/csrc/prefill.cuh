@@ -4,8 +4,8 @@
 
 namespace nvllm {
 
-// Who stores packed rows: nobody, a warp that has nothing else to do, or the epilogue warps from the key tiles in
-// shared memory.
+// Who stores packed rows: nobody, a warp that has nothing else to do, or from the key tiles in shared memory the epilogue
+// warps, in blocks of three to an SM that warp.
 enum class Store { None, Spare, Tiles };
 
 // Where the key tiles of new rows are, for a prefill through the block table (prefill_route.cu).  Every cache block that

@@ -8,10 +8,11 @@ namespace nvllm {
 
 namespace tc {
 constexpr int BM = 128, BN = 64, KST = 2;
-constexpr int TMEM_COLS = 256;              // S/P buffers: [0,64) and [64,128); O: [128,256)
+constexpr int TMEM_COLS = 256;              // of two blocks to an SM: S/P buffers [0,64) and [64,128), O [128,256)
 constexpr float kRescaleThreshold = 8.f;    // log2 units
-// One tcgen05.commit per MMA group, each completion signalled once and shared by all its waiters.  QK_DONE[s]: S buffer s holds S_j (softmax) and K stage s is free
-// (producer).  PV_DONE[s]: V stage s is free (producer), O includes tile j (rescale, epilogue).
+// One tcgen05.commit per MMA group, each completion signalled once and shared by all its waiters.  QK_DONE[s]: S of a tile
+// of stage s is there (softmax) and K stage s is free (producer).  PV_DONE[s]: V stage s is free (producer), O includes
+// tile j (rescale, epilogue; three blocks to an SM: P may be written again).
 enum Bar {
   Q_FULL = 0, K_FULL0, K_FULL1, V_FULL0, V_FULL1, QK_DONE0, QK_DONE1, PV_DONE0, PV_DONE1,
   P_FULL0, P_FULL1, DRAIN, NUM_BARS

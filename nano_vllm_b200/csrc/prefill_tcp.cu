@@ -4,10 +4,14 @@
 //
 // Tile pipeline: 128 query rows x 64-key tiles; S = Q K^T (SS form, both operands K-major in
 // shared memory) into one of two S buffers in TMEM; the softmax warps (thread = query row) read
-// their row of S with tcgen05.ld, write P as packed bf16 over it with tcgen05.st; O += P V (TS
+// their row of S with tcgen05.ld, write P as packed bf16 over it (three blocks to an SM: one S buffer, P
+// beside it) with tcgen05.st; O += P V (TS
 // form: P from TMEM, V as an MN-major shared-memory operand); Q, K, V arrive by TMA tile loads
 // (128-byte swizzle, no multicast) into a two-stage ring; one tcgen05.commit per MMA group.
-// Twelve warps (eight in the form of three blocks to an SM, see Geo): 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
+// Two forms, see Geo and three_blocks: two blocks of twelve warps to an SM, which the following describes, or at head_dim 64
+// three of eight, without the epilogue warps: there the softmax warps write an item's results and the copy warp stores rows
+// from the key tiles.
+// Twelve warps: 0-3 softmax / correction (thread = query row), 4-7 epilogue (same rows: when an
 // item's last P V product is done they normalise O and store it while the softmax warps are
 // already in the next item's first tile, and write packed K/V rows to the cache from the key tiles), warp 8 = TMA producer of
 // Q and K, warp 9 = MMA issuer, warp 10 = TMA producer of V (one elected lane each), warp 11 = a copy of rows that no
@@ -26,15 +30,16 @@
 // Order of the items: sequences longest first (ranked in shared memory by every block at start-up,
 // for batches of up to SORT_BATCH sequences), a sequence's long tiles first, head groups fastest.
 // The blocks that are still busy when the counter runs out are then working on the cheapest
-// items, so the launch ends without a tail of half-idle SMs.  Where there are no more items than blocks, of prompts of
-// about one length, all sequences' long tiles go first instead.
+// items, so the launch ends without a tail of half-idle SMs.  At head_dim 128 where there are no more items than blocks, of
+// prompts of about one length, and with three blocks to an SM where prompts have the same number of query tiles, all
+// sequences' long tiles go first instead.
 //
 // Item hand-off: the producer lane decodes an item into one of two descriptor slots in shared
 // memory (ITEM_FULL / ITEM_FREE barriers).  All rings keep running across items: tile t of the
 // block's life uses stage t&1 and barrier phase (t>>1)&1, so the next item's first K/V tiles
 // are fetched under the current item's last products.  The first P V product of an item waits
-// for the previous item's O to be read (O_FREE); the softmax warps leave each row's 1 / sum in
-// shared memory (EPI_FULL) and move on.  The epilogue needs no block-wide buffer: an epilogue
+// for the previous item's O to be read (O_FREE; by the softmax warps themselves where there are no others); the softmax
+// warps leave each row's 1 / sum in shared memory (EPI_FULL) and move on.  The epilogue needs no block-wide buffer: an epilogue
 // warp owns the same 32 rows in TMEM and in the output, and passes them 32 columns at a time
 // through a private 2 KB patch of shared memory to turn row-per-lane registers into 64-byte row
 // segments.

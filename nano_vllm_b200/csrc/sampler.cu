@@ -22,7 +22,8 @@
 // the largest is taken.  Ties go to the lowest index.
 //
 // What bounds it: not the one read of the logits (78 MB at batch 256, 12 us) but the instructions
-// per element.  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
+// per element: the generator alone, at 768 threads to an SM and without a load, takes 24.7 us of the 43.5 there, 21 of
+// them its 18 wide products for four logits (29 a clock and SM).  Ten Philox rounds for four elements and two logarithms for each came to 74 us there
 // (now 43.5; greedy rows 32 -> 16; batch 1, 12.7 -> 5.7).  The logarithms are only needed for elements that
 // can still win: since e >= v, where v is the uniform
 // draw, element i can beat a score b only if v < exp(x_i - b), x_i = logit_i / T.  One exponential of
@@ -315,8 +316,8 @@ __global__ void __launch_bounds__(1024, 1) sample_kernel(const SampleParams p) {
       auto limit_of = [&](const uint4& raw, float bar) { return fast_exp2(fmaf(G::max(raw), x_scale, -bar)); };
       float bar = bar_of(-INFINITY);
       int seen = ordered(-INFINITY);
-      // One group at a time: two, with twice as many generator chains in flight, are slower below some 400
-      // rows (17.4 / 19.7 us at batch 64), and so are fewer registers and more warps.
+      // One group at a time: two, with twice as many generator chains in flight, were slower below some 400
+      // rows, and so were fewer registers and more warps.
       for_groups<A, 1>(first, n_groups, tid, nthreads, [&](const uint4 (&raw)[1], int g, int, auto full) {
         const bool live = decltype(full)::value || g < n_groups;
         const int now = *static_cast<volatile int*>(&s_best);
@@ -447,6 +448,8 @@ static Shape in_waves(int batch, int vocab, int sms) {
 // instead of 85, but take 29.3 instead of 25.7 for 450 greedy ones), and long ones of which SMs would have one or two (200
 // 36.4, 41.7 at once; fp32 45.6, 50.5, though greedy 25.1, 22.4).  Rows shorter than kLongRow have too little for the merges of
 // four blocks of 256 threads and more (112 rows of 32000 10.2 -> 8.7 us, of 18992 greedy fp32 4.8 -> 4.0).
+// Blocks that are not spread by force land 15 % unevenly: with 1 for the 1.15 below 200 sampled rows take 40.8 us instead of 38.3
+// (greedy 14.5 instead of 17.1), over 480 launches 1, 1.15 and 1.3 are the same to 0.1 %.
 // All for 151936 logits and T = 0.6 unless said, in waves -> now, us: 1 row 6.05 -> 5.4, 16 10.35 -> 8.15, 64 16.1 -> 14.4, 100 24.8 ->
 // 21.7, 148 30.6 -> 23.6, 180 35.6 -> 31.4, 256 43.9 -> 42.3.  Of 980 launches (1-512 rows of 1000-151936 logits of both types,
 // sampled and greedy) in a chain the mean is 11 % faster; 32 are 4 % slower or more, four of them by over 0.4 us (56 greedy
