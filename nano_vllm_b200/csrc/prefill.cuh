@@ -85,6 +85,7 @@ int launch_prefill_tcp(const PrefillParams& p, int64_t total_q, int64_t total_k,
 // n_new) and whether through the block table, with the route's tables or without (block_tables, route.jobs).
 struct PrefillPlan {
   int blocks, grid;  // to an SM (three at head_dim 64 only), of the launch
+  int pack;          // query heads in a tile
   int spread_from;   // see PrefillParams
   Store store;
 };

@@ -904,9 +904,13 @@ static int heads_per_tile(int g) {
   return pack;
 }
 
-int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch) {
-  const int pack = heads_per_tile(hq / hkv), bmt = tc::BM / pack;
+static int64_t max_items_of(int hq, int pack, int max_seqlen_q, int batch) {
+  const int bmt = tc::BM / pack;
   return static_cast<int64_t>((max_seqlen_q + bmt - 1) / bmt) * (hq / pack) * batch;
+}
+
+int64_t prefill_max_items(int hq, int hkv, int max_seqlen_q, int batch) {
+  return max_items_of(hq, heads_per_tile(hq / hkv), max_seqlen_q, batch);
 }
 
 // Prompts of less than four key tiles are the two-block form's: a block of three has no warps to write an item's results while
@@ -939,8 +943,8 @@ static bool same_tiles(const PrefillParams& p, int64_t total_q, int bmt) {
 // 2000-4096 (4.4 times) 108 -> 114, 16 of 1000-1024 (6.4 times) 62.7 -> 66.1; one head to a tile, 48 of 200-400 (8 times) 46.8 -> 51.3.
 // Of 237 launches that the rule takes (six pairs of heads, 256 to 4096 tokens) the mean is 6 % faster; 21 are slower, six of them
 // by 3-8 % (32 / 8 heads, 7 of 256 13.1 -> 14.1; 16 / 16, 3 of 1024 22.0 -> 23.0).
-static bool three_blocks(const PrefillParams& p, int64_t total_q, int sms) {
-  const int pack = heads_per_tile(p.g), bmt = tc::BM / pack;
+static bool three_blocks(const PrefillParams& p, int64_t total_q, int sms, int pack) {
+  const int bmt = tc::BM / pack;
   const double mean = static_cast<double>(total_q) / p.batch;
   const double items = static_cast<double>(total_q) / bmt * (p.hq / pack), tiles = items * (mean / 2 + tc::BN / 2) / tc::BN;
   if (mean < kTrioTokens) return false;
@@ -950,12 +954,13 @@ static bool three_blocks(const PrefillParams& p, int64_t total_q, int sms) {
 }
 
 PrefillPlan prefill_plan(const PrefillParams& p, int64_t total_q, int sms) {
-  const int bmt = tc::BM / heads_per_tile(p.g);
-  const bool routed = p.route.jobs > 0;
   PrefillPlan plan;
-  plan.blocks = p.d == 64 && three_blocks(p, total_q, sms) ? 3 : 2;
+  plan.pack = heads_per_tile(p.g);  // reads the environment: once to a launch
+  const int bmt = tc::BM / plan.pack;
+  const bool routed = p.route.jobs > 0;
+  plan.blocks = p.d == 64 && three_blocks(p, total_q, sms, plan.pack) ? 3 : 2;
   // an upper bound of the work items known to the host: no more blocks than that
-  const int64_t max_items = prefill_max_items(p.hq, p.hkv, p.max_seqlen_q, p.batch);
+  const int64_t max_items = max_items_of(p.hq, plan.pack, p.max_seqlen_q, p.batch);
   plan.grid = plan.blocks * sms;
   // With an item to a block and more items than SMs, blocks that share an SM with those of long tiles get short ones by
   // another order: 6 prompts of 300 tokens 15.1 -> 13.4 us, 10 of 100 11.4 -> 10.4, 3 of 500 14.6 -> 14.1.  Which blocks
@@ -1014,7 +1019,7 @@ static int launch_prefill_tcp_t(const PrefillParams& p_in, const PrefillPlan& pl
   }
   PrefillParams p = p_in;
   const bool routed = p.route.jobs > 0;
-  p.pack = heads_per_tile(p.g);
+  p.pack = plan.pack;
   const int pack = p.pack, bmt = tc::BM / pack;
   p.tile_tokens = bmt;
   p.inv_pack = 65536 / pack + 1;  // exact for rows of a tile
