@@ -419,6 +419,49 @@ def test_three_blocks_to_an_sm_whose_spare_warps_store_rows(cuda, lib, d_heads, 
     assert _lib.read_status() == 0
 
 
+@pytest.mark.parametrize("hq,hkv,batch", [(14, 2, 70), (7, 1, 140), (16, 4, 70)])
+@pytest.mark.parametrize("table", [False, True])
+def test_three_blocks_to_an_sm_store_rows_from_the_key_tiles(cuda, lib, hq, hkv, batch, table):
+    """Rows stored by one warp of each block: ends around a tile's, sequences of one token and of none, rows in front and behind,
+    scattered slots; through the table with blocks that others fill.  Cache and output against the reference."""
+    d, r = 64, random.Random(batch + table)
+    lens = [r.choice([512, 511, 449, 448, 447, 321, 1 if not table else 300, 512] + [0] * (not table)) for _ in range(batch - 1)] + [512]
+    if table:
+        shared = [(i % 4 == 3) * min(1, min(lens[i - 1], lens[i] - 1) // 256) for i in range(batch)]
+        c = W.make_prefill_case(89, batch, 1, 1, hq, hkv, d, lengths=lens, shared_blocks=shared)
+        q, k, v, cu_q, cu_k, slots, bt, k_cache, v_cache = c.q, c.k, c.v, c.cu_seqlens_q, c.cu_seqlens_k, c.slot_mapping, c.block_tables, c.k_cache, c.v_cache
+        max_q, max_k, n, n_k = c.max_seqlen_q, c.max_seqlen_k, q.shape[0], k.shape[0]
+    else:
+        front, behind, bt = 3, 70, None
+        n, n_k, max_q, max_k = sum(lens), front + sum(lens) + behind, 512, 512
+        gen = torch.Generator().manual_seed(batch)
+        rand = lambda *shape: torch.randn(*shape, generator=gen).bfloat16()
+        q, k, v = rand(n, hq, d), rand(n_k, hkv, d), rand(n_k, hkv, d)
+        cu_q = torch.tensor([0] + lens).cumsum(0).int()
+        cu_k = cu_q + front
+        blocks = n_k // 256 + 3
+        slots = torch.randperm(blocks * 256, generator=gen)[:n_k].int()
+        slots[::11] = -1
+        k_cache, v_cache = rand(blocks, 256, hkv, d), rand(blocks, 256, hkv, d)
+    out = [ctypes.c_int32() for _ in range(3)]
+    sms = torch.cuda.get_device_properties(cuda).multi_processor_count
+    assert lib.nvllm_prefill_plan(n, n_k, batch, max_q, max_k, hq, hkv, d, 2 if table else 1, sms, *(ctypes.byref(x) for x in out)) == 0
+    assert [x.value for x in out] == [3, 1 << 30, TILES] or sms != 148
+    layer = A.Attention(hq, d, d ** -0.5, hkv)
+    layer.k_cache, layer.v_cache = k_cache.to(cuda), v_cache.to(cuda)
+    C.set_context(True, cu_q.to(cuda), cu_k.to(cuda), max_q, max_k, slots.to(cuda), None, bt.to(cuda) if table else None)
+    for _ in range(2):
+        got = layer(q.to(cuda).flatten(1), k.to(cuda).flatten(1), v.to(cuda).flatten(1))
+    C.reset_context()
+    torch.cuda.synchronize()
+    R.store_kvcache_ref(k, v, k_cache, v_cache, slots)
+    assert torch.equal(layer.k_cache.cpu().view(torch.int16), k_cache.view(torch.int16))
+    assert torch.equal(layer.v_cache.cpu().view(torch.int16), v_cache.view(torch.int16))
+    ref = R.prefill_ref(q, k_cache, v_cache, cu_q, cu_k, d ** -0.5, bt) if table else R.prefill_ref(q, k, v, cu_q, cu_k, d ** -0.5)
+    assert_close_to_oracle(got.view(n, hq, d), ref, f"{batch} sequences hq{hq}")
+    assert _lib.read_status() == 0
+
+
 @pytest.mark.parametrize("hq,hkv", FORM_64)
 @pytest.mark.parametrize("table", [False, True])
 def test_three_blocks_to_an_sm_see_nothing_behind_a_sequence(cuda, lib, hq, hkv, table):
